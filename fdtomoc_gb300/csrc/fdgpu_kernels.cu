@@ -163,6 +163,7 @@ struct Shared {
     unsigned gfaces;
     long long gM;
     unsigned ctxm[6], innm[6];
+    unsigned rel[6][27];     /* see relation_word */
     void *gsm;
     unsigned long long red[FD_BLOCK / 32];
     unsigned long long bcast;
@@ -181,7 +182,7 @@ __device__ __forceinline__ void wfence(const Shared &sh)
     if (sh.cs > 1)
         asm volatile("fence.acq_rel.cluster;" ::: "memory");
     else
-        __threadfence_block();
+        asm volatile("fence.acq_rel.cta;" ::: "memory");
 }
 
 #ifndef FD_BAR_SPINS
@@ -714,11 +715,20 @@ struct GRect {
     short face, layer, ulo, uhi, vlo, vhi, nuf, pad;
 };
 
-/* in the dynamic shared memory after the warp areas (the face walks' dependency bytes otherwise) */
+/* In the dynamic shared memory after the warp areas (the face walks' dependency bytes otherwise).
+ *
+ * lay[a][c]: when the box's walls reach coordinate c of axis a, as an owner word (below): the instance
+ * whose wall stands there, FD_IN_BOX if the sweep starts with c inside the box, FD_NEVER if no wall
+ * gets there.  A node joins the box when the last of its three coordinates does, so its owner is the
+ * largest of three entries: three shared-memory loads and two comparisons, where a search through the
+ * six faces' instances and their rectangles took about a hundred instructions, divergent ones. */
+#define FD_IN_BOX ((short)-1)
+#define FD_NEVER ((short)0x7fff)
 struct GraphSmem {
-    short lay2inst[FDN_NFACE][FD_LMAX];   /* instance of face f at layer l, -1 if none */
+    short lay[3][FD_LMAX + 2];   /* entry c + 1 for coordinate c, FD_NEVER on both sides of the grid */
     GRect rect[FD_IMAX];
 };
+static_assert((FD_IMAX << 3) + 7 < 0x7fff, "owner words in a short");
 
 /* the warp areas and the sweep-graph tables fit one CTA's 227 KB, with 2 KB left for the static
  * shared memory of fd_solve */
@@ -727,10 +737,15 @@ static_assert(kSmemBase + sizeof(GraphSmem) + 2048 <= 227 * 1024, "shared memory
 __device__ __forceinline__ GraphSmem &gsmem(const Shared &sh) { return *reinterpret_cast<GraphSmem *>(sh.gsm); }
 
 /* Neighbour offsets (dx,dy,dz) are numbered k = (dz+1)*9 + (dy+1)*3 + (dx+1), 13 being the node
- * itself; the opposite offset is 26 - k.  An owner word holds (face << 24) | instance, -1 for a
+ * itself; the opposite offset is 26 - k.  An owner word holds (instance << 3) | face, -1 for a
  * node no instance of the sweep computes. */
-__device__ __forceinline__ int own_inst(int w) { return w & 0xFFFFFF; }
-__device__ __forceinline__ int own_face(int w) { return w >> 24; }
+__device__ __forceinline__ int own_inst(int w) { return w >> 3; }
+__device__ __forceinline__ int own_face(int w) { return w & 7; }
+__device__ __forceinline__ int owner_word(int lx, int ly, int lz)
+{
+    const int w = max(max(lx, ly), lz);
+    return w == FD_NEVER ? -1 : w;
+}
 
 /* masks of the offsets a node of face f reads (own plane and inner plane) and of its inner plane */
 __device__ void relation_masks(int f, unsigned &ctx, unsigned &inn)
@@ -746,39 +761,32 @@ __device__ void relation_masks(int f, unsigned &ctx, unsigned &inn)
     }
 }
 
+/* What the node at offset k from a node of face F has to do with it.  Bits 0-5: it waits for that node
+ * if it belongs to a later instance of face (bit) — it reads that node, or that node reads it; bits 6-11:
+ * through its inner block; bit 12: k lies in F's plane, and then bits 16-19: its place in the inner 3x3
+ * block relative to the centre, plus 4; bit 20: it comes later if the inner-layer times are equal. */
+__device__ unsigned relation_word(const Shared &sh, int F, int k)
+{
+    unsigned w = 0;
+    for (int f = 0; f < 6; f++) {
+        if (((sh.ctxm[F] >> k) & 1u) || ((sh.ctxm[f] >> (26 - k)) & 1u)) w |= 1u << f;
+        if ((sh.innm[f] >> (26 - k)) & 1u) w |= 1u << (6 + f);
+    }
+    const fdn_frame fr = frame_of(F);
+    const int dx = k % 3 - 1, dy = (k / 3) % 3 - 1, dz = k / 9 - 1;
+    if (coord(fr.axis_n, dx, dy, dz) == 0) {
+        const int du = coord(fr.axis_u, dx, dy, dz), dv = coord(fr.axis_v, dx, dy, dz);
+        w |= 1u << 12 | (unsigned)(dv * 3 + du + 4) << 16 | (dv > 0 || (dv == 0 && du > 0) ? 1u << 20 : 0u);
+    }
+    return w;
+}
+
 __device__ __forceinline__ int rect_n(const GRect &r) { return r.nuf * (r.vhi - r.vlo + 1); }
 
 /* owner word of node (x,y,z), which must lie in the grid */
-__device__ __forceinline__ int owner_of(const GraphSmem &gs, unsigned faces, int x, int y, int z)
+__device__ __forceinline__ int owner_of(const GraphSmem &gs, int x, int y, int z)
 {
-#pragma unroll
-    for (int f = 0; f < 6; f++) {
-        if (!((faces >> f) & 1u)) continue;
-        const fdn_frame fr = frame_of(f);
-        const int I = gs.lay2inst[f][coord(fr.axis_n, x, y, z)];
-        if (I < 0) continue;
-        const GRect &r = gs.rect[I];
-        const int u = coord(fr.axis_u, x, y, z), v = coord(fr.axis_v, x, y, z);
-        if (u >= r.ulo && u <= r.uhi && v >= r.vlo && v <= r.vhi) return (f << 24) | I;
-    }
-    return -1;
-}
-
-/* owner word of node (x,y,z) when face F is the likely owner: F's instance at the node's layer is
- * looked at first (one table entry and one rectangle), the full search only if it is not F's.  Each
- * node belongs to at most one instance of a sweep, so the answer is owner_of's. */
-__device__ __forceinline__ int owner_near(const GraphSmem &gs, unsigned faces, int F, int x, int y, int z)
-{
-    const fdn_frame fr = frame_of(F);
-    if ((faces >> F) & 1u) {
-        const int I = gs.lay2inst[F][coord(fr.axis_n, x, y, z)];
-        if (I >= 0) {
-            const GRect &r = gs.rect[I];
-            const int u = coord(fr.axis_u, x, y, z), v = coord(fr.axis_v, x, y, z);
-            if (u >= r.ulo && u <= r.uhi && v >= r.vlo && v <= r.vhi) return (F << 24) | I;
-        }
-    }
-    return owner_of(gs, faces, x, y, z);
+    return owner_word(gs.lay[0][x + 1], gs.lay[1][y + 1], gs.lay[2][z + 1]);
 }
 
 /* node index of point j of instance r */
@@ -796,6 +804,13 @@ __device__ __forceinline__ unsigned long long inst_key(const fd_station_dev &sd,
     const fdn_frame fr = frame_of(r.face);
     const long long p = inst_node(sd, r, j) + fr.inner * t_stride(sd, fr.axis_n);
     return node_key(vload(sd.T[p]), j);
+}
+
+/* the in-face neighbour (du,dv) of a node comes later in its instance's order: inner-layer time (as
+ * okey32 images), then fill index, which grows with dv and, within a row, with du */
+__device__ __forceinline__ bool later_key(unsigned nb, unsigned own, int du, int dv)
+{
+    return nb > own || (nb == own && (dv > 0 || (dv == 0 && du > 0)));
 }
 
 /* fill index of node (x,y,z) in instance r */
@@ -820,9 +835,8 @@ __device__ void fire_event(const fd_station_dev &sd, Shared &sh, int I, int kind
     }
 }
 
-/* Key event of node j of instance I (its inner block is final): its earlier same-instance
- * neighbours, recorded, and the later ones dropped from its counter.  Returns the counter word
- * after the update. */
+/* Key event of node j of instance I (its inner block is final): its later same-instance neighbours
+ * are dropped from its counter.  Returns the counter word after the update. */
 __device__ unsigned key_event(const fd_station_dev &sd, Shared &sh, int I, int j, long long q)
 {
     const GRect &r = gsmem(sh).rect[I];
@@ -840,20 +854,18 @@ __device__ unsigned key_event(const fd_station_dev &sd, Shared &sh, int I, int j
         const long long qk = qin + du * su + dv * sv;
         tn[k] = (((inr >> k) & 1u) && FD_OK(qk, (long long)sd.g.nx * sd.g.ny * sd.g.nz, 12)) ? vload(sd.T[qk]) : 0.f;
     }
-    const unsigned long long kj = node_key(vload(sd.T[qin]), j);
-    unsigned em = 0;
+    const unsigned kj = okey32(vload(sd.T[qin]));
+    unsigned lat = 0;
 #pragma unroll
     for (int k = 0; k < 8; k++) {
         int du, dv;
         nb_off(k, du, dv);
-        if (((inr >> k) & 1u) && node_key(tn[k], j + du + dv * r.nuf) < kj) em |= 1u << k;
+        if (((inr >> k) & 1u) && later_key(okey32(tn[k]), kj, du, dv)) lat++;
     }
     if (!FD_OK(q, (long long)sd.g.nx * sd.g.ny * sd.g.nz, 13) || !FD_OK(qin, (long long)sd.g.nx * sd.g.ny * sd.g.nz, 29)
         || !FD_OK(I, sd.scr.ginst_cap, 14))
         return 0u;
-    sd.scr.gemask[q] = (unsigned char)em;
     wfence(sh);
-    const unsigned lat = (unsigned)__popc(inr & ~em);
     const unsigned add = FD_KEYED - (lat << 8);
     const unsigned nw = atomicAdd(&sd.scr.gcnt[q], add) + add;
     if (!sh.nodefer && atomicAdd(&sd.scr.ginst[I].nkeyed, 1) == n - 1) fire_event(sd, sh, I, 1);
@@ -867,35 +879,17 @@ __device__ __forceinline__ void graph_ready(const fd_station_dev &sd, Shared &sh
     enqueue_to(sd.scr.gqueue + sh.w->qbase[face], sh.w->qtail[face], sh.w->qcap[face], sh, (int)q);
 }
 
-/* drop one inner-block (inner) or other-instance dependency of node q (instance oq, face fq) */
-__device__ __forceinline__ void graph_dec(const fd_station_dev &sd, Shared &sh, long long q, int oq, int fq,
-                                          int qx, int qy, int qz, bool inner)
+/* node p (instance I, fill index i) is final: its record, and the points that wait for it */
+__device__ void graph_record(const fd_station_dev &sd, Shared &sh, long long p, int I, int i, bool writer, float st0,
+                             float st4, float tin)
 {
-    const unsigned dec = inner ? 1u : (1u << 16);
-    if (!FD_OK(q, (long long)sd.g.nx * sd.g.ny * sd.g.nz, 19)) return;
-    const unsigned nw = atomicSub(&sd.scr.gcnt[q], dec) - dec;
-    if (inner && (nw & 0xFFu) == 0u) {
-        /* q's inner block is complete: its key and in-face order are now known */
-        if (ready_word(key_event(sd, sh, oq, inst_fill(gsmem(sh).rect[oq], qx, qy, qz), q))) graph_ready(sd, sh, fq, q);
-    } else if (ready_word(nw)) {
-        graph_ready(sd, sh, fq, q);
-    }
-}
-
-/* node p (instance I, face F, fill index i) is final: record, release what waits on it */
-__device__ void graph_release(const fd_station_dev &sd, Shared &sh, int F, long long p, int x, int y, int z, int I,
-                              int i, bool writer, float st0, float st4, float tin)
-{
-    const GraphSmem &gs = gsmem(sh);
     if (!FD_OK(p, (long long)sd.g.nx * sd.g.ny * sd.g.nz, 15) || !FD_OK(I, sd.scr.ginst_cap, 16)) return;
-    const GRect &r = gs.rect[I];
-    fd_ginst &gi = sd.scr.ginst[I];
     /* records: of every point when a point may need an earlier one's; else only the last instance's,
      * for the state the sweep leaves */
     if (!sh.nodefer || I == sh.ninst - 1) {
         if (writer) {
             sd.scr.grec[p] = make_float2(st0, st4);
-            atomicMax(&gi.exitkey, node_key(tin, i));
+            atomicMax(&sd.scr.ginst[I].exitkey, node_key(tin, i));
         } else {
             sd.scr.grec[p] = make_float2(__int_as_float(0x7fc00000), __int_as_float(0x7fc00000));
         }
@@ -909,52 +903,158 @@ __device__ void graph_release(const fd_station_dev &sd, Shared &sh, int F, long 
             if (vload(sd.scr.gwait[k].x) == (int)p && atomicCAS(&sd.scr.gwait[k].x, (int)p, -1) == (int)p)
                 enqueue_to(sd.scr.grq, sh.w->rqtail, sh.w->rqcap, sh, vload(sd.scr.gwait[k].y));
     }
+}
+
+/* nodes of a chunk up to which a release gives each neighbour a lane (more: each node), in a sweep of
+ * several faces and of one */
+#ifndef FD_FEW
+#define FD_FEW 12
+#endif
+#ifndef FD_FEW1
+#define FD_FEW1 6
+#endif
+
+/* a final node as its release needs it: packed coordinates, grid index, instance, its lane */
+struct RelNode {
+    int xyz, p, inst, slot;
+};
+
+/* what the node with owner word w at an offset with relation word rw drops from its counter when a
+ * node of instance I is final (t13: that node's inner block centre) */
+__device__ __forceinline__ unsigned release_dec(int w, int I, unsigned rw, const float *t13)
+{
+    const int oi = own_inst(w);
+    if (w == FD_NEVER || oi < I) return 0u;
+    if (oi == I) {
+        /* a neighbour in the same instance waits only if it comes later */
+        const unsigned a = okey32(t13[(int)((rw >> 16) & 15u) - 4]), b = okey32(*t13);
+        return a > b || (a == b && (rw >> 20) & 1u) ? 1u << 8 : 0u;
+    }
+    const unsigned f = rw >> own_face(w);
+    return !(f & 1u) ? 0u : (f & (1u << 6)) ? 1u : 1u << 16;
+}
+
+/* drop dec from the counter of node q; a node that becomes ready is queued, one whose inner block is now
+ * complete goes on the list of key events */
+__device__ __forceinline__ void release_one(const fd_station_dev &sd, Shared &sh, int q, int fq, unsigned dec, int *keyq,
+                                            int *nkey)
+{
+    if (!FD_OK(q, (long long)sd.g.nx * sd.g.ny * sd.g.nz, 19)) return;
+    const unsigned nw = atomicSub(&sd.scr.gcnt[q], dec) - dec;
+    if (dec == 1u && (nw & 0xFFu) == 0u)
+        keyq[atomicAdd(nkey, 1)] = q;
+    else if (ready_word(nw))
+        graph_ready(sd, sh, fq, q);
+}
+
+/* Release what waits on the chunk's final nodes (fin, wh: this lane's node).  All 32 lanes call.
+ *
+ * What bounds a release is instructions: a warp of this kernel issues one about every ten cycles, so
+ * what matters is how many the warp steps through.  A chunk of a forward sweep holds two to nine nodes;
+ * each node's 26 neighbours then go to 26 lanes, so that a node costs one pass, and what depends on the
+ * neighbour's offset alone (its relation word, its index offset) is set up once per chunk.  With more
+ * nodes each lane walks the neighbours of its own node, with the offsets known at compile time (in a
+ * one-face sweep only the 9 nodes of the next instance and the 8 of its own).  Nodes whose inner block
+ * the chunk completes are collected (in the trial values' area, free after the commit) and take their
+ * keys together: a key event is three more round trips to memory.
+ *
+ * Measured, commit and release of one chunk: 55 -> 28 thousand cycles at 3.8 nodes (27x20x21), 80 -> 50 at
+ * 29 nodes (141x121x57), against a loop over the neighbours with a search of the six faces for each
+ * owner and a key event inside it.  The two forms cost the same at about 12 nodes of a forward sweep (27
+ * steps of the second form against 12 of the first) and at 6 of a one-face sweep (17 steps). */
+__device__ void graph_release(const fd_station_dev &sd, Shared &sh, WarpSmem &ws, int F, bool fin, const Where &wh)
+{
+    const int lane = threadIdx.x & 31;
+    const GraphSmem &gs = gsmem(sh);
+    const unsigned mask = __ballot_sync(0xffffffffu, fin);
+    const int m = __popc(mask);
+    if (!m) return;
+    int *keyq = reinterpret_cast<int *>(&ws.res[0][0]);
+    int *nkey = reinterpret_cast<int *>(&ws.cnt[5]);
     const int nx = sd.g.nx, ny = sd.g.ny;
-    const fdn_frame fr = frame_of(F);
-    if (sh.single) {
-        /* one face: the next instance's nodes whose inner block holds p */
-        if (I + 1 < sh.ninst && gs.rect[I + 1].layer == r.layer - fr.inner) {
-            const GRect &rn = gs.rect[I + 1];
-            const int u0 = coord(fr.axis_u, x, y, z), v0 = coord(fr.axis_v, x, y, z);
-            for (int dv = -1; dv <= 1; dv++)
-                for (int du = -1; du <= 1; du++) {
-                    const int u = u0 + du, v = v0 + dv;
-                    if (u < rn.ulo || u > rn.uhi || v < rn.vlo || v > rn.vhi) continue;
-                    int qx, qy, qz;
-                    place(fr, u, v, rn.layer, qx, qy, qz);
-                    const long long q = ((long long)qz * ny + qy) * nx + qx;
-                    graph_dec(sd, sh, q, I + 1, F, qx, qy, qz, true);
-                }
+    const bool few = m <= (sh.single ? FD_FEW1 : FD_FEW);
+    RelNode *rn = reinterpret_cast<RelNode *>(ws.s0);   /* s0, s4, z, y: free after the commit */
+    if (few && fin)
+        rn[__popc(mask & ((1u << lane) - 1u))] = {wh.x | (wh.y << 10) | (wh.z << 20), (int)wh.p, wh.inst, lane};
+    if (lane == 0) *nkey = 0;
+    __syncwarp();
+    wfence(sh);
+    if (few) {
+        if (lane < 26) {
+            const int k = lane + (lane >= 13);
+            const int kx = k % 3, ky = (k / 3) % 3, kz = k / 9;
+            const int off = ((kz - 1) * ny + ky - 1) * nx + kx - 1;
+            const unsigned rw = sh.rel[F][k];
+            for (int j = 0; j < m; j++) {
+                const RelNode n = rn[j];
+                const int w = max(max(gs.lay[0][(n.xyz & 1023) + kx], gs.lay[1][((n.xyz >> 10) & 1023) + ky]),
+                                  gs.lay[2][(n.xyz >> 20) + kz]);
+                const unsigned dec = release_dec(w, n.inst, rw, &ws.t[n.slot][13]);
+                if (dec) release_one(sd, sh, n.p + off, own_face(w), dec, keyq, nkey);
+            }
+        }
+    } else if (sh.single) {
+        if (fin) {
+            const fdn_frame fr = frame_of(F);
+            const GRect r = gs.rect[wh.inst];
+            const int su = (int)t_stride(sd, fr.axis_u), sv = (int)t_stride(sd, fr.axis_v);
+            const int p = (int)wh.p, pn = p - fr.inner * (int)t_stride(sd, fr.axis_n);
+            const float *t13 = &ws.t[lane][13];
+            const unsigned own = okey32(*t13);
+            /* columns (bits 0-2) and rows (3-5) of the 3x3 block inside a rectangle */
+            auto inside = [&](const GRect &q) {
+                const int u = wh.r.u, v = wh.r.v;
+                return (u - 1 >= q.ulo && u - 1 <= q.uhi ? 1u : 0u) | (u >= q.ulo && u <= q.uhi ? 2u : 0u)
+                       | (u + 1 >= q.ulo && u + 1 <= q.uhi ? 4u : 0u) | (v - 1 >= q.vlo && v - 1 <= q.vhi ? 8u : 0u)
+                       | (v >= q.vlo && v <= q.vhi ? 16u : 0u) | (v + 1 >= q.vlo && v + 1 <= q.vhi ? 32u : 0u);
+            };
+            const unsigned mine = inside(r);
+            const bool adj = wh.inst + 1 < sh.ninst && gs.rect[wh.inst + 1].layer == r.layer - fr.inner;
+            const unsigned next = adj ? inside(gs.rect[wh.inst + 1]) : 0u;
+#pragma unroll
+            for (int k = 0; k < 9; k++) {
+                const int du = k % 3 - 1, dv = k / 3 - 1;
+                const unsigned bits = 1u << (du + 1) | 8u << (dv + 1);
+                const int o = du * su + dv * sv;
+                if ((next & bits) == bits) release_one(sd, sh, pn + o, F, 1u, keyq, nkey);
+                if (k != 4 && (mine & bits) == bits && later_key(okey32(t13[dv * 3 + du]), own, du, dv))
+                    release_one(sd, sh, p + o, F, 1u << 8, keyq, nkey);
+            }
         }
     } else {
-        /* nodes of later instances that read p, or that p read */
-        const unsigned myctx = sh.ctxm[F];
-        for (int k = 0; k < 27; k++) {
-            if (k == 13) continue;
-            const int qx = x + k % 3 - 1, qy = y + (k / 3) % 3 - 1, qz = z + k / 9 - 1;
-            if (qx < 0 || qx >= nx || qy < 0 || qy >= ny || qz < 0 || qz >= sd.g.nz) continue;
-            const int w = owner_near(gs, sh.gfaces, F, qx, qy, qz);
-            if (w < 0 || own_inst(w) <= I) continue;
-            const int fq = own_face(w);
-            if (!((myctx >> k) & 1u) && !((sh.ctxm[fq] >> (26 - k)) & 1u)) continue;
-            const long long q = ((long long)qz * ny + qy) * nx + qx;
-            graph_dec(sd, sh, q, own_inst(w), fq, qx, qy, qz, (sh.innm[fq] >> (26 - k)) & 1u);
+        if (fin) {
+            int lx[3], ly[3], lz[3];
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                lx[k] = gs.lay[0][wh.x + k];
+                ly[k] = gs.lay[1][wh.y + k];
+                lz[k] = gs.lay[2][wh.z + k];
+            }
+            const int p = (int)wh.p, nxy = nx * ny;
+            const float *t13 = &ws.t[lane][13];
+#pragma unroll
+            for (int k = 0; k < 27; k++) {
+                if (k == 13) continue;
+                const int w = max(max(lx[k % 3], ly[(k / 3) % 3]), lz[k / 9]);
+                const unsigned dec = release_dec(w, wh.inst, sh.rel[F][k], t13);
+                if (dec)
+                    release_one(sd, sh, p + (k / 9 - 1) * nxy + ((k / 3) % 3 - 1) * nx + k % 3 - 1, own_face(w), dec, keyq,
+                                nkey);
+            }
         }
     }
-    /* later neighbours in the same instance */
-    const int nvf = r.vhi - r.vlo + 1, iu = i % r.nuf, iv = i / r.nuf;
-    const unsigned char gem = sh.cs > 1 ? __ldcg(&sd.scr.gemask[p]) : sd.scr.gemask[p];
-    unsigned later = inrect_mask(iu, iv, r.nuf, nvf) & ~(unsigned)gem;
-    while (later) {
-        const int k = __ffs(later) - 1;
-        later &= later - 1;
-        int du, dv;
-        nb_off(k, du, dv);
-        const long long q = p + du * t_stride(sd, fr.axis_u) + dv * t_stride(sd, fr.axis_v);
-        if (!FD_OK(q, (long long)sd.g.nx * sd.g.ny * sd.g.nz, 17)) continue;
-        const unsigned nw = atomicSub(&sd.scr.gcnt[q], 1u << 8) - (1u << 8);
-        if (ready_word(nw)) graph_ready(sd, sh, F, q);
+    __syncwarp();
+    wfence(sh);
+    /* inner blocks now complete: these nodes' keys and in-face order are known */
+    const int nk = *nkey;
+    for (int j = lane; j < nk; j += 32) {
+        const int q = keyq[j];
+        const int qxy = q / nx, qx = q - qxy * nx, qz = qxy / ny, qy = qxy - qz * ny;
+        const int w = owner_of(gs, qx, qy, qz);
+        if (ready_word(key_event(sd, sh, own_inst(w), inst_fill(gs.rect[own_inst(w)], qx, qy, qz), q)))
+            graph_ready(sd, sh, own_face(w), q);
     }
+    __syncwarp();
 }
 
 /* point w waits for an event of instance I (kind 1: all keys final, 2: all points done) (lane 0) */
@@ -998,8 +1098,8 @@ __device__ bool wait_point(const fd_station_dev &sd, Shared &sh, int w, long lon
 
 /* The reference's sequential minimum over the 22 trials of one node, from the values computed
  * by the warp (new-edge and new-face values that were not precomputed are evaluated here — they
- * are needed only at first contact), then the commit (src/sphfd.c:1756-1760), the node's
- * stencil-state record and the release of the nodes that wait on it.
+ * are needed only at first contact), then the commit (src/sphfd.c:1756-1760) and the node's
+ * stencil-state record; a face walk also releases the nodes that wait on it here.
  *
  * `permissive`: the node makes no writer call before its 2-D trials, so those test against a
  * stencil state left by an earlier point; their values were computed with no stale floor.  A
@@ -1065,7 +1165,7 @@ __device__ bool commit_node(const fd_station_dev &sd, Shared &sh, const TrialDes
         }
     }
     if (sh.graph)
-        graph_release(sd, sh, F, wh.p, wh.x, wh.y, wh.z, wh.inst, wh.i, writers != 0, st0, st4, t18[13]);
+        graph_record(sd, sh, wh.p, wh.inst, wh.i, writers != 0, st0, st4, t18[13]);
     else
         face_release(sd, sh, dag, wh.i, writers != 0, st0, st4);
     return true;
@@ -1084,7 +1184,7 @@ __device__ __forceinline__ Where locate(const fd_station_dev &sd, const Shared &
         wh.x = e - exy * nx;
         wh.z = exy / ny;
         wh.y = exy - wh.z * ny;
-        const int w = owner_near(gsmem(sh), sh.gfaces, F, wh.x, wh.y, wh.z);
+        const int w = owner_of(gsmem(sh), wh.x, wh.y, wh.z);
         if (w < 0) {
             ok = false;
             return wh;
@@ -1192,6 +1292,7 @@ __device__ void warp_chunk(const fd_station_dev &sd, Shared &sh, const CtaSmem &
                 enqueue_to(sh.graph ? sd.scr.grq : sd.scr.rq, sh.w->rqtail, sh.w->rqcap, sh, e);
         }
     }
+    if (sh.graph) graph_release(sd, sh, ws, F, fin, wh);
     if (sh.graph && !sh.nodefer) {
         /* points done per face instance, one atomic per instance in the chunk; the instance
          * complete wakes points waiting for its last writer */
@@ -1295,7 +1396,7 @@ __device__ void resume_graph(const fd_station_dev &sd, Shared &sh, const CtaSmem
     if (!FD_OK(w, (long long)sd.g.nx * sd.g.ny * sd.g.nz, 20)) return;
     const int wxy = w / nx;
     const int wx = w - wxy * nx, wy = wxy % ny, wz = wxy / ny;
-    const int ow = owner_of(gs, sh.gfaces, wx, wy, wz);
+    const int ow = owner_of(gs, wx, wy, wz);
     if (ow < 0) {
         if (lane == 0) atomicCAS(&sh.w->status, 0, 14);
         return;
@@ -1623,7 +1724,13 @@ __device__ void graph_sweep(const fd_station_dev &sd, Shared &sh, CtaSmem &cs, W
     const int nx = sd.g.nx, ny = sd.g.ny, nz = sd.g.nz;
     GraphSmem &gs = gsmem(sh);
     FD_TIC(t0);
-    for (int k = tid; k < FDN_NFACE * FD_LMAX; k += blockDim.x) (&gs.lay2inst[0][0])[k] = -1;
+    /* walls: 0 z1, 1 z2, 2 x2, 3 x1, 4 y1, 5 y2 */
+    for (int k = tid; k < FD_LMAX + 2; k += blockDim.x) {
+        const int c = k - 1;
+        gs.lay[0][k] = c >= 0 && c < nx && c > sh.wall[3] && c < sh.wall[2] ? FD_IN_BOX : FD_NEVER;
+        gs.lay[1][k] = c >= 0 && c < ny && c > sh.wall[4] && c < sh.wall[5] ? FD_IN_BOX : FD_NEVER;
+        gs.lay[2][k] = c >= 0 && c < nz && c > sh.wall[0] && c < sh.wall[1] ? FD_IN_BOX : FD_NEVER;
+    }
     __syncthreads();
     /* the sweep's face instances, as the radius loop visits them */
     if (tid == 0) {
@@ -1650,11 +1757,15 @@ __device__ void graph_sweep(const fd_station_dev &sd, Shared &sh, CtaSmem &cs, W
                         gr.face = (short)face; gr.layer = (short)sh.layer;
                         gr.ulo = (short)sh.ulo; gr.uhi = (short)sh.uhi; gr.vlo = (short)sh.vlo; gr.vhi = (short)sh.vhi;
                         gr.nuf = (short)sh.nuf; gr.pad = 0;
-                        gs.lay2inst[face][sh.layer] = (short)ninst;
+                        gs.lay[frame_of(face).axis_n][sh.layer + 1] = (short)((ninst << 3) | face);
                         ninst++;
                         M += sh.n;
                         per_face[face] += sh.n;
                         faces |= 1u << face;
+                    } else {
+                        /* a wall that moves while its rectangle is empty owns no node: its nodes join
+                         * with a later wall, and any word between the instances around it does */
+                        gs.lay[frame_of(face).axis_n][sh.layer + 1] = (short)(((ninst - 1) << 3) | 7);
                     }
                     /* move the wall outward (e.g. src/sphfd.c:1762-1764) */
                     const int inner = frame_of(face).inner;
@@ -1728,12 +1839,18 @@ __device__ void graph_sweep(const fd_station_dev &sd, Shared &sh, CtaSmem &cs, W
                     }
                 } else {
                     const int pi = (int)p, pxy = pi / nx;
-                    const int x = pi - pxy * nx, y = pxy % ny, z = pxy / ny;
+                    const int x = pi - pxy * nx, z = pxy / ny, y = pxy - z * ny;
+                    int lx[3], ly[3], lz[3];
+#pragma unroll
+                    for (int k = 0; k < 3; k++) {
+                        lx[k] = gs.lay[0][x + k];
+                        ly[k] = gs.lay[1][y + k];
+                        lz[k] = gs.lay[2][z + k];
+                    }
+#pragma unroll
                     for (int k = 0; k < 27; k++) {
                         if (k == 13) continue;
-                        const int qx = x + k % 3 - 1, qy = y + (k / 3) % 3 - 1, qz = z + k / 9 - 1;
-                        if (qx < 0 || qx >= nx || qy < 0 || qy >= ny || qz < 0 || qz >= nz) continue;
-                        const int w = owner_near(gs, sh.gfaces, r.face, qx, qy, qz);
+                        const int w = owner_word(lx[k % 3], ly[(k / 3) % 3], lz[k / 9]);
                         if (w < 0 || own_inst(w) > I) continue;
                         if (own_inst(w) == I) { c2++; continue; }
                         if (!((myctx >> k) & 1u) && !((sh.ctxm[own_face(w)] >> (26 - k)) & 1u)) continue;
@@ -1891,6 +2008,7 @@ __device__ __forceinline__ void solve_station(const fd_station_dev &sd, int dag_
         sh.gfaces = 0;
     }
     csync(sh, 6);
+    for (int k = tid; k < 6 * 27; k += blockDim.x) sh.rel[k / 27][k % 27] = relation_word(sh, k / 27, k % 27);
     if ((tid & 31) < 6) ws.cnt[tid & 31] = 0ull;
     __syncwarp();
     Counters cn;

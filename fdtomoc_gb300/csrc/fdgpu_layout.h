@@ -102,11 +102,10 @@ typedef struct {
     /* sweep graphs (gcnt NULL: not available, every face is walked on its own).  Per grid node:
      * dependency counter word (inner block pending in bits 0-7, same-instance neighbours in 8-15,
      * other instances' nodes in 16-23, a point waits on it bit 29, done bit 30, sort key final
-     * bit 31), ready queue, earlier-neighbour byte, stencil-state record.  Small tables: the
-     * sweep's face instances, wait pairs, parked points, resume queue. */
+     * bit 31), ready queue, stencil-state record.  Small tables: the sweep's face instances,
+     * wait pairs, parked points, resume queue. */
     unsigned *gcnt;
     int *gqueue;
-    unsigned char *gemask;
     float2 *grec;
     fd_ginst *ginst;
     int ginst_cap;

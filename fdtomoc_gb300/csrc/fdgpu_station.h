@@ -38,9 +38,9 @@ inline long long max_face(const fdgpu_station &s)
 constexpr size_t kFacePerPoint = 8 + 4 + 4 + 4 + 8 + 4 + 2;
 inline size_t face_bytes(const fdgpu_station &s) { return align256(((size_t)max_face(s) + 16) * kFacePerPoint); }
 
-/* sweep-graph arrays per grid node: stencil-state record, counter, queue, earlier-neighbour byte;
- * then the face instances, wait pairs, parked points and resume queue */
-constexpr size_t kGraphPerNode = 8 + 4 + 4 + 1;
+/* sweep-graph arrays per grid node: stencil-state record, counter, queue; then the face instances,
+ * wait pairs, parked points and resume queue */
+constexpr size_t kGraphPerNode = 8 + 4 + 4;
 inline size_t graph_node_bytes(size_t nn) { return align256(nn * kGraphPerNode); }
 inline int graph_instances(const fdgpu_station &s) { return s.nx + s.ny + s.nz + 8; }
 inline size_t graph_bytes(const fdgpu_station &s)
@@ -195,12 +195,11 @@ inline void fill_station(fd_station_dev &d, const fdgpu_station &s, const GeoPtr
     d.scr.rq = reinterpret_cast<int *>(face + 24 * m);
     d.scr.dag = reinterpret_cast<unsigned char *>(face + 32 * m);
     if (graph) {
-        /* 8-byte records first, then the 4-byte arrays, then the bytes */
+        /* 8-byte records first, then the 4-byte arrays */
         const size_t nn = (size_t)s.nx * s.ny * s.nz;
         d.scr.grec = reinterpret_cast<float2 *>(graph);
         d.scr.gcnt = reinterpret_cast<unsigned *>(graph + 8 * nn);
         d.scr.gqueue = reinterpret_cast<int *>(graph + 12 * nn);
-        d.scr.gemask = reinterpret_cast<unsigned char *>(graph + 16 * nn);
         char *tb = graph + graph_node_bytes(nn);
         d.scr.ginst_cap = graph_instances(s);
         d.scr.ginst = reinterpret_cast<fd_ginst *>(tb);
