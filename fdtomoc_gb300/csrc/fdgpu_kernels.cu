@@ -79,7 +79,7 @@ __global__ void fd_geo_build(int nx, int ny, int nz, double h, double dq, double
         double *o = node + k * FD_N_N;
         o[FD_N_RSDF] = rsdf;
         o[FD_N_INV_RSDF] = 1.0 / rsdf;
-        o[FD_N_RDFS] = (r * df) * s;
+        *reinterpret_cast<float2 *>(o + FD_N_INV32) = make_float2(d2f_trunc(1.0 / rdq), d2f_trunc(1.0 / rsdf));
         const double is_s = 1.0 / (rsdf * rsdf), is_q = 1.0 / (rdq * rdq);
         const double a_sh = is_s + is_h, a_qh = is_q + is_h, a_sq = is_s + is_q;
         o[FD_N_A_SH] = a_sh;
@@ -397,9 +397,8 @@ constexpr unsigned guard_need(int K)
 }
 
 /* what the code below takes for granted about the trial tables: the corner trials look at the quadrants
- * (+,+) (-,+) (+,-) (-,-), whose seven other cell nodes are their floor; the first 1-D trial looks at the inner
- * node and the others at the own-plane neighbours; a non-zero test is on such a neighbour; and only
- * in-plane trials (2-D and 1-D) can be head waves */
+ * (+,+) (-,+) (+,-) (-,-), whose seven other cell nodes are their floor; a non-zero test is on an own-plane
+ * neighbour; and only in-plane trials (2-D and 1-D) can be head waves (steps_as_assumed has the 1-D trials) */
 constexpr bool trials_as_assumed()
 {
     for (int f = 0; f < FDN_NFACE; f++)
@@ -417,19 +416,16 @@ constexpr bool trials_as_assumed()
                 }
                 if (__builtin_popcount(cell) != 7 || (cell >> 4) & 1u) return false;
             }
-            if (tr.kind == FDN_1D && k == TK_1D0 && nb_index(tr.t[0]) != 13) return false;
-            if (tr.kind == FDN_1D && k > TK_1D0 && (tr.t[0].w != 0 || (tr.t[0].du != 0) == (tr.t[0].dv != 0))) return false;
             if (tr.head && !(k >= TK_2D0 && k < TK_NF) && !(k > TK_1D0)) return false;
         }
     return true;
 }
 static_assert(trials_as_assumed(), "trial tables");
 
-/* per face: each trial's needed facts; two bits per trial of 1-D trials 18-21, the neighbour's dir_index;
- * and the head trials */
+/* per face: each trial's needed facts, and the head trials */
 struct FaceGuards {
     unsigned need[FDN_NTRIAL];
-    unsigned dir1d, head;
+    unsigned head;
 };
 template <int F>
 constexpr FaceGuards make_guards()
@@ -437,7 +433,6 @@ constexpr FaceGuards make_guards()
     FaceGuards g{};
     for (int k = 0; k < FDN_NTRIAL; k++) {
         g.need[k] = guard_need<F>(k);
-        if (k > TK_1D0) g.dir1d |= (unsigned)dir_index(fd_face_trials[F][k].t[0].du, fd_face_trials[F][k].t[0].dv) << (2 * (k - TK_1D0 - 1));
         if (fd_face_trials[F][k].head) g.head |= 1u << k;
     }
     return g;
@@ -484,10 +479,7 @@ __device__ __forceinline__ void guards(int face, const float (&t)[NB_N], unsigne
         if (fl < tp || high) can |= 1u << K;
     }
     const unsigned lower = (t[5] < tp ? 1u : 0u) | (t[3] < tp ? 2u : 0u) | (t[7] < tp ? 4u : 0u) | (t[1] < tp ? 8u : 0u);
-    if (t[13] < tp) can |= 1u << TK_1D0;
-#pragma unroll
-    for (int K = TK_1D0 + 1; K < FDN_NTRIAL; K++)
-        can |= ((lower >> ((fg.dir1d >> (2 * (K - TK_1D0 - 1))) & 3u)) & 1u) << K;
+    can |= (t[13] < tp ? 1u << TK_1D0 : 0u) | lower << (TK_1D0 + 1);
     em = gm & can;
     if (!(gm & 0xFu) && tp > 1.0e9f) em |= gm & 0xF0u;   /* their floors are looked at by ne_prune */
 }
@@ -518,8 +510,9 @@ __device__ __forceinline__ int push_items(unsigned short *items, int n, unsigned
     }
     return n;
 }
-constexpr unsigned kBefore2d = 0xFFu | 0x1Fu << TK_1D0;   /* corner, new-edge and 1-D trials */
+constexpr unsigned kWriters = 0xFFu;                /* corner and new-edge trials */
 constexpr unsigned k2d = 0xFFu << TK_2D0;
+constexpr unsigned k1d = 0x1Fu << TK_1D0;
 
 /* evaluate items[0..n) with the warp's lanes; a 2-D value is stored after the causality selection
  * against its floor, which includes the stencil state entering the 2-D block (src/sphfd.c:6116-6121) */
@@ -559,11 +552,13 @@ __device__ void eval_items(const fd_station_dev &sd, const TrialDesc *dsc, WarpS
 }
 
 /* Replay of the corner and new-edge trials (every writer of the stencil state comes before the
- * 2-D block): the running minimum entering the 2-D block — an upper bound for every 2-D trial's
- * turn — and the stale (t0,t4) those trials test against.  Returns the 2-D trials that can still
- * lower the minimum. */
-__device__ unsigned stale_pair(const TrialDesc *dsc, WarpSmem &ws, int slot, unsigned gm, unsigned em, float it0,
-                               float it4)
+ * 2-D block): the running minimum entering the 2-D block — an upper bound for every later trial's
+ * turn — and the stale (t0,t4) the 2-D trials test against.  Returns em with the 2-D trials that can still
+ * lower the minimum, and without the 1-D trials that cannot: nearly all lose to the corners by far more
+ * than FP32 rounding, so their time is bounded from below in FP32 (step lengths truncated, products
+ * rounded down and shortened by 2^-20, which covers the FP64 chain's rounding). */
+__device__ unsigned stale_pair(const fd_station_dev &sd, const TrialDesc *dsc, WarpSmem &ws, int slot, int F,
+                               unsigned gm, unsigned em, float it0, float it4)
 {
     const float *t18 = ws.t[slot];
     double g1 = f2d(t18[NB_POINT]);
@@ -599,7 +594,24 @@ __device__ unsigned stale_pair(const TrialDesc *dsc, WarpSmem &ws, int slot, uns
         const float fl = fmaxf(fmaxf(t18[d.slot[1]], t18[d.slot[2]]), fmaxf(t18[d.slot[3]], s04));
         if (!prunable(fl, g1)) add |= 1u << K;
     }
-    return add;
+    const float gf = d2f_trunc(g1), gup = __int_as_float(__float_as_int(gf) + 1);   /* above g1; NaN stays NaN */
+    if ((em & k1d) && gup <= 99999997952.f) {
+        const fdn_frame fr = frame_of(F);
+        const int z = ws.z[slot], y = ws.y[slot];
+        const float *s18 = ws.s[slot];
+        const float dx = d2f_trunc(node_row(sd.g, z, y)[FD_N_RSDF]);
+        const float dy = d2f_trunc(sd.g.zrow[(long long)(FD_OK(z, sd.g.nz, 8) ? z : 0) * FD_Z_N + FD_Z_RDQ]);
+        const float dz = d2f_trunc(sd.g.h);
+#pragma unroll
+        for (int k = 0; k < 5; k++) {
+            const int nb = k == 0 ? 13 : k == 1 ? 5 : k == 2 ? 3 : k == 3 ? 7 : 1;
+            const int axis = k == 0 ? fr.axis_n : k < 3 ? fr.axis_u : fr.axis_v;
+            const float len = axis == 0 ? dx : axis == 1 ? dy : dz;
+            const float step = __fmul_rd(__fmul_rd(0.5f * (s18[NB_POINT] + s18[nb]), len), 0.99999904632568359375f);
+            if (__fadd_rd(t18[nb], step) >= gup) em &= ~(1u << (TK_1D0 + k));
+        }
+    }
+    return em | add;
 }
 
 /* Drop the queued 2-D items whose single-precision lower bound shows they cannot lower the
@@ -1313,7 +1325,7 @@ __device__ void warp_chunk(const fd_station_dev &sd, Shared &sh, const CtaSmem &
         permissive = !have_inherit && (gm & 0xFu) == 0 && !((gm & 0xF0u) && t[NB_POINT] > 1.0e9f) && (gm & 0xFF00u);
     }
     __syncwarp();
-    const int n1 = push_items(ws.items, 0, em, kBefore2d, lane);
+    const int n1 = push_items(ws.items, 0, em, kWriters, lane);
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncwarp();
     FD_TOC(1, ta);
@@ -1322,11 +1334,12 @@ __device__ void warp_chunk(const fd_station_dev &sd, Shared &sh, const CtaSmem &
     __syncwarp();
     const float lo = __int_as_float(0xff800000);   /* -inf: no stale floor */
     const float p0 = permissive ? lo : it0, p4 = permissive ? lo : it4;
-    if (valid) em |= stale_pair(dsc, ws, lane, gm, em, p0, p4);
+    if (valid) em = stale_pair(sd, dsc, ws, lane, F, gm, em, p0, p4);
     __syncwarp();
     int n2 = push_items(ws.items, 0, em, k2d, lane);
     __syncwarp();
     n2 = filter_2d(sd, dsc, ws, n2, lane);
+    n2 = push_items(ws.items, n2, em, k1d, lane);
     __syncwarp();
     eval_items(sd, dsc, ws, n2, lane, cn);
     __syncwarp();

@@ -14,8 +14,8 @@
  * only touches travel times and slownesses:
  *   zrow[z][FD_Z*]      radius rc(z) and rc(z)*dq with its reciprocal;
  *   ysin[y]             sin(qc(y)), evaluated by the host C library (the reference calls sin());
- *   node[z][y][FD_N*]   the products r*sin(q)*df and r*df*sin(q), reciprocals, and the "a"
- *                       coefficient (with 1/(2a)) for the three distance pairs that the
+ *   node[z][y][FD_N*]   the product r*sin(q)*df and its reciprocal, both distances' reciprocals as
+ *                       floats, and the "a" coefficient (with 1/(2a)) for the three distance pairs that the
  *                       new-edge and 2-D stencils use;
  *   cell[zc][yc][FD_C*] every fdsph3d coefficient for the cell with corner (yc, zc): the
  *                       quadratic's a for each of the cell's four (r,q) corners and 1/(2a),
@@ -32,7 +32,7 @@ enum { FD_Z_R = 0, FD_Z_RDQ, FD_Z_INV_RDQ, FD_Z_N };
 enum {
     FD_N_RSDF = 0,   /* (rc(z)*sin(qc(y)))*df */
     FD_N_INV_RSDF,   /* 1/that, correctly rounded */
-    FD_N_RDFS,       /* (rc(z)*df)*sin(qc(y)) */
+    FD_N_INV32,      /* two floats: 1/(rc(z)*dq) and 1/RSDF, truncated (the bounds' tables) */
     FD_N_A_SH,       /* 1/RSDF^2 + 1/h^2           (each term as the reference rounds it) */
     FD_N_I2A_SH,     /* 1/(2a) */
     FD_N_A_QH,       /* 1/RDQ^2 + 1/h^2 */

@@ -134,26 +134,45 @@ constexpr bool kinds_uniform()
         }
     return true;
 }
+
+/* the 1-D trials step along one axis from the point itself: the inner neighbour, then +u -u +v -v, with the
+ * factors h (z), r dq (y), r df s or r s df (x) in this order */
+template <int F>
+constexpr bool steps_as_assumed()
+{
+    constexpr int du[5] = {0, 1, -1, 0, 0}, dv[5] = {0, 0, 0, 1, -1};
+    for (int k = 0; k < 5; k++) {
+        const fdn_trial tr = fd_face_trials[F][TK_1D0 + k];
+        if (tr.t[0].du != du[k] || tr.t[0].dv != dv[k] || tr.t[0].w != (k == 0)) return false;
+        const int axis = k == 0 ? FaceT<F>::AN : k < 3 ? FaceT<F>::AU : FaceT<F>::AV;
+        const TrialDesc d = make_desc<F>(TK_1D0 + k);
+        if (d.vn != 3 - axis) return false;
+        if (axis == 2 && d.vk[0] != FK_H) return false;
+        if (axis < 2 && d.vk[0] != FK_R) return false;
+        if (axis == 1 && d.vk[1] != FK_DQ) return false;
+        if (axis == 0 && !((d.vk[1] == FK_DF && d.vk[2] == FK_S) || (d.vk[1] == FK_S && d.vk[2] == FK_DF))) return false;
+        for (int j = 0; j < d.vn; j++)
+            if (d.vdz[j] != 0 || d.vdy[j] != 0) return false;
+    }
+    return true;
+}
+static_assert(steps_as_assumed<0>() && steps_as_assumed<1>() && steps_as_assumed<2>() && steps_as_assumed<3>()
+                  && steps_as_assumed<4>() && steps_as_assumed<5>(),
+              "1-D trials");
 static_assert(kinds_uniform(), "every face runs 4 corner, 4 new-edge, 8 2-D, 1 new-face, 5 1-D trials in that order");
 
 /* ---------------------------------------------------------------------------------------------- */
 /* geometry accessors at run time                                                                  */
 
+/* a distance and its reciprocal: both tabulated kinds are two doubles side by side, so one address is
+ * selected and nothing branches (for CH_H the descriptor's offsets are zero and the loads are unused) */
 __device__ __forceinline__ void dist_rt(const fd_geo_dev &g, int cls, int z, int y, double &d, double &inv)
 {
-    if (cls == CH_H) {
-        d = g.h;
-        inv = g.inv_h;
-    } else if (cls == CH_RDQ) {
-        if (!FD_OK(z, g.nz, 3)) z = 0;
-        const double *zr = g.zrow + (long long)z * FD_Z_N;
-        d = zr[FD_Z_RDQ];
-        inv = zr[FD_Z_INV_RDQ];
-    } else {
-        const double *nr = node_row(g, z, y);
-        d = nr[FD_N_RSDF];
-        inv = nr[FD_N_INV_RSDF];
-    }
+    if (!FD_OK(z, g.nz, 3)) z = 0;
+    const double *p = cls == CH_RDQ ? g.zrow + (long long)z * FD_Z_N + FD_Z_RDQ : node_row(g, z, y) + FD_N_RSDF;
+    const double pd = p[0], pi = p[1];
+    d = cls == CH_H ? g.h : pd;
+    inv = cls == CH_H ? g.inv_h : pi;
 }
 
 __device__ __forceinline__ void apair_rt(const fd_geo_dev &g, int ap, int z, int y, double &a, double &i2a)
@@ -298,13 +317,21 @@ __device__ __forceinline__ double eval_nf(const TrialDesc &d, const float *t18, 
     return flt(x, f2d(tchk)) ? 1.e11 : x;
 }
 
-/* straight edge: t_nbr + 0.5*(s_point + s_nbr) * f1 * f2 * f3 (e.g. src/sphfd.c:1727-1755) */
+/* straight edge: t_nbr + 0.5*(s_point + s_nbr) times the step's factors (e.g. src/sphfd.c:1727-1755): along
+ * z, h; along y, r then dq; along x, r then df and s (s first on the EAST and WEST faces) */
 __device__ __forceinline__ double eval_1d(const TrialDesc &d, const float *t18, const float *s18,
                                           const fd_geo_dev &g, int z, int y)
 {
     const float ssum = s18[NB_POINT] + s18[d.slot[0]];
     double x = scale2k<-1>(f2d(ssum));
-    for (int j = 0; j < d.vn; j++) x = x * factor_rt(g, d.vk[j], z + d.vdz[j], y + d.vdy[j], 0.f);
+    if (d.vn == 1) {
+        x = x * g.h;
+    } else {
+        x = x * g.zrow[(long long)(FD_OK(z, g.nz, 4) ? z : 0) * FD_Z_N + FD_Z_R];
+        const double s = g.ysin[FD_OK(y, g.ny, 5) ? y : 0];
+        x = x * (d.vn == 2 ? g.dq : d.vk[1] == FK_S ? s : g.df);
+        if (d.vn == 3) x = x * (d.vk[1] == FK_S ? g.df : s);
+    }
     return f2d(t18[d.slot[0]]) + x;
 }
 
