@@ -327,11 +327,6 @@ __device__ __forceinline__ void place(const fdn_frame &fr, int u, int v, int n, 
 __constant__ TrialDesc c_desc[FDN_NFACE * FDN_NTRIAL] = {FD_DESC_ROW(0), FD_DESC_ROW(1), FD_DESC_ROW(2),
                                                          FD_DESC_ROW(3), FD_DESC_ROW(4), FD_DESC_ROW(5)};
 
-__device__ __forceinline__ int kind_of(int K)
-{
-    return K < TK_NE0 ? 0 : K < TK_2D0 ? 1 : K < TK_NF ? 2 : K < TK_1D0 ? 3 : 4;
-}
-
 /* shared by the CTA: the trial descriptors of all six faces */
 struct CtaSmem {
     TrialDesc desc[FDN_NFACE][FDN_NTRIAL];
@@ -510,26 +505,199 @@ __device__ __forceinline__ int push_items(unsigned short *items, int n, unsigned
     }
     return n;
 }
-constexpr unsigned kWriters = 0xFFu;                /* corner and new-edge trials */
 constexpr unsigned k2d = 0xFFu << TK_2D0;
 constexpr unsigned k1d = 0x1Fu << TK_1D0;
 
-/* evaluate items[0..n) with the warp's lanes; a 2-D value is stored after the causality selection
- * against its floor, which includes the stencil state entering the 2-D block (src/sphfd.c:6116-6121) */
-__device__ void eval_items(const fd_station_dev &sd, const TrialDesc *dsc, WarpSmem &ws, int n, int lane, Counters cn)
+/* ---- evaluation of the queued items ----
+ *
+ * An FP64 instruction occupies its sub-partition for 64 cycles whatever the number of active lanes, so a
+ * stencil evaluated by one lane holds it for its whole serial length: 116 instructions for a corner, 70 for
+ * a new-edge or a 2-D trial.  That is the right form for a warp full of items.  A chunk of a forward
+ * sweep has one to five corners and rarely more than one of the others; there four lanes share an
+ * item, each taking the products, divisions or sums that do not depend on one another, in the
+ * reference's order within every sum: 49 and 38 instructions for up to eight items.  FD_QUAD is where
+ * two such passes would cost as much as one of the other form. */
+#ifndef FD_QUAD
+#define FD_QUAD 8
+#endif
+
+__device__ __forceinline__ double shfl_d(double x, int src) { return __shfl_sync(0xffffffffu, x, src); }
+
+/* the accepted root of fdsphne / fdsph2d and of fdsph3d (tie rules of roots_2 and roots_3d) */
+__device__ __forceinline__ double pick_2(double x1, double x2, double tmx)
 {
-    for (int j = lane; j < n; j += 32) {
-        const unsigned it = ws.items[j];
+    const bool bad1 = flt(x1, tmx), bad2 = flt(x2, tmx);
+    return bad1 ? (bad2 ? 1.e11 : x2) : (bad2 ? x1 : (flt(x2, x1) ? x2 : x1));
+}
+__device__ __forceinline__ double pick_3(double x1, double x2, double tmx)
+{
+    const bool bad1 = flt(x1, tmx), bad2 = flt(x2, tmx);
+    return bad1 ? (bad2 ? 1.e11 : x2) : (bad2 ? x1 : (flt(x1, x2) ? x1 : x2));
+}
+
+/* Up to eight corner items (fdsph3d, as eval_3d), lanes 4g .. 4g+3 on item g.  Lane r holds terms r and
+ * r+4 of the seven; the pair sums' rows go 0 | 1 and 5 | 2 and 4 | 3 to the lanes, six products each; then lane
+ * 0 adds up b, lane 1 c and lane 2 the slownesses, side by side.  Terms pass through the trial values'
+ * columns from the 2-D trials on, which hold nothing yet: rows 4g .. 4g+3, T then R | S | P | Q.
+ * Groups beyond n repeat the first item and store nothing. */
+__device__ void eval_corners_quad(const fd_station_dev &sd, const TrialDesc *dsc, WarpSmem &ws, const unsigned short *items,
+                                  int n, int lane)
+{
+    const int g = lane >> 2, r = lane & 3, lead = lane & ~3;
+    const unsigned it = items[g < n ? g : 0];
+    const int slot = (int)(it >> 5), K = (int)(it & 31);
+    const TrialDesc &d = dsc[K];
+    const float *t18 = ws.t[slot], *s18 = ws.s[slot];
+    double *T = &ws.res[lead][TK_2D0], *R = T + 7, *S = &ws.res[lead + 1][TK_2D0], *P = &ws.res[lead + 2][TK_2D0],
+           *Q = &ws.res[lead + 3][TK_2D0];
+    int zc = ws.z[slot] + d.zmin, yc = ws.y[slot] + d.ymin;
+    if (!FD_OK(zc, sd.g.nz - 1, 6) || !FD_OK(yc, sd.g.ny - 1, 7)) { zc = 0; yc = 0; }
+    const double *C = sd.g.cell + ((long long)zc * (sd.g.ny - 1) + yc) * FD_C_N;
+    const double a = C[d.a_idx], i2a = C[d.i2a_idx];
+    float tm = 0.f;
+    double tr = 0.0;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const int i = r + 4 * h;   /* term 7: the point itself, a slowness only */
+        const int nb = i < 7 ? d.slot[i] : NB_POINT;
+        S[i] = f2d(s18[nb]);
+        if (i < 7) {
+            const double t = f2d(t18[nb]);
+            if (h == 0) tr = t;
+            tm = h == 0 ? t18[nb] : fmaxf(tm, t18[nb]);
+            T[i] = t;
+            P[i] = t * C[d.prow[i]];
+            Q[i] = (t * t) * C[d.diag[i]];
+        }
+    }
+    tm = fmaxf(tm, __shfl_xor_sync(0xffffffffu, tm, 1));
+    tm = fmaxf(tm, __shfl_xor_sync(0xffffffffu, tm, 2));
+    __syncwarp();
+    const int len = 6 - r, first = r == 0 ? 0 : r == 1 ? 6 : r == 2 ? 11 : 15;   /* row r's terms in the pair list */
+    double acc = 0.0, acc2 = 0.0;
+#pragma unroll
+    for (int k = 0; k < 6; k++) {
+        const bool in = k < len;
+        const double x = T[in ? r + 1 + k : k == 4 ? 5 : 6] * C[d.pair[in ? first + k : k + (r == 1 ? 15 : 14)]];
+        if (k == 0) {
+            acc = x;
+        } else {
+            const double y = (in ? acc : acc2) + x;
+            if (in) acc = y;
+            else acc2 = k == len ? x : y;
+        }
+    }
+    const double r1 = acc * tr, r2 = acc2 * T[r == 1 ? 5 : 4];
+    R[r] = r1;
+    if (r == 1) R[5] = r2;
+    if (r == 2) R[4] = r2;
+    __syncwarp();
+    const double *ch = r == 0 ? P : r == 1 ? Q : S;
+    double v = ch[0];
+#pragma unroll
+    for (int k = 1; k < 7; k++) v = v + ch[k];
+#pragma unroll
+    for (int k = 0; k < 6; k++) {
+        const double x = r == 1 ? R[k] : S[7];
+        if (r == 1 || (r > 1 && k == 0)) v = v + x;
+    }
+    /* b*b in lane 0, 2 sum (sum / 8) in lane 2 */
+    const double m = (r == 0 ? v : scale2k<1>(v)) * (r == 0 ? v : scale2k<-3>(v));
+    const double b = shfl_d(v, lead), bb = shfl_d(m, lead);
+    const double c = shfl_d(v, lead + 1) - shfl_d(m, lead + 2);
+    const double rad = bb - scale2k<2>(a) * c;
+    const bool none = not_ge0(rad);
+    const double sq = __dsqrt_rn(none ? 0.0 : rad);
+    const double x = div_rn(-b + (r & 1 ? -sq : sq), scale2k<1>(a), i2a);
+    const double x1 = shfl_d(x, lead), x2 = shfl_d(x, lead + 1);
+    if (r == 0 && g < n) ws.res[slot][K] = none ? 1.e11 : pick_3(x1, x2, f2d(tm));
+    __syncwarp();
+}
+
+/* Up to eight new-edge or 2-D items (fdsphne and fdsph2d, as eval_ne and eval_2d), lanes 4g .. 4g+3 on item
+ * g.  Both solve the same form, with X, Y, Z = t4, t2, t1 (new edge) or t1, t2, t3 (2-D):
+ *   p = (X - Z)/dp - Y/dy,  q = (Y - Z)/dq - X/dx,  b = 2 (p/dy + q/dx),  c = p^2 + q^2 [+ ((t0 - t3)/d01)^2] - sum^2/4.
+ * Lanes 0 to 3 take the four quotients, then 1 and 3 the two of b and 0 the new edge's third square. */
+__device__ void eval_edges_quad(const fd_station_dev &sd, const TrialDesc *dsc, WarpSmem &ws, const unsigned short *items,
+                                int n, int lane)
+{
+    const int g = lane >> 2, r = lane & 3, lead = lane & ~3;
+    const unsigned it = items[g < n ? g : 0];
+    const int slot = (int)(it >> 5), K = (int)(it & 31);
+    const bool ne = K < TK_2D0;
+    const TrialDesc &d = dsc[K];
+    const float *t18 = ws.t[slot], *s18 = ws.s[slot];
+    const int z = ws.z[slot], y = ws.y[slot];
+    const int j = (ne ? 0x4132 : 0x0312) >> (4 * r) & 15;   /* this lane's distance: dp dy dq dx */
+    double dd, iv, a, i2a;
+    dist_rt(sd.g, d.dcls[j], z + d.ddz[j], y + d.ddy[j], dd, iv);
+    apair_rt(sd.g, d.apair, z, y, a, i2a);
+    const float fx = t18[d.slot[ne ? 4 : 1]], fy = t18[d.slot[2]], fz = t18[d.slot[ne ? 1 : 3]];
+    float fl = fmaxf(fmaxf(fx, fy), fz);
+    const double tz = f2d(fz), ta = f2d(r == 0 || r == 3 ? fx : fy);
+    const double df = ta - tz;
+    const double q1 = div_rn(r & 1 ? ta : df, dd, iv);
+    const double pq = q1 - shfl_d(q1, lane ^ 1);      /* p in lane 0, q in lane 2 */
+    double v = shfl_d(pq, lane & ~1);                 /* p in lanes 0 and 1, q in 2 and 3 */
+    double d3 = 0.0;
+    if (ne) {
+        const float f0 = t18[d.slot[0]], f3 = t18[d.slot[3]];
+        fl = fmaxf(fl, fmaxf(f0, f3));
+        d3 = f2d(f0) - f2d(f3);
+        if (r == 0) dist_rt(sd.g, d.dcls[0], z + d.ddz[0], y + d.ddy[0], dd, iv);
+    } else {
+        fl = fmaxf(fl, fmaxf(ws.s0[slot], ws.s4[slot]));
+    }
+    const double q2 = div_rn(r == 0 ? d3 : v, dd, iv);
+    if (r == 0) v = q2;                               /* the new edge's third term; zero for a 2-D trial */
+    const double b = scale2k<1>(shfl_d(q2, lead + 1) + shfl_d(q2, lead + 3));
+    /* slownesses in the reference's order, one conversion a lane */
+    const int so = ne ? (r == 3 ? NB_POINT : d.slot[r == 0 ? 1 : r == 1 ? 2 : 4]) : (r == 0 ? NB_POINT : d.slot[r]);
+    const double sl = f2d(s18[so]);
+    const double sum = ((shfl_d(sl, lead) + shfl_d(sl, lead + 1)) + shfl_d(sl, lead + 2)) + shfl_d(sl, lead + 3);
+    const double m = (r == 2 ? sum : v) * (r == 2 ? scale2k<-2>(sum) : v);
+    const double c = ((shfl_d(m, lead + 1) + shfl_d(m, lead + 3)) + shfl_d(m, lead)) - shfl_d(m, lead + 2);
+    const double rad = b * b - scale2k<2>(a) * c;
+    const bool none = not_ge0(rad);
+    const double sq = __dsqrt_rn(none ? 0.0 : rad);
+    const double x = div_rn(-b + (r & 1 ? -sq : sq), scale2k<1>(a), i2a);
+    const double x1 = shfl_d(x, lead), x2 = shfl_d(x, lead + 1);
+    if (r == 0 && g < n) ws.res[slot][K] = none ? 1.e11 : pick_2(x1, x2, f2d(fl));
+    __syncwarp();
+}
+
+/* Evaluate items[0..n), all corner trials (kind 0), new-edge (1), 2-D (2) or 1-D (4), with the warp's lanes; a
+ * 2-D value is stored after the causality selection against its floor, which includes the stencil
+ * state entering the 2-D block (src/sphfd.c:6116-6121) */
+template <int KIND>
+__device__ __forceinline__ void eval_items(const fd_station_dev &sd, const TrialDesc *dsc, WarpSmem &ws,
+                                           const unsigned short *items, int n, int lane)
+{
+    if (lane == 0) ws.cnt[KIND] += (unsigned)n;
+    int j0 = 0;
+    if constexpr (KIND < 3) {
+        const int rest = n & 31;   /* whole warps of items, and a remainder above FD_QUAD, one lane each */
+        if (rest && rest <= FD_QUAD) {
+            for (; j0 < rest; j0 += 8) {
+                const int m = rest - j0 < 8 ? rest - j0 : 8;
+                if constexpr (KIND == 0) eval_corners_quad(sd, dsc, ws, items + j0, m, lane);
+                else eval_edges_quad(sd, dsc, ws, items + j0, m, lane);
+            }
+            j0 = rest;
+        }
+    }
+    for (int j = j0 + lane; j < n; j += 32) {
+        const unsigned it = items[j];
         const int slot = (int)(it >> 5), K = (int)(it & 31);
         const TrialDesc &d = dsc[K];
         const int z = ws.z[slot], y = ws.y[slot];
         const float *t18 = ws.t[slot], *s18 = ws.s[slot];
-        const int kind = kind_of(K);
         double v;
-        switch (kind) {
-        case 0: v = eval_3d(d, t18, s18, sd.g, z, y); break;
-        case 1: v = eval_ne(d, t18, s18, sd.g, z, y); break;
-        case 2: {
+        if constexpr (KIND == 0) {
+            v = eval_3d(d, t18, s18, sd.g, z, y);
+        } else if constexpr (KIND == 1) {
+            v = eval_ne(d, t18, s18, sd.g, z, y);
+        } else if constexpr (KIND == 2) {
             double x1, x2;
             eval_2d(d, t18, s18, sd.g, z, y, x1, x2);
             if ((__double_as_longlong(x1) & 0x7fffffffffffffffll) > 0x7ff0000000000000ll) {   /* NaN: no root */
@@ -537,17 +705,12 @@ __device__ void eval_items(const fd_station_dev &sd, const TrialDesc *dsc, WarpS
             } else {
                 const float fl = fmaxf(fmaxf(fmaxf(t18[d.slot[1]], t18[d.slot[2]]), fmaxf(t18[d.slot[3]], ws.s0[slot])),
                                        ws.s4[slot]);
-                const double f = f2d(fl);
-                const bool bad1 = flt(x1, f), bad2 = flt(x2, f);
-                v = bad1 ? (bad2 ? 1.e11 : x2) : (bad2 ? x1 : (flt(x2, x1) ? x2 : x1));
+                v = pick_2(x1, x2, f2d(fl));
             }
-            break;
-        }
-        case 3: v = eval_nf(d, t18, s18, sd.g, z, y); break;
-        default: v = eval_1d(d, t18, s18, sd.g, z, y); break;
+        } else {
+            v = eval_1d(d, t18, s18, sd.g, z, y);
         }
         ws.res[slot][K] = v;
-        count_eval(cn, kind);
     }
 }
 
@@ -1325,12 +1488,14 @@ __device__ void warp_chunk(const fd_station_dev &sd, Shared &sh, const CtaSmem &
         permissive = !have_inherit && (gm & 0xFu) == 0 && !((gm & 0xF0u) && t[NB_POINT] > 1.0e9f) && (gm & 0xFF00u);
     }
     __syncwarp();
-    const int n1 = push_items(ws.items, 0, em, kWriters, lane);
+    const int n3 = push_items(ws.items, 0, em, 0xFu, lane);
+    const int n1 = push_items(ws.items, n3, em, 0xF0u, lane);
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncwarp();
     FD_TOC(1, ta);
     FD_TIC(tb);
-    eval_items(sd, dsc, ws, n1, lane, cn);
+    eval_items<0>(sd, dsc, ws, ws.items, n3, lane);
+    eval_items<1>(sd, dsc, ws, ws.items + n3, n1 - n3, lane);
     __syncwarp();
     const float lo = __int_as_float(0xff800000);   /* -inf: no stale floor */
     const float p0 = permissive ? lo : it0, p4 = permissive ? lo : it4;
@@ -1339,9 +1504,10 @@ __device__ void warp_chunk(const fd_station_dev &sd, Shared &sh, const CtaSmem &
     int n2 = push_items(ws.items, 0, em, k2d, lane);
     __syncwarp();
     n2 = filter_2d(sd, dsc, ws, n2, lane);
-    n2 = push_items(ws.items, n2, em, k1d, lane);
+    const int n4 = push_items(ws.items, n2, em, k1d, lane);
     __syncwarp();
-    eval_items(sd, dsc, ws, n2, lane, cn);
+    eval_items<2>(sd, dsc, ws, ws.items, n2, lane);
+    eval_items<4>(sd, dsc, ws, ws.items + n2, n4 - n2, lane);
     __syncwarp();
     FD_TOC(2, tb);
     FD_TIC(tc);
