@@ -899,13 +899,15 @@ __device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long x)
 /* is the sort order of the inner-layer times, known once a node's inner block is final (its inner */
 /* block holds the inner nodes of all its in-face neighbours).  Every node keeps one counter word: */
 /* inner block pending (bits 0-7), same-instance neighbours pending (8-15), other-instance nodes    */
-/* pending (16-23), a point waits on it (bit 29), done (bit 30), key final (bit 31).  After a      */
+/* pending (16-23), it made a writer call (bit 28), a point waits on it (bit 29), done (bit 30), key */
+/* final (bit 31).  After a                                                                        */
 /* restart (one face) this is a plane pipeline; in the forward sweep it lets all six faces and     */
 /* successive wall positions advance together.                                                     */
 /*                                                                                                 */
 /* Inherited stencil state: a point whose 2-D trials need the state an earlier point left, and    */
 /* whose result depends on it, waits for the last point before it (in the reference's order) that  */
-/* made a writer call: the predecessor by key in its own instance once all keys there are final,   */
+/* made a writer call: the last such point in its own instance, once all keys there are final, or  */
+/* the last one not yet done if that comes after it (then it looks again when that one is done),   */
 /* else the last writer of the nearest earlier instance once that instance is complete.  Waits    */
 /* are registered on a point (a wait pair and the counter's wait bit) or on an instance event (all */
 /* keys final, all points done; a parked-point entry).                                            */
@@ -915,6 +917,7 @@ __device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long x)
 #define FD_GRAPH_FORWARD 1           /* the first sweep as a graph too */
 #endif
 #define FD_IMAX 3088                 /* face instances: at most nx + ny + nz + 8 */
+#define FD_WRITERB 0x10000000u       /* done, and it made a writer call */
 #define FD_WAITB 0x20000000u
 #define FD_DONEB 0x40000000u
 
@@ -1027,18 +1030,17 @@ __device__ __forceinline__ int inst_fill(const GRect &r, int x, int y, int z)
     return (coord(fr.axis_v, x, y, z) - r.vlo) * r.nuf + (coord(fr.axis_u, x, y, z) - r.ulo);
 }
 
-/* points parked on instance I's event `kind` (1: all keys final, 2: all done) go to the resume queue */
+/* Points parked on instance I's event `kind` (1: all keys final, 2: all done) go to the resume queue.  The
+ * event's word heads a list of them through gpark, and says so once the event has fired; the one
+ * thread whose count completes the event takes the list. */
 __device__ void fire_event(const fd_station_dev &sd, Shared &sh, int I, int kind)
 {
     wfence(sh);
-    if (!(vload(sd.scr.ginst[I].evwait) & kind)) return;
-    const int st = (kind << 24) | I;
-    const int np = min(vload(sh.w->npark), FD_GPARK_CAP);
-    for (int k = 0; k < np; k++) {
-        if (vload(sd.scr.gpark[k].y) == st && atomicCAS(&sd.scr.gpark[k].y, st, -2) == st) {
-            wfence(sh);
-            enqueue_to(sd.scr.grq, sh.w->rqtail, sh.w->rqcap, sh, vload(sd.scr.gpark[k].x));
-        }
+    int k = atomicExch(&sd.scr.ginst[I].ev[kind - 1], FD_EV_FIRED);
+    wfence(sh);
+    while (k >= 0) {
+        enqueue_to(sd.scr.grq, sh.w->rqtail, sh.w->rqcap, sh, vload(sd.scr.gpark[k].x));
+        k = vload(sd.scr.gpark[k].y);
     }
 }
 
@@ -1086,6 +1088,26 @@ __device__ __forceinline__ void graph_ready(const fd_station_dev &sd, Shared &sh
     enqueue_to(sd.scr.gqueue + sh.w->qbase[face], sh.w->qtail[face], sh.w->qcap[face], sh, (int)q);
 }
 
+/* Points that wait for a point: (awaited, waiting) pairs in a hash table probed one slot on at a time.  The
+ * first word of a slot is -1 (free), -2 (being filled), -3 (taken back or woken) or the awaited point; a slot
+ * never becomes free again within a sweep, so the pairs of a point lie between its hash slot and the
+ * first free one.  (A list of all the sweep's pairs, searched for every awaited point, cost up to half a
+ * million cycles a wake-up on windows with thousands of waits.) */
+__device__ __forceinline__ unsigned wait_slot(int p) { return ((unsigned)p * 2654435761u) >> 16; }
+static_assert(FD_GWAIT_CAP == 1 << 16, "wait_slot");
+
+__device__ void wake_waiters(const fd_station_dev &sd, Shared &sh, int p)
+{
+    wfence(sh);
+    unsigned k = wait_slot(p);
+    for (int n = 0; n < FD_GWAIT_CAP; n++, k = (k + 1) & (FD_GWAIT_CAP - 1)) {
+        const int x = vload(sd.scr.gwait[k].x);
+        if (x == -1) break;
+        if (x == p && atomicCAS(&sd.scr.gwait[k].x, p, -3) == p)
+            enqueue_to(sd.scr.grq, sh.w->rqtail, sh.w->rqcap, sh, vload(sd.scr.gwait[k].y));
+    }
+}
+
 /* node p (instance I, fill index i) is final: its record, and the points that wait for it */
 __device__ void graph_record(const fd_station_dev &sd, Shared &sh, long long p, int I, int i, bool writer, float st0,
                              float st4, float tin)
@@ -1103,13 +1125,7 @@ __device__ void graph_record(const fd_station_dev &sd, Shared &sh, long long p, 
     }
     wfence(sh);
     /* done; a point waiting for the stencil state left before it resumes its search */
-    if (!sh.nodefer && (atomicOr(&sd.scr.gcnt[p], FD_DONEB) & FD_WAITB)) {
-        wfence(sh);
-        const int nw = min(vload(sh.w->nwait), FD_GWAIT_CAP);
-        for (int k = 0; k < nw; k++)
-            if (vload(sd.scr.gwait[k].x) == (int)p && atomicCAS(&sd.scr.gwait[k].x, (int)p, -1) == (int)p)
-                enqueue_to(sd.scr.grq, sh.w->rqtail, sh.w->rqcap, sh, vload(sd.scr.gwait[k].y));
-    }
+    if (!sh.nodefer && (atomicOr(&sd.scr.gcnt[p], FD_DONEB | (writer ? FD_WRITERB : 0u)) & FD_WAITB)) wake_waiters(sd, sh, (int)p);
 }
 
 /* nodes of a chunk up to which a release gives each neighbour a lane (more: each node), in a sweep of
@@ -1272,32 +1288,38 @@ __device__ void wait_event(const fd_station_dev &sd, Shared &sh, int w, int I, i
         atomicCAS(&sh.w->status, 0, 15);
         return;
     }
-    const int st = (kind << 24) | I;
+    int *head = &sd.scr.ginst[I].ev[kind - 1];
     sd.scr.gpark[k].x = w;
-    wfence(sh);
-    atomicExch(&sd.scr.gpark[k].y, st);
-    atomicOr(&sd.scr.ginst[I].evwait, kind);
-    wfence(sh);
-    const int n = rect_n(gsmem(sh).rect[I]);
-    const bool now = kind == 1 ? vload(sd.scr.ginst[I].nkeyed) >= n : vload(sd.scr.ginst[I].ndone) >= n;
-    if (now && atomicCAS(&sd.scr.gpark[k].y, st, -2) == st) enqueue_to(sd.scr.grq, sh.w->rqtail, sh.w->rqcap, sh, w);
+    for (int h = vload(*head);;) {
+        if (h == FD_EV_FIRED) {   /* it has happened already */
+            enqueue_to(sd.scr.grq, sh.w->rqtail, sh.w->rqcap, sh, w);
+            return;
+        }
+        sd.scr.gpark[k].y = h;
+        wfence(sh);
+        const int old = atomicCAS(head, h, k);
+        if (old == h) return;
+        h = old;
+    }
 }
 
 /* point w waits for point p to be done (lane 0).  Returns false if p is already done (no wait). */
 __device__ bool wait_point(const fd_station_dev &sd, Shared &sh, int w, long long p)
 {
-    const int k = atomicAdd(&sh.w->nwait, 1);
-    if (k >= FD_GWAIT_CAP) {
+    if (atomicAdd(&sh.w->nwait, 1) >= FD_GWAIT_CAP) {
         atomicCAS(&sh.w->status, 0, 15);
         return true;
     }
+    unsigned k = wait_slot((int)p);
+    for (int n = 0; n < FD_GWAIT_CAP; n++, k = (k + 1) & (FD_GWAIT_CAP - 1))
+        if (vload(sd.scr.gwait[k].x) == -1 && atomicCAS(&sd.scr.gwait[k].x, -1, -2) == -1) break;
     sd.scr.gwait[k].y = w;
     wfence(sh);
     atomicExch(&sd.scr.gwait[k].x, (int)p);
     wfence(sh);
     if (!(atomicOr(&sd.scr.gcnt[p], FD_WAITB) & FD_DONEB)) return true;
     /* p finished meanwhile: take the pair back unless p's release already took it (and queued w) */
-    return atomicCAS(&sd.scr.gwait[k].x, (int)p, -1) != (int)p;
+    return atomicCAS(&sd.scr.gwait[k].x, (int)p, -3) != (int)p;
 }
 
 /* ---------------------------------------------------------------------------------------------- */
@@ -1638,31 +1660,57 @@ __device__ void resume_graph(const fd_station_dev &sd, Shared &sh, const CtaSmem
         if (lane == 0) wait_event(sd, sh, w, I, 1);
         return;
     }
-    unsigned long long kc = inst_key(sd, r, inst_fill(r, wx, wy, wz));
+    const unsigned long long kc = inst_key(sd, r, inst_fill(r, wx, wy, wz));
+    const fdn_frame fr = frame_of(r.face);
+    const int su = (int)t_stride(sd, fr.axis_u), sv = (int)t_stride(sd, fr.axis_v);
+    const int base = (int)inst_node(sd, r, 0), in = fr.inner * (int)t_stride(sd, fr.axis_n);
+    const int dv = 32 / r.nuf, du = 32 - dv * r.nuf;   /* 32 points on in fill order */
     for (int guard = 0; guard <= 2 * n + 2; guard++) {
-        /* predecessor in the instance */
-        unsigned long long best = 0ull;
-        for (int j = lane; j < n; j += 32) {
-            const unsigned long long k = inst_key(sd, r, j);
-            if (k < kc && k > best) best = k;
+        /* among the instance's earlier points: the last writer that is done, and the last point that is
+         * not (it may yet be a writer); four points a lane at a time, so that their loads overlap */
+        unsigned long long done = 0ull, pend = 0ull;
+        int u = lane % r.nuf, v = lane / r.nuf;
+        for (int j0 = lane; j0 < n; j0 += 128) {
+            int q[4];
+            unsigned long long key[4];
+            unsigned cnt[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                q[k] = base + u * su + v * sv;
+                const int j = j0 + 32 * k;
+                key[k] = j < n ? node_key(vload(sd.T[q[k] + in]), j) : ~0ull;
+                u += du;
+                v += dv;
+                if (u >= r.nuf) { u -= r.nuf; v++; }
+            }
+#pragma unroll
+            for (int k = 0; k < 4; k++) cnt[k] = key[k] < kc ? vload(sd.scr.gcnt[q[k]]) : 0u;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                if (key[k] >= kc) continue;
+                if (!(cnt[k] & FD_DONEB)) pend = key[k] > pend ? key[k] : pend;
+                else if (cnt[k] & FD_WRITERB) done = key[k] > done ? key[k] : done;
+            }
         }
-        best = warp_max_u64(best);
-        int verdict = 0;   /* 0 continue below best, 1 found, 2 waiting */
+        done = warp_max_u64(done);
+        pend = warp_max_u64(pend);
+        int verdict = 0;   /* 0 look again, 1 found, 2 waiting */
         float t0 = sh.carry_t0, t4 = sh.carry_t4;
         if (lane == 0) {
-            if (best) {
-                const long long p = inst_node(sd, r, (int)(best & 0xffffffffu));
-                if (!FD_OK((long long)(best & 0xffffffffu), n, 21)) {
-                    verdict = 2;
-                } else if (!(vload(sd.scr.gcnt[p]) & FD_DONEB) && wait_point(sd, sh, w, p)) {
+            if (pend > done) {
+                if (wait_point(sd, sh, w, inst_node(sd, r, (int)(pend & 0xffffffffu)))) verdict = 2;
+            } else if (done) {
+                const long long p = inst_node(sd, r, (int)(done & 0xffffffffu));
+                if (!FD_OK((long long)(done & 0xffffffffu), n, 21)) {
                     verdict = 2;
                 } else {
                     wfence(sh);
-                    const float r0 = vload(sd.scr.grec[p].x), r4 = vload(sd.scr.grec[p].y);
-                    if (!isnan(r0)) { verdict = 1; t0 = r0; t4 = r4; }
+                    verdict = 1;
+                    t0 = vload(sd.scr.grec[p].x);
+                    t4 = vload(sd.scr.grec[p].y);
                 }
             } else {
-                /* no earlier point in the instance: the last writer of an earlier instance */
+                /* no writer before it in the instance: the last writer of an earlier instance */
                 verdict = 1;
                 for (int J = I - 1; J >= 0; J--) {
                     const GRect &rj = gs.rect[J];
@@ -1687,7 +1735,6 @@ __device__ void resume_graph(const fd_station_dev &sd, Shared &sh, const CtaSmem
             warp_chunk(sd, sh, cs, ws, r.face, lane == 0 ? w : -1, true, t0, t4, nullptr, cn);
             return;
         }
-        kc = best;
     }
     if (lane == 0) atomicCAS(&sh.w->status, 0, 12);
 }
@@ -1981,7 +2028,7 @@ __device__ void graph_sweep(const fd_station_dev &sd, Shared &sh, CtaSmem &cs, W
                             gi.face = face; gi.layer = sh.layer;
                             gi.ulo = sh.ulo; gi.uhi = sh.uhi; gi.vlo = sh.vlo; gi.vhi = sh.vhi;
                             gi.nuf = sh.nuf; gi.n = sh.n;
-                            gi.nkeyed = 0; gi.ndone = 0; gi.evwait = 0; gi.pad = 0; gi.exitkey = 0ull;
+                            gi.nkeyed = 0; gi.ndone = 0; gi.ev[0] = gi.ev[1] = FD_EV_NONE; gi.exitkey = 0ull;
                         }
                         GRect &gr = gs.rect[ninst];
                         gr.face = (short)face; gr.layer = (short)sh.layer;
@@ -2109,10 +2156,9 @@ __device__ void graph_sweep(const fd_station_dev &sd, Shared &sh, CtaSmem &cs, W
     }
     /* the small tables back to their empty state for the next sweep */
     {
-        const int nw = min(vload(sh.w->nwait), FD_GWAIT_CAP), np = min(vload(sh.w->npark), FD_GPARK_CAP);
+        const int nw = vload(sh.w->nwait) > 0 ? FD_GWAIT_CAP : 0;
         const int nr = min(vload(sh.w->rqtail), FD_GRQ_CAP);
         for (int k = gt; k < nw; k += gstride) sd.scr.gwait[k] = make_int2(-1, -1);
-        for (int k = gt; k < np; k += gstride) sd.scr.gpark[k] = make_int2(-1, -2);
         for (int k = gt; k < nr; k += gstride) sd.scr.grq[k] = -1;
     }
     if (tid == 0) {
@@ -2203,7 +2249,6 @@ __device__ __forceinline__ void solve_station(const fd_station_dev &sd, int dag_
         if (gok) {
             /* the sweep-graph tables start empty */
             for (int k = tid; k < FD_GWAIT_CAP; k += blockDim.x) sd.scr.gwait[k] = make_int2(-1, -1);
-            for (int k = tid; k < FD_GPARK_CAP; k += blockDim.x) sd.scr.gpark[k] = make_int2(-1, -2);
             for (int k = tid; k < FD_GRQ_CAP; k += blockDim.x) sd.scr.grq[k] = -1;
         }
         if (sd.init_mode == 0) init_field(sd);

@@ -80,13 +80,17 @@ typedef struct {
 typedef struct {
     int face, layer, ulo, uhi, vlo, vhi, nuf, n;
     int nkeyed, ndone;             /* points whose sort key is final; points done */
-    int evwait, pad;               /* bit 1: points wait for all keys, bit 2: for all points done */
+    int ev[2];                     /* events "all keys final", "all points done": the first parked
+                                      point waiting for it (gpark index), FD_EV_NONE, FD_EV_FIRED */
     unsigned long long exitkey;    /* largest key of a point that made a writer call (0: none) */
 } fd_ginst;
 
+#define FD_EV_NONE (-1)
+#define FD_EV_FIRED (-2)
+
 /* sizes of the small sweep-graph tables */
-#define FD_GWAIT_CAP 65536   /* (awaited point, waiting point) pairs */
-#define FD_GPARK_CAP 65536   /* points parked on an instance event, and their wait states */
+#define FD_GWAIT_CAP 65536   /* (awaited point, waiting point) pairs, a hash table */
+#define FD_GPARK_CAP 65536   /* points parked on an instance event: (point, next in the event's list) */
 #define FD_GRQ_CAP 262144    /* resume queue */
 
 /* Face-walk scratch of one station, sized for its largest face m (34 bytes per point):
@@ -101,8 +105,8 @@ typedef struct {
                                   not fit in shared memory */
     /* sweep graphs (gcnt NULL: not available, every face is walked on its own).  Per grid node:
      * dependency counter word (inner block pending in bits 0-7, same-instance neighbours in 8-15,
-     * other instances' nodes in 16-23, a point waits on it bit 29, done bit 30, sort key final
-     * bit 31), ready queue, stencil-state record.  Small tables: the sweep's face instances,
+     * other instances' nodes in 16-23, made a writer call bit 28, a point waits on it bit 29, done
+     * bit 30, sort key final bit 31), ready queue, stencil-state record.  Small tables: the sweep's face instances,
      * wait pairs, parked points, resume queue. */
     unsigned *gcnt;
     int *gqueue;
