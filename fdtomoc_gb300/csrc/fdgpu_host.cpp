@@ -30,12 +30,11 @@
 extern "C" cudaError_t fdk_launch_geo_build(int nx, int ny, int nz, double h, double dq, double df, double z0r,
                                             const double *ysin, double *zrow, double *node, double *cell,
                                             cudaStream_t stream);
-extern "C" cudaError_t fdk_launch_solve(const fd_station_dev *stations, int nst, long long max_face_pad, int cluster,
-                                        cudaStream_t stream);
+extern "C" cudaError_t fdk_launch_solve(const fd_station_dev *stations, int nst, long long max_face_pad, int lmax,
+                                        int imax, cudaStream_t stream);
 extern "C" cudaError_t fdk_launch_v2s(const float *v, float *s, long long n, cudaStream_t stream);
-extern "C" cudaError_t fdk_solve_config(int nst, long long max_face_pad, int cluster, long long *bytes_out,
-                                        int *csz_out);
-extern "C" cudaError_t fdk_solve_launch(const fd_station_dev *stations, int nst, long long bytes, int cs,
+extern "C" cudaError_t fdk_solve_config(long long max_face_pad, int lmax, int imax, long long *bytes_out);
+extern "C" cudaError_t fdk_solve_launch(const fd_station_dev *stations, int nst, long long bytes, int lmax, int imax,
                                         cudaStream_t stream);
 extern "C" cudaError_t fdk_probe_fp64(double *scratch, int blocks, int threads, int iters, float *ms, cudaStream_t s);
 
@@ -334,10 +333,10 @@ std::string station_key(const fdgpu_station &s)
 }
 
 /* Check the stations and lay out their records in bufs (queued on cs): everything a launch of
- * fd_solve reads, except the fields and the slowness it points at.  *max_pad: the largest face. */
+ * fd_solve reads, except the fields and the slowness it points at. */
 int prepare_batch(fdgpu_ctx *ctx, int n, const fdgpu_station *st, const float *slowness, long long s_sy,
                   long long s_sz, float *const *d_times, int times_initialised, BatchBufs &bufs, cudaStream_t cs,
-                  long long *max_pad_out)
+                  fdh::SolveShape *shape)
 {
     if (((uintptr_t)slowness & 3u) != 0) return FDGPU_EINVAL;
     for (int k = 0; k < n; k++) {
@@ -356,7 +355,7 @@ int prepare_batch(fdgpu_ctx *ctx, int n, const fdgpu_station *st, const float *s
     for (int k = 0; k < n; k++) maxt = std::max(maxt, fdh::box_trig_count(st[k]));
     FD_CU(ctx, bufs.trig.ensure(sizeof(double) * (size_t)maxt * n + 8));
     std::vector<fd_station_dev> hs(n);
-    long long max_pad = 16;
+    *shape = fdh::SolveShape();
     std::vector<double> trig((size_t)maxt * n, 0.0);
     for (int k = 0; k < n; k++) {
         const fdgpu_station &s = st[k];
@@ -371,7 +370,7 @@ int prepare_batch(fdgpu_ctx *ctx, int n, const fdgpu_station *st, const float *s
                           bufs.trig.as<double>() + (size_t)maxt * k, bufs.stats.as<fd_station_stats>() + k);
         hs[k].wait_cycles = ctx->wait_cycles;
         hs[k].walk_cycles = ctx->walk_cycles;
-        max_pad = std::max(max_pad, hs[k].max_face_pad);
+        shape->add(s, true);
     }
     /* Launch order: largest grids first.  CTA i solves record i, and CTAs beyond the resident ones
      * start as earlier ones finish, so a batch of uneven windows ends sooner when the long solves
@@ -398,7 +397,6 @@ int prepare_batch(fdgpu_ctx *ctx, int n, const fdgpu_station *st, const float *s
     FD_CU(ctx, cudaMemcpyAsync(bufs.stations.p, hs.data(), sizeof(fd_station_dev) * n, cudaMemcpyHostToDevice, cs));
     /* the host vectors go away on return: the copies must have left them */
     FD_CU(ctx, cudaStreamSynchronize(cs));
-    *max_pad_out = max_pad;
     return FDGPU_OK;
 }
 
@@ -456,9 +454,8 @@ struct fdgpu_batch {
     fdgpu_ctx *ctx = nullptr;
     int n = 0;
     std::vector<fdgpu_station> stations;   /* the caller's stations, in its order */
-    long long max_pad = 16;
-    long long smem_bytes = 0;   /* launch shape, fixed at creation */
-    int csz = 1;
+    fdh::SolveShape shape;      /* launch shape, fixed at creation */
+    long long smem_bytes = 0;
     long long recorded = -1;    /* the run whose times the order table holds (see record_run) */
     BatchBufs bufs;
 };
@@ -473,10 +470,11 @@ extern "C" int fdgpu_solve_device(fdgpu_ctx *ctx, int n, const fdgpu_station *st
     FD_CU(ctx, dev_.err);
     cudaStream_t cs = stream ? (cudaStream_t)stream : ctx->stream;
     BatchBufs &bufs = ctx->batch;
-    long long max_pad = 16;
-    int rc = prepare_batch(ctx, n, st, slowness, s_sy, s_sz, d_times, times_initialised, bufs, cs, &max_pad);
+    fdh::SolveShape shape;
+    int rc = prepare_batch(ctx, n, st, slowness, s_sy, s_sz, d_times, times_initialised, bufs, cs, &shape);
     if (rc == FDGPU_OK) {
-        const cudaError_t e = fdk_launch_solve(bufs.stations.as<fd_station_dev>(), n, max_pad, ctx->cluster, cs);
+        const cudaError_t e = fdk_launch_solve(bufs.stations.as<fd_station_dev>(), n, shape.max_face_pad, shape.lmax,
+                                               shape.imax, cs);
         rc = e ? cuda_fail(ctx, e, "fdk_launch_solve") : read_stats(ctx, bufs.stats, n, stats, cs, st, nullptr);
     }
     return rc;
@@ -497,9 +495,9 @@ extern "C" int fdgpu_batch_create(fdgpu_ctx *ctx, int n, const fdgpu_station *st
     b->n = n;
     b->stations.assign(st, st + n);
     int rc = prepare_batch(ctx, n, st, slowness, s_sy, s_sz, d_times, times_initialised, b->bufs, ctx->stream,
-                           &b->max_pad);
+                           &b->shape);
     if (!rc) {
-        const cudaError_t e = fdk_solve_config(n, b->max_pad, ctx->cluster, &b->smem_bytes, &b->csz);
+        const cudaError_t e = fdk_solve_config(b->shape.max_face_pad, b->shape.lmax, b->shape.imax, &b->smem_bytes);
         if (e) rc = cuda_fail(ctx, e, "fdk_solve_config");
     }
     if (rc) {
@@ -517,7 +515,8 @@ extern "C" int fdgpu_batch_run(fdgpu_batch *b, void *stream)
     cudaStream_t cs = stream ? (cudaStream_t)stream : ctx->stream;
     FdDeviceScope dev_(ctx->device);   /* switches nothing when the device is already current */
     FD_CU(ctx, dev_.err);
-    FD_CU(ctx, fdk_solve_launch(b->bufs.stations.as<fd_station_dev>(), b->n, b->smem_bytes, b->csz, cs));
+    FD_CU(ctx, fdk_solve_launch(b->bufs.stations.as<fd_station_dev>(), b->n, b->smem_bytes, b->shape.lmax, b->shape.imax,
+                                cs));
     return FDGPU_OK;
 }
 

@@ -24,7 +24,6 @@
  * counters (see "warp workers" below); every wait among them is bounded and ends in an error
  * status, never in a hang.
  */
-#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -35,12 +34,6 @@
 #include "fdgpu_layout.h"
 
 #define FD_WARPS 12                 /* independent workers per station */
-/* Largest cluster of CTAs one station may use.  Multi-CTA solving (the walk state shared through
- * distributed shared memory) passed the bit-exactness tests but hung or faulted intermittently on
- * this GPU; until the cause is found every station runs on one CTA. */
-#ifndef FD_MAX_CLUSTER
-#define FD_MAX_CLUSTER 1
-#endif
 #define FD_BLOCK (FD_WARPS * 32)
 
 /* optional per-phase cycle counters (thread 0, between barriers) for profiling builds */
@@ -53,6 +46,9 @@
 #define FD_TOC(k, v) do { } while (0)
 #endif
 #define FD_HEADTEST 1.e-3
+
+/* rarely called: kept out of the worker loop's code, whose registers and instruction fetches they would cost */
+#define FD_COLD __device__ __noinline__
 
 namespace fdk {
 
@@ -128,8 +124,7 @@ __global__ void fd_geo_build(int nx, int ny, int nz, double h, double dq, double
 /* ---------------------------------------------------------------------------------------------- */
 /* per-CTA state                                                                                   */
 
-/* state of the current walk that all CTAs of a station's cluster share; it lives in the shared
- * memory of the cluster's first CTA and the others reach it through distributed shared memory */
+/* state of the current walk */
 struct WalkShared {
     /* ready queues (one per face in a sweep graph; a face walk uses queue 0), the queue of points
      * resuming a search for an inherited stencil state, idle workers, finished nodes, parked points
@@ -142,14 +137,11 @@ struct WalkShared {
     unsigned long long exitkey;
     long long rounds, deferred;
     unsigned long long st[5];
-    int bar_count;            /* cluster barrier: arrivals so far */
 };
 
 struct Shared {
-    WalkShared wl;
-    WalkShared *w;           /* the cluster's shared walk state (wl of rank 0) */
-    int cs, rank;            /* CTAs per station, this CTA's rank */
-    int stat;                /* the station's status as this CTA read it at its last barrier */
+    WalkShared w;
+    int stat;                /* the station's status at the last csync */
     int wall[6], dflag[6];
     int radius, rad0, reverse, headpref;
     float carry_t0, carry_t4;
@@ -164,7 +156,7 @@ struct Shared {
     long long gM;
     unsigned ctxm[6], innm[6];
     unsigned rel[6][27];     /* see relation_word */
-    void *gsm;
+    int lstride, imax;       /* layout of the sweep-graph tables (see GraphSmem) */
     unsigned long long red[FD_BLOCK / 32];
     unsigned long long bcast;
     /* statistics */
@@ -175,46 +167,14 @@ struct Shared {
     long long gsweeps;
 };
 
-/* ordering of a worker's global and shared stores before the counters that publish them, at the
- * scope of the CTAs that share the walk */
-__device__ __forceinline__ void wfence(const Shared &sh)
-{
-    if (sh.cs > 1)
-        asm volatile("fence.acq_rel.cluster;" ::: "memory");
-    else
-        asm volatile("fence.acq_rel.cta;" ::: "memory");
-}
+/* ordering of a worker's global and shared stores before the counters that publish them */
+__device__ __forceinline__ void wfence(const Shared &) { asm volatile("fence.acq_rel.cta;" ::: "memory"); }
 
-#ifndef FD_BAR_SPINS
-#define FD_BAR_SPINS (1ll << 26)   /* polls (about 64 ns apart) before a cluster barrier gives up */
-#endif
-
-/* Barrier of all threads of the station's CTAs: the CTA's threads meet, its thread 0 meets the other
- * CTAs' at an arrival counter in the first CTA's shared memory that only grows (barrier k is passed
- * once it reaches (k+1) * CTAs, so no arrival can be lost to a reset).  The wait is bounded: a CTA
- * that waits too long records which barrier (site) gave up in the station's status and goes on, so
- * a fault in the schedule ends in an error, never in a hang.  Thread 0 then takes the station's
- * status for the whole CTA (sh.stat), so every branch that depends on it is taken by all threads. */
-__device__ __forceinline__ void csync(Shared &sh, int site)
+/* barrier after which every branch that depends on the station's status (sh.stat) is taken by all threads */
+__device__ __forceinline__ void csync(Shared &sh)
 {
     __syncthreads();
-    if (threadIdx.x == 0) {
-        if (sh.cs > 1) {
-            asm volatile("fence.acq_rel.cluster;" ::: "memory");
-            const int my = atomicAdd(&sh.w->bar_count, 1);
-            const int target = (my / sh.cs + 1) * sh.cs;
-            long long spins = 0;
-            while (*const_cast<volatile int *>(&sh.w->bar_count) < target) {
-                __nanosleep(64);
-                if (++spins > FD_BAR_SPINS) {
-                    atomicCAS(&sh.w->status, 0, 100 + site);
-                    break;
-                }
-            }
-            asm volatile("fence.acq_rel.cluster;" ::: "memory");
-        }
-        sh.stat = *const_cast<volatile int *>(&sh.w->status);
-    }
+    if (threadIdx.x == 0) sh.stat = *const_cast<volatile int *>(&sh.w.status);
     __syncthreads();
 }
 
@@ -333,6 +293,9 @@ struct CtaSmem {
 };
 constexpr int kCtaSmemBytes = (int)((sizeof(CtaSmem) + 15) & ~(size_t)15);
 
+/* the longest list: the 2-D and 1-D trials of 32 nodes */
+constexpr int kItems = (TK_NF - TK_2D0 + FDN_NTRIAL - TK_1D0) * 32;
+
 /* one warp's chunk of up to 32 nodes; slot = lane of the node */
 struct WarpSmem {
     double res[32][FDN_NTRIAL];            /* trial values (2-D: after the causality selection) */
@@ -340,7 +303,7 @@ struct WarpSmem {
     float s[32][NB_PAD];                   /* 18-node slowness context */
     float s0[32], s4[32];                  /* stencil state entering the 2-D block */
     int z[32], y[32];                      /* grid z and y of the node */
-    unsigned short items[FDN_NTRIAL * 32]; /* (slot << 5 | trial) to evaluate, trial-major */
+    unsigned short items[kItems];          /* (slot << 5 | trial) to evaluate, trial-major */
     unsigned long long cnt[6];             /* stencil evaluations by kind (5 used) */
 };
 static_assert(sizeof(WarpSmem) % 16 == 0, "keeps the dependency bytes after the warp areas aligned");
@@ -841,7 +804,7 @@ __device__ __forceinline__ void enqueue_to(int *queue, int &tail, int cap, Share
     if (pos < cap)
         *const_cast<volatile int *>(&queue[pos]) = e;   /* a strong store: readers synchronise on it */
     else
-        atomicCAS(&sh.w->status, 0, 10);
+        atomicCAS(&sh.w.status, 0, 10);
 }
 
 /* ---------------------------------------------------------------------------------------------- */
@@ -853,14 +816,14 @@ __device__ void face_release(const fd_station_dev &sd, Shared &sh, unsigned char
 {
     if (writer) {
         sd.scr.rec[i] = make_float2(st0, st4);
-        atomicMax(&sh.w->exitkey, sd.scr.key[i]);
+        atomicMax(&sh.w.exitkey, sd.scr.key[i]);
     } else {
         sd.scr.rec[i] = make_float2(__int_as_float(0x7fc00000), __int_as_float(0x7fc00000));
     }
     wfence(sh);
     /* done; a point waiting for the stencil state left before it resumes its search */
     const int waiter = atomicExch(&sd.scr.pst[i], -2);
-    if (waiter >= 0) enqueue_to(sd.scr.rq, sh.w->rqtail, sh.w->rqcap, sh, waiter);
+    if (waiter >= 0) enqueue_to(sd.scr.rq, sh.w.rqtail, sh.w.rqcap, sh, waiter);
     const int nvf = sh.n / sh.nuf, iu = i % sh.nuf, iv = i / sh.nuf;
     const unsigned char *emask = dag + sh.n_pad;
     unsigned later = inrect_mask(iu, iv, sh.nuf, nvf) & ~(unsigned)emask[i];
@@ -873,7 +836,7 @@ __device__ void face_release(const fd_station_dev &sd, Shared &sh, unsigned char
         const int j = (iv + dv) * sh.nuf + iu + du;
         const unsigned sh8 = (j & 3) * 8;
         const unsigned old = atomicSub(reinterpret_cast<unsigned *>(dag) + (j >> 2), 1u << sh8);
-        if (((old >> sh8) & 0xFFu) == 1u) enqueue_to(sd.scr.queue, sh.w->qtail[0], sh.w->qcap[0], sh, j);
+        if (((old >> sh8) & 0xFFu) == 1u) enqueue_to(sd.scr.queue, sh.w.qtail[0], sh.w.qcap[0], sh, j);
     }
 }
 
@@ -912,11 +875,9 @@ __device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long x)
 /* are registered on a point (a wait pair and the counter's wait bit) or on an instance event (all */
 /* keys final, all points done; a parked-point entry).                                            */
 
-#define FD_LMAX 1024                 /* largest grid extent a sweep graph handles */
 #ifndef FD_GRAPH_FORWARD
 #define FD_GRAPH_FORWARD 1           /* the first sweep as a graph too */
 #endif
-#define FD_IMAX 3088                 /* face instances: at most nx + ny + nz + 8 */
 #define FD_WRITERB 0x10000000u       /* done, and it made a writer call */
 #define FD_WAITB 0x20000000u
 #define FD_DONEB 0x40000000u
@@ -935,16 +896,30 @@ struct GRect {
 #define FD_IN_BOX ((short)-1)
 #define FD_NEVER ((short)0x7fff)
 struct GraphSmem {
-    short lay[3][FD_LMAX + 2];   /* entry c + 1 for coordinate c, FD_NEVER on both sides of the grid */
-    GRect rect[FD_IMAX];
+    short *lay[3];   /* entry c + 1 for coordinate c, FD_NEVER on both sides of the grid */
+    GRect *rect;
 };
 static_assert((FD_IMAX << 3) + 7 < 0x7fff, "owner words in a short");
 
-/* the warp areas and the sweep-graph tables fit one CTA's 227 KB, with 2 KB left for the static
- * shared memory of fd_solve */
-static_assert(kSmemBase + sizeof(GraphSmem) + 2048 <= 227 * 1024, "shared memory of one CTA");
+/* bytes of the tables for extents up to lmax and imax instances.  A launch asks for what its largest
+ * station needs and no more: what shared memory leaves of the SM's 256 KB is L1, which the solver reads
+ * its tables, times and keys through (28 KB beside the largest tables, 60 to 92 KB beside those of a
+ * window; a 141x121x57 station 219 -> 177 ms). */
+__host__ __device__ constexpr long long graph_smem_bytes(int lmax, int imax)
+{
+    return ((3ll * (lmax + 2) * 2 + 15) & ~15ll) + (long long)imax * (long long)sizeof(GRect);
+}
 
-__device__ __forceinline__ GraphSmem &gsmem(const Shared &sh) { return *reinterpret_cast<GraphSmem *>(sh.gsm); }
+/* the tables of the largest grids, the warp areas and 2.5 KB of static shared memory fit a CTA's 227 KB */
+static_assert(kSmemBase + graph_smem_bytes(FD_LMAX, FD_IMAX) + 2560 <= 227 * 1024, "shared memory of one CTA");
+
+__device__ __forceinline__ GraphSmem gsmem(const Shared &sh)
+{
+    extern __shared__ __align__(16) unsigned char fd_dyn_smem[];
+    short *l = reinterpret_cast<short *>(fd_dyn_smem + kSmemBase);
+    const int n = sh.lstride;
+    return {{l, l + n, l + 2 * n}, reinterpret_cast<GRect *>(fd_dyn_smem + kSmemBase + ((3 * n * 2 + 15) & ~15))};
+}
 
 /* Neighbour offsets (dx,dy,dz) are numbered k = (dz+1)*9 + (dy+1)*3 + (dx+1), 13 being the node
  * itself; the opposite offset is 26 - k.  An owner word holds (instance << 3) | face, -1 for a
@@ -1033,13 +1008,13 @@ __device__ __forceinline__ int inst_fill(const GRect &r, int x, int y, int z)
 /* Points parked on instance I's event `kind` (1: all keys final, 2: all done) go to the resume queue.  The
  * event's word heads a list of them through gpark, and says so once the event has fired; the one
  * thread whose count completes the event takes the list. */
-__device__ void fire_event(const fd_station_dev &sd, Shared &sh, int I, int kind)
+FD_COLD void fire_event(const fd_station_dev &sd, Shared &sh, int I, int kind)
 {
     wfence(sh);
     int k = atomicExch(&sd.scr.ginst[I].ev[kind - 1], FD_EV_FIRED);
     wfence(sh);
     while (k >= 0) {
-        enqueue_to(sd.scr.grq, sh.w->rqtail, sh.w->rqcap, sh, vload(sd.scr.gpark[k].x));
+        enqueue_to(sd.scr.grq, sh.w.rqtail, sh.w.rqcap, sh, vload(sd.scr.gpark[k].x));
         k = vload(sd.scr.gpark[k].y);
     }
 }
@@ -1085,7 +1060,7 @@ __device__ __forceinline__ bool ready_word(unsigned w) { return (w & ~FD_WAITB) 
 
 __device__ __forceinline__ void graph_ready(const fd_station_dev &sd, Shared &sh, int face, long long q)
 {
-    enqueue_to(sd.scr.gqueue + sh.w->qbase[face], sh.w->qtail[face], sh.w->qcap[face], sh, (int)q);
+    enqueue_to(sd.scr.gqueue + sh.w.qbase[face], sh.w.qtail[face], sh.w.qcap[face], sh, (int)q);
 }
 
 /* Points that wait for a point: (awaited, waiting) pairs in a hash table probed one slot on at a time.  The
@@ -1096,7 +1071,7 @@ __device__ __forceinline__ void graph_ready(const fd_station_dev &sd, Shared &sh
 __device__ __forceinline__ unsigned wait_slot(int p) { return ((unsigned)p * 2654435761u) >> 16; }
 static_assert(FD_GWAIT_CAP == 1 << 16, "wait_slot");
 
-__device__ void wake_waiters(const fd_station_dev &sd, Shared &sh, int p)
+FD_COLD void wake_waiters(const fd_station_dev &sd, Shared &sh, int p)
 {
     wfence(sh);
     unsigned k = wait_slot(p);
@@ -1104,7 +1079,7 @@ __device__ void wake_waiters(const fd_station_dev &sd, Shared &sh, int p)
         const int x = vload(sd.scr.gwait[k].x);
         if (x == -1) break;
         if (x == p && atomicCAS(&sd.scr.gwait[k].x, p, -3) == p)
-            enqueue_to(sd.scr.grq, sh.w->rqtail, sh.w->rqcap, sh, vload(sd.scr.gwait[k].y));
+            enqueue_to(sd.scr.grq, sh.w.rqtail, sh.w.rqcap, sh, vload(sd.scr.gwait[k].y));
     }
 }
 
@@ -1188,7 +1163,7 @@ __device__ __forceinline__ void release_one(const fd_station_dev &sd, Shared &sh
 __device__ void graph_release(const fd_station_dev &sd, Shared &sh, WarpSmem &ws, int F, bool fin, const Where &wh)
 {
     const int lane = threadIdx.x & 31;
-    const GraphSmem &gs = gsmem(sh);
+    const GraphSmem gs = gsmem(sh);
     const unsigned mask = __ballot_sync(0xffffffffu, fin);
     const int m = __popc(mask);
     if (!m) return;
@@ -1281,18 +1256,18 @@ __device__ void graph_release(const fd_station_dev &sd, Shared &sh, WarpSmem &ws
 }
 
 /* point w waits for an event of instance I (kind 1: all keys final, 2: all points done) (lane 0) */
-__device__ void wait_event(const fd_station_dev &sd, Shared &sh, int w, int I, int kind)
+FD_COLD void wait_event(const fd_station_dev &sd, Shared &sh, int w, int I, int kind)
 {
-    const int k = atomicAdd(&sh.w->npark, 1);
+    const int k = atomicAdd(&sh.w.npark, 1);
     if (k >= FD_GPARK_CAP) {
-        atomicCAS(&sh.w->status, 0, 15);
+        atomicCAS(&sh.w.status, 0, 15);
         return;
     }
     int *head = &sd.scr.ginst[I].ev[kind - 1];
     sd.scr.gpark[k].x = w;
     for (int h = vload(*head);;) {
         if (h == FD_EV_FIRED) {   /* it has happened already */
-            enqueue_to(sd.scr.grq, sh.w->rqtail, sh.w->rqcap, sh, w);
+            enqueue_to(sd.scr.grq, sh.w.rqtail, sh.w.rqcap, sh, w);
             return;
         }
         sd.scr.gpark[k].y = h;
@@ -1304,10 +1279,10 @@ __device__ void wait_event(const fd_station_dev &sd, Shared &sh, int w, int I, i
 }
 
 /* point w waits for point p to be done (lane 0).  Returns false if p is already done (no wait). */
-__device__ bool wait_point(const fd_station_dev &sd, Shared &sh, int w, long long p)
+FD_COLD bool wait_point(const fd_station_dev &sd, Shared &sh, int w, long long p)
 {
-    if (atomicAdd(&sh.w->nwait, 1) >= FD_GWAIT_CAP) {
-        atomicCAS(&sh.w->status, 0, 15);
+    if (atomicAdd(&sh.w.nwait, 1) >= FD_GWAIT_CAP) {
+        atomicCAS(&sh.w.status, 0, 15);
         return true;
     }
     unsigned k = wait_slot((int)p);
@@ -1391,7 +1366,7 @@ __device__ bool commit_node(const fd_station_dev &sd, Shared &sh, const TrialDes
         sd.T[wh.p] = __double2float_rn(guess);
         if (lastK >= 0) {
             /* only the last head trial that lowered the minimum sets the measure that is tested */
-            if (head_wave(last_gb - last_v, head_den(dsc[lastK], s18, sd.g, z, y))) atomicAdd(&sh.w->headw[frame_of(F).headw], 1);
+            if (head_wave(last_gb - last_v, head_den(dsc[lastK], s18, sd.g, z, y))) atomicAdd(&sh.w.headw[frame_of(F).headw], 1);
         }
     }
     const float st0 = writer < 0 ? it0 : t18[dsc[writer].slot[0]], st4 = writer < 0 ? it4 : t18[dsc[writer].slot[4]];
@@ -1463,7 +1438,7 @@ __device__ void warp_chunk(const fd_station_dev &sd, Shared &sh, const CtaSmem &
         bool ok;
         wh = locate(sd, sh, F, e, ok);
         if (!ok) {
-            atomicCAS(&sh.w->status, 0, 14);   /* a queued node no face instance owns */
+            atomicCAS(&sh.w.status, 0, 14);   /* a queued node no face instance owns */
             e = -1;
         }
     }
@@ -1487,11 +1462,9 @@ __device__ void warp_chunk(const fd_station_dev &sd, Shared &sh, const CtaSmem &
             const unsigned bits = 1u << (du + 1) | 8u << (dv + 1);
             t[nb] = 0.f;
             if ((inside & bits) == bits) {
-                /* with several CTAs, through L2: another SM may have written it since this SM last
-                 * read it; one CTA's own stores keep its L1 current */
                 const long long o = du * su + dv * sv + (w ? inner_t : 0ll);
                 if (FD_OK(wh.p + o, (long long)sd.g.nx * sd.g.ny * sd.g.nz, 27)) {
-                    t[nb] = sh.cs > 1 ? __ldcg(pT + o) : pT[o];
+                    t[nb] = pT[o];   /* the CTA's own stores keep its L1 current */
                     copy_async4(&sr[nb], pS + (du * ssu + dv * ssv + (w ? inner_s : 0ll)));
                 }
             } else {
@@ -1537,11 +1510,11 @@ __device__ void warp_chunk(const fd_station_dev &sd, Shared &sh, const CtaSmem &
     if (valid) {
         fin = commit_node(sd, sh, dsc, ws, lane, F, wh, gm, em, p0, p4, permissive, dag, cn);
         if (!fin) {
-            atomicAdd(reinterpret_cast<unsigned long long *>(&sh.w->deferred), 1ull);
+            atomicAdd(reinterpret_cast<unsigned long long *>(&sh.w.deferred), 1ull);
             if (sh.nodefer)
-                atomicCAS(&sh.w->status, 0, 6);   /* excluded by the sweep's precondition */
+                atomicCAS(&sh.w.status, 0, 6);   /* excluded by the sweep's precondition */
             else
-                enqueue_to(sh.graph ? sd.scr.grq : sd.scr.rq, sh.w->rqtail, sh.w->rqcap, sh, e);
+                enqueue_to(sh.graph ? sd.scr.grq : sd.scr.rq, sh.w.rqtail, sh.w.rqcap, sh, e);
         }
     }
     if (sh.graph) graph_release(sd, sh, ws, F, fin, wh);
@@ -1559,7 +1532,7 @@ __device__ void warp_chunk(const fd_station_dev &sd, Shared &sh, const CtaSmem &
     const unsigned done = __ballot_sync(0xffffffffu, fin);
     if (lane == 0 && done) {
         wfence(sh);
-        atomicAdd(&sh.w->ndone, __popc(done));
+        atomicAdd(&sh.w.ndone, __popc(done));
     }
     __syncwarp();
     FD_TOC(3, tc);
@@ -1595,9 +1568,8 @@ __device__ int predecessor(const fd_station_dev &sd, int n, int c, int lane)
  * non-writer passes the search to its predecessor; a point not yet done takes w as its waiter and
  * queues it again when it finishes (a point has at most one waiter: waiters lie between it and the
  * next pending point).  Before the face's first point the state is the one the face started with.
- * Keys fall along the walk, so waits cannot form a cycle.  One warp; evaluates w when found. */
-__device__ void resume_waiter(const fd_station_dev &sd, Shared &sh, const CtaSmem &cs, WarpSmem &ws, int w,
-                              unsigned char *dag, Counters cn)
+ * Keys fall along the walk, so waits cannot form a cycle.  One warp; true with the state when found. */
+FD_COLD bool resume_waiter(const fd_station_dev &sd, Shared &sh, int w, float *st0, float *st4)
 {
     const int lane = threadIdx.x & 31;
     int c = w;
@@ -1613,7 +1585,7 @@ __device__ void resume_waiter(const fd_station_dev &sd, Shared &sh, const CtaSme
                     const int old = atomicCAS(&sd.scr.pst[p], -1, w);
                     if (old == -1) verdict = 2;
                     else if (old == -2) verdict = 3;
-                    else { atomicCAS(&sh.w->status, 0, 11); verdict = 2; }   /* a second waiter */
+                    else { atomicCAS(&sh.w.status, 0, 11); verdict = 2; }   /* a second waiter */
                 }
                 if (verdict == 0 || verdict == 3) {
                     wfence(sh);
@@ -1624,41 +1596,40 @@ __device__ void resume_waiter(const fd_station_dev &sd, Shared &sh, const CtaSme
             }
         }
         verdict = __shfl_sync(0xffffffffu, verdict, 0);
-        if (verdict == 2) return;
+        if (verdict == 2) return false;
         if (verdict == 1) {
-            t0 = __shfl_sync(0xffffffffu, t0, 0);
-            t4 = __shfl_sync(0xffffffffu, t4, 0);
-            warp_chunk(sd, sh, cs, ws, sh.face, lane == 0 ? w : -1, true, t0, t4, dag, cn);
-            return;
+            *st0 = __shfl_sync(0xffffffffu, t0, 0);
+            *st4 = __shfl_sync(0xffffffffu, t4, 0);
+            return true;
         }
         c = p;
     }
-    if (lane == 0) atomicCAS(&sh.w->status, 0, 12);
+    if (lane == 0) atomicCAS(&sh.w.status, 0, 12);
+    return false;
 }
 
 /* Sweep graph: the same search for point w (a grid index), by the reference's order of face
  * instances and, within one, of keys.  Registers w on an instance event or a point when the
- * answer is not yet known.  One warp; evaluates w when found. */
-__device__ void resume_graph(const fd_station_dev &sd, Shared &sh, const CtaSmem &cs, WarpSmem &ws, int w,
-                             Counters cn)
+ * answer is not yet known.  One warp; true with the state and w's face when found. */
+FD_COLD bool resume_graph(const fd_station_dev &sd, Shared &sh, int w, float *st0, float *st4, int *face)
 {
     const int lane = threadIdx.x & 31;
-    const GraphSmem &gs = gsmem(sh);
+    const GraphSmem gs = gsmem(sh);
     const int nx = sd.g.nx, ny = sd.g.ny;
-    if (!FD_OK(w, (long long)sd.g.nx * sd.g.ny * sd.g.nz, 20)) return;
+    if (!FD_OK(w, (long long)sd.g.nx * sd.g.ny * sd.g.nz, 20)) return false;
     const int wxy = w / nx;
     const int wx = w - wxy * nx, wy = wxy % ny, wz = wxy / ny;
     const int ow = owner_of(gs, wx, wy, wz);
     if (ow < 0) {
-        if (lane == 0) atomicCAS(&sh.w->status, 0, 14);
-        return;
+        if (lane == 0) atomicCAS(&sh.w.status, 0, 14);
+        return false;
     }
     const int I = own_inst(ow);
     const GRect &r = gs.rect[I];
     const int n = rect_n(r);
     if (vload(sd.scr.ginst[I].nkeyed) < n) {   /* keys below w's not all known yet */
         if (lane == 0) wait_event(sd, sh, w, I, 1);
-        return;
+        return false;
     }
     const unsigned long long kc = inst_key(sd, r, inst_fill(r, wx, wy, wz));
     const fdn_frame fr = frame_of(r.face);
@@ -1728,15 +1699,16 @@ __device__ void resume_graph(const fd_station_dev &sd, Shared &sh, const CtaSmem
             }
         }
         verdict = __shfl_sync(0xffffffffu, verdict, 0);
-        if (verdict == 2) return;
+        if (verdict == 2) return false;
         if (verdict == 1) {
-            t0 = __shfl_sync(0xffffffffu, t0, 0);
-            t4 = __shfl_sync(0xffffffffu, t4, 0);
-            warp_chunk(sd, sh, cs, ws, r.face, lane == 0 ? w : -1, true, t0, t4, nullptr, cn);
-            return;
+            *st0 = __shfl_sync(0xffffffffu, t0, 0);
+            *st4 = __shfl_sync(0xffffffffu, t4, 0);
+            *face = r.face;
+            return true;
         }
     }
-    if (lane == 0) atomicCAS(&sh.w->status, 0, 12);
+    if (lane == 0) atomicCAS(&sh.w.status, 0, 12);
+    return false;
 }
 
 /* ---------------------------------------------------------------------------------------------- */
@@ -1745,18 +1717,18 @@ __device__ void resume_graph(const fd_station_dev &sd, Shared &sh, const CtaSmem
 /* nothing queued, every worker idle, and all queues unchanged across the idle count (lane 0) */
 __device__ __forceinline__ bool quiescent(Shared &sh)
 {
-    int t0[6], r0 = vload(sh.w->rqtail);
-    for (int k = 0; k < sh.w->nq; k++) {
-        t0[k] = vload(sh.w->qtail[k]);
-        if (vload(sh.w->qhead[k]) != t0[k]) return false;
+    int t0[6], r0 = vload(sh.w.rqtail);
+    for (int k = 0; k < sh.w.nq; k++) {
+        t0[k] = vload(sh.w.qtail[k]);
+        if (vload(sh.w.qhead[k]) != t0[k]) return false;
     }
-    if (vload(sh.w->rqhead) != r0) return false;
+    if (vload(sh.w.rqhead) != r0) return false;
     wfence(sh);
-    if (vload(sh.w->idle) != sh.cs * FD_WARPS) return false;
+    if (vload(sh.w.idle) != FD_WARPS) return false;
     wfence(sh);
-    for (int k = 0; k < sh.w->nq; k++)
-        if (vload(sh.w->qtail[k]) != t0[k] || vload(sh.w->qhead[k]) != t0[k]) return false;
-    return vload(sh.w->rqtail) == r0 && vload(sh.w->rqhead) == r0;
+    for (int k = 0; k < sh.w.nq; k++)
+        if (vload(sh.w.qtail[k]) != t0[k] || vload(sh.w.qhead[k]) != t0[k]) return false;
+    return vload(sh.w.rqtail) == r0 && vload(sh.w.rqhead) == r0;
 }
 
 /* read a claimed queue entry: spins briefly for an entry whose writer is between its two
@@ -1769,7 +1741,7 @@ __device__ __forceinline__ int read_entry(const int *queue, int pos, Shared &sh)
         __nanosleep(32);
         e = *q;
     }
-    if (e < 0) atomicCAS(&sh.w->status, 0, 9);   /* a claimed entry never written */
+    if (e < 0) atomicCAS(&sh.w.status, 0, 9);   /* a claimed entry never written */
     return e;
 }
 
@@ -1791,36 +1763,36 @@ __device__ void run_walk(const fd_station_dev &sd, Shared &sh, const CtaSmem &cs
     for (;;) {
         int act = 0, h = 0, m = 0, qf = 0;   /* act: 0 wait, 1 chunk, 2 resume a waiter, 3 leave */
         if (lane == 0) {
-            if (vload(sh.w->status) != 0 || vload(sh.w->ndone) >= total) {
+            if (vload(sh.w.status) != 0 || vload(sh.w.ndone) >= total) {
                 act = 3;
             } else {
-                const int rh = vload(sh.w->rqhead), rt0 = vload(sh.w->rqtail), rt = rt0 < sh.w->rqcap ? rt0 : sh.w->rqcap;
+                const int rh = vload(sh.w.rqhead), rt0 = vload(sh.w.rqtail), rt = rt0 < sh.w.rqcap ? rt0 : sh.w.rqcap;
                 if (rh < rt) {
-                    if (idle) { atomicSub(&sh.w->idle, 1); idle = false; }
-                    if (atomicCAS(&sh.w->rqhead, rh, rh + 1) == rh) { act = 2; h = read_entry(rq, rh, sh); }
+                    if (idle) { atomicSub(&sh.w.idle, 1); idle = false; }
+                    if (atomicCAS(&sh.w.rqhead, rh, rh + 1) == rh) { act = 2; h = read_entry(rq, rh, sh); }
                 } else {
                     /* the fullest queue, starting the scan at a warp-dependent face */
                     int best = -1, bavail = 0, bhead = 0;
-                    for (int k0 = 0; k0 < sh.w->nq; k0++) {
-                        const int k = (k0 + warp) % sh.w->nq;
-                        const int hd = vload(sh.w->qhead[k]), qt = vload(sh.w->qtail[k]);
-                        const int tl = qt < sh.w->qcap[k] ? qt : sh.w->qcap[k];
+                    for (int k0 = 0; k0 < sh.w.nq; k0++) {
+                        const int k = (k0 + warp) % sh.w.nq;
+                        const int hd = vload(sh.w.qhead[k]), qt = vload(sh.w.qtail[k]);
+                        const int tl = qt < sh.w.qcap[k] ? qt : sh.w.qcap[k];
                         if (tl - hd > bavail) { bavail = tl - hd; best = k; bhead = hd; }
                     }
                     if (best >= 0) {
-                        if (idle) { atomicSub(&sh.w->idle, 1); idle = false; }
+                        if (idle) { atomicSub(&sh.w.idle, 1); idle = false; }
                         const int want = bavail < 32 ? bavail : 32;
-                        if (atomicCAS(&sh.w->qhead[best], bhead, bhead + want) == bhead) {
-                            act = 1; h = sh.w->qbase[best] + bhead; m = want; qf = best;
+                        if (atomicCAS(&sh.w.qhead[best], bhead, bhead + want) == bhead) {
+                            act = 1; h = sh.w.qbase[best] + bhead; m = want; qf = best;
                         }
                     } else {
-                        if (!idle) { wfence(sh); atomicAdd(&sh.w->idle, 1); idle = true; idle_polls = 0; }
+                        if (!idle) { wfence(sh); atomicAdd(&sh.w.idle, 1); idle = true; idle_polls = 0; }
                         /* all idle with nothing queued and nodes left: nothing can release them.  The
                          * check (two fences and a scan of every queue) runs on every 64th idle poll
                          * only: idle warps are most of the CTA in a forward sweep, and their polls
                          * share the SM's shared-memory pipe with the working warps */
-                        if ((++idle_polls & 63u) == 0u && quiescent(sh) && vload(sh.w->ndone) < total) {
-                            atomicCAS(&sh.w->status, 0, 3);
+                        if ((++idle_polls & 63u) == 0u && quiescent(sh) && vload(sh.w.ndone) < total) {
+                            atomicCAS(&sh.w.status, 0, 3);
                             act = 3;
                         }
                     }
@@ -1828,11 +1800,11 @@ __device__ void run_walk(const fd_station_dev &sd, Shared &sh, const CtaSmem &cs
                 if (act == 1 || act == 2) {
                     since = clock64();
                 } else if (act == 0 && clock64() - since > wait_lim) {
-                    atomicCAS(&sh.w->status, 0, 8);   /* no work for this worker for too long */
+                    atomicCAS(&sh.w.status, 0, 8);   /* no work for this worker for too long */
                     act = 3;
                 }
                 if (act != 3 && clock64() - started > walk_lim) {
-                    atomicCAS(&sh.w->status, 0, 17);   /* the walk as a whole ran far too long */
+                    atomicCAS(&sh.w.status, 0, 17);   /* the walk as a whole ran far too long */
                     act = 3;
                 }
             }
@@ -1840,10 +1812,12 @@ __device__ void run_walk(const fd_station_dev &sd, Shared &sh, const CtaSmem &cs
         act = __shfl_sync(0xffffffffu, act, 0);
         if (act == 3) break;
         h = __shfl_sync(0xffffffffu, h, 0);
+        int e = -1, face = sh.face;
+        float in0 = 0.f, in4 = 0.f;
         if (act == 1) {
             m = __shfl_sync(0xffffffffu, m, 0);
             qf = __shfl_sync(0xffffffffu, qf, 0);
-            int e = -1;
+            if (sh.graph) face = qf;
             if (lane < m) {
                 const volatile int *q = queue + h + lane;
                 e = *q;
@@ -1851,49 +1825,44 @@ __device__ void run_walk(const fd_station_dev &sd, Shared &sh, const CtaSmem &cs
                     __nanosleep(32);
                     e = *q;
                 }
-                if (e < 0) atomicCAS(&sh.w->status, 0, 9);   /* a claimed entry never written */
+                if (e < 0) atomicCAS(&sh.w.status, 0, 9);   /* a claimed entry never written */
                 /* an entry outside the walk's nodes ends the walk with a status instead of an access */
                 const long long bound = sh.graph ? (long long)sd.g.nx * sd.g.ny * sd.g.nz : (long long)sh.n;
                 if (e >= bound) {
                     (void)FD_OK(e, bound, 23);
-                    atomicCAS(&sh.w->status, 0, 18);
+                    atomicCAS(&sh.w.status, 0, 18);
                     e = -1;
                 }
             }
             wfence(sh);
-            warp_chunk(sd, sh, cs, ws, sh.graph ? qf : sh.face, e, false, 0.f, 0.f, dag, cn);
             chunks++;
-            continue;
-        }
-        if (act == 2) {
+        } else if (act == 2) {
             wfence(sh);
             const long long bound = sh.graph ? (long long)sd.g.nx * sd.g.ny * sd.g.nz : (long long)sh.n;
             if (h >= bound) {
                 (void)FD_OK(h, bound, 24);
-                if (lane == 0) atomicCAS(&sh.w->status, 0, 18);
+                if (lane == 0) atomicCAS(&sh.w.status, 0, 18);
                 h = -1;
             }
-            if (h >= 0) {
-                if (sh.graph)
-                    resume_graph(sd, sh, cs, ws, h, cn);
-                else
-                    resume_waiter(sd, sh, cs, ws, h, dag, cn);
-            }
+            if (h < 0 || !(sh.graph ? resume_graph(sd, sh, h, &in0, &in4, &face) : resume_waiter(sd, sh, h, &in0, &in4))) continue;
+            if (lane == 0) e = h;
+        } else {
+            __nanosleep(64);
             continue;
         }
-        __nanosleep(64);
+        warp_chunk(sd, sh, cs, ws, face, e, act == 2, in0, in4, dag, cn);
     }
-    if (lane == 0 && chunks) atomicAdd(reinterpret_cast<unsigned long long *>(&sh.w->rounds), (unsigned long long)chunks);
+    if (lane == 0 && chunks) atomicAdd(reinterpret_cast<unsigned long long *>(&sh.w.rounds), (unsigned long long)chunks);
 }
 
 /* reset the walk counters (thread 0) */
 __device__ void walk_reset(Shared &sh, int nq, int rqcap)
 {
-    sh.w->nq = nq;
-    for (int k = 0; k < 6; k++) { sh.w->qhead[k] = 0; sh.w->qtail[k] = 0; sh.w->qcap[k] = 0; sh.w->qbase[k] = 0; }
-    sh.w->rqhead = sh.w->rqtail = sh.w->idle = sh.w->ndone = sh.w->npark = 0;
-    sh.w->rqcap = rqcap;
-    sh.w->exitkey = 0ull;
+    sh.w.nq = nq;
+    for (int k = 0; k < 6; k++) { sh.w.qhead[k] = 0; sh.w.qtail[k] = 0; sh.w.qcap[k] = 0; sh.w.qbase[k] = 0; }
+    sh.w.rqhead = sh.w.rqtail = sh.w.idle = sh.w.ndone = sh.w.npark = 0;
+    sh.w.rqcap = rqcap;
+    sh.w.exitkey = 0ull;
 }
 
 /* Walk the current face (parameters in sh) in dependency order. */
@@ -1920,7 +1889,7 @@ __device__ void face_walk(const fd_station_dev &sd, Shared &sh, CtaSmem &cs, War
     }
     if (tid == 0) {
         walk_reset(sh, 1, 2 * n);
-        sh.w->qcap[0] = n;
+        sh.w.qcap[0] = n;
         sh.graph = 0;
     }
     __syncthreads();
@@ -1939,7 +1908,7 @@ __device__ void face_walk(const fd_station_dev &sd, Shared &sh, CtaSmem &cs, War
         }
         emask[i] = (unsigned char)em;
         dag[i] = (unsigned char)__popc(em);
-        if (em == 0) enqueue_to(queue, sh.w->qtail[0], sh.w->qcap[0], sh, i);
+        if (em == 0) enqueue_to(queue, sh.w.qtail[0], sh.w.qcap[0], sh, i);
     }
     __syncthreads();
     FD_TOC(0, t0);
@@ -1948,8 +1917,8 @@ __device__ void face_walk(const fd_station_dev &sd, Shared &sh, CtaSmem &cs, War
     __syncthreads();
     FD_TOC(4, tw);
     if (tid == 0) {
-        if (sh.w->exitkey) {
-            const float2 r = sd.scr.rec[(int)(sh.w->exitkey & 0xffffffffu)];
+        if (sh.w.exitkey) {
+            const float2 r = sd.scr.rec[(int)(sh.w.exitkey & 0xffffffffu)];
             sh.carry_t0 = r.x;
             sh.carry_t4 = r.y;
         }
@@ -1995,14 +1964,11 @@ __device__ void setup_face(const fd_station_dev &sd, Shared &sh, int face)
 __device__ void graph_sweep(const fd_station_dev &sd, Shared &sh, CtaSmem &cs, WarpSmem &ws, Counters cn)
 {
     const int tid = threadIdx.x;
-    /* the station's threads over all its CTAs, for loops over nodes */
-    const int gt = sh.rank * blockDim.x + tid, gstride = sh.cs * blockDim.x;
-    const bool lead = sh.rank == 0;
     const int nx = sd.g.nx, ny = sd.g.ny, nz = sd.g.nz;
-    GraphSmem &gs = gsmem(sh);
+    const GraphSmem gs = gsmem(sh);
     FD_TIC(t0);
     /* walls: 0 z1, 1 z2, 2 x2, 3 x1, 4 y1, 5 y2 */
-    for (int k = tid; k < FD_LMAX + 2; k += blockDim.x) {
+    for (int k = tid; k < sh.lstride; k += blockDim.x) {
         const int c = k - 1;
         gs.lay[0][k] = c >= 0 && c < nx && c > sh.wall[3] && c < sh.wall[2] ? FD_IN_BOX : FD_NEVER;
         gs.lay[1][k] = c >= 0 && c < ny && c > sh.wall[4] && c < sh.wall[5] ? FD_IN_BOX : FD_NEVER;
@@ -2011,7 +1977,7 @@ __device__ void graph_sweep(const fd_station_dev &sd, Shared &sh, CtaSmem &cs, W
     __syncthreads();
     /* the sweep's face instances, as the radius loop visits them */
     if (tid == 0) {
-        const int cap = sd.scr.ginst_cap < FD_IMAX ? sd.scr.ginst_cap : FD_IMAX;
+        const int cap = sd.scr.ginst_cap < sh.imax ? sd.scr.ginst_cap : sh.imax;
         int ninst = 0;
         long long M = 0, per_face[6] = {0, 0, 0, 0, 0, 0};
         unsigned faces = 0;
@@ -2023,13 +1989,11 @@ __device__ void graph_sweep(const fd_station_dev &sd, Shared &sh, CtaSmem &cs, W
                     setup_face(sd, sh, face);
                     if (sh.n > 0) {
                         if (ninst >= cap) { over = true; break; }
-                        if (lead) {
-                            fd_ginst &gi = sd.scr.ginst[ninst];
-                            gi.face = face; gi.layer = sh.layer;
-                            gi.ulo = sh.ulo; gi.uhi = sh.uhi; gi.vlo = sh.vlo; gi.vhi = sh.vhi;
-                            gi.nuf = sh.nuf; gi.n = sh.n;
-                            gi.nkeyed = 0; gi.ndone = 0; gi.ev[0] = gi.ev[1] = FD_EV_NONE; gi.exitkey = 0ull;
-                        }
+                        fd_ginst &gi = sd.scr.ginst[ninst];
+                        gi.face = face; gi.layer = sh.layer;
+                        gi.ulo = sh.ulo; gi.uhi = sh.uhi; gi.vlo = sh.vlo; gi.vhi = sh.vhi;
+                        gi.nuf = sh.nuf; gi.n = sh.n;
+                        gi.nkeyed = 0; gi.ndone = 0; gi.ev[0] = gi.ev[1] = FD_EV_NONE; gi.exitkey = 0ull;
                         GRect &gr = gs.rect[ninst];
                         gr.face = (short)face; gr.layer = (short)sh.layer;
                         gr.ulo = (short)sh.ulo; gr.uhi = (short)sh.uhi; gr.vlo = (short)sh.vlo; gr.vhi = (short)sh.vhi;
@@ -2062,15 +2026,13 @@ __device__ void graph_sweep(const fd_station_dev &sd, Shared &sh, CtaSmem &cs, W
         sh.nodefer = 0;
         sh.graph = 1;
         sh.gM = M;
-        if (lead) {
-            if (over) sh.w->status = 13;
-            walk_reset(sh, 6, FD_GRQ_CAP);
-            sh.w->nwait = 0;
-            long long b = 0;
-            for (int f = 0; f < 6; f++) { sh.w->qbase[f] = (int)b; sh.w->qcap[f] = (int)per_face[f]; b += per_face[f]; }
-        }
+        if (over) sh.w.status = 13;
+        walk_reset(sh, 6, FD_GRQ_CAP);
+        sh.w.nwait = 0;
+        long long b = 0;
+        for (int f = 0; f < 6; f++) { sh.w.qbase[f] = (int)b; sh.w.qcap[f] = (int)per_face[f]; b += per_face[f]; }
     }
-    csync(sh, 1);
+    csync(sh);
     const int ninst = sh.ninst;
     const long long M = sh.gM;
     if (sh.single) {
@@ -2091,7 +2053,7 @@ __device__ void graph_sweep(const fd_station_dev &sd, Shared &sh, CtaSmem &cs, W
         __syncthreads();
     }
     if (M > 0 && sh.stat == 0) {
-        for (long long k = gt; k < M; k += gstride) sd.scr.gqueue[k] = -1;
+        for (long long k = tid; k < M; k += blockDim.x) sd.scr.gqueue[k] = -1;
         /* dependency counters */
         for (int I = 0; I < ninst; I++) {
             const GRect r = gs.rect[I];
@@ -2099,7 +2061,7 @@ __device__ void graph_sweep(const fd_station_dev &sd, Shared &sh, CtaSmem &cs, W
             const int n = rect_n(r), nvf = r.vhi - r.vlo + 1;
             const unsigned myctx = sh.ctxm[r.face], myinn = sh.innm[r.face];
             const bool prev = sh.single && I > 0 && gs.rect[I - 1].layer == r.layer + fr.inner;
-            for (int j = gt; j < n; j += gstride) {
+            for (int j = tid; j < n; j += blockDim.x) {
                 const long long p = inst_node(sd, r, j);
                 if (!FD_OK(p, (long long)nx * ny * nz, 25)) continue;
                 unsigned cin = 0, c2 = 0, cx = 0;
@@ -2137,29 +2099,29 @@ __device__ void graph_sweep(const fd_station_dev &sd, Shared &sh, CtaSmem &cs, W
                 sd.scr.gcnt[p] = cin | (c2 << 8) | (cx << 16);
             }
         }
-        csync(sh, 2);
+        csync(sh);
         /* nodes whose inner block is final take their key now */
         for (int I = 0; I < ninst; I++) {
             const GRect r = gs.rect[I];
             const int n = rect_n(r);
-            for (int j = gt; j < n; j += gstride) {
+            for (int j = tid; j < n; j += blockDim.x) {
                 const long long p = inst_node(sd, r, j);
                 if ((sd.scr.gcnt[p] & 0xFFu) == 0u && ready_word(key_event(sd, sh, I, j, p))) graph_ready(sd, sh, r.face, p);
             }
         }
-        csync(sh, 3);
+        csync(sh);
         FD_TOC(0, t0);
         FD_TIC(tw);
         run_walk(sd, sh, cs, ws, (int)M, nullptr, cn);
-        csync(sh, 4);
+        csync(sh);
         FD_TOC(4, tw);
     }
     /* the small tables back to their empty state for the next sweep */
     {
-        const int nw = vload(sh.w->nwait) > 0 ? FD_GWAIT_CAP : 0;
-        const int nr = min(vload(sh.w->rqtail), FD_GRQ_CAP);
-        for (int k = gt; k < nw; k += gstride) sd.scr.gwait[k] = make_int2(-1, -1);
-        for (int k = gt; k < nr; k += gstride) sd.scr.grq[k] = -1;
+        const int nw = vload(sh.w.nwait) > 0 ? FD_GWAIT_CAP : 0;
+        const int nr = min(vload(sh.w.rqtail), FD_GRQ_CAP);
+        for (int k = tid; k < nw; k += blockDim.x) sd.scr.gwait[k] = make_int2(-1, -1);
+        for (int k = tid; k < nr; k += blockDim.x) sd.scr.grq[k] = -1;
     }
     if (tid == 0) {
         /* the stencil state after the sweep: the record of its last writer */
@@ -2177,7 +2139,7 @@ __device__ void graph_sweep(const fd_station_dev &sd, Shared &sh, CtaSmem &cs, W
         sh.gsweeps++;
         sh.graph = 0;
     }
-    csync(sh, 5);
+    csync(sh);
 }
 
 /* ---------------------------------------------------------------------------------------------- */
@@ -2220,39 +2182,27 @@ __device__ void init_field(const fd_station_dev &sd)
 /* ---------------------------------------------------------------------------------------------- */
 /* the sweep loop (src/sphfd.c:1008-5678)                                                          */
 
-/* The solve of one station by this CTA, or by this cluster of csz CTAs (csz > 1 only for sweep
- * graphs: face walks run in one CTA).  sd is the station record in this CTA's shared memory. */
-__device__ __forceinline__ void solve_station(const fd_station_dev &sd, int dag_smem_bytes, int csz, Shared &sh)
+/* The solve of one station by this CTA.  sd is the station record in this CTA's shared memory; lmax and imax
+ * are the extent and the instances that the launch's sweep-graph tables have room for. */
+__device__ __forceinline__ void solve_station(const fd_station_dev &sd, int dag_smem_bytes, int lmax, int imax, Shared &sh)
 {
     extern __shared__ __align__(16) unsigned char fd_dyn_smem[];
     CtaSmem &cs = *reinterpret_cast<CtaSmem *>(fd_dyn_smem);
     WarpSmem &ws = reinterpret_cast<WarpSmem *>(fd_dyn_smem + kCtaSmemBytes)[threadIdx.x >> 5];
     const int tid = threadIdx.x;
-    const int rank = csz > 1 ? (int)cooperative_groups::this_cluster().block_rank() : 0;
     unsigned long long t_start = 0;
     if (tid == 0) asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_start));
     /* the dependency bytes of the station's largest face go to shared memory when they fit */
     unsigned char *dag = 2ll * sd.max_face_pad <= dag_smem_bytes ? fd_dyn_smem + kSmemBase : sd.scr.dag;
     const int gdim = sd.g.nx > sd.g.ny ? (sd.g.nx > sd.g.nz ? sd.g.nx : sd.g.nz) : (sd.g.ny > sd.g.nz ? sd.g.ny : sd.g.nz);
-    const bool gok = sd.scr.gcnt && gdim <= FD_LMAX && (int)sizeof(GraphSmem) <= dag_smem_bytes;
-    /* without sweep graphs the first CTA solves alone (the launcher does not ask for more) */
-    if (!gok && rank > 0) return;
-    sh.cs = gok ? csz : 1;
-    sh.rank = rank;
-    sh.w = sh.cs > 1 ? cooperative_groups::this_cluster().map_shared_rank(&sh.wl, 0) : &sh.wl;
-    if (tid == 0 && rank == 0) sh.wl.bar_count = 0;
+    const bool gok = sd.scr.gcnt && gdim <= lmax && sd.scr.ginst_cap <= imax && graph_smem_bytes(lmax, imax) <= dag_smem_bytes;
     if (tid == 0) sh.stat = 0;
-    /* once, before any CTA touches another's shared memory: every CTA of the cluster has started and
-     * the barrier counter is set; every CTA reaches this line */
-    if (sh.cs > 1) cooperative_groups::this_cluster().sync();
-    if (rank == 0) {
-        if (gok) {
-            /* the sweep-graph tables start empty */
-            for (int k = tid; k < FD_GWAIT_CAP; k += blockDim.x) sd.scr.gwait[k] = make_int2(-1, -1);
-            for (int k = tid; k < FD_GRQ_CAP; k += blockDim.x) sd.scr.grq[k] = -1;
-        }
-        if (sd.init_mode == 0) init_field(sd);
+    if (gok) {
+        /* the sweep-graph tables start empty */
+        for (int k = tid; k < FD_GWAIT_CAP; k += blockDim.x) sd.scr.gwait[k] = make_int2(-1, -1);
+        for (int k = tid; k < FD_GRQ_CAP; k += blockDim.x) sd.scr.grq[k] = -1;
     }
+    if (sd.init_mode == 0) init_field(sd);
     for (int k = tid; k < FDN_NFACE * FDN_NTRIAL; k += blockDim.x) (&cs.desc[0][0])[k] = c_desc[k];
     if (tid == 0) {
         for (int f = 0; f < 6; f++) { sh.wall[f] = sd.wall[f]; sh.dflag[f] = sd.dflag[f]; }
@@ -2262,13 +2212,11 @@ __device__ __forceinline__ void solve_station(const fd_station_dev &sd, int dag_
         sh.headpref = sd.headpref;
         sh.carry_t0 = sd.carry_t0;
         sh.carry_t4 = sd.carry_t4;
-        if (rank == 0) {
-            sh.w->status = 0;
-            sh.w->rounds = sh.w->deferred = 0;
-            for (int k = 0; k < 5; k++) sh.w->st[k] = 0;
-            sh.w->nwait = 0;
-            sh.w->npark = 0;
-        }
+        sh.w.status = 0;
+        sh.w.rounds = sh.w.deferred = 0;
+        for (int k = 0; k < 5; k++) sh.w.st[k] = 0;
+        sh.w.nwait = 0;
+        sh.w.npark = 0;
         sh.faces = sh.node_updates = 0;
         sh.sweeps = 0;
         for (int k = 0; k < 8; k++) sh.restart_wall[k] = 0;
@@ -2276,13 +2224,14 @@ __device__ __forceinline__ void solve_station(const fd_station_dev &sd, int dag_
         sh.graph = 0;
         sh.gsweeps = 0;
         for (int f = 0; f < 6; f++) relation_masks(f, sh.ctxm[f], sh.innm[f]);
-        sh.gsm = fd_dyn_smem + kSmemBase;
+        sh.lstride = lmax + 2;
+        sh.imax = imax;
         sh.gok = gok;
         sh.single = 0;
         sh.nodefer = 0;
         sh.gfaces = 0;
     }
-    csync(sh, 6);
+    csync(sh);
     for (int k = tid; k < 6 * 27; k += blockDim.x) sh.rel[k / 27][k % 27] = relation_word(sh, k / 27, k % 27);
     if ((tid & 31) < 6) ws.cnt[tid & 31] = 0ull;
     __syncwarp();
@@ -2291,8 +2240,8 @@ __device__ __forceinline__ void solve_station(const fd_station_dev &sd, int dag_
     const int nx = sd.g.nx, ny = sd.g.ny, nz = sd.g.nz;
     int guard_sweeps = 0;
     while (sh.reverse > -1 && sh.stat == 0) {
-        if (tid == 0 && rank == 0) for (int k = 0; k < 8; k++) sh.w->headw[k] = 0;
-        csync(sh, 7);
+        if (tid == 0) for (int k = 0; k < 8; k++) sh.w.headw[k] = 0;
+        csync(sh);
         FD_TIC(tsweep);
         const bool as_graph = sh.gok && (FD_GRAPH_FORWARD || sh.sweeps > 0);
         if (as_graph) graph_sweep(sd, sh, cs, ws, cn);
@@ -2321,13 +2270,13 @@ __device__ __forceinline__ void solve_station(const fd_station_dev &sd, int dag_
                 sh.radius++;
                 if (sh.radius == sd.maxrad) sh.rad0 = 0;
             }
-            csync(sh, 10);
+            csync(sh);
         }
         if (tid == 0) {
             if (sh.sweeps == 0) FD_TOC(5, tsweep);   /* profiling builds: the first sweep's cycles */
             sh.sweeps++;
             /* restart test (src/sphfd.c:5570-5676) */
-            const int *hw = sh.w->headw;
+            const int *hw = sh.w.headw;
             if (!hw[1] && !hw[2] && !hw[3] && !hw[4] && !hw[5] && !hw[6]) {
                 sh.reverse = 0;
             } else {
@@ -2349,23 +2298,22 @@ __device__ __forceinline__ void solve_station(const fd_station_dev &sd, int dag_
             }
             sh.reverse--;
         }
-        /* every CTA has read this sweep's head-wave counts before the next sweep clears them */
-        csync(sh, 8);
-        if (++guard_sweeps > 1000000) { if (tid == 0 && rank == 0) sh.w->status = 4; break; }
+        csync(sh);
+        if (++guard_sweeps > 1000000) { if (tid == 0) sh.w.status = 4; break; }
     }
     /* statistics */
     __syncwarp();
-    if ((tid & 31) < 5) atomicAdd(&sh.w->st[tid & 31], ws.cnt[tid & 31]);
-    csync(sh, 9);
-    if (tid == 0 && rank == 0 && sd.stats) {
+    if ((tid & 31) < 5) atomicAdd(&sh.w.st[tid & 31], ws.cnt[tid & 31]);
+    csync(sh);
+    if (tid == 0 && sd.stats) {
         fd_station_stats *o = sd.stats;
-        o->status = sh.w->status;
+        o->status = sh.w.status;
         o->sweeps = sh.sweeps;
         o->node_updates = sh.node_updates;
         o->faces = sh.faces;
-        o->rounds = sh.w->rounds;
-        o->deferred = sh.w->deferred;
-        for (int k = 0; k < 5; k++) o->stencils[k] = (int64_t)sh.w->st[k];
+        o->rounds = sh.w.rounds;
+        o->deferred = sh.w.deferred;
+        for (int k = 0; k < 5; k++) o->stencils[k] = (int64_t)sh.w.st[k];
         for (int k = 0; k < 8; k++) o->restart_wall[k] = sh.restart_wall[k];
         for (int k = 0; k < 6; k++) o->phase_cycles[k] = sh.cyc[k];
         unsigned long long t_end;
@@ -2377,9 +2325,6 @@ __device__ __forceinline__ void solve_station(const fd_station_dev &sd, int dag_
         asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
         o->sm = (int32_t)smid;
     }
-    /* no CTA leaves while another may still read the first CTA's shared memory; every wait before
-     * this line is bounded, so every CTA reaches it */
-    if (sh.cs > 1) cooperative_groups::this_cluster().sync();
 }
 
 /* a station record copied into shared memory by the whole CTA; cache-volatile loads, because a
@@ -2438,18 +2383,18 @@ __device__ int serve_claim(const fd_serve_queue &q, unsigned long long *gen)
     }
 }
 
-/* Batch mode (q == nullptr): station blockIdx.x / csz of `stations`, one launch per batch.
+/* Batch mode (q == nullptr): station blockIdx.x of `stations`, one launch per batch.
  * Serving mode: a long-running grid of one CTA per SM; each CTA solves the requests it claims from
- * q one after another (csz 1), and writes exitf[cta_id0 + blockIdx.x] when it leaves. */
+ * q one after another, and writes exitf[cta_id0 + blockIdx.x] when it leaves. */
 __global__ void __launch_bounds__(FD_BLOCK, 1) fd_solve(const fd_station_dev *stations, int nst, int dag_smem_bytes,
-                                                       int csz, const fd_serve_queue *q, int cta_id0)
+                                                       int lmax, int imax, const fd_serve_queue *q, int cta_id0)
 {
     __shared__ Shared sh;
     __shared__ fd_station_dev rec;
     __shared__ int entry;
     __shared__ unsigned long long gen;
-    const int station = (int)blockIdx.x / csz;
-    if (!q && station >= nst) return;   /* a whole cluster: its CTAs are consecutive */
+    const int station = (int)blockIdx.x;
+    if (!q && station >= nst) return;
     for (;;) {
         if (q) {
             if (threadIdx.x == 0) entry = serve_claim(*q, &gen);
@@ -2458,7 +2403,7 @@ __global__ void __launch_bounds__(FD_BLOCK, 1) fd_solve(const fd_station_dev *st
         }
         load_record(rec, q ? q->desc + entry : stations + station);
         __syncthreads();
-        solve_station(rec, dag_smem_bytes, q ? 1 : csz, sh);
+        solve_station(rec, dag_smem_bytes, lmax, imax, sh);
         if (!q) return;
         /* every thread's field writes, then the statistics, then the flag the host waits for */
         __syncthreads();
@@ -2497,83 +2442,46 @@ static size_t dyn_smem_limit_margin()
     return margin;
 }
 
-/* cluster: CTAs per station; 0 picks more than one when the stations alone would leave SMs idle,
- * up to 8 (1 keeps every station on one CTA).  Reduced until every cluster of the launch is
- * co-resident. */
-/* Launch shape of a batch: dynamic shared memory (the warp areas, plus the sweep-graph tables or the
- * face's dependency bytes, whichever is larger and fits) and CTAs per station; sets the kernel's
- * shared-memory limit.  Host calls only (no stream work): done once per batch, outside any capture. */
-extern "C" cudaError_t fdk_solve_config(int nst, long long max_face_pad, int cluster, long long *bytes_out,
-                                        int *csz_out)
+/* Launch shape of a batch: dynamic shared memory for the warp areas and the larger of the sweep-graph tables
+ * (extents up to lmax, imax instances; 0: no station has a sweep graph) and, where stations walk their faces one at
+ * a time, the largest such face's dependency bytes (max_face_pad points; left to global memory when they do not
+ * fit).  Sets the kernel's shared-memory limit.  Host calls only (no stream work): done once per batch, outside any
+ * capture. */
+extern "C" cudaError_t fdk_solve_config(long long max_face_pad, int lmax, int imax, long long *bytes_out)
 {
-    int dev = 0, optin = 0, sms = 0;
+    int dev = 0, optin = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const long long room = optin - (long long)dyn_smem_limit_margin();
     const long long base = (long long)fdk::kSmemBase;
-    const long long graph = (long long)sizeof(fdk::GraphSmem);
+    const long long graph = imax > 0 ? fdk::graph_smem_bytes(lmax, imax) : 0;
     const long long dagb = 2 * max_face_pad > graph ? 2 * max_face_pad : graph;
     const long long bytes = base + dagb <= room ? base + dagb : (base + graph <= room ? base + graph : base);
     /* the attribute is an upper bound shared by every launch of the kernel (a serving session may
      * launch it from another thread): always the largest */
-    cudaError_t e = cudaFuncSetAttribute(fdk::fd_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room);
+    const cudaError_t e = cudaFuncSetAttribute(fdk::fd_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room);
     if (e != cudaSuccess) return e;
-    /* CTAs per station: with clusters of 2 any two SMs of a GPC serve; clusters of 4 and 8 are taken
-     * only with room to spare, so that every cluster of the launch is co-resident (launches whose
-     * clusters of 8 ran in several waves faulted once on this GPU; they are not made) */
-    auto fits = [&](int c) {
-        const long long ctas = (long long)nst * c;
-        return c == 1 || (c == 2 && ctas <= sms) || (c == 4 && 4 * ctas <= 3ll * sms) || (c == 8 && 2 * ctas <= sms);
-    };
-    int cs = cluster;
-    if (cs <= 0) {
-        cs = 1;
-        while (cs < 8 && fits(cs * 2) && (long long)nst * cs * 2 <= sms) cs *= 2;
-    }
-    while (cs > 1 && !fits(cs)) cs /= 2;
-    if (cs > FD_MAX_CLUSTER) cs = FD_MAX_CLUSTER;
-    if (bytes - base < graph) cs = 1;   /* no room for the sweep-graph tables: face walks, one CTA */
     *bytes_out = bytes;
-    *csz_out = cs;
     return cudaSuccess;
 }
 
 /* One launch of a configured batch: queues the kernel only (capturable in a CUDA graph). */
-extern "C" cudaError_t fdk_solve_launch(const fd_station_dev *stations, int nst, long long bytes, int cs,
+extern "C" cudaError_t fdk_solve_launch(const fd_station_dev *stations, int nst, long long bytes, int lmax, int imax,
                                         cudaStream_t stream)
 {
     if (nst <= 0) return cudaSuccess;
-    const long long base = (long long)fdk::kSmemBase;
-    if (cs == 1) {
-        fdk::fd_solve<<<nst, FD_BLOCK, (size_t)bytes, stream>>>(stations, nst, (int)(bytes - base), 1, nullptr, 0);
-        return cudaGetLastError();
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(nst * cs));
-    cfg.blockDim = dim3(FD_BLOCK);
-    cfg.dynamicSmemBytes = (size_t)bytes;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)cs;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, fdk::fd_solve, stations, nst, (int)(bytes - base), cs,
-                                             static_cast<const fd_serve_queue *>(nullptr), 0);
-    return e == cudaSuccess ? cudaGetLastError() : e;
+    fdk::fd_solve<<<nst, FD_BLOCK, (size_t)bytes, stream>>>(stations, nst, (int)(bytes - fdk::kSmemBase), lmax, imax,
+                                                           nullptr, 0);
+    return cudaGetLastError();
 }
 
-extern "C" cudaError_t fdk_launch_solve(const fd_station_dev *stations, int nst, long long max_face_pad, int cluster,
-                                        cudaStream_t stream)
+extern "C" cudaError_t fdk_launch_solve(const fd_station_dev *stations, int nst, long long max_face_pad, int lmax,
+                                        int imax, cudaStream_t stream)
 {
     if (nst <= 0) return cudaSuccess;
     long long bytes = 0;
-    int cs = 1;
-    const cudaError_t e = fdk_solve_config(nst, max_face_pad, cluster, &bytes, &cs);
-    return e != cudaSuccess ? e : fdk_solve_launch(stations, nst, bytes, cs, stream);
+    const cudaError_t e = fdk_solve_config(max_face_pad, lmax, imax, &bytes);
+    return e != cudaSuccess ? e : fdk_solve_launch(stations, nst, bytes, lmax, imax, stream);
 }
 
 /* The long-running grid of a serving session: nctas CTAs (one per SM), numbered cta_id0 onward in
@@ -2587,11 +2495,11 @@ extern "C" cudaError_t fdk_launch_serve(const fd_serve_queue *q, int nctas, int 
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     const long long bytes = optin - (long long)dyn_smem_limit_margin();
     const long long base = (long long)fdk::kSmemBase;
-    if (bytes - base < (long long)sizeof(fdk::GraphSmem)) return cudaErrorInvalidConfiguration;
+    if (bytes - base < fdk::graph_smem_bytes(FD_LMAX, FD_IMAX)) return cudaErrorInvalidConfiguration;
     /* the same bound as every other launch of the kernel */
     cudaError_t e = cudaFuncSetAttribute(fdk::fd_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e != cudaSuccess) return e;
-    fdk::fd_solve<<<nctas, FD_BLOCK, (size_t)bytes, stream>>>(nullptr, 0, (int)(bytes - base), 1, q, cta_id0);
+    fdk::fd_solve<<<nctas, FD_BLOCK, (size_t)bytes, stream>>>(nullptr, 0, (int)(bytes - base), FD_LMAX, FD_IMAX, q, cta_id0);
     return cudaGetLastError();
 }
 

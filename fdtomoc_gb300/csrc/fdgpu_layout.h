@@ -85,6 +85,11 @@ typedef struct {
     unsigned long long exitkey;    /* largest key of a point that made a writer call (0: none) */
 } fd_ginst;
 
+/* the largest sweep graph: grid extent, face instances (at most nx + ny + nz + 8); larger grids walk their
+ * faces one at a time */
+#define FD_LMAX 1024
+#define FD_IMAX 3088
+
 #define FD_EV_NONE (-1)
 #define FD_EV_FIRED (-2)
 

@@ -50,6 +50,24 @@ inline size_t graph_bytes(const fdgpu_station &s)
            + 8 * (size_t)FD_GWAIT_CAP + 8 * (size_t)FD_GPARK_CAP + 4 * (size_t)FD_GRQ_CAP;
 }
 
+/* what a launch's shared memory has to hold for its stations: the sweep-graph tables of the largest ones that
+ * have a sweep graph, the largest face of those that walk their faces one at a time */
+struct SolveShape {
+    long long max_face_pad = 0;
+    int lmax = 0, imax = 0;
+
+    void add(const fdgpu_station &s, bool graph)
+    {
+        const int g = std::max({s.nx, s.ny, s.nz});
+        if (graph && g <= FD_LMAX) {
+            lmax = std::max(lmax, g);
+            imax = std::max(imax, graph_instances(s));
+        } else {
+            max_face_pad = std::max(max_face_pad, (max_face(s) + 15) & ~15LL);
+        }
+    }
+};
+
 /* geometry tables of one grid geometry: ysin | zrow | node | cell */
 inline size_t geo_bytes(int ny, int nz)
 {
