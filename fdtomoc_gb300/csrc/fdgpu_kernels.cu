@@ -301,7 +301,7 @@ struct WarpSmem {
     double res[32][FDN_NTRIAL];            /* trial values (2-D: after the causality selection) */
     float t[32][NB_PAD];                   /* 18-node time context */
     float s[32][NB_PAD];                   /* 18-node slowness context */
-    float s0[32], s4[32];                  /* stencil state entering the 2-D block */
+    float s0[32], s4[32];                  /* stencil state entering the 2-D block; before it, step lengths */
     int z[32], y[32];                      /* grid z and y of the node */
     unsigned short items[kItems];          /* (slot << 5 | trial) to evaluate, trial-major */
     unsigned long long cnt[6];             /* stencil evaluations by kind (5 used) */
@@ -454,19 +454,20 @@ __device__ __forceinline__ unsigned ne_prune(const TrialDesc *dsc, const float *
     return em;
 }
 
-/* append the items (lane, K) for the trials K of `of` whose bit is set in the lane's em, trial-major */
+/* append the items (lane, K) for the trials K of `of` whose bit is set in the lane's em, node by node */
 __device__ __forceinline__ int push_items(unsigned short *items, int n, unsigned em, unsigned of, int lane)
 {
-    const unsigned below = (1u << lane) - 1u;
     em &= of;
-    for (unsigned any = __reduce_or_sync(0xffffffffu, em); any; any &= any - 1) {
-        const int K = __ffs(any) - 1;
-        const bool on = (em >> K) & 1u;
-        const unsigned b = __ballot_sync(0xffffffffu, on);
-        if (on) items[n + __popc(b & below)] = (unsigned short)((lane << 5) | K);
-        n += __popc(b);
+    const int mine = __popc(em);
+    int end = mine;   /* items of the lanes up to this one */
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, end, o);
+        if (lane >= o) end += x;
     }
-    return n;
+    unsigned short *to = items + n + end - mine;
+    for (; em; em &= em - 1) *to++ = (unsigned short)((lane << 5) | (__ffs(em) - 1));
+    return n + __shfl_sync(0xffffffffu, end, 31);
 }
 constexpr unsigned k2d = 0xFFu << TK_2D0;
 constexpr unsigned k1d = 0x1Fu << TK_1D0;
@@ -687,6 +688,7 @@ __device__ unsigned stale_pair(const fd_station_dev &sd, const TrialDesc *dsc, W
                                unsigned gm, unsigned em, float it0, float it4)
 {
     const float *t18 = ws.t[slot];
+    const float dx = ws.s0[slot], dy = ws.s4[slot], dz = d2f_trunc(sd.g.h);   /* step lengths, put there with the context */
     double g1 = f2d(t18[NB_POINT]);
     float s0 = it0, s4 = it4;
     /* the last writer's slots are what remains of the writers before it */
@@ -723,11 +725,7 @@ __device__ unsigned stale_pair(const fd_station_dev &sd, const TrialDesc *dsc, W
     const float gf = d2f_trunc(g1), gup = __int_as_float(__float_as_int(gf) + 1);   /* above g1; NaN stays NaN */
     if ((em & k1d) && gup <= 99999997952.f) {
         const fdn_frame fr = frame_of(F);
-        const int z = ws.z[slot], y = ws.y[slot];
         const float *s18 = ws.s[slot];
-        const float dx = d2f_trunc(node_row(sd.g, z, y)[FD_N_RSDF]);
-        const float dy = d2f_trunc(sd.g.zrow[(long long)(FD_OK(z, sd.g.nz, 8) ? z : 0) * FD_Z_N + FD_Z_RDQ]);
-        const float dz = d2f_trunc(sd.g.h);
 #pragma unroll
         for (int k = 0; k < 5; k++) {
             const int nb = k == 0 ? 13 : k == 1 ? 5 : k == 2 ? 3 : k == 3 ? 7 : 1;
@@ -882,8 +880,12 @@ __device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long x)
 #define FD_WAITB 0x20000000u
 #define FD_DONEB 0x40000000u
 
+/* a face instance: face and layer, and its rectangle */
 struct GRect {
-    short face, layer, ulo, uhi, vlo, vhi, nuf, pad;
+    short fl, ulo, uhi, vlo, vhi, pad;
+    __device__ __forceinline__ int face() const { return fl & 7; }
+    __device__ __forceinline__ int layer() const { return fl >> 3; }
+    __device__ __forceinline__ int nuf() const { return uhi - ulo + 1; }
 };
 
 /* In the dynamic shared memory after the warp areas (the face walks' dependency bytes otherwise).
@@ -898,6 +900,7 @@ struct GRect {
 struct GraphSmem {
     short *lay[3];   /* entry c + 1 for coordinate c, FD_NEVER on both sides of the grid */
     GRect *rect;
+    int *nkeyed, *ndone;   /* per instance: points whose sort key is final, points done */
 };
 static_assert((FD_IMAX << 3) + 7 < 0x7fff, "owner words in a short");
 
@@ -907,7 +910,7 @@ static_assert((FD_IMAX << 3) + 7 < 0x7fff, "owner words in a short");
  * window; a 141x121x57 station 219 -> 177 ms). */
 __host__ __device__ constexpr long long graph_smem_bytes(int lmax, int imax)
 {
-    return ((3ll * (lmax + 2) * 2 + 15) & ~15ll) + (long long)imax * (long long)sizeof(GRect);
+    return ((3ll * (lmax + 2) * 2 + 15) & ~15ll) + (long long)imax * (long long)(sizeof(GRect) + 2 * sizeof(int));
 }
 
 /* the tables of the largest grids, the warp areas and 2.5 KB of static shared memory fit a CTA's 227 KB */
@@ -918,7 +921,9 @@ __device__ __forceinline__ GraphSmem gsmem(const Shared &sh)
     extern __shared__ __align__(16) unsigned char fd_dyn_smem[];
     short *l = reinterpret_cast<short *>(fd_dyn_smem + kSmemBase);
     const int n = sh.lstride;
-    return {{l, l + n, l + 2 * n}, reinterpret_cast<GRect *>(fd_dyn_smem + kSmemBase + ((3 * n * 2 + 15) & ~15))};
+    GRect *r = reinterpret_cast<GRect *>(fd_dyn_smem + kSmemBase + ((3 * n * 2 + 15) & ~15));
+    int *c = reinterpret_cast<int *>(r + sh.imax);   /* GRect is 12 bytes */
+    return {{l, l + n, l + 2 * n}, r, c, c + sh.imax};
 }
 
 /* Neighbour offsets (dx,dy,dz) are numbered k = (dz+1)*9 + (dy+1)*3 + (dx+1), 13 being the node
@@ -966,7 +971,7 @@ __device__ unsigned relation_word(const Shared &sh, int F, int k)
     return w;
 }
 
-__device__ __forceinline__ int rect_n(const GRect &r) { return r.nuf * (r.vhi - r.vlo + 1); }
+__device__ __forceinline__ int rect_n(const GRect &r) { return r.nuf() * (r.vhi - r.vlo + 1); }
 
 /* owner word of node (x,y,z), which must lie in the grid */
 __device__ __forceinline__ int owner_of(const GraphSmem &gs, int x, int y, int z)
@@ -974,35 +979,30 @@ __device__ __forceinline__ int owner_of(const GraphSmem &gs, int x, int y, int z
     return owner_word(gs.lay[0][x + 1], gs.lay[1][y + 1], gs.lay[2][z + 1]);
 }
 
-/* node index of point j of instance r */
-__device__ __forceinline__ long long inst_node(const fd_station_dev &sd, const GRect &r, int j)
+/* a node's coordinates in one word: what the queues and lists of a sweep graph hold (extents are at most
+ * FD_LMAX), so that nothing divides to get them back */
+__device__ __forceinline__ int pack_xyz(int x, int y, int z) { return x | (y << 10) | (z << 20); }
+static_assert(FD_LMAX <= 1024, "pack_xyz");
+__device__ __forceinline__ int node_of(const fd_station_dev &sd, int xyz)
 {
-    const fdn_frame fr = frame_of(r.face);
-    int x, y, z;
-    place(fr, r.ulo + j % r.nuf, r.vlo + j / r.nuf, r.layer, x, y, z);
-    return ((long long)z * sd.g.ny + y) * sd.g.nx + x;
+    return ((xyz >> 20) * sd.g.ny + ((xyz >> 10) & 1023)) * sd.g.nx + (xyz & 1023);
 }
 
-/* sort key of point j of instance r: time of its inner-layer node, then fill index */
-__device__ __forceinline__ unsigned long long inst_key(const fd_station_dev &sd, const GRect &r, int j)
+/* coordinates of point j of instance r, its node index */
+__device__ __forceinline__ int inst_xyz(const GRect &r, int j)
 {
-    const fdn_frame fr = frame_of(r.face);
-    const long long p = inst_node(sd, r, j) + fr.inner * t_stride(sd, fr.axis_n);
-    return node_key(vload(sd.T[p]), j);
+    const int nuf = r.nuf(), iv = j / nuf;
+    int x, y, z;
+    place(frame_of(r.face()), r.ulo + j - iv * nuf, r.vlo + iv, r.layer(), x, y, z);
+    return pack_xyz(x, y, z);
 }
+__device__ __forceinline__ int inst_node(const fd_station_dev &sd, const GRect &r, int j) { return node_of(sd, inst_xyz(r, j)); }
 
 /* the in-face neighbour (du,dv) of a node comes later in its instance's order: inner-layer time (as
  * okey32 images), then fill index, which grows with dv and, within a row, with du */
 __device__ __forceinline__ bool later_key(unsigned nb, unsigned own, int du, int dv)
 {
     return nb > own || (nb == own && (dv > 0 || (dv == 0 && du > 0)));
-}
-
-/* fill index of node (x,y,z) in instance r */
-__device__ __forceinline__ int inst_fill(const GRect &r, int x, int y, int z)
-{
-    const fdn_frame fr = frame_of(r.face);
-    return (coord(fr.axis_v, x, y, z) - r.vlo) * r.nuf + (coord(fr.axis_u, x, y, z) - r.ulo);
 }
 
 /* Points parked on instance I's event `kind` (1: all keys final, 2: all done) go to the resume queue.  The
@@ -1019,32 +1019,36 @@ FD_COLD void fire_event(const fd_station_dev &sd, Shared &sh, int I, int kind)
     }
 }
 
-/* Key event of node j of instance I (its inner block is final): its later same-instance neighbours
- * are dropped from its counter.  Returns the counter word after the update. */
-__device__ unsigned key_event(const fd_station_dev &sd, Shared &sh, int I, int j, long long q)
+/* Key event of a node (coordinates xyz, grid index q, instance I): its inner block is final, and its
+ * later same-instance neighbours are dropped from its counter.  Returns the counter word after the
+ * update. */
+__device__ __forceinline__ unsigned key_event(const fd_station_dev &sd, Shared &sh, int I, int xyz, int q)
 {
-    const GRect &r = gsmem(sh).rect[I];
-    const fdn_frame fr = frame_of(r.face);
-    const int n = rect_n(r), nvf = r.vhi - r.vlo + 1, iv = j / r.nuf, iu = j - iv * r.nuf;
-    const long long su = t_stride(sd, fr.axis_u), sv = t_stride(sd, fr.axis_v);
-    const long long qin = q + fr.inner * t_stride(sd, fr.axis_n);   /* q's inner-layer node */
-    const unsigned inr = inrect_mask(iu, iv, r.nuf, nvf);
+    const GraphSmem gs = gsmem(sh);
+    const GRect r = gs.rect[I];
+    const fdn_frame fr = frame_of(r.face());
+    const int x = xyz & 1023, y = (xyz >> 10) & 1023, z = xyz >> 20;
+    const int u = coord(fr.axis_u, x, y, z), v = coord(fr.axis_v, x, y, z);
+    const int su = (int)t_stride(sd, fr.axis_u), sv = (int)t_stride(sd, fr.axis_v);
+    const int qin = q + fr.inner * (int)t_stride(sd, fr.axis_n);   /* q's inner-layer node */
+    /* columns and rows of the 3x3 block inside the rectangle */
+    const unsigned in = (u > r.ulo ? 1u : 0u) | 2u | (u < r.uhi ? 4u : 0u) | (v > r.vlo ? 8u : 0u) | 16u | (v < r.vhi ? 32u : 0u);
     /* the inner-layer times of q and of its in-rectangle neighbours, all loads issued together */
-    float tn[8];
+    float tn[9];
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
-        int du, dv;
-        nb_off(k, du, dv);
-        const long long qk = qin + du * su + dv * sv;
-        tn[k] = (((inr >> k) & 1u) && FD_OK(qk, (long long)sd.g.nx * sd.g.ny * sd.g.nz, 12)) ? vload(sd.T[qk]) : 0.f;
+    for (int k = 0; k < 9; k++) {
+        const int du = k % 3 - 1, dv = k / 3 - 1;
+        const unsigned bits = 1u << (du + 1) | 8u << (dv + 1);
+        const int qk = qin + du * su + dv * sv;
+        tn[k] = ((in & bits) == bits && FD_OK(qk, (long long)sd.g.nx * sd.g.ny * sd.g.nz, 12)) ? sd.T[qk] : 0.f;
     }
-    const unsigned kj = okey32(vload(sd.T[qin]));
+    const unsigned kj = okey32(tn[4]);
     unsigned lat = 0;
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
-        int du, dv;
-        nb_off(k, du, dv);
-        if (((inr >> k) & 1u) && later_key(okey32(tn[k]), kj, du, dv)) lat++;
+    for (int k = 0; k < 9; k++) {
+        const int du = k % 3 - 1, dv = k / 3 - 1;
+        const unsigned bits = 1u << (du + 1) | 8u << (dv + 1);
+        if (k != 4 && (in & bits) == bits && later_key(okey32(tn[k]), kj, du, dv)) lat++;
     }
     if (!FD_OK(q, (long long)sd.g.nx * sd.g.ny * sd.g.nz, 13) || !FD_OK(qin, (long long)sd.g.nx * sd.g.ny * sd.g.nz, 29)
         || !FD_OK(I, sd.scr.ginst_cap, 14))
@@ -1052,15 +1056,15 @@ __device__ unsigned key_event(const fd_station_dev &sd, Shared &sh, int I, int j
     wfence(sh);
     const unsigned add = FD_KEYED - (lat << 8);
     const unsigned nw = atomicAdd(&sd.scr.gcnt[q], add) + add;
-    if (!sh.nodefer && atomicAdd(&sd.scr.ginst[I].nkeyed, 1) == n - 1) fire_event(sd, sh, I, 1);
+    if (!sh.nodefer && atomicAdd(&gs.nkeyed[I], 1) == rect_n(r) - 1) fire_event(sd, sh, I, 1);
     return nw;
 }
 
 __device__ __forceinline__ bool ready_word(unsigned w) { return (w & ~FD_WAITB) == FD_KEYED; }
 
-__device__ __forceinline__ void graph_ready(const fd_station_dev &sd, Shared &sh, int face, long long q)
+__device__ __forceinline__ void graph_ready(const fd_station_dev &sd, Shared &sh, int face, int xyz)
 {
-    enqueue_to(sd.scr.gqueue + sh.w.qbase[face], sh.w.qtail[face], sh.w.qcap[face], sh, (int)q);
+    enqueue_to(sd.scr.gqueue + sh.w.qbase[face], sh.w.qtail[face], sh.w.qcap[face], sh, xyz);
 }
 
 /* Points that wait for a point: (awaited, waiting) pairs in a hash table probed one slot on at a time.  The
@@ -1083,11 +1087,13 @@ FD_COLD void wake_waiters(const fd_station_dev &sd, Shared &sh, int p)
     }
 }
 
-/* node p (instance I, fill index i) is final: its record, and the points that wait for it */
-__device__ void graph_record(const fd_station_dev &sd, Shared &sh, long long p, int I, int i, bool writer, float st0,
-                             float st4, float tin)
+/* node p (instance I, fill index i) is final: its record.  Returns its counter word as it was when it was
+ * marked done: FD_WAITB if a point waits for it (the caller wakes those once it has used the time the
+ * word takes to arrive). */
+__device__ __forceinline__ unsigned graph_record(const fd_station_dev &sd, Shared &sh, long long p, int I, int i, bool writer,
+                                                 float st0, float st4, float tin)
 {
-    if (!FD_OK(p, (long long)sd.g.nx * sd.g.ny * sd.g.nz, 15) || !FD_OK(I, sd.scr.ginst_cap, 16)) return;
+    if (!FD_OK(p, (long long)sd.g.nx * sd.g.ny * sd.g.nz, 15) || !FD_OK(I, sd.scr.ginst_cap, 16)) return 0u;
     /* records: of every point when a point may need an earlier one's; else only the last instance's,
      * for the state the sweep leaves */
     if (!sh.nodefer || I == sh.ninst - 1) {
@@ -1099,8 +1105,7 @@ __device__ void graph_record(const fd_station_dev &sd, Shared &sh, long long p, 
         }
     }
     wfence(sh);
-    /* done; a point waiting for the stencil state left before it resumes its search */
-    if (!sh.nodefer && (atomicOr(&sd.scr.gcnt[p], FD_DONEB | (writer ? FD_WRITERB : 0u)) & FD_WAITB)) wake_waiters(sd, sh, (int)p);
+    return sh.nodefer ? 0u : atomicOr(&sd.scr.gcnt[p], FD_DONEB | (writer ? FD_WRITERB : 0u));
 }
 
 /* nodes of a chunk up to which a release gives each neighbour a lane (more: each node), in a sweep of
@@ -1132,20 +1137,21 @@ __device__ __forceinline__ unsigned release_dec(int w, int I, unsigned rw, const
     return !(f & 1u) ? 0u : (f & (1u << 6)) ? 1u : 1u << 16;
 }
 
-/* drop dec from the counter of node q; a node that becomes ready is queued, one whose inner block is now
- * complete goes on the list of key events */
-__device__ __forceinline__ void release_one(const fd_station_dev &sd, Shared &sh, int q, int fq, unsigned dec, int *keyq,
-                                            int *nkey)
+/* drop dec from the counter of node q (coordinates xyz); a node that becomes ready is queued, one whose
+ * inner block is now complete goes on the list of key events */
+__device__ __forceinline__ void release_one(const fd_station_dev &sd, Shared &sh, int q, int xyz, int fq, unsigned dec,
+                                            int *keyq, int *nkey)
 {
     if (!FD_OK(q, (long long)sd.g.nx * sd.g.ny * sd.g.nz, 19)) return;
     const unsigned nw = atomicSub(&sd.scr.gcnt[q], dec) - dec;
     if (dec == 1u && (nw & 0xFFu) == 0u)
-        keyq[atomicAdd(nkey, 1)] = q;
+        keyq[atomicAdd(nkey, 1)] = xyz;
     else if (ready_word(nw))
-        graph_ready(sd, sh, fq, q);
+        graph_ready(sd, sh, fq, xyz);
 }
 
-/* Release what waits on the chunk's final nodes (fin, wh: this lane's node).  All 32 lanes call.
+/* Release what waits on the chunk's final nodes (fin, was, wh: this lane's node, graph_record's word).  All 32
+ * lanes call.
  *
  * What bounds a release is instructions: a warp of this kernel issues one about every ten cycles, so
  * what matters is how many the warp steps through.  A chunk of a forward sweep holds two to nine nodes;
@@ -1160,7 +1166,8 @@ __device__ __forceinline__ void release_one(const fd_station_dev &sd, Shared &sh
  * 29 nodes (141x121x57), against a loop over the neighbours with a search of the six faces for each
  * owner and a key event inside it.  The two forms cost the same at about 12 nodes of a forward sweep (27
  * steps of the second form against 12 of the first) and at 6 of a one-face sweep (17 steps). */
-__device__ void graph_release(const fd_station_dev &sd, Shared &sh, WarpSmem &ws, int F, bool fin, const Where &wh)
+__device__ void graph_release(const fd_station_dev &sd, Shared &sh, WarpSmem &ws, int F, bool fin, unsigned was,
+                              const Where &wh)
 {
     const int lane = threadIdx.x & 31;
     const GraphSmem gs = gsmem(sh);
@@ -1173,7 +1180,7 @@ __device__ void graph_release(const fd_station_dev &sd, Shared &sh, WarpSmem &ws
     const bool few = m <= (sh.single ? FD_FEW1 : FD_FEW);
     RelNode *rn = reinterpret_cast<RelNode *>(ws.s0);   /* s0, s4, z, y: free after the commit */
     if (few && fin)
-        rn[__popc(mask & ((1u << lane) - 1u))] = {wh.x | (wh.y << 10) | (wh.z << 20), (int)wh.p, wh.inst, lane};
+        rn[__popc(mask & ((1u << lane) - 1u))] = {pack_xyz(wh.x, wh.y, wh.z), (int)wh.p, wh.inst, lane};
     if (lane == 0) *nkey = 0;
     __syncwarp();
     wfence(sh);
@@ -1181,14 +1188,14 @@ __device__ void graph_release(const fd_station_dev &sd, Shared &sh, WarpSmem &ws
         if (lane < 26) {
             const int k = lane + (lane >= 13);
             const int kx = k % 3, ky = (k / 3) % 3, kz = k / 9;
-            const int off = ((kz - 1) * ny + ky - 1) * nx + kx - 1;
+            const int off = ((kz - 1) * ny + ky - 1) * nx + kx - 1, oxyz = kx - 1 + (ky - 1) * 1024 + (kz - 1) * (1 << 20);
             const unsigned rw = sh.rel[F][k];
             for (int j = 0; j < m; j++) {
                 const RelNode n = rn[j];
                 const int w = max(max(gs.lay[0][(n.xyz & 1023) + kx], gs.lay[1][((n.xyz >> 10) & 1023) + ky]),
                                   gs.lay[2][(n.xyz >> 20) + kz]);
                 const unsigned dec = release_dec(w, n.inst, rw, &ws.t[n.slot][13]);
-                if (dec) release_one(sd, sh, n.p + off, own_face(w), dec, keyq, nkey);
+                if (dec) release_one(sd, sh, n.p + off, n.xyz + oxyz, own_face(w), dec, keyq, nkey);
             }
         }
     } else if (sh.single) {
@@ -1197,6 +1204,8 @@ __device__ void graph_release(const fd_station_dev &sd, Shared &sh, WarpSmem &ws
             const GRect r = gs.rect[wh.inst];
             const int su = (int)t_stride(sd, fr.axis_u), sv = (int)t_stride(sd, fr.axis_v);
             const int p = (int)wh.p, pn = p - fr.inner * (int)t_stride(sd, fr.axis_n);
+            const int hu = 1 << (10 * fr.axis_u), hv = 1 << (10 * fr.axis_v);   /* steps of packed coordinates */
+            const int xyz = pack_xyz(wh.x, wh.y, wh.z), xyzn = xyz - fr.inner * (1 << (10 * fr.axis_n));
             const float *t13 = &ws.t[lane][13];
             const unsigned own = okey32(*t13);
             /* columns (bits 0-2) and rows (3-5) of the 3x3 block inside a rectangle */
@@ -1207,16 +1216,16 @@ __device__ void graph_release(const fd_station_dev &sd, Shared &sh, WarpSmem &ws
                        | (v >= q.vlo && v <= q.vhi ? 16u : 0u) | (v + 1 >= q.vlo && v + 1 <= q.vhi ? 32u : 0u);
             };
             const unsigned mine = inside(r);
-            const bool adj = wh.inst + 1 < sh.ninst && gs.rect[wh.inst + 1].layer == r.layer - fr.inner;
+            const bool adj = wh.inst + 1 < sh.ninst && gs.rect[wh.inst + 1].layer() == r.layer() - fr.inner;
             const unsigned next = adj ? inside(gs.rect[wh.inst + 1]) : 0u;
 #pragma unroll
             for (int k = 0; k < 9; k++) {
                 const int du = k % 3 - 1, dv = k / 3 - 1;
                 const unsigned bits = 1u << (du + 1) | 8u << (dv + 1);
-                const int o = du * su + dv * sv;
-                if ((next & bits) == bits) release_one(sd, sh, pn + o, F, 1u, keyq, nkey);
+                const int o = du * su + dv * sv, oh = du * hu + dv * hv;
+                if ((next & bits) == bits) release_one(sd, sh, pn + o, xyzn + oh, F, 1u, keyq, nkey);
                 if (k != 4 && (mine & bits) == bits && later_key(okey32(t13[dv * 3 + du]), own, du, dv))
-                    release_one(sd, sh, p + o, F, 1u << 8, keyq, nkey);
+                    release_one(sd, sh, p + o, xyz + oh, F, 1u << 8, keyq, nkey);
             }
         }
     } else {
@@ -1228,7 +1237,7 @@ __device__ void graph_release(const fd_station_dev &sd, Shared &sh, WarpSmem &ws
                 ly[k] = gs.lay[1][wh.y + k];
                 lz[k] = gs.lay[2][wh.z + k];
             }
-            const int p = (int)wh.p, nxy = nx * ny;
+            const int p = (int)wh.p, nxy = nx * ny, xyz = pack_xyz(wh.x, wh.y, wh.z);
             const float *t13 = &ws.t[lane][13];
 #pragma unroll
             for (int k = 0; k < 27; k++) {
@@ -1236,21 +1245,21 @@ __device__ void graph_release(const fd_station_dev &sd, Shared &sh, WarpSmem &ws
                 const int w = max(max(lx[k % 3], ly[(k / 3) % 3]), lz[k / 9]);
                 const unsigned dec = release_dec(w, wh.inst, sh.rel[F][k], t13);
                 if (dec)
-                    release_one(sd, sh, p + (k / 9 - 1) * nxy + ((k / 3) % 3 - 1) * nx + k % 3 - 1, own_face(w), dec, keyq,
-                                nkey);
+                    release_one(sd, sh, p + (k / 9 - 1) * nxy + ((k / 3) % 3 - 1) * nx + k % 3 - 1,
+                                xyz + (k / 9 - 1) * (1 << 20) + ((k / 3) % 3 - 1) * 1024 + k % 3 - 1, own_face(w), dec,
+                                keyq, nkey);
             }
         }
     }
     __syncwarp();
     wfence(sh);
+    if (was & FD_WAITB) wake_waiters(sd, sh, (int)wh.p);
     /* inner blocks now complete: these nodes' keys and in-face order are known */
     const int nk = *nkey;
     for (int j = lane; j < nk; j += 32) {
         const int q = keyq[j];
-        const int qxy = q / nx, qx = q - qxy * nx, qz = qxy / ny, qy = qxy - qz * ny;
-        const int w = owner_of(gs, qx, qy, qz);
-        if (ready_word(key_event(sd, sh, own_inst(w), inst_fill(gs.rect[own_inst(w)], qx, qy, qz), q)))
-            graph_ready(sd, sh, own_face(w), q);
+        const int w = owner_of(gs, q & 1023, (q >> 10) & 1023, q >> 20);
+        if (ready_word(key_event(sd, sh, own_inst(w), q, node_of(sd, q)))) graph_ready(sd, sh, own_face(w), q);
     }
     __syncwarp();
 }
@@ -1323,7 +1332,7 @@ __device__ __forceinline__ bool head_wave(double num, double den)
  * returns false without committing. */
 __device__ bool commit_node(const fd_station_dev &sd, Shared &sh, const TrialDesc *dsc, WarpSmem &ws, int slot,
                             int F, const Where &wh, unsigned gm, unsigned em, float it0, float it4, bool permissive,
-                            unsigned char *dag, Counters cn)
+                            unsigned char *dag, unsigned &was, Counters cn)
 {
     const float *t18 = ws.t[slot], *s18 = ws.s[slot];
     const double told = f2d(t18[NB_POINT]);
@@ -1371,13 +1380,13 @@ __device__ bool commit_node(const fd_station_dev &sd, Shared &sh, const TrialDes
     }
     const float st0 = writer < 0 ? it0 : t18[dsc[writer].slot[0]], st4 = writer < 0 ? it4 : t18[dsc[writer].slot[4]];
     if (sh.graph)
-        graph_record(sd, sh, wh.p, wh.inst, wh.i, writer >= 0, st0, st4, t18[13]);
+        was = graph_record(sd, sh, wh.p, wh.inst, wh.i, writer >= 0, st0, st4, t18[13]);
     else
         face_release(sd, sh, dag, wh.i, writer >= 0, st0, st4);
     return true;
 }
 
-/* where the node of queue entry e lies: a fill index in a face walk, a grid index in a graph;
+/* where the node of queue entry e lies: a fill index in a face walk, packed coordinates in a graph;
  * ok false for a graph node no instance owns */
 __device__ __forceinline__ Where locate(const fd_station_dev &sd, const Shared &sh, int F, int e, bool &ok)
 {
@@ -1385,22 +1394,21 @@ __device__ __forceinline__ Where locate(const fd_station_dev &sd, const Shared &
     Where wh;
     ok = true;
     if (sh.graph) {
-        wh.p = e;
-        const int nx = sd.g.nx, ny = sd.g.ny, exy = e / nx;
-        wh.x = e - exy * nx;
-        wh.z = exy / ny;
-        wh.y = exy - wh.z * ny;
+        wh.p = node_of(sd, e);
+        wh.x = e & 1023;
+        wh.y = (e >> 10) & 1023;
+        wh.z = e >> 20;
         const int w = owner_of(gsmem(sh), wh.x, wh.y, wh.z);
         if (w < 0) {
             ok = false;
             return wh;
         }
         wh.inst = own_inst(w);
-        const GRect &gr = gsmem(sh).rect[wh.inst];
+        const GRect gr = gsmem(sh).rect[wh.inst];
         wh.r.u = coord(fr.axis_u, wh.x, wh.y, wh.z);
         wh.r.v = coord(fr.axis_v, wh.x, wh.y, wh.z);
         wh.r.ulo = gr.ulo; wh.r.uhi = gr.uhi; wh.r.vlo = gr.vlo; wh.r.vhi = gr.vhi;
-        wh.i = inst_fill(gr, wh.x, wh.y, wh.z);
+        wh.i = (wh.r.v - gr.vlo) * gr.nuf() + wh.r.u - gr.ulo;
     } else {
         wh.i = e;
         wh.inst = -1;
@@ -1478,6 +1486,9 @@ __device__ void warp_chunk(const fd_station_dev &sd, Shared &sh, const CtaSmem &
             if (t[nb] < 1.e9f) below |= 1u << nb;
         }
         guards(F, t, below, wh.r, gm, em);
+        /* the point's step lengths along x and y for the 1-D bounds (see stale_pair) */
+        ws.s0[lane] = d2f_trunc(node_row(sd.g, wh.z, wh.y)[FD_N_RSDF]);
+        ws.s4[lane] = d2f_trunc(sd.g.zrow[(long long)(FD_OK(wh.z, sd.g.nz, 8) ? wh.z : 0) * FD_Z_N + FD_Z_RDQ]);
         if (em & 0xF0u) em = ne_prune(dsc, tr, em);
         /* a 2-D trial before any corner / new-edge call reads the state an earlier point left */
         permissive = !have_inherit && (gm & 0xFu) == 0 && !((gm & 0xF0u) && t[NB_POINT] > 1.0e9f) && (gm & 0xFF00u);
@@ -1507,8 +1518,9 @@ __device__ void warp_chunk(const fd_station_dev &sd, Shared &sh, const CtaSmem &
     FD_TOC(2, tb);
     FD_TIC(tc);
     bool fin = false;
+    unsigned was = 0;   /* graph_record's word */
     if (valid) {
-        fin = commit_node(sd, sh, dsc, ws, lane, F, wh, gm, em, p0, p4, permissive, dag, cn);
+        fin = commit_node(sd, sh, dsc, ws, lane, F, wh, gm, em, p0, p4, permissive, dag, was, cn);
         if (!fin) {
             atomicAdd(reinterpret_cast<unsigned long long *>(&sh.w.deferred), 1ull);
             if (sh.nodefer)
@@ -1517,7 +1529,7 @@ __device__ void warp_chunk(const fd_station_dev &sd, Shared &sh, const CtaSmem &
                 enqueue_to(sh.graph ? sd.scr.grq : sd.scr.rq, sh.w.rqtail, sh.w.rqcap, sh, e);
         }
     }
-    if (sh.graph) graph_release(sd, sh, ws, F, fin, wh);
+    if (sh.graph) graph_release(sd, sh, ws, F, fin, was, wh);
     if (sh.graph && !sh.nodefer) {
         /* points done per face instance, one atomic per instance in the chunk; the instance
          * complete wakes points waiting for its last writer */
@@ -1525,7 +1537,7 @@ __device__ void warp_chunk(const fd_station_dev &sd, Shared &sh, const CtaSmem &
         const unsigned peers = __match_any_sync(0xffffffffu, key);
         if (fin && lane == __ffs(peers) - 1) {
             const int c = __popc(peers);
-            const int old = atomicAdd(&sd.scr.ginst[key].ndone, c);
+            const int old = atomicAdd(&gsmem(sh).ndone[key], c);
             if (old + c == rect_n(gsmem(sh).rect[key])) fire_event(sd, sh, key, 2);
         }
     }
@@ -1608,39 +1620,37 @@ FD_COLD bool resume_waiter(const fd_station_dev &sd, Shared &sh, int w, float *s
     return false;
 }
 
-/* Sweep graph: the same search for point w (a grid index), by the reference's order of face
+/* Sweep graph: the same search for point w (packed coordinates), by the reference's order of face
  * instances and, within one, of keys.  Registers w on an instance event or a point when the
  * answer is not yet known.  One warp; true with the state and w's face when found. */
 FD_COLD bool resume_graph(const fd_station_dev &sd, Shared &sh, int w, float *st0, float *st4, int *face)
 {
     const int lane = threadIdx.x & 31;
     const GraphSmem gs = gsmem(sh);
-    const int nx = sd.g.nx, ny = sd.g.ny;
-    if (!FD_OK(w, (long long)sd.g.nx * sd.g.ny * sd.g.nz, 20)) return false;
-    const int wxy = w / nx;
-    const int wx = w - wxy * nx, wy = wxy % ny, wz = wxy / ny;
+    const int wx = w & 1023, wy = (w >> 10) & 1023, wz = w >> 20;
     const int ow = owner_of(gs, wx, wy, wz);
     if (ow < 0) {
         if (lane == 0) atomicCAS(&sh.w.status, 0, 14);
         return false;
     }
     const int I = own_inst(ow);
-    const GRect &r = gs.rect[I];
-    const int n = rect_n(r);
-    if (vload(sd.scr.ginst[I].nkeyed) < n) {   /* keys below w's not all known yet */
+    const GRect r = gs.rect[I];
+    const int n = rect_n(r), nuf = r.nuf();
+    if (vload(gs.nkeyed[I]) < n) {   /* keys below w's not all known yet */
         if (lane == 0) wait_event(sd, sh, w, I, 1);
         return false;
     }
-    const unsigned long long kc = inst_key(sd, r, inst_fill(r, wx, wy, wz));
-    const fdn_frame fr = frame_of(r.face);
+    const fdn_frame fr = frame_of(r.face());
     const int su = (int)t_stride(sd, fr.axis_u), sv = (int)t_stride(sd, fr.axis_v);
-    const int base = (int)inst_node(sd, r, 0), in = fr.inner * (int)t_stride(sd, fr.axis_n);
-    const int dv = 32 / r.nuf, du = 32 - dv * r.nuf;   /* 32 points on in fill order */
+    const int base = inst_node(sd, r, 0), in = fr.inner * (int)t_stride(sd, fr.axis_n);
+    const int wu = coord(fr.axis_u, wx, wy, wz) - r.ulo, wv = coord(fr.axis_v, wx, wy, wz) - r.vlo;
+    const unsigned long long kc = node_key(vload(sd.T[base + wu * su + wv * sv + in]), wv * nuf + wu);
+    const int dv = 32 / nuf, du = 32 - dv * nuf;   /* 32 points on in fill order */
     for (int guard = 0; guard <= 2 * n + 2; guard++) {
         /* among the instance's earlier points: the last writer that is done, and the last point that is
          * not (it may yet be a writer); four points a lane at a time, so that their loads overlap */
         unsigned long long done = 0ull, pend = 0ull;
-        int u = lane % r.nuf, v = lane / r.nuf;
+        int v = lane / nuf, u = lane - v * nuf;
         for (int j0 = lane; j0 < n; j0 += 128) {
             int q[4];
             unsigned long long key[4];
@@ -1649,10 +1659,10 @@ FD_COLD bool resume_graph(const fd_station_dev &sd, Shared &sh, int w, float *st
             for (int k = 0; k < 4; k++) {
                 q[k] = base + u * su + v * sv;
                 const int j = j0 + 32 * k;
-                key[k] = j < n ? node_key(vload(sd.T[q[k] + in]), j) : ~0ull;
+                key[k] = j < n ? node_key(sd.T[q[k] + in], j) : ~0ull;   /* final: every key is */
                 u += du;
                 v += dv;
-                if (u >= r.nuf) { u -= r.nuf; v++; }
+                if (u >= nuf) { u -= nuf; v++; }
             }
 #pragma unroll
             for (int k = 0; k < 4; k++) cnt[k] = key[k] < kc ? vload(sd.scr.gcnt[q[k]]) : 0u;
@@ -1685,7 +1695,7 @@ FD_COLD bool resume_graph(const fd_station_dev &sd, Shared &sh, int w, float *st
                 verdict = 1;
                 for (int J = I - 1; J >= 0; J--) {
                     const GRect &rj = gs.rect[J];
-                    if (vload(sd.scr.ginst[J].ndone) < rect_n(rj)) { wait_event(sd, sh, w, J, 2); verdict = 2; break; }
+                    if (vload(gs.ndone[J]) < rect_n(rj)) { wait_event(sd, sh, w, J, 2); verdict = 2; break; }
                     wfence(sh);
                     const unsigned long long ek = vload(sd.scr.ginst[J].exitkey);
                     if (ek) {
@@ -1703,7 +1713,7 @@ FD_COLD bool resume_graph(const fd_station_dev &sd, Shared &sh, int w, float *st
         if (verdict == 1) {
             *st0 = __shfl_sync(0xffffffffu, t0, 0);
             *st4 = __shfl_sync(0xffffffffu, t4, 0);
-            *face = r.face;
+            *face = r.face();
             return true;
         }
     }
@@ -1761,94 +1771,83 @@ __device__ void run_walk(const fd_station_dev &sd, Shared &sh, const CtaSmem &cs
     long long chunks = 0;
     unsigned idle_polls = 0;
     for (;;) {
-        int act = 0, h = 0, m = 0, qf = 0;   /* act: 0 wait, 1 chunk, 2 resume a waiter, 3 leave */
-        if (lane == 0) {
-            if (vload(sh.w.status) != 0 || vload(sh.w.ndone) >= total) {
-                act = 3;
-            } else {
-                const int rh = vload(sh.w.rqhead), rt0 = vload(sh.w.rqtail), rt = rt0 < sh.w.rqcap ? rt0 : sh.w.rqcap;
-                if (rh < rt) {
-                    if (idle) { atomicSub(&sh.w.idle, 1); idle = false; }
-                    if (atomicCAS(&sh.w.rqhead, rh, rh + 1) == rh) { act = 2; h = read_entry(rq, rh, sh); }
-                } else {
-                    /* the fullest queue, starting the scan at a warp-dependent face */
-                    int best = -1, bavail = 0, bhead = 0;
-                    for (int k0 = 0; k0 < sh.w.nq; k0++) {
-                        const int k = (k0 + warp) % sh.w.nq;
-                        const int hd = vload(sh.w.qhead[k]), qt = vload(sh.w.qtail[k]);
-                        const int tl = qt < sh.w.qcap[k] ? qt : sh.w.qcap[k];
-                        if (tl - hd > bavail) { bavail = tl - hd; best = k; bhead = hd; }
-                    }
-                    if (best >= 0) {
-                        if (idle) { atomicSub(&sh.w.idle, 1); idle = false; }
-                        const int want = bavail < 32 ? bavail : 32;
-                        if (atomicCAS(&sh.w.qhead[best], bhead, bhead + want) == bhead) {
-                            act = 1; h = sh.w.qbase[best] + bhead; m = want; qf = best;
-                        }
-                    } else {
-                        if (!idle) { wfence(sh); atomicAdd(&sh.w.idle, 1); idle = true; idle_polls = 0; }
-                        /* all idle with nothing queued and nodes left: nothing can release them.  The
-                         * check (two fences and a scan of every queue) runs on every 64th idle poll
-                         * only: idle warps are most of the CTA in a forward sweep, and their polls
-                         * share the SM's shared-memory pipe with the working warps */
-                        if ((++idle_polls & 63u) == 0u && quiescent(sh) && vload(sh.w.ndone) < total) {
-                            atomicCAS(&sh.w.status, 0, 3);
-                            act = 3;
-                        }
-                    }
-                }
-                if (act == 1 || act == 2) {
-                    since = clock64();
-                } else if (act == 0 && clock64() - since > wait_lim) {
-                    atomicCAS(&sh.w.status, 0, 8);   /* no work for this worker for too long */
-                    act = 3;
-                }
-                if (act != 3 && clock64() - started > walk_lim) {
-                    atomicCAS(&sh.w.status, 0, 17);   /* the walk as a whole ran far too long */
-                    act = 3;
-                }
-            }
+        /* One look at all counters, a queue per lane (0-5 ready nodes by face, 6 resuming points): what every
+         * chunk of a latency-bound sweep waits for, so it is kept to a few dozen instructions (a
+         * loop over the queues in lane 0 took about 400). */
+        int hd = 0, avail = 0;
+        bool stop = false;
+        if (lane < 6) {
+            hd = vload(sh.w.qhead[lane]);
+            const int qt = vload(sh.w.qtail[lane]);
+            avail = min(qt, sh.w.qcap[lane]) - hd;
+        } else if (lane == 6) {
+            hd = vload(sh.w.rqhead);
+            const int qt = vload(sh.w.rqtail);
+            avail = min(qt, sh.w.rqcap) - hd;
+        } else if (lane == 7) {
+            stop = vload(sh.w.status) != 0 || vload(sh.w.ndone) >= total;
         }
-        act = __shfl_sync(0xffffffffu, act, 0);
-        if (act == 3) break;
-        h = __shfl_sync(0xffffffffu, h, 0);
+        if (__any_sync(0xffffffffu, stop)) break;
+        /* resuming points first, else the fullest queue, ties in a warp-dependent order */
+        const int pref = avail <= 0 ? 0 : lane == 6 ? 0x7fffffff : lane < 6 ? avail << 3 | ((lane + warp) & 7) : 0;
+        const int best = __reduce_max_sync(0xffffffffu, pref);
+        int act = 0, h = 0, m = 0, qf = 0;   /* act: 0 nothing, 1 chunk, 2 resume a waiter */
+        if (best) {
+            qf = __ffs(__ballot_sync(0xffffffffu, pref == best)) - 1;
+            if (idle && lane == 0) atomicSub(&sh.w.idle, 1);
+            idle = false;
+            if (lane == qf) {
+                m = lane == 6 ? 1 : min(avail, 32);
+                int *head = lane == 6 ? &sh.w.rqhead : &sh.w.qhead[lane];
+                if (atomicCAS(head, hd, hd + m) == hd) act = lane == 6 ? 2 : 1;
+                h = lane == 6 ? hd : sh.w.qbase[lane] + hd;
+            }
+            act = __shfl_sync(0xffffffffu, act, qf);
+            h = __shfl_sync(0xffffffffu, h, qf);
+            m = __shfl_sync(0xffffffffu, m, qf);
+        } else {
+            if (!idle) {
+                wfence(sh);
+                if (lane == 0) atomicAdd(&sh.w.idle, 1);
+                idle = true;
+                idle_polls = 0;
+            }
+            /* all idle with nothing queued and nodes left: nothing can release them.  The
+             * check (two fences and a scan of every queue) runs on every 64th idle poll
+             * only: idle warps are most of the CTA in a forward sweep, and their polls
+             * share the SM's shared-memory pipe with the working warps */
+            if ((++idle_polls & 63u) == 0u && lane == 0 && quiescent(sh) && vload(sh.w.ndone) < total)
+                atomicCAS(&sh.w.status, 0, 3);
+        }
+        if (lane == 0) {
+            const long long now = clock64();
+            if (act) since = now;
+            else if (now - since > wait_lim) atomicCAS(&sh.w.status, 0, 8);   /* no work for this worker for too long */
+            if (now - started > walk_lim) atomicCAS(&sh.w.status, 0, 17);     /* the walk as a whole ran far too long */
+        }
+        if (!act) {
+            if (!best) __nanosleep(64);
+            continue;
+        }
         int e = -1, face = sh.face;
         float in0 = 0.f, in4 = 0.f;
+        if (lane < m) {
+            e = read_entry((act == 1 ? queue : rq) + h, lane, sh);
+            /* an entry outside the walk's nodes ends the walk with a status instead of an access */
+            const bool ok = sh.graph ? (e & 1023) < sd.g.nx && ((e >> 10) & 1023) < sd.g.ny && (e >> 20) < sd.g.nz : e < sh.n;
+            if (e >= 0 && !ok) {
+                (void)FD_OK(e, 0, 23);
+                atomicCAS(&sh.w.status, 0, 18);
+                e = -1;
+            }
+        }
+        wfence(sh);
         if (act == 1) {
-            m = __shfl_sync(0xffffffffu, m, 0);
-            qf = __shfl_sync(0xffffffffu, qf, 0);
             if (sh.graph) face = qf;
-            if (lane < m) {
-                const volatile int *q = queue + h + lane;
-                e = *q;
-                for (int spin = 0; e < 0 && spin < FD_QSPIN; spin++) {
-                    __nanosleep(32);
-                    e = *q;
-                }
-                if (e < 0) atomicCAS(&sh.w.status, 0, 9);   /* a claimed entry never written */
-                /* an entry outside the walk's nodes ends the walk with a status instead of an access */
-                const long long bound = sh.graph ? (long long)sd.g.nx * sd.g.ny * sd.g.nz : (long long)sh.n;
-                if (e >= bound) {
-                    (void)FD_OK(e, bound, 23);
-                    atomicCAS(&sh.w.status, 0, 18);
-                    e = -1;
-                }
-            }
-            wfence(sh);
             chunks++;
-        } else if (act == 2) {
-            wfence(sh);
-            const long long bound = sh.graph ? (long long)sd.g.nx * sd.g.ny * sd.g.nz : (long long)sh.n;
-            if (h >= bound) {
-                (void)FD_OK(h, bound, 24);
-                if (lane == 0) atomicCAS(&sh.w.status, 0, 18);
-                h = -1;
-            }
-            if (h < 0 || !(sh.graph ? resume_graph(sd, sh, h, &in0, &in4, &face) : resume_waiter(sd, sh, h, &in0, &in4))) continue;
-            if (lane == 0) e = h;
         } else {
-            __nanosleep(64);
-            continue;
+            h = __shfl_sync(0xffffffffu, e, 0);
+            if (h < 0 || !(sh.graph ? resume_graph(sd, sh, h, &in0, &in4, &face) : resume_waiter(sd, sh, h, &in0, &in4))) continue;
         }
         warp_chunk(sd, sh, cs, ws, face, e, act == 2, in0, in4, dag, cn);
     }
@@ -1990,14 +1989,12 @@ __device__ void graph_sweep(const fd_station_dev &sd, Shared &sh, CtaSmem &cs, W
                     if (sh.n > 0) {
                         if (ninst >= cap) { over = true; break; }
                         fd_ginst &gi = sd.scr.ginst[ninst];
-                        gi.face = face; gi.layer = sh.layer;
-                        gi.ulo = sh.ulo; gi.uhi = sh.uhi; gi.vlo = sh.vlo; gi.vhi = sh.vhi;
-                        gi.nuf = sh.nuf; gi.n = sh.n;
-                        gi.nkeyed = 0; gi.ndone = 0; gi.ev[0] = gi.ev[1] = FD_EV_NONE; gi.exitkey = 0ull;
+                        gi.ev[0] = gi.ev[1] = FD_EV_NONE; gi.exitkey = 0ull;
                         GRect &gr = gs.rect[ninst];
-                        gr.face = (short)face; gr.layer = (short)sh.layer;
+                        gr.fl = (short)(sh.layer << 3 | face);
                         gr.ulo = (short)sh.ulo; gr.uhi = (short)sh.uhi; gr.vlo = (short)sh.vlo; gr.vhi = (short)sh.vhi;
-                        gr.nuf = (short)sh.nuf; gr.pad = 0;
+                        gs.nkeyed[ninst] = 0;
+                        gs.ndone[ninst] = 0;
                         gs.lay[frame_of(face).axis_n][sh.layer + 1] = (short)((ninst << 3) | face);
                         ninst++;
                         M += sh.n;
@@ -2057,18 +2054,18 @@ __device__ void graph_sweep(const fd_station_dev &sd, Shared &sh, CtaSmem &cs, W
         /* dependency counters */
         for (int I = 0; I < ninst; I++) {
             const GRect r = gs.rect[I];
-            const fdn_frame fr = frame_of(r.face);
-            const int n = rect_n(r), nvf = r.vhi - r.vlo + 1;
-            const unsigned myctx = sh.ctxm[r.face], myinn = sh.innm[r.face];
-            const bool prev = sh.single && I > 0 && gs.rect[I - 1].layer == r.layer + fr.inner;
+            const fdn_frame fr = frame_of(r.face());
+            const int n = rect_n(r), nuf = r.nuf(), nvf = r.vhi - r.vlo + 1;
+            const unsigned myctx = sh.ctxm[r.face()], myinn = sh.innm[r.face()];
+            const bool prev = sh.single && I > 0 && gs.rect[I - 1].layer() == r.layer() + fr.inner;
             for (int j = tid; j < n; j += blockDim.x) {
-                const long long p = inst_node(sd, r, j);
+                const int xyz = inst_xyz(r, j), p = node_of(sd, xyz);
                 if (!FD_OK(p, (long long)nx * ny * nz, 25)) continue;
                 unsigned cin = 0, c2 = 0, cx = 0;
                 if (sh.single) {
                     /* one face: the same-instance neighbours and the previous plane's inner block */
-                    const int iu = j % r.nuf, iv = j / r.nuf;
-                    c2 = (unsigned)__popc(inrect_mask(iu, iv, r.nuf, nvf));
+                    const int iv = j / nuf, iu = j - iv * nuf;
+                    c2 = (unsigned)__popc(inrect_mask(iu, iv, nuf, nvf));
                     if (prev) {
                         const GRect &rp = gs.rect[I - 1];
                         const int u0 = r.ulo + iu, v0 = r.vlo + iv;
@@ -2077,8 +2074,7 @@ __device__ void graph_sweep(const fd_station_dev &sd, Shared &sh, CtaSmem &cs, W
                                 if (u0 + du >= rp.ulo && u0 + du <= rp.uhi && v0 + dv >= rp.vlo && v0 + dv <= rp.vhi) cin++;
                     }
                 } else {
-                    const int pi = (int)p, pxy = pi / nx;
-                    const int x = pi - pxy * nx, z = pxy / ny, y = pxy - z * ny;
+                    const int x = xyz & 1023, y = (xyz >> 10) & 1023, z = xyz >> 20;
                     int lx[3], ly[3], lz[3];
 #pragma unroll
                     for (int k = 0; k < 3; k++) {
@@ -2105,8 +2101,8 @@ __device__ void graph_sweep(const fd_station_dev &sd, Shared &sh, CtaSmem &cs, W
             const GRect r = gs.rect[I];
             const int n = rect_n(r);
             for (int j = tid; j < n; j += blockDim.x) {
-                const long long p = inst_node(sd, r, j);
-                if ((sd.scr.gcnt[p] & 0xFFu) == 0u && ready_word(key_event(sd, sh, I, j, p))) graph_ready(sd, sh, r.face, p);
+                const int xyz = inst_xyz(r, j), p = node_of(sd, xyz);
+                if ((sd.scr.gcnt[p] & 0xFFu) == 0u && ready_word(key_event(sd, sh, I, xyz, p))) graph_ready(sd, sh, r.face(), xyz);
             }
         }
         csync(sh);

@@ -75,11 +75,8 @@ typedef struct {
     int32_t sm;              /* the SM whose CTA ran the solve */
 } fd_station_stats;
 
-/* One face instance of a sweep graph: a face walked at one wall position, with its point
- * rectangle and its completion state. */
+/* One face instance of a sweep graph (a face walked at one wall position): what its points leave and wait for */
 typedef struct {
-    int face, layer, ulo, uhi, vlo, vhi, nuf, n;
-    int nkeyed, ndone;             /* points whose sort key is final; points done */
     int ev[2];                     /* events "all keys final", "all points done": the first parked
                                       point waiting for it (gpark index), FD_EV_NONE, FD_EV_FIRED */
     unsigned long long exitkey;    /* largest key of a point that made a writer call (0: none) */
