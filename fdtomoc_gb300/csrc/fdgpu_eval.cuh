@@ -35,19 +35,15 @@ namespace fdk {
 /* ---------------------------------------------------------------------------------------------- */
 /* exact helpers                                                                                   */
 
-/* float -> double on the integer pipe (normal numbers and zeros; anything else converts normally) */
+/* The solver's code is several times the SM's instruction caches, so the helpers that are inlined in dozens of
+ * places are kept as short as they can be: one test for the operands that need the general instruction. */
+
+/* float -> double on the integer pipe (normal numbers; zeros and anything else convert normally) */
 __device__ __forceinline__ double f2d(float f)
 {
     const unsigned b = __float_as_uint(f);
-    const unsigned e = (b >> 23) & 0xffu;
-    if (e - 1u < 254u) {
-        const unsigned long long d = ((unsigned long long)(b & 0x80000000u) << 32)
-                                     | ((unsigned long long)(e + 896u) << 52)
-                                     | ((unsigned long long)(b & 0x7fffffu) << 29);
-        return __longlong_as_double((long long)d);
-    }
-    if ((b << 1) == 0u) return __longlong_as_double((long long)((unsigned long long)(b & 0x80000000u) << 32));
-    return (double)f;
+    if (((b >> 23) & 0xffu) - 1u >= 254u) return (double)f;
+    return __hiloint2double((int)(((b & 0x7fffffffu) >> 3) + 0x38000000u | (b & 0x80000000u)), (int)(b << 29));
 }
 
 /* Comparisons of finite doubles on the integer pipe (an FP64 compare occupies this GPU's FP64 unit
@@ -72,13 +68,13 @@ __device__ __forceinline__ bool not_ge0(double x)
 }
 
 /* x * 2^k, exact: exponent arithmetic on the integer pipe when x and the result are normal;
- * zeros and subnormals take the floating-point multiply (never reached with physical inputs) */
+ * zeros and subnormals take the floating-point multiply */
 template <int K>
 __device__ __forceinline__ double scale2k(double x)
 {
-    const long long b = __double_as_longlong(x);
-    const int e = (int)((b >> 52) & 0x7ff);
-    if (e != 0 && e + K >= 1 && e + K <= 2046) return __longlong_as_double(b + ((long long)K << 52));
+    const int hi = __double2hiint(x), e = (hi >> 20) & 0x7ff;
+    constexpr int lo = K < 0 ? 1 - K : 1, n = 2046 - (K > 0 ? K : 0) - lo;
+    if ((unsigned)(e - lo) <= (unsigned)n) return __hiloint2double(hi + K * (1 << 20), __double2loint(x));
     constexpr double p2 = K >= 0 ? (double)(1ll << (K >= 0 ? K : 0)) : 1.0 / (double)(1ll << (K < 0 ? -K : 0));
     return x * p2;
 }
@@ -87,12 +83,12 @@ __device__ __forceinline__ double scale2k(double x)
  * its sign, as a true division would. */
 __device__ __forceinline__ double div_rn(double x, double d, double inv)
 {
-    if ((__double_as_longlong(x) << 1) == 0) return __dmul_rn(x, inv);
-    double q = __dmul_rn(x, inv);
-    double e = __fma_rn(-d, q, x);
-    q = __fma_rn(e, inv, q);
+    const double q0 = __dmul_rn(x, inv);
+    double e = __fma_rn(-d, q0, x);
+    const double q = __fma_rn(e, inv, q0);
     e = __fma_rn(-d, q, x);
-    return __fma_rn(e, inv, q);
+    const double r = __fma_rn(e, inv, q);
+    return (__double_as_longlong(x) << 1) == 0 ? q0 : r;
 }
 
 /* ---------------------------------------------------------------------------------------------- */

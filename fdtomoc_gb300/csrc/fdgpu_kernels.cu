@@ -479,11 +479,9 @@ constexpr unsigned k1d = 0x1Fu << TK_1D0;
  * a new-edge or a 2-D trial.  That is the right form for a warp full of items.  A chunk of a forward
  * sweep has one to five corners and rarely more than one of the others; there four lanes share an
  * item, each taking the products, divisions or sums that do not depend on one another, in the
- * reference's order within every sum: 49 and 38 instructions for up to eight items.  FD_QUAD is where
- * two such passes would cost as much as one of the other form. */
-#ifndef FD_QUAD
+ * reference's order within every sum: 49 and 38 instructions for up to eight items (two such passes for
+ * nine to sixteen corners cost as much as one of the other form). */
 #define FD_QUAD 8
-#endif
 
 __device__ __forceinline__ double shfl_d(double x, int src) { return __shfl_sync(0xffffffffu, x, src); }
 
@@ -632,49 +630,32 @@ __device__ void eval_edges_quad(const fd_station_dev &sd, const TrialDesc *dsc, 
 
 /* Evaluate items[0..n), all corner trials (kind 0), new-edge (1), 2-D (2) or 1-D (4), with the warp's lanes; a
  * 2-D value is stored after the causality selection against its floor, which includes the stencil
- * state entering the 2-D block (src/sphfd.c:6116-6121) */
+ * state entering the 2-D block (src/sphfd.c:6116-6121).  Corners come in warps: whole warps of them, and a
+ * remainder above FD_QUAD, take a lane each.  New-edge and 2-D items are rarely more than eight. */
 template <int KIND>
 __device__ __forceinline__ void eval_items(const fd_station_dev &sd, const TrialDesc *dsc, WarpSmem &ws,
                                            const unsigned short *items, int n, int lane)
 {
+    if (n == 0) return;
     if (lane == 0) ws.cnt[KIND] += (unsigned)n;
-    int j0 = 0;
-    if constexpr (KIND < 3) {
-        const int rest = n & 31;   /* whole warps of items, and a remainder above FD_QUAD, one lane each */
-        if (rest && rest <= FD_QUAD) {
-            for (; j0 < rest; j0 += 8) {
-                const int m = rest - j0 < 8 ? rest - j0 : 8;
-                if constexpr (KIND == 0) eval_corners_quad(sd, dsc, ws, items + j0, m, lane);
-                else eval_edges_quad(sd, dsc, ws, items + j0, m, lane);
-            }
-            j0 = rest;
-        }
-    }
-    for (int j = j0 + lane; j < n; j += 32) {
-        const unsigned it = items[j];
-        const int slot = (int)(it >> 5), K = (int)(it & 31);
-        const TrialDesc &d = dsc[K];
-        const int z = ws.z[slot], y = ws.y[slot];
-        const float *t18 = ws.t[slot], *s18 = ws.s[slot];
-        double v;
+    if constexpr (KIND == 1 || KIND == 2) {
+        for (int j0 = 0; j0 < n; j0 += 8) eval_edges_quad(sd, dsc, ws, items + j0, n - j0 < 8 ? n - j0 : 8, lane);
+    } else {
+        int j0 = 0;
         if constexpr (KIND == 0) {
-            v = eval_3d(d, t18, s18, sd.g, z, y);
-        } else if constexpr (KIND == 1) {
-            v = eval_ne(d, t18, s18, sd.g, z, y);
-        } else if constexpr (KIND == 2) {
-            double x1, x2;
-            eval_2d(d, t18, s18, sd.g, z, y, x1, x2);
-            if ((__double_as_longlong(x1) & 0x7fffffffffffffffll) > 0x7ff0000000000000ll) {   /* NaN: no root */
-                v = 1.e11;
-            } else {
-                const float fl = fmaxf(fmaxf(fmaxf(t18[d.slot[1]], t18[d.slot[2]]), fmaxf(t18[d.slot[3]], ws.s0[slot])),
-                                       ws.s4[slot]);
-                v = pick_2(x1, x2, f2d(fl));
+            const int rest = n & 31;
+            if (rest && rest <= FD_QUAD) {
+                eval_corners_quad(sd, dsc, ws, items, rest, lane);
+                j0 = rest;
             }
-        } else {
-            v = eval_1d(d, t18, s18, sd.g, z, y);
         }
-        ws.res[slot][K] = v;
+        for (int j = j0 + lane; j < n; j += 32) {
+            const unsigned it = items[j];
+            const int slot = (int)(it >> 5), K = (int)(it & 31);
+            const int z = ws.z[slot], y = ws.y[slot];
+            if constexpr (KIND == 0) ws.res[slot][K] = eval_3d(dsc[K], ws.t[slot], ws.s[slot], sd.g, z, y);
+            else ws.res[slot][K] = eval_1d(dsc[K], ws.t[slot], ws.s[slot], sd.g, z, y);
+        }
     }
 }
 
@@ -1230,24 +1211,30 @@ __device__ void graph_release(const fd_station_dev &sd, Shared &sh, WarpSmem &ws
         }
     } else {
         if (fin) {
-            int lx[3], ly[3], lz[3];
-#pragma unroll
-            for (int k = 0; k < 3; k++) {
-                lx[k] = gs.lay[0][wh.x + k];
-                ly[k] = gs.lay[1][wh.y + k];
-                lz[k] = gs.lay[2][wh.z + k];
-            }
-            const int p = (int)wh.p, nxy = nx * ny, xyz = pack_xyz(wh.x, wh.y, wh.z);
+            /* (a loop, not 26 copies: the solver's code is larger than the instruction caches, and the copies
+             * cost the sweeps that never get here more than the loop costs this one) */
+            const int xyz = pack_xyz(wh.x, wh.y, wh.z), nxy = nx * ny;
             const float *t13 = &ws.t[lane][13];
-#pragma unroll
+            const short *ax = gs.lay[0] + wh.x, *ay = gs.lay[1] + wh.y, *az = gs.lay[2] + wh.z;
+            int kx = 0, ky = 0, kz = 0, q = (int)wh.p - nxy - nx - 1, o = -(1 << 20) - 1024 - 1;
+#pragma unroll 1
             for (int k = 0; k < 27; k++) {
-                if (k == 13) continue;
-                const int w = max(max(lx[k % 3], ly[(k / 3) % 3]), lz[k / 9]);
-                const unsigned dec = release_dec(w, wh.inst, sh.rel[F][k], t13);
-                if (dec)
-                    release_one(sd, sh, p + (k / 9 - 1) * nxy + ((k / 3) % 3 - 1) * nx + k % 3 - 1,
-                                xyz + (k / 9 - 1) * (1 << 20) + ((k / 3) % 3 - 1) * 1024 + k % 3 - 1, own_face(w), dec,
-                                keyq, nkey);
+                const int w = max(max(ax[kx], ay[ky]), az[kz]);
+                const unsigned dec = k == 13 ? 0u : release_dec(w, wh.inst, sh.rel[F][k], t13);
+                if (dec) release_one(sd, sh, q, xyz + o, own_face(w), dec, keyq, nkey);
+                q++;
+                o++;
+                if (++kx == 3) {
+                    kx = 0;
+                    q += nx - 3;
+                    o += 1024 - 3;
+                    if (++ky == 3) {
+                        ky = 0;
+                        kz++;
+                        q += nxy - 3 * nx;
+                        o += (1 << 20) - 3 * 1024;
+                    }
+                }
             }
         }
     }
@@ -1309,15 +1296,31 @@ FD_COLD bool wait_point(const fd_station_dev &sd, Shared &sh, int w, long long p
 /* ---------------------------------------------------------------------------------------------- */
 /* evaluation of one chunk                                                                         */
 
-/* num / den > FD_HEADTEST for num >= 0, den > 0, as the double division rounds it.  Almost every quotient
- * is far from the threshold: both operands truncated to float (on the integer pipe, within 2^-23) tell
- * unless the quotient is within 2^-18 of it, and only then is the division made (17 FP64 instructions). */
-__device__ __forceinline__ bool head_wave(double num, double den)
+/* the head-wave measure of trial d against its threshold, as the reference forms it */
+FD_COLD bool head_wave_exact(const fd_station_dev &sd, const TrialDesc &d, const float *s18, int z, int y, double num)
 {
-    const float n = d2f_trunc(num), t = 1.e-3f * d2f_trunc(den);
+    return num / head_den(d, s18, sd.g, z, y) > FD_HEADTEST;
+}
+
+/* num / (length * slowness) > FD_HEADTEST for num >= 0.  Almost every quotient is far from the threshold: in
+ * FP32 (num and the reciprocal length truncated, each within 2^-23) it tells unless the quotient is within
+ * 2^-18 of it, and only then is the reference's product and division made (20 FP64 instructions). */
+__device__ __forceinline__ bool head_wave(const fd_station_dev &sd, const TrialDesc &d, const float *s18, int z, int y,
+                                          double num)
+{
+    const float2 f = inv32_at(sd.g, z + d.ddz[0], y + d.ddy[0]);
+    const float iv = d.dcls[0] == CH_H ? d2f_trunc(sd.g.inv_h) : d.dcls[0] == CH_RDQ ? f.x : f.y;
+    const float n = d2f_trunc(num) * iv, t = 1.e-3f * s18[NB_POINT];
     if (n > t * 1.0000038146972656f) return true;
     if (n < t * 0.9999961853027344f) return false;
-    return num / den > FD_HEADTEST;
+    return head_wave_exact(sd, d, s18, z, y, num);
+}
+
+/* a new-edge or new-face value that was not computed with the chunk's items */
+FD_COLD double contact_value(const fd_station_dev &sd, const TrialDesc &d, const float *t18, const float *s18, int z, int y,
+                             bool nf)
+{
+    return nf ? eval_nf(d, t18, s18, sd.g, z, y) : eval_ne(d, t18, s18, sd.g, z, y);
 }
 
 /* The reference's sequential minimum over the 22 trials of one node, from the values computed
@@ -1359,7 +1362,7 @@ __device__ bool commit_node(const fd_station_dev &sd, Shared &sh, const TrialDes
         float fl = t18[d.slot[0]];
         for (int k = 1; k < 5; k++) fl = fmaxf(fl, t18[d.slot[k]]);
         if (prunable(fl, guess)) return;
-        take(K, K == TK_NF ? eval_nf(d, t18, s18, sd.g, z, y) : eval_ne(d, t18, s18, sd.g, z, y));
+        take(K, contact_value(sd, d, t18, s18, z, y, K == TK_NF));
         count_eval(cn, K == TK_NF ? 3 : 1);
     };
     if (gm & 0xFu) writer = 31 - __clz((int)(gm & 0xFu));
@@ -1375,7 +1378,7 @@ __device__ bool commit_node(const fd_station_dev &sd, Shared &sh, const TrialDes
         sd.T[wh.p] = __double2float_rn(guess);
         if (lastK >= 0) {
             /* only the last head trial that lowered the minimum sets the measure that is tested */
-            if (head_wave(last_gb - last_v, head_den(dsc[lastK], s18, sd.g, z, y))) atomicAdd(&sh.w.headw[frame_of(F).headw], 1);
+            if (head_wave(sd, dsc[lastK], s18, z, y, last_gb - last_v)) atomicAdd(&sh.w.headw[frame_of(F).headw], 1);
         }
     }
     const float st0 = writer < 0 ? it0 : t18[dsc[writer].slot[0]], st4 = writer < 0 ? it4 : t18[dsc[writer].slot[4]];

@@ -32,7 +32,7 @@ struct TrialDesc {
     /* fdsph3d */
     unsigned char prow[7], diag[7], pair[21], a_idx, i2a_idx;
     signed char zmin, ymin;
-    /* distances of ne / 2-D / nf, in the stencil's argument order */
+    /* distances of ne / 2-D / nf, in the stencil's argument order; 1-D: the step's */
     unsigned char dcls[5];
     signed char ddz[5], ddy[5];
     unsigned char apair;
@@ -103,6 +103,7 @@ constexpr TrialDesc make_desc(int K)
         if (tr.kind == FDN_2D) d.apair = (unsigned char)apair_of<F>(tr.d[0], tr.d[1]);
     }
     if (tr.kind == FDN_1D) {
+        d.dcls[0] = (unsigned char)(tr.d[0].n == 1 ? CH_H : tr.d[0].n == 2 ? CH_RDQ : CH_RSDF);   /* the step's length */
         d.vn = tr.d[0].n;
         for (int j = 0; j < tr.d[0].n; j++) {
             d.vk[j] = tr.d[0].f[j].kind;
