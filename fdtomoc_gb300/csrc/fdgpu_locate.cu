@@ -9,14 +9,20 @@
  * trial point scored by the standard deviation of its weighted residuals, then (d) drops outliers or
  * recovers phases and repeats (a)-(c) if that changed the phase set (:1086-1128).
  *
- * GPU form: one thread per trial point and event, every event of the batch in the same launch
- * (grid.y).  Each thread keeps the reference's sequential per-phase accumulation, so the statistics
- * match bit for bit; the "first strictly smaller" scan over trial points becomes an atomicMin on
+ * GPU form: a thread keeps the reference's sequential per-phase accumulation of its trial points, every
+ * event of the batch in the same launch, so the statistics match bit for bit; the "first strictly smaller" scan over trial points becomes an atomicMin on
  * (float bits of the deviation << 32 | trial index in loop order), which picks the same point.  A
- * one-thread-per-event kernel between stages takes the minimum, updates the event's best point the
+ * kernel between stages takes the minimum, updates the event's best point the
  * way the sequential scan would, and lays out the next stage's window; a last one recomputes the
  * residuals at the final point and runs the outlier / recovery step.  The host repeats the stages
  * for the events that asked for another pass.
+ *
+ * Refinements.  The reference interpolates each phase's time in double and rounds the residual to float:
+ * 26 FP64 instructions a phase and trial, which held the FP64 units (2 lanes a clock on an SM) 86 % busy.
+ * Here the residual along a row of trials is A - b f in pairs of floats (about 46 bits), A and b formed once per
+ * row, cell and phase; its float is certain unless the value lies within the pairs' error of
+ * a rounding boundary (res_pair), and only such residuals, about one in ten thousand, are formed in double.
+ * The floats that enter the statistics are the reference's either way.
  *
  * Arithmetic: statistics in float, positions and trilinear weights in double, as the reference;
  * compiled with --fmad=false and IEEE float division and square root.  At grid nodes the residual
@@ -49,6 +55,8 @@ struct LocEvent {
     double exm, eym, ezm;
     double x0i, y0i, z0i, sx, sy, sz;   /* current refinement window: origin and steps */
     int nsx, nsy, nsz;
+    int nlist;                  /* accepted phases of this pass, listed from obs0 on */
+    float facs;                 /* their weights' sum, in phase order (the same at every trial point) */
     unsigned long long best;    /* (deviation bits << 32) | trial index; ~0: none */
 };
 
@@ -56,6 +64,14 @@ struct LocObsDev {
     const float *field;
     float obstime, pwt;
     int s_scaled;   /* S phase whose time is the P field times vpvs (ivs 0) */
+};
+
+/* a trial coordinate along one axis of an event's window: its cell and its place in the cell, as find_cell
+ * forms it, and that place as a pair of floats */
+struct AxisPos {
+    double f;
+    float fh, fl;
+    int cell;
 };
 
 __device__ __forceinline__ unsigned long long trial_key(float std, unsigned idx)
@@ -76,24 +92,8 @@ struct Cell {
     double w[8];
 };
 
-__device__ __forceinline__ void find_cell(const fdgpu_loc_grid &g, double x, double yy, double z, Cell &c)
+__device__ __forceinline__ void cell_weights(Cell &c, double fx, double fy, double fz)
 {
-    int i = (int)((x - g.x0) / g.df);
-    int j = (int)((yy - g.y0) / g.dq);
-    int k = (int)((z - g.z0) / g.h);
-    i = i < 0 ? 0 : i;
-    j = j < 0 ? 0 : j;
-    k = k < 0 ? 0 : k;
-    i = i > g.nx - 2 ? g.nx - 2 : i;
-    j = j > g.ny - 2 ? g.ny - 2 : j;
-    k = k > g.nz - 2 ? g.nz - 2 : k;
-    const double xi = g.x0 + g.df * i, yj = g.y0 + g.dq * j, zk = g.z0 + g.h * k;
-    c.a = (long long)g.nx * g.ny * k;
-    c.b = (long long)g.nx * j;
-    c.a2 = (long long)g.nx * g.ny * (k + 1);
-    c.b2 = (long long)g.nx * (j + 1);
-    c.i = i;
-    const double fx = (x - xi) / g.df, fy = (yy - yj) / g.dq, fz = (z - zk) / g.h;
     c.w[0] = (1.0 - fx) * (1.0 - fy) * (1.0 - fz);
     c.w[1] = fx * (1.0 - fy) * (1.0 - fz);
     c.w[2] = (1.0 - fx) * fy * (1.0 - fz);
@@ -102,6 +102,29 @@ __device__ __forceinline__ void find_cell(const fdgpu_loc_grid &g, double x, dou
     c.w[5] = fx * (1.0 - fy) * fz;
     c.w[6] = (1.0 - fx) * fy * fz;
     c.w[7] = fx * fy * fz;
+}
+
+/* the cell of coordinate x on an axis of n nodes at o + d i, clamped to the grid, and x's place in it */
+__device__ __forceinline__ int axis_cell(double x, double o, double d, int n, double *f)
+{
+    int i = (int)((x - o) / d);
+    i = i < 0 ? 0 : i;
+    i = i > n - 2 ? n - 2 : i;
+    *f = (x - (o + d * i)) / d;
+    return i;
+}
+
+__device__ __forceinline__ void find_cell(const fdgpu_loc_grid &g, double x, double yy, double z, Cell &c)
+{
+    double fx, fy, fz;
+    const int i = axis_cell(x, g.x0, g.df, g.nx, &fx), j = axis_cell(yy, g.y0, g.dq, g.ny, &fy);
+    const int k = axis_cell(z, g.z0, g.h, g.nz, &fz);
+    c.a = (long long)g.nx * g.ny * k;
+    c.b = (long long)g.nx * j;
+    c.a2 = (long long)g.nx * g.ny * (k + 1);
+    c.b2 = (long long)g.nx * (j + 1);
+    c.i = i;
+    cell_weights(c, fx, fy, fz);
 }
 
 /* the trilinear time of one field in that cell: the reference's sum, term by term */
@@ -126,16 +149,13 @@ __device__ __forceinline__ float residual_d(const LocObsDev &o, double tp, float
     return (float)((double)o.obstime - tp);
 }
 
-/* the accumulation of :750-770 for one phase */
-__device__ __forceinline__ void accumulate(float res, float wt, bool good, float &avres, float &rsq, float &facs)
+/* the accumulation of :750-770 for one accepted phase (facs: LocEvent) */
+__device__ __forceinline__ void accumulate(float res, float wt, float &avres, float &rsq)
 {
-    if (good) {
-        const float r1 = res * wt;
-        const float r2 = r1 * res;
-        avres += r1;
-        rsq += r2;
-        facs += wt;
-    }
+    const float r1 = res * wt;
+    const float r2 = r1 * res;
+    avres += r1;
+    rsq += r2;
 }
 
 /* :771-777 */
@@ -144,6 +164,31 @@ __device__ __forceinline__ float deviation(float avres, float rsq, float facs, i
     const float avwt = facs / (float)ngood;
     const float deb = (rsq - avres * avres / facs) / ((float)(ngood - 4) * avwt);
     return sqrtf(fabsf(deb));
+}
+
+/* Whether a trial's deviation is certainly above the smallest one found so far, `best` (any earlier value of the
+ * event's minimum serves).  It is formed without the divisions and the square root of deviation(), within
+ * 2^-20 rsq / den of its square; NaN and infinite values answer no.
+ * Almost every trial ends here: two divisions and a square root cost as much as the sums of several phases. */
+struct Hopeless {
+    float rf, rd, b2;
+    __device__ __forceinline__ Hopeless(float facs, int ngood, unsigned long long best)
+    {
+        const float b = __uint_as_float((unsigned)(best >> 32));
+        rf = 1.0f / facs;
+        rd = 1.0f / ((float)(ngood - 4) * (facs / (float)ngood));
+        b2 = best == ~0ull ? INFINITY : b * b * 1.00000191f + 1e-36f;
+    }
+    __device__ __forceinline__ bool operator()(float avres, float rsq) const
+    {
+        const float q = rsq * rd;
+        return (rsq - avres * avres * rf) * rd - 1.9073486e-06f * fabsf(q) > b2;
+    }
+};
+
+__device__ __forceinline__ unsigned long long load_best(const LocEvent &ev)
+{
+    return *const_cast<const volatile unsigned long long *>(&ev.best);
 }
 
 /* the block's smallest key into the event's minimum */
@@ -166,72 +211,274 @@ __device__ __forceinline__ void reduce_key(unsigned long long key, unsigned long
     }
 }
 
-/* the event's phases in shared memory */
-struct ObsTile {
-    const float *field[kMaxObs];
-    float obstime[kMaxObs], pwt[kMaxObs];
-    unsigned char good[kMaxObs], s_scaled[kMaxObs];
-};
-
-__device__ void load_obs(ObsTile &ot, const LocObsDev *obs, const unsigned char *good, const LocEvent &ev)
+/* obstime - t * vpvs as the reference forms it (in double, then float) */
+__device__ __noinline__ float residual_scaled(float obstime, float t, float vpvs)
 {
-    for (int q = threadIdx.x; q < ev.nobs; q += blockDim.x) {
-        const LocObsDev o = obs[ev.obs0 + q];
-        ot.field[q] = o.field;
-        ot.obstime[q] = o.obstime;
-        ot.pwt[q] = o.pwt;
-        ot.s_scaled[q] = (unsigned char)o.s_scaled;
-        ot.good[q] = good[ev.obs0 + q];
-    }
-    __syncthreads();
+    return (float)((double)obstime - (double)t * (double)vpvs);
 }
 
-/* (a) coarse search: trial c is grid node nx*ny*kmin + c, in the reference's loop order */
-__global__ void __launch_bounds__(kLocBlock) loc_coarse(fdgpu_loc_grid g, const LocObsDev *obs,
-                                                          const unsigned char *good, LocEvent *evs,
-                                                          const int *active, long long ncand)
+/* The same without FP64: the product and the difference are exact as pairs of floats, but for a last
+ * rounding within 2^-46 of their size (the reference rounds once more to double: 2^-53); where that
+ * could change the float, the reference's form decides. */
+__device__ __forceinline__ float residual_scaled_pair(float obstime, float t, float vpvs)
 {
-    __shared__ ObsTile ot;
-    LocEvent &ev = evs[active[blockIdx.y]];
-    if ((long long)blockIdx.x * kLocBlock >= ncand) return;
-    load_obs(ot, obs, good, ev);
-    const long long c = (long long)blockIdx.x * kLocBlock + threadIdx.x;
-    unsigned long long key = ~0ull;
-    if (c < ncand) {
-        const long long n = (long long)g.nx * g.ny * g.kmin + c;
-        float avres = 0.0f, rsq = 0.0f, facs = 0.0f;
-        /* the phases' times are loaded eight at a time, so that eight loads are in flight, and then
-         * accumulated in phase order */
-        constexpr int kBatch = 8;
-        for (int q0 = 0; q0 < ev.nobs; q0 += kBatch) {
-            float tv[kBatch];
+    const float p = t * vpvs, e = fmaf(t, vpvs, -p);
+    const float d = obstime - p, v = d - obstime, er = (obstime - (d - v)) + (-p - v);
+    const float low = er - e, m = 1.4210854715202004e-14f * (fabsf(obstime) + fabsf(p));
+    const float up = d + (low + m), dn = d + (low - m);
+    return up == dn ? up : residual_scaled(obstime, t, vpvs);
+}
+
+/* a phase as the coarse search reads it from shared memory, in one 16-byte load */
+struct __align__(16) CoarseObs {
+    const float *field;   /* at the block's first node */
+    float obstime, pwt;
+};
+
+/* the statistics of nodes n .. n+3 over the event's accepted phases */
+template <bool SCALED>
+__device__ __forceinline__ void coarse_sums(const CoarseObs *ob, const unsigned char *scaled, int nl, int at, bool wide, int left,
+                                            float vpvs, float av[4], float rs[4])
+{
+    constexpr int kBatch = 4;   /* phases whose loads are in flight together */
+    auto load = [&](const CoarseObs &o) {
+        const float *f = o.field + at;
+        if (wide) return __ldg(reinterpret_cast<const float4 *>(f));
+        return make_float4(f[0], left > 1 ? f[1] : 0.f, left > 2 ? f[2] : 0.f, left > 3 ? f[3] : 0.f);
+    };
+    auto add = [&](const CoarseObs &o, int q, const float4 &tv) {
+        const float t[4] = {tv.x, tv.y, tv.z, tv.w};
+        const bool sc = SCALED && scaled[q];
 #pragma unroll
-            for (int u = 0; u < kBatch; u++) tv[u] = q0 + u < ev.nobs ? ot.field[q0 + u][n] : 0.0f;
+        for (int i = 0; i < 4; i++) accumulate(sc ? residual_scaled_pair(o.obstime, t[i], vpvs) : o.obstime - t[i], o.pwt, av[i], rs[i]);
+    };
+    int q = 0;
+    for (; q + kBatch <= nl; q += kBatch) {
+        CoarseObs o[kBatch];
+        float4 tv[kBatch];
 #pragma unroll
-            for (int u = 0; u < kBatch; u++) {
-                const int q = q0 + u;
-                if (q >= ev.nobs) break;
-                const float t = tv[u];
-                const float res = ot.s_scaled[q] ? (float)((double)ot.obstime[q] - (double)t * (double)g.vpvs)
-                                                 : ot.obstime[q] - t;
-                accumulate(res, ot.pwt[q], ot.good[q] != 0, avres, rsq, facs);
-            }
+        for (int u = 0; u < kBatch; u++) {
+            o[u] = ob[q + u];
+            tv[u] = load(o[u]);
         }
-        key = trial_key(deviation(avres, rsq, facs, ev.ngood), (unsigned)c);
+#pragma unroll
+        for (int u = 0; u < kBatch; u++) add(o[u], q + u, tv[u]);
+    }
+    for (; q < nl; q++) {
+        const CoarseObs o = ob[q];
+        add(o, q, load(o));
+    }
+}
+
+/* (a) Coarse search: trial c is grid node n0 + c, in the reference's loop order.  What bounds it is reading a
+ * time per phase and node, and five float operations on it.  A thread takes four nodes, one 16-byte load per
+ * phase, and consecutive blocks take the same nodes for successive events, so that the events of a catalog,
+ * which share their stations' fields, find them in L2.  128 events x 32 phases on 201x201x81: 10.5 -> 4.7 ms a
+ * pass against a node a thread with the events one after another (52 GB of DRAM reads, 0.8 GB now). */
+__global__ void __launch_bounds__(kLocBlock) loc_coarse(fdgpu_loc_grid g, const LocObsDev *list, LocEvent *evs,
+                                                          const int *active, int nact, long long n0, long long n1,
+                                                          int aligned)
+{
+    __shared__ CoarseObs ob[kMaxObs];
+    __shared__ unsigned char scaled[kMaxObs];
+    LocEvent &ev = evs[active[blockIdx.x % (unsigned)nact]];
+    const int nl = ev.nlist;
+    /* nodes first + 4 threadIdx.x ..; the first group may begin before n0, the last end after n1 */
+    const long long first = (n0 & ~3ll) + 4ll * (blockIdx.x / (unsigned)nact) * kLocBlock;
+    bool any = false;
+    for (int q = threadIdx.x; q < nl; q += blockDim.x) {
+        const LocObsDev o = list[ev.obs0 + q];
+        ob[q] = CoarseObs{o.field + first, o.obstime, o.pwt};
+        scaled[q] = (unsigned char)o.s_scaled;
+        any = any || o.s_scaled;
+    }
+    any = __syncthreads_or(any);
+    const unsigned long long best = load_best(ev);
+    const int at = 4 * threadIdx.x;
+    const long long n = first + at;
+    unsigned long long key = ~0ull;
+    if (n < n1) {
+        float av[4] = {0.f, 0.f, 0.f, 0.f}, rs[4] = {0.f, 0.f, 0.f, 0.f};
+        const int left = n1 - n > 4 ? 4 : (int)(n1 - n);
+        if (any) coarse_sums<true>(ob, scaled, nl, at, aligned && left > 3, left, g.vpvs, av, rs);
+        else coarse_sums<false>(ob, scaled, nl, at, aligned && left > 3, left, g.vpvs, av, rs);
+        const Hopeless hopeless(ev.facs, ev.ngood, best);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            if (n + i < n0 || i >= left || hopeless(av[i], rs[i])) continue;
+            const unsigned long long k = trial_key(deviation(av[i], rs[i], ev.facs, ev.ngood), (unsigned)(n + i - n0));
+            key = k < key ? k : key;
+        }
     }
     reduce_key(key, &ev.best);
 }
 
-/* (b), (c) refinements: trial c = (k * nsy + j) * nsx + i of the event's window */
-__global__ void __launch_bounds__(kLocBlock) loc_refine(fdgpu_loc_grid g, const LocObsDev *obs,
-                                                          const unsigned char *good, LocEvent *evs,
-                                                          const int *active)
+/* one phase's residual at place (fx,fy,fz) of the cell with corner times at t: the reference's (find_time) */
+__device__ __noinline__ float residual_exact(const LocObsDev &o, const float *t, int nx, int nxy, double fx, double fy,
+                                             double fz, float vpvs)
 {
-    __shared__ ObsTile ot;
+    Cell c;
+    c.a = 0;
+    c.b = 0;
+    c.a2 = nxy;
+    c.b2 = nx;
+    c.i = 0;
+    cell_weights(c, fx, fy, fz);
+    return residual_d(o, cell_time(c, t), vpvs);
+}
+
+/* a pair of floats (h + l) */
+struct FF {
+    float h, l;
+};
+__device__ __forceinline__ FF ff_one_minus(FF f)
+{
+    const float h = 1.f - f.h;
+    return {h, ((1.f - h) - f.h) - f.l};
+}
+__device__ __forceinline__ FF ff_mul(FF a, FF b)
+{
+    const float p = a.h * b.h;
+    return {p, fmaf(a.h, b.h, -p) + fmaf(a.h, b.l, a.l * b.h)};
+}
+__device__ __forceinline__ FF ff_add(FF a, FF b)
+{
+    const float h = a.h + b.h, v = h - a.h;
+    return {h, ((a.h - (h - v)) + (b.h - v)) + (a.l + b.l)};
+}
+__device__ __forceinline__ FF ff_neg(FF a) { return {-a.h, -a.l}; }
+/* a - b, exact */
+__device__ __forceinline__ FF ff_diff(float a, float b) { return ff_add(FF{a, 0.f}, FF{-b, 0.f}); }
+__device__ __forceinline__ FF ff_scale(FF a, float s)
+{
+    const float p = a.h * s;
+    return {p, fmaf(a.l, s, fmaf(a.h, s, -p))};
+}
+
+/* A cell's residual along a row of trials: A - b f, from the times of the row's cell at t (x), t + nx (y), t + nxy
+ * (z) and the row's weights.  Times enter as their differences from the corner's, t0: they are exact and of a
+ * step's size, so the pairs' error is too.  It is within 100 u^2 D + 10 u^2 |obs - t0| (u = 2^-24, D the largest
+ * difference: weights, products and sums, term by term), the reference's own within 2^-49 of the largest time:
+ * m is above their sum. */
+__device__ __forceinline__ void row_coefficients(const LocObsDev &o, const float *t, int nx, int nxy, const FF w[4], float vpvs,
+                                                 float4 *ab, float *m)
+{
+    const float t0 = t[0];
+    float big = fabsf(t0), dmax = 0.f;
+    FF v[2] = {{0.f, 0.f}, {0.f, 0.f}};
+#pragma unroll
+    for (int k = 1; k < 8; k++) {
+        const float tk = t[(k & 1) + (k & 2 ? nx : 0) + (k & 4 ? nxy : 0)];
+        const FF d = ff_diff(tk, t0);
+        big = fmaxf(big, fabsf(tk));
+        dmax = fmaxf(dmax, fabsf(d.h));
+        v[k & 1] = ff_add(v[k & 1], ff_mul(w[k >> 1], d));
+    }
+    FF c = {t0, 0.f}, a = v[0], b = ff_add(v[1], ff_neg(v[0]));
+    float mag = 1.f;
+    if (o.s_scaled) {
+        c = ff_scale(c, vpvs);
+        a = ff_scale(a, vpvs);
+        b = ff_scale(b, vpvs);
+        mag = fmaxf(1.f, fabsf(vpvs));
+    }
+    c = ff_add(FF{o.obstime, 0.f}, ff_neg(c));
+    const FF A = ff_add(c, ff_neg(a));
+    *ab = make_float4(A.h, A.l, b.h, b.l);
+    *m = mag * (4.547473508864641e-13f * dmax + 3.552713678800501e-15f * big) + 5.684341886080802e-14f * fabsf(c.h);
+}
+
+/* The residual A - b f rounded to float, f = fh + fl: true and the reference's float if that is certain, that
+ * is if A - b f - m and A - b f + m round to the same float; else the caller forms the residual in double. */
+__device__ __forceinline__ bool res_pair(const float4 &ab, float m, float fh, float fl, float *res)
+{
+    const float p = ab.z * fh, e = fmaf(ab.w, fh, fmaf(ab.z, fl, fmaf(ab.z, fh, -p)));
+    const float d = ab.x - p, v = d - ab.x;
+    const float low = ((ab.x - (d - v)) + (-p - v)) + (ab.y - e);
+    const float up = d + (low + m);
+    *res = up;
+    return up == d + (low - m);
+}
+
+/* (b), (c) refinements: trial c = (k * nsy + j) * nsx + i of the event's window (header comment).  A block's
+ * consecutive trials lie on a few rows (j, k) and in at most three cells of each (segments); the phases go
+ * through in tiles whose coefficients, a pair of floats for a and b and the margin m per segment, fit shared
+ * memory.  128 events x 32 phases, 41^3 trials: 14.7 -> 2.0 ms in the first refinement and
+ * 0.6 in the second, against FP64. */
+constexpr int kCoef = 1024;   /* coefficients of a tile: segments x phases */
+constexpr int kDivMax = 64;   /* largest divisions of the axis tables; finer windows take loc_refine_fp64 */
+
+__global__ void __launch_bounds__(kLocBlock) loc_refine(fdgpu_loc_grid g, const LocObsDev *list, LocEvent *evs,
+                                                          const int *active, const AxisPos *axes, int naxis)
+{
+    __shared__ float4 cab[kCoef];
+    __shared__ float cm[kCoef];
+    __shared__ FF wrow[kLocBlock + 2][4];
+    __shared__ int orow[kLocBlock + 2];
+    const int e = active[blockIdx.y];
+    LocEvent &ev = evs[e];
+    const int nsx = ev.nsx, nsy = ev.nsy, ncand = nsx * nsy * ev.nsz;
+    const int c0 = blockIdx.x * kLocBlock;
+    if (c0 >= ncand) return;
+    const AxisPos *ax = axes + (size_t)e * 3 * naxis, *ay = ax + naxis, *az = ay + naxis;
+    const LocObsDev *ob = list + ev.obs0;
+    const int nl = ev.nlist, nx = g.nx, nxy = g.nx * g.ny;
+    const int c = c0 + threadIdx.x, clast = min(c0 + kLocBlock, ncand) - 1;
+    const int row0 = c0 / nsx, nrows = clast / nsx - row0 + 1;
+    const int cmin = ax[0].cell, ncx = ax[nsx - 1].cell - cmin + 1;
+    const int segs = nrows * ncx, tile = min(16, kCoef / segs);
+    for (int r = threadIdx.x; r < nrows; r += kLocBlock) {
+        const int row = row0 + r, k = row / nsy, j = row - k * nsy;
+        const FF fy = {ay[j].fh, ay[j].fl}, fz = {az[k].fh, az[k].fl}, gy = ff_one_minus(fy), gz = ff_one_minus(fz);
+        wrow[r][0] = ff_mul(gy, gz);
+        wrow[r][1] = ff_mul(fy, gz);
+        wrow[r][2] = ff_mul(gy, fz);
+        wrow[r][3] = ff_mul(fy, fz);
+        orow[r] = az[k].cell * nxy + ay[j].cell * nx;
+    }
+    float avres = 0.0f, rsq = 0.0f, fh = 0.f, fl = 0.f;
+    int seg = 0, i = 0, row = 0;
+    if (c < ncand) {
+        row = c / nsx;
+        i = c - row * nsx;
+        fh = ax[i].fh;
+        fl = ax[i].fl;
+        seg = (row - row0) * ncx + ax[i].cell - cmin;
+    }
+    for (int q0 = 0; q0 < nl; q0 += tile) {
+        const int nq = min(tile, nl - q0);
+        __syncthreads();
+        for (int x = threadIdx.x; x < nq * segs; x += kLocBlock) {
+            const int q = x / segs, sg = x - q * segs, r = sg / ncx;
+            const LocObsDev o = ob[q0 + q];
+            row_coefficients(o, o.field + orow[r] + cmin + (sg - r * ncx), nx, nxy, wrow[r], g.vpvs, &cab[x], &cm[x]);
+        }
+        __syncthreads();
+        if (c < ncand) {
+            for (int q = 0; q < nq; q++) {
+                const LocObsDev &o = ob[q0 + q];
+                float res;
+                if (!res_pair(cab[q * segs + seg], cm[q * segs + seg], fh, fl, &res)) {
+                    const int k = row / nsy, j = row - k * nsy;
+                    res = residual_exact(o, o.field + orow[row - row0] + ax[i].cell, nx, nxy, ax[i].f, ay[j].f, az[k].f, g.vpvs);
+                }
+                accumulate(res, o.pwt, avres, rsq);
+            }
+        }
+    }
+    unsigned long long key = ~0ull;
+    if (c < ncand) key = trial_key(deviation(avres, rsq, ev.facs, ev.ngood), (unsigned)c);
+    reduce_key(key, &ev.best);
+}
+
+/* the refinements in double throughout, for windows finer than the axis tables hold */
+__global__ void __launch_bounds__(kLocBlock) loc_refine_fp64(fdgpu_loc_grid g, const LocObsDev *list, LocEvent *evs,
+                                                               const int *active)
+{
     LocEvent &ev = evs[active[blockIdx.y]];
     const long long ncand = (long long)ev.nsx * ev.nsy * ev.nsz;
     if ((long long)blockIdx.x * kLocBlock >= ncand) return;
-    load_obs(ot, obs, good, ev);
+    const LocObsDev *ob = list + ev.obs0;
     const long long c = (long long)blockIdx.x * kLocBlock + threadIdx.x;
     unsigned long long key = ~0ull;
     if (c < ncand) {
@@ -239,23 +486,16 @@ __global__ void __launch_bounds__(kLocBlock) loc_refine(fdgpu_loc_grid g, const 
         const double zp = ev.z0i + ev.sz * k, yp = ev.y0i + ev.sy * j, xp = ev.x0i + ev.sx * i;
         Cell cell;
         find_cell(g, xp, yp, zp, cell);
-        float avres = 0.0f, rsq = 0.0f, facs = 0.0f;
-        for (int q = 0; q < ev.nobs; q++) {
-            const LocObsDev o{ot.field[q], ot.obstime[q], ot.pwt[q], ot.s_scaled[q]};
-            const float res = residual_d(o, cell_time(cell, o.field), g.vpvs);
-            accumulate(res, ot.pwt[q], ot.good[q] != 0, avres, rsq, facs);
-        }
-        key = trial_key(deviation(avres, rsq, facs, ev.ngood), (unsigned)c);
+        float avres = 0.0f, rsq = 0.0f;
+        for (int q = 0; q < ev.nlist; q++) accumulate(residual_d(ob[q], cell_time(cell, ob[q].field), g.vpvs), ob[q].pwt, avres, rsq);
+        key = trial_key(deviation(avres, rsq, ev.facs, ev.ngood), (unsigned)c);
     }
     reduce_key(key, &ev.best);
 }
 
 /* Take the stage's minimum (stage 0 coarse, 1, 2) and lay out the next window. */
-__global__ void loc_plan(fdgpu_loc_grid g, LocEvent *evs, const int *active, int nact, int stage)
+__device__ void plan_stage(const fdgpu_loc_grid &g, LocEvent &ev, int stage)
 {
-    const int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= nact) return;
-    LocEvent &ev = evs[active[a]];
     const unsigned long long key = ev.best;
     ev.best = ~0ull;
     const float std = __uint_as_float((unsigned)(key >> 32));
@@ -336,77 +576,96 @@ __global__ void loc_plan(fdgpu_loc_grid g, LocEvent *evs, const int *active, int
     }
 }
 
-/* Residuals at the final point, then the outlier / recovery step (:1086-1128). */
+/* A block per event: the stage's minimum and the next window, then (axes given) the window's coordinates along
+ * each axis, whose cells and places in them every trial of the window shares. */
+__global__ void loc_plan(fdgpu_loc_grid g, LocEvent *evs, const int *active, int stage, AxisPos *axes, int naxis)
+{
+    const int e = active[blockIdx.x];
+    __shared__ LocEvent ev;
+    if (threadIdx.x == 0) {
+        ev = evs[e];
+        plan_stage(g, ev, stage);
+        evs[e] = ev;
+    }
+    __syncthreads();
+    if (!axes) return;
+    AxisPos *at = axes + (size_t)e * 3 * naxis;
+    for (int t = threadIdx.x; t < 3 * naxis; t += blockDim.x) {
+        const int axis = t / naxis, i = t - axis * naxis;
+        AxisPos p;
+        if (axis == 0) p.cell = axis_cell(ev.x0i + ev.sx * i, g.x0, g.df, g.nx, &p.f);
+        else if (axis == 1) p.cell = axis_cell(ev.y0i + ev.sy * i, g.y0, g.dq, g.ny, &p.f);
+        else p.cell = axis_cell(ev.z0i + ev.sz * i, g.z0, g.h, g.nz, &p.f);
+        p.fh = (float)p.f;
+        p.fl = (float)(p.f - (double)p.fh);
+        at[t] = p;
+    }
+}
+
+/* Residuals at the final point, then the outlier / recovery step (:1086-1128).  A warp per event: a lane
+ * per phase, sums in phase order. */
 __global__ void loc_finish(fdgpu_loc_grid g, const LocObsDev *obs, unsigned char *good, LocEvent *evs,
                            const int *active, int nact, float *resmin, float *tps)
 {
-    const int a = blockIdx.x * blockDim.x + threadIdx.x;
+    const int a = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (a >= nact) return;
     LocEvent &ev = evs[active[a]];
-    float avres = 0.0f, rsq = 0.0f, facs = 0.0f;
     const bool found = ev.stdmin < INFINITY;
+    const int obs0 = ev.obs0, nobs = ev.nobs, wstage = ev.wstage, iretry = ev.iretry;
     const long long node = (long long)g.nx * g.ny * ev.nzz + (long long)g.nx * ev.nyy + ev.nxx;
+    float avres = 0.0f;
     Cell cell;
-    find_cell(g, ev.exm, ev.eym, ev.ezm, cell);
-    for (int q = 0; q < ev.nobs; q++) {
-        const int o = ev.obs0 + q;
-        const LocObsDev d = obs[o];
-        float res;
-        if (ev.wstage == 0)
-            res = d.s_scaled ? (float)((double)d.obstime - (double)d.field[node] * (double)g.vpvs) : d.obstime - d.field[node];
-        else
-            res = residual_d(d, cell_time(cell, d.field), g.vpvs);
-        accumulate(res, d.pwt, good[o] != 0, avres, rsq, facs);
-        /* where no trial became the minimum in this pass the reference keeps the previous pass's
-         * values (zero before the first) */
-        if (found) {
-            resmin[o] = res;
-            tps[o] = d.obstime - res;
-        }
-    }
-    ev.avrmin = found ? avres / facs : 0.0f;
-    int ngood = 0, redo = 0;
-    for (int q = 0; q < ev.nobs; q++) {
-        const int o = ev.obs0 + q;
-        if (!good[o]) continue;
-        const float absres = fabsf(resmin[o] - ev.avrmin);
-        const float perc = 100.0f * absres / tps[o];
-        if (absres <= g.resthres || perc <= g.resthrep)
-            ngood++;
-        else {
-            good[o] = 0;
-            redo = 1;
-        }
-    }
-    ev.ngood = ngood;
-    if (ngood < g.nthres) {
-        ev.state = kTooFew;
-        return;
-    }
-    if (redo) {
-        ev.state = kRedo;
-        return;
-    }
-    if (ev.iretry < 1) {
-        ev.iretry++;
-        for (int q = 0; q < ev.nobs; q++) {
-            const int o = ev.obs0 + q;
-            if (good[o]) continue;
-            const float absres = fabsf(resmin[o] - ev.avrmin);
-            const float perc = 100.0f * absres / tps[o];
-            if (absres <= g.resthres || perc <= g.resthrep) {
-                ngood++;
-                good[o] = 1;
-                redo = 1;
+    if (wstage != 0) find_cell(g, ev.exm, ev.eym, ev.ezm, cell);
+    for (int q0 = 0; q0 < nobs; q0 += 32) {
+        const int o = obs0 + q0 + lane;
+        float r1 = 0.f;
+        bool in = false;
+        if (q0 + lane < nobs) {
+            const LocObsDev d = obs[o];
+            float res;
+            if (wstage == 0)
+                res = d.s_scaled ? residual_scaled(d.obstime, d.field[node], g.vpvs) : d.obstime - d.field[node];
+            else
+                res = residual_d(d, cell_time(cell, d.field), g.vpvs);
+            in = good[o] != 0;
+            r1 = res * d.pwt;
+            /* where no trial became the minimum in this pass the reference keeps the previous pass's
+             * values (zero before the first) */
+            if (found) {
+                resmin[o] = res;
+                tps[o] = d.obstime - res;
             }
         }
-        ev.ngood = ngood;
-        if (redo) {
-            ev.state = kRedo;
-            return;
-        }
+        for (unsigned b = __ballot_sync(0xffffffffu, in); b; b &= b - 1) avres += __shfl_sync(0xffffffffu, r1, __ffs(b) - 1);
     }
-    ev.state = ev.stdmin <= g.stdmax ? kAccepted : kStdHigh;
+    const float avrmin = found ? avres / ev.facs : 0.0f;
+    /* a phase whose residual is off by too much is dropped; on the second look, one dropped before whose
+     * residual has come in is taken back */
+    int ngood = 0;
+    bool redo = false;
+    for (int look = 0; look < 2; look++) {
+        for (int q0 = 0; q0 < nobs; q0 += 32) {
+            const int o = obs0 + q0 + lane;
+            bool kept = false, changed = false;
+            if (q0 + lane < nobs && (good[o] != 0) == (look == 0)) {
+                const float absres = fabsf(resmin[o] - avrmin);
+                const float perc = 100.0f * absres / tps[o];
+                const bool near = absres <= g.resthres || perc <= g.resthrep;
+                kept = near;
+                changed = near != (look == 0);
+                if (changed) good[o] = look == 0 ? 0 : 1;
+            }
+            ngood += __popc(__ballot_sync(0xffffffffu, kept));
+            redo = __any_sync(0xffffffffu, changed) || redo;
+        }
+        if (look == 0 && (ngood < g.nthres || redo || iretry >= 1)) break;
+        if (look == 0 && lane == 0) ev.iretry = iretry + 1;
+    }
+    if (lane == 0) {
+        ev.avrmin = avrmin;
+        ev.ngood = ngood;
+        ev.state = ngood < g.nthres ? kTooFew : redo ? kRedo : ev.stdmin <= g.stdmax ? kAccepted : kStdHigh;
+    }
 }
 
 __global__ void loc_init(LocEvent *evs, const int *offs, int nev)
@@ -423,14 +682,33 @@ __global__ void loc_init(LocEvent *evs, const int *offs, int nev)
     ev.best = ~0ull;
 }
 
-__global__ void loc_begin_pass(LocEvent *evs, const int *active, int nact)
+/* A warp per event: its state for the pass, and the phases accepted so far, listed in order. */
+__global__ void loc_begin_pass(LocEvent *evs, const int *active, int nact, const LocObsDev *obs, const unsigned char *good,
+                               LocObsDev *list)
 {
-    const int a = blockIdx.x * blockDim.x + threadIdx.x;
+    const int a = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (a >= nact) return;
     LocEvent &ev = evs[active[a]];
-    ev.passes++;
-    ev.state = kActive;
-    ev.best = ~0ull;
+    const int obs0 = ev.obs0, nobs = ev.nobs;
+    int nl = 0;
+    float facs = 0.0f;
+    for (int q0 = 0; q0 < nobs; q0 += 32) {
+        const int o = obs0 + q0 + lane;
+        const bool in = q0 + lane < nobs && good[o] != 0;
+        LocObsDev d{};
+        if (in) d = obs[o];
+        unsigned b = __ballot_sync(0xffffffffu, in);
+        if (in) list[obs0 + nl + __popc(b & ((1u << lane) - 1u))] = d;
+        nl += __popc(b);
+        for (; b; b &= b - 1) facs += __shfl_sync(0xffffffffu, d.pwt, __ffs(b) - 1);
+    }
+    if (lane == 0) {
+        ev.nlist = nl;
+        ev.facs = facs;
+        ev.passes++;
+        ev.state = kActive;
+        ev.best = ~0ull;
+    }
 }
 
 __global__ void loc_results(const LocEvent *evs, int nev, fdgpu_loc_result *out)
@@ -576,13 +854,18 @@ extern "C" int fdgpu_locate(fdgpu_ctx *ctx, const fdgpu_loc_grid *g, const float
         hgood[k] = obs[k].good ? 1 : 0;
     }
     DevArena mem(st);
-    LocObsDev *dobs;
+    LocObsDev *dobs, *dlist;
+    AxisPos *daxes = nullptr;
     unsigned char *dgood;
     LocEvent *devs;
     int *doffs, *dact, *dstate;
     float *dres, *dtps;
     fdgpu_loc_result *dout;
     LOC_CU(mem.get(&dobs, nobs));
+    LOC_CU(mem.get(&dlist, nobs));
+    /* the windows' axis tables (see loc_refine) */
+    const int ndmax = g->ndiv > g->ndiv2 ? g->ndiv : g->ndiv2, naxis = 2 * ndmax + 1;
+    if (ndmax <= kDivMax) LOC_CU(mem.get(&daxes, (size_t)nev * 3 * naxis));
     LOC_CU(mem.get(&dgood, nobs));
     LOC_CU(mem.get(&devs, nev));
     LOC_CU(mem.get(&doffs, nev + 1));
@@ -600,38 +883,44 @@ extern "C" int fdgpu_locate(fdgpu_ctx *ctx, const fdgpu_loc_grid *g, const float
     LOC_CU(cudaGetLastError());
 
     const fdgpu_loc_grid G = *g;
-    const long long ncoarse = g->kmin < g->nz ? (long long)(g->nz - g->kmin) * g->nx * g->ny : 0;
-    const long long nwin1 = (long long)(2 * g->ndiv + 1) * (2 * g->ndiv + 1) * (2 * g->ndiv + 1);
-    const long long nwin2 = (long long)(2 * g->ndiv2 + 1) * (2 * g->ndiv2 + 1) * (2 * g->ndiv2 + 1);
+    const long long n0 = (long long)g->kmin * g->nx * g->ny, n1 = (long long)g->nz * g->nx * g->ny;
+    const long long ncoarse = n0 < n1 ? (n1 - (n0 & ~3ll) + 3) / 4 : 0;   /* threads: four nodes each */
+    const long long nwin[2] = {(long long)(2 * g->ndiv + 1) * (2 * g->ndiv + 1) * (2 * g->ndiv + 1),
+                               (long long)(2 * g->ndiv2 + 1) * (2 * g->ndiv2 + 1) * (2 * g->ndiv2 + 1)};
+    /* 16-byte loads of four nodes need every field on a 16-byte boundary */
+    int aligned = 1;
+    for (int k = 0; k < nobs; k++)
+        if ((reinterpret_cast<uintptr_t>(hobs[k].field) & 15u) != 0) aligned = 0;
     std::vector<int> act(nev), state(nev);
     for (int e = 0; e < nev; e++) act[e] = e;
     for (int pass = 0; !act.empty(); pass++) {
         if (pass > 2 * kMaxObs + 4) return FDGPU_ESCHED;   /* each redo drops or recovers a phase */
         const int nact = (int)act.size();
         LOC_CU(cudaMemcpyAsync(dact, act.data(), sizeof(int) * nact, cudaMemcpyHostToDevice, st));
-        const int tb = (nact + 127) / 128;
-        loc_begin_pass<<<tb, 128, 0, st>>>(devs, dact, nact);
-        /* grid.y carries the events; more than 65535 go in slices */
-        for (int a0 = 0; a0 < nact; a0 += 65535) {
-            const int na = nact - a0 < 65535 ? nact - a0 : 65535;
-            if (ncoarse > 0)
-                loc_coarse<<<dim3((unsigned)((ncoarse + kLocBlock - 1) / kLocBlock), na), kLocBlock, 0, st>>>(
-                    G, dobs, dgood, devs, dact + a0, ncoarse);
+        const int tw = (nact + 3) / 4;   /* a warp per event */
+        loc_begin_pass<<<tw, 128, 0, st>>>(devs, dact, nact, dobs, dgood, dlist);
+        if (ncoarse > 0) {
+            /* blocks of one launch: tiles x events, within the grid's limit of 2^31 - 1 */
+            const long long tiles = (ncoarse + kLocBlock - 1) / kLocBlock;
+            const long long most = 0x7fffffffll / tiles;
+            for (int a0 = 0; a0 < nact;) {
+                const int na = (int)(nact - a0 < most ? nact - a0 : most);
+                loc_coarse<<<(unsigned)(tiles * na), kLocBlock, 0, st>>>(G, dlist, devs, dact + a0, na, n0, n1, aligned);
+                a0 += na;
+            }
         }
-        loc_plan<<<tb, 128, 0, st>>>(G, devs, dact, nact, 0);
-        for (int a0 = 0; a0 < nact; a0 += 65535) {
-            const int na = nact - a0 < 65535 ? nact - a0 : 65535;
-            loc_refine<<<dim3((unsigned)((nwin1 + kLocBlock - 1) / kLocBlock), na), kLocBlock, 0, st>>>(
-                G, dobs, dgood, devs, dact + a0);
+        loc_plan<<<nact, 128, 0, st>>>(G, devs, dact, 0, daxes, naxis);
+        for (int stage = 1; stage <= 2; stage++) {
+            /* grid.y carries the events; more than 65535 go in slices */
+            for (int a0 = 0; a0 < nact; a0 += 65535) {
+                const int na = nact - a0 < 65535 ? nact - a0 : 65535;
+                const dim3 grid((unsigned)((nwin[stage - 1] + kLocBlock - 1) / kLocBlock), na);
+                if (daxes) loc_refine<<<grid, kLocBlock, 0, st>>>(G, dlist, devs, dact + a0, daxes, naxis);
+                else loc_refine_fp64<<<grid, kLocBlock, 0, st>>>(G, dlist, devs, dact + a0);
+            }
+            loc_plan<<<nact, 128, 0, st>>>(G, devs, dact, stage, stage == 1 ? daxes : nullptr, naxis);
         }
-        loc_plan<<<tb, 128, 0, st>>>(G, devs, dact, nact, 1);
-        for (int a0 = 0; a0 < nact; a0 += 65535) {
-            const int na = nact - a0 < 65535 ? nact - a0 : 65535;
-            loc_refine<<<dim3((unsigned)((nwin2 + kLocBlock - 1) / kLocBlock), na), kLocBlock, 0, st>>>(
-                G, dobs, dgood, devs, dact + a0);
-        }
-        loc_plan<<<tb, 128, 0, st>>>(G, devs, dact, nact, 2);
-        loc_finish<<<tb, 128, 0, st>>>(G, dobs, dgood, devs, dact, nact, dres, dtps);
+        loc_finish<<<tw, 128, 0, st>>>(G, dobs, dgood, devs, dact, nact, dres, dtps);
         loc_states<<<(nev + 127) / 128, 128, 0, st>>>(devs, nev, dstate);
         LOC_CU(cudaGetLastError());
         LOC_CU(cudaMemcpyAsync(state.data(), dstate, sizeof(int) * nev, cudaMemcpyDeviceToHost, st));
