@@ -6,7 +6,7 @@
  * Why: FP64 instructions issue once in 64 cycles per scheduler here and a double-double sine takes some 250 of
  * them; 64-bit integer products are four full-rate instructions.
  *
- * Method: unsigned 128-bit fixed point (fdx_u: hi, lo), a value v at scale s held as v 2^s.
+ * Method: unsigned 128-bit fixed point (fdx_u), a value v at scale s held as v 2^s.
  *  - sin, cos: x = k pi/128 + r exactly to 2^-111, |r| <= pi/256; 1 - cos r and sin r from their Taylor series with
  *    w = r^2, the leading terms in two words and the later ones, which are below 2^-21, in one word or half of one;
  *    then the addition theorem with a table of sin(j pi/128), j = 0..64.
@@ -30,9 +30,7 @@
 #define FDX_TABLE static const
 #endif
 
-typedef struct {
-    uint64_t hi, lo;
-} fdx_u;
+typedef unsigned __int128 fdx_u;
 
 /* sin(j pi/128) at scale 126 */
 FDX_TABLE uint64_t fdx_sin_table[65][2] = {
@@ -132,62 +130,22 @@ FDX_FN int fdx_clz(uint64_t a)   /* a != 0 */
 #endif
 }
 
-FDX_FN fdx_u fdx_make(uint64_t hi, uint64_t lo)
-{
-    fdx_u r;
-    r.hi = hi;
-    r.lo = lo;
-    return r;
-}
+FDX_FN fdx_u fdx_make(uint64_t hi, uint64_t lo) { return ((fdx_u)hi << 64) | lo; }
+FDX_FN uint64_t fdx_hi(fdx_u a) { return (uint64_t)(a >> 64); }
+FDX_FN uint64_t fdx_lo(fdx_u a) { return (uint64_t)a; }
 
-FDX_FN fdx_u fdx_add(fdx_u a, fdx_u b)
-{
-    fdx_u r;
-    r.lo = a.lo + b.lo;
-    r.hi = a.hi + b.hi + (r.lo < a.lo);
-    return r;
-}
+/* -a if neg */
+FDX_FN fdx_u fdx_neg_if(fdx_u a, int neg) { return neg ? -a : a; }
 
-FDX_FN fdx_u fdx_sub(fdx_u a, fdx_u b)
-{
-    fdx_u r;
-    r.lo = a.lo - b.lo;
-    r.hi = a.hi - b.hi - (a.lo < b.lo);
-    return r;
-}
-
-FDX_FN fdx_u fdx_shl(fdx_u a, int n)   /* 0 < n < 64 */
-{
-    return fdx_make((a.hi << n) | (a.lo >> (64 - n)), a.lo << n);
-}
-
-FDX_FN fdx_u fdx_shr(fdx_u a, int n)   /* 0 < n < 64 */
-{
-    return fdx_make(a.hi >> n, (a.lo >> n) | (a.hi << (64 - n)));
-}
-
-/* a 2^n for a one-word a, 0 < n < 64 */
-FDX_FN fdx_u fdx_word_shl(uint64_t a, int n) { return fdx_make(a >> (64 - n), a << n); }
-
-/* two's complement: -a if neg */
-FDX_FN fdx_u fdx_neg_if(fdx_u a, int neg)
-{
-    const uint64_t m = neg ? ~0ull : 0ull;
-    fdx_u r;
-    r.lo = (a.lo ^ m) - m;
-    r.hi = (a.hi ^ m) + (neg && r.lo == 0);
-    return r;
-}
-
-FDX_FN fdx_u fdx_mul_ww(uint64_t a, uint64_t b) { return fdx_make(fdx_mulhi(a, b), a * b); }
+FDX_FN fdx_u fdx_mul_ww(uint64_t a, uint64_t b) { return (fdx_u)a * b; }
 
 /* floor(w a / 2^64), within 1 */
-FDX_FN fdx_u fdx_mul_wu(uint64_t w, fdx_u a) { return fdx_add(fdx_mul_ww(w, a.hi), fdx_make(0, fdx_mulhi(w, a.lo))); }
+FDX_FN fdx_u fdx_mul_wu(uint64_t w, fdx_u a) { return fdx_mul_ww(w, fdx_hi(a)) + fdx_mulhi(w, fdx_lo(a)); }
 
 /* a b / 2^128, within 3 */
 FDX_FN fdx_u fdx_mul_uu(fdx_u a, fdx_u b)
 {
-    return fdx_add(fdx_add(fdx_mul_ww(a.hi, b.hi), fdx_make(0, fdx_mulhi(a.hi, b.lo))), fdx_make(0, fdx_mulhi(a.lo, b.hi)));
+    return fdx_mul_ww(fdx_hi(a), fdx_hi(b)) + fdx_mulhi(fdx_hi(a), fdx_lo(b)) + fdx_mulhi(fdx_lo(a), fdx_hi(b));
 }
 
 FDX_FN uint64_t fdx_bits(double v)
@@ -200,14 +158,14 @@ FDX_FN uint64_t fdx_bits(double v)
 /* (-1)^neg v 2^-scale rounded to double; 0 if a midpoint of doubles lies within 2^guard of v */
 FDX_FN int fdx_round(fdx_u v, int neg, int scale, int guard, double *out)
 {
-    if (v.hi == 0) return 0;
-    const int lz = fdx_clz(v.hi);
+    if (fdx_hi(v) == 0) return 0;
+    const int lz = fdx_clz(fdx_hi(v));
     if (guard + lz >= 73) return 0;
-    const fdx_u t = lz ? fdx_shl(v, lz) : v;
-    const uint64_t rest = (t.hi << 53) | (t.lo >> 11);   /* below the last place of the result; half a place is 2^63 */
+    const fdx_u t = lz ? (v << lz) : v;
+    const uint64_t rest = (fdx_hi(t) << 53) | (fdx_lo(t) >> 11);   /* below the last place of the result; half a place is 2^63 */
     const uint64_t near = (guard + lz > 11 ? 1ull << (guard + lz - 11) : 1ull) + 2;
     if (rest - (0x8000000000000000ull - near) <= 2 * near) return 0;
-    const uint64_t u = ((uint64_t)(1023 + 127 - 1 - scale - lz) << 52) + (t.hi >> 11) + (rest >> 63) + ((uint64_t)neg << 63);
+    const uint64_t u = ((uint64_t)(1023 + 127 - 1 - scale - lz) << 52) + (fdx_hi(t) >> 11) + (rest >> 63) + ((uint64_t)neg << 63);
     memcpy(out, &u, sizeof u);
     return 1;
 }
@@ -223,40 +181,40 @@ FDX_FN int fdx_sincos(double x, double *s, double *c)
     /* |x| at scale 120: m 2^(68 + e) */
     const int sh = 68 + e;
     const fdx_u X = sh >= 64 ? fdx_make(m << (sh - 64), 0) : fdx_make(m >> (64 - sh), m << sh);
-    /* k = |x| 128/pi to the nearest: X.hi at scale 56 times 128/pi at scale 57 */
-    const unsigned k = (unsigned)((fdx_mulhi(X.hi, 0x517cc1b727220a95ull) + (1ull << 48)) >> 49);
-    const fdx_u kp = fdx_add(fdx_make(k * 0x0006487ed5110b46ull, 0), fdx_mul_ww(k, 0x11a62633145c06e1ull));
-    fdx_u r = fdx_sub(X, kp);
-    const int rneg = (int)(r.hi >> 63);
+    /* k = |x| 128/pi to the nearest: fdx_hi(X) at scale 56 times 128/pi at scale 57 */
+    const unsigned k = (unsigned)((fdx_mulhi(fdx_hi(X), 0x517cc1b727220a95ull) + (1ull << 48)) >> 49);
+    const fdx_u kp = fdx_make(0x0006487ed5110b46ull, 0x11a62633145c06e1ull) * k;
+    fdx_u r = X - kp;
+    const int rneg = (int)(fdx_hi(r) >> 63);
     r = fdx_neg_if(r, rneg);
     /* w = r^2 at scale 140, its first word wh at scale 76, w32 at scale 44 */
-    const uint64_t rh = (r.hi << 14) | (r.lo >> 50), rl = r.lo << 14;   /* scales 70 and 134 */
+    const uint64_t rh = (fdx_hi(r) << 14) | (fdx_lo(r) >> 50), rl = fdx_lo(r) << 14;   /* scales 70 and 134 */
     const uint64_t cross = fdx_mulhi(rh, rl);
-    const fdx_u W = fdx_add(fdx_mul_ww(rh, rh), fdx_make(cross >> 63, cross << 1));
-    const uint64_t wh = W.hi;
+    const fdx_u W = fdx_mul_ww(rh, rh) + ((fdx_u)cross << 1);
+    const uint64_t wh = fdx_hi(W);
     const uint32_t w32 = (uint32_t)(wh >> 32);
     /* 1 - cos r = w/2 - w^2 (1/4! - w (1/6! - w (1/8! - w/10!))) at scale 124 */
     const uint32_t u1 = 0xd00d00d0u - (fdx_mulhi32(0x93f27dbcu, w32) >> 18);
     const uint64_t u2 = 0xb60b60b60b60b60bull - (((uint64_t)w32 * u1) >> 18);
     const uint64_t u3 = 0xaaaaaaaaaaaaaaabull - (fdx_mulhi(wh, u2) >> 17);
     const uint64_t u4 = fdx_mulhi(fdx_mulhi(wh, wh), u3);   /* scale 92 */
-    const fdx_u V = fdx_sub(fdx_shr(W, 17), fdx_word_shl(u4, 32));
+    const fdx_u V = (W >> 17) - ((fdx_u)u4 << 32);
     /* sin |r| = r - r w (1/3! - w (1/5! - w (1/7! - w/9!))) at scale 124 */
     const uint32_t v1 = 0xd00d00d0u - (fdx_mulhi32(0xb8ef1d2bu, w32) >> 18);
     const uint64_t v2 = 0x8888888888888889ull - (((uint64_t)w32 * v1) >> 18);
     const uint64_t v3 = 0xaaaaaaaaaaaaaaabull - (fdx_mulhi(wh, v2) >> 16);
     const uint64_t rz = fdx_mulhi(rh, fdx_mulhi(wh, v3));   /* scale 84 */
-    const fdx_u sr = fdx_sub(fdx_shl(r, 4), fdx_word_shl(rz, 40));
+    const fdx_u sr = (r << 4) - ((fdx_u)rz << 40);
     /* sin and cos of i pi/128 + r, i = k mod 64, at scale 122 */
     const int i = (int)(k & 63), q = (int)((k >> 6) & 3);
     const fdx_u A = fdx_make(fdx_sin_table[i][0], fdx_sin_table[i][1]);
     const fdx_u B = fdx_make(fdx_sin_table[64 - i][0], fdx_sin_table[64 - i][1]);
-    fdx_u s0 = fdx_sub(fdx_shr(A, 4), fdx_mul_uu(A, V));
-    fdx_u c0 = fdx_sub(fdx_shr(B, 4), fdx_mul_uu(B, V));
+    fdx_u s0 = (A >> 4) - fdx_mul_uu(A, V);
+    fdx_u c0 = (B >> 4) - fdx_mul_uu(B, V);
     const fdx_u bs = fdx_mul_uu(B, sr), as = fdx_mul_uu(A, sr);
-    s0 = fdx_add(s0, fdx_neg_if(bs, rneg));
-    c0 = fdx_add(c0, fdx_neg_if(as, !rneg));
-    const int sneg = (int)(s0.hi >> 63), cneg = (int)(c0.hi >> 63);   /* below 0 by r */
+    s0 += fdx_neg_if(bs, rneg);
+    c0 += fdx_neg_if(as, !rneg);
+    const int sneg = (int)(fdx_hi(s0) >> 63), cneg = (int)(fdx_hi(c0) >> 63);   /* below 0 by r */
     s0 = fdx_neg_if(s0, sneg);
     c0 = fdx_neg_if(c0, cneg);
     const int odd = q & 1;
@@ -277,30 +235,30 @@ FDX_FN int fdx_atan2(double y, double x, double *out)
     const uint64_t a = ((ua & 0xfffffffffffffull) | 0x10000000000000ull) << 10;
     const uint64_t bm = ((ub & 0xfffffffffffffull) | 0x10000000000000ull) << 10;
     const fdx_u b = d ? fdx_make(bm >> d, bm << (64 - d)) : fdx_make(bm, 0);
-    const float t0 = (float)(uint32_t)(b.hi >> 32) / (float)(uint32_t)(a >> 32);
+    const float t0 = (float)(uint32_t)(fdx_hi(b) >> 32) / (float)(uint32_t)(a >> 32);
     const int k = (int)(atanf(t0) * 40.743665f + 0.5f);
     const fdx_u S = fdx_make(fdx_sin_table[k][0], fdx_sin_table[k][1]);
     const fdx_u C = fdx_make(fdx_sin_table[64 - k][0], fdx_sin_table[64 - k][1]);
     /* numerator and denominator at scale 124; t <= tan(pi/256 + 2^-20) */
-    fdx_u N = fdx_sub(fdx_mul_uu(b, C), fdx_mul_wu(a, S));
-    const fdx_u D = fdx_add(fdx_mul_wu(a, C), fdx_mul_uu(b, S));
-    const int nneg = (int)(N.hi >> 63);
+    fdx_u N = fdx_mul_uu(b, C) - fdx_mul_wu(a, S);
+    const fdx_u D = fdx_mul_wu(a, C) + fdx_mul_uu(b, S);
+    const int nneg = (int)(fdx_hi(N) >> 63);
     N = fdx_neg_if(N, nneg);
     /* y2 = 1/D at scale 62 within 2^-58 of it, from a float and two Newton steps on dh = D at scale 62 */
-    const uint64_t dh = (D.hi << 2) | (D.lo >> 62);
+    const uint64_t dh = (fdx_hi(D) << 2) | (fdx_lo(D) >> 62);
     const uint64_t y0 = (uint64_t)(uint32_t)(1152921504606846976.0f / (float)(uint32_t)(dh >> 32)) << 32;
     const int64_t e0 = (int64_t)((1ull << 60) - fdx_mulhi(dh, y0));
     const uint64_t y1 = y0 + (uint64_t)fdx_mulhi_s((int64_t)y0, e0 * 16);
     const int64_t e1 = (int64_t)((1ull << 60) - fdx_mulhi(dh, y1));
     const uint64_t y2 = y1 + (uint64_t)fdx_mulhi_s((int64_t)y1, e1 * 16);
     /* t = q0 + remainder / D, at scale 123 */
-    const uint64_t q0 = fdx_mulhi((N.hi << 8) | (N.lo >> 56), y2);   /* scales 68 + 62 - 64 */
-    const fdx_u rem = fdx_sub(fdx_shl(N, 2), fdx_mul_wu(q0, D));     /* scale 126 */
-    const int64_t rem2 = (int64_t)((rem.hi << 62) | (rem.lo >> 2));  /* scale 124 */
+    const uint64_t q0 = fdx_mulhi((fdx_hi(N) << 8) | (fdx_lo(N) >> 56), y2);   /* scales 68 + 62 - 64 */
+    const fdx_u rem = (N << 2) - fdx_mul_wu(q0, D);     /* scale 126 */
+    const int64_t rem2 = (int64_t)((fdx_hi(rem) << 62) | (fdx_lo(rem) >> 2));  /* scale 124 */
     const int64_t t1 = 2 * fdx_mulhi_s(rem2, (int64_t)y2);
-    const fdx_u t = fdx_add(fdx_word_shl(q0, 57), fdx_make((uint64_t)(t1 >> 63), (uint64_t)t1));
+    const fdx_u t = ((fdx_u)q0 << 57) + (fdx_u)(__int128)t1;
     /* atan t = t - t w (1/3 - w (1/5 - w (1/7 - w (1/9 - w (1/11 - w/13))))) */
-    const uint64_t th = (t.hi << 11) | (t.lo >> 53);   /* scale 70 */
+    const uint64_t th = (fdx_hi(t) << 11) | (fdx_lo(t) >> 53);   /* scale 70 */
     const uint64_t wh = fdx_mulhi(th, th);
     const uint32_t w32 = (uint32_t)(wh >> 32);
     const uint32_t g1 = 0xba2e8ba3u - (fdx_mulhi32(0x9d89d89eu, w32) >> 12);
@@ -309,10 +267,10 @@ FDX_FN int fdx_atan2(double y, double x, double *out)
     const uint64_t g4 = 0xcccccccccccccccdull - (fdx_mulhi(wh, g3) >> 12);
     const uint64_t g5 = 0xaaaaaaaaaaaaaaabull - (fdx_mulhi(wh, g4) >> 13);
     const uint64_t tz = fdx_mulhi(th, fdx_mulhi(wh, g5));   /* scale 83 */
-    fdx_u v = fdx_sub(t, fdx_word_shl(tz, 40));
-    v = fdx_add(fdx_add(fdx_make((unsigned)k * 0x003243f6a8885a30ull, 0), fdx_mul_ww((unsigned)k, 0x8d313198a2e03707ull)), fdx_neg_if(v, nneg));
-    if (swap) v = fdx_sub(fdx_make(0x0c90fdaa22168c23ull, 0x4c4c6628b80dc1cdull), v);
-    if (ux >> 63) v = fdx_sub(fdx_make(0x1921fb54442d1846ull, 0x9898cc51701b839aull), v);
+    fdx_u v = t - ((fdx_u)tz << 40);
+    v = fdx_make(0x003243f6a8885a30ull, 0x8d313198a2e03707ull) * (unsigned)k + fdx_neg_if(v, nneg);
+    if (swap) v = fdx_make(0x0c90fdaa22168c23ull, 0x4c4c6628b80dc1cdull) - v;
+    if (ux >> 63) v = fdx_make(0x1921fb54442d1846ull, 0x9898cc51701b839aull) - v;
     return fdx_round(v, (int)(uy >> 63), 123, 44, out);
 }
 
