@@ -3,8 +3,8 @@
  * slowness derivatives on the coarse metagrid (reference src/sphrayderv.c:1054-2232,
  * lib/sphrayderv/dfind.c, pmin.c), against travel-time fields already on the device.
  *
- * A lane traces a ray: a ray is a chain of dependent cell crossings, and the observations of a run
- * are independent.  A second warp beside it adds the segments to the rays' derivative lists.  Every intermediate keeps the C type the reference gives it (the type
+ * Two lanes trace a ray: a ray is a chain of dependent cell crossings, and the observations of a run
+ * are independent.  Another warp beside them adds the segments to the rays' derivative lists.  Every intermediate keeps the C type the reference gives it (the type
  * decides the rounding), the build has no fused multiply-add contraction, and sin/cos/atan2 are
  * correctly rounded (fd_trig_fx.h, fd_trig.h), so the results are bit-identical to the oracle's
  * double-double mode.  A ray's derivatives go to its own list of (coarse node, value) in the order
@@ -72,61 +72,80 @@ __device__ __noinline__ double atan2_rn(double y, double x)
 /* (int) of a double as x86-64 converts it: truncation, INT_MIN for NaN and out-of-range values */
 __device__ __forceinline__ int trunc_i(double v)
 {
-    if (!(v > -2147483649.0 && v < 2147483648.0)) return INT_MIN;
-    return (int)v;
+    return ((__double2hiint(v) >> 20) & 2047) >= 1023 + 31 ? INT_MIN : (int)v;
 }
 
-__device__ __forceinline__ double pmin(double d1, double d2)
+/* v < 0, v > 0, v != 0 by the bits: a comparison in FP64 takes as long as a product */
+__device__ __forceinline__ bool below0(double v)
+{
+    const unsigned long long u = __double_as_longlong(v);
+    return u > 0x8000000000000000ull && u <= 0xfff0000000000000ull;
+}
+__device__ __forceinline__ bool above0(double v)
+{
+    const unsigned long long u = __double_as_longlong(v);
+    return u != 0 && u <= 0x7ff0000000000000ull;
+}
+__device__ __forceinline__ bool not0(double v) { return __double_as_longlong(v) << 1 != 0; }
+
+/* The distances to a cell's three walls are floats, zero or more, or "none", which the reference writes as the double
+ * -1e20 (lib/sphrayderv/pmin.c, dfind.c) and which is kNone here */
+constexpr float kNone = -1.f;
+
+__device__ __forceinline__ float pmin(float d1, float d2)
 {
     if (d1 >= 0) return (d2 >= 0) ? (d1 < d2 ? d1 : d2) : d1;
-    return d2 >= 0 ? d2 : -1e20;
+    return d2 >= 0 ? d2 : kNone;
 }
 
-__device__ __forceinline__ void dfind(const double dd[3], double *d, int *md, double tolmin, double tolmax)
+/* the order of the distances' magnitudes, 1e20 for none */
+__device__ __forceinline__ unsigned magnitude(float d)
 {
-    int mn, mid, mx;
-    const double a0 = fabs(dd[0]), a1 = fabs(dd[1]), a2 = fabs(dd[2]);
-    if (a0 <= a1 && a0 <= a2) {
-        mn = 0;
-        if (a1 <= a2) { mid = 1; mx = 2; } else { mid = 2; mx = 1; }
-    } else if (a1 <= a2) {
-        mn = 1;
-        if (a0 <= a2) { mid = 0; mx = 2; } else { mid = 2; mx = 0; }
-    } else {
-        mn = 2;
-        if (a0 <= a1) { mid = 0; mx = 1; } else { mid = 1; mx = 0; }
-    }
-    *d = dd[mn];
-    *md = mn;
-    if (dd[mn] < tolmin) {
-        if (dd[mid] < tolmin) {
-            if (dd[mx] < tolmax) { *d = dd[mx]; *md = mx; }
-            else { *d = dd[mid]; *md = mid; }
-        } else if (dd[mid] < tolmax) {
-            *d = dd[mid];
-            *md = mid;
-        }
-    }
+    return d == kNone ? 2u * 0x60ad78ecu - 1u : 2u * (__float_as_uint(d) & 0x7fffffffu);
 }
 
-/* corner indices of fine cell (ie, je, ke); false if one falls outside the field */
-__device__ __forceinline__ bool corners(const RayGridDev &g, int ie, int je, int ke, long long ipt[8])
+/* tolmin, tolmax: rounded up to float, which compares with floats as the double itself */
+__device__ __forceinline__ void dfind(const float dd[3], float *d, int *md, float tolmin, float tolmax)
+{
+    const unsigned a0 = magnitude(dd[0]), a1 = magnitude(dd[1]), a2 = magnitude(dd[2]);
+    const int mn = a0 <= a1 && a0 <= a2 ? 0 : a1 <= a2 ? 1 : 2;
+    int mid, mx;
+    if (mn == 0) {
+        mid = a1 <= a2 ? 1 : 2;
+        mx = 3 - mid;
+    } else if (mn == 1) {
+        mid = a0 <= a2 ? 0 : 2;
+        mx = 2 - mid;
+    } else {
+        mid = a0 <= a1 ? 0 : 1;
+        mx = 1 - mid;
+    }
+    auto at = [&](int q) { return q == 0 ? dd[0] : q == 1 ? dd[1] : dd[2]; };
+    int m = mn;
+    if (at(mn) < tolmin) {
+        if (at(mid) < tolmin) m = at(mx) < tolmax ? mx : mid;
+        else if (at(mid) < tolmax) m = mid;
+    }
+    *d = at(m);
+    *md = m;
+}
+
+/* the times at the corners of fine cell (ie, je, ke); false if one falls outside the field */
+__device__ __forceinline__ bool corners(const RayGridDev &g, const float *t, int ie, int je, int ke, float tv[8])
 {
     const long long nxy = (long long)g.nx * g.ny, n = nxy * g.nz;
-    const long long nk = nxy * ke, nj = (long long)g.nx * je, nk2 = nxy * ((long long)ke + 1),
-                    nj2 = (long long)g.nx * ((long long)je + 1);
-    ipt[0] = nk + nj + ie;
-    ipt[1] = nk + nj + ie + 1;
-    ipt[2] = nk + nj2 + ie;
-    ipt[3] = nk + nj2 + ie + 1;
-    ipt[4] = nk2 + nj + ie;
-    ipt[5] = nk2 + nj + ie + 1;
-    ipt[6] = nk2 + nj2 + ie;
-    ipt[7] = nk2 + nj2 + ie + 1;
-    bool ok = true;
-#pragma unroll
-    for (int q = 0; q < 8; q++) ok = ok && ipt[q] >= 0 && ipt[q] < n;
-    return ok;
+    const long long at = nxy * ke + (long long)g.nx * je + ie;   /* the smallest index */
+    if (at < 0 || at + nxy + g.nx + 1 >= n) return false;
+    const float *c = t + at, *c2 = c + nxy;
+    tv[0] = c[0];
+    tv[1] = c[1];
+    tv[2] = c[g.nx];
+    tv[3] = c[g.nx + 1];
+    tv[4] = c2[0];
+    tv[5] = c2[1];
+    tv[6] = c2[g.nx];
+    tv[7] = c2[g.nx + 1];
+    return true;
 }
 
 /* sin and cos of the cell-wall angles a ray meets: rows y(j) = dq j + y0 and y(j) + dq, columns
@@ -155,39 +174,23 @@ __global__ void ray_wall_trig(RayGridDev g, double4 *row, double4 *col)
     }
 }
 
-/* (sin, cos) of y(je) (second = 0) or y(je) + dq (second = 1); a direct call off the table */
-__device__ __forceinline__ void row_trig(const RayGridDev &g, const WallTrig &w, int je, int second, double *sn,
-                                         double *cs)
+/* a table's row, or a direct call off the table */
+__device__ __forceinline__ double4 walls(const double4 *table, int n, int i, double step, double origin)
 {
-    if (je >= 0 && je <= g.ny) {
-        const double4 v = w.row[je];
-        *sn = second ? v.z : v.x;
-        *cs = second ? v.w : v.y;
-        return;
-    }
-    const double yj = g.dq * je + g.y0;
-    sincos_rn(second ? yj + g.dq : yj, sn, cs);
+    if (i >= 0 && i <= n) return table[i];
+    const double a = step * i + origin;
+    double4 v;
+    sincos_rn(a, &v.x, &v.y);
+    sincos_rn(a + step, &v.z, &v.w);
+    return v;
 }
 
-__device__ __forceinline__ void col_trig(const RayGridDev &g, const WallTrig &w, int ie, int second, double *sn,
-                                         double *cs)
-{
-    if (ie >= 0 && ie <= g.nx) {
-        const double4 v = w.col[ie];
-        *sn = second ? v.z : v.x;
-        *cs = second ? v.w : v.y;
-        return;
-    }
-    const double xi = g.df * ie + g.x0;
-    sincos_rn(second ? xi + g.df : xi, sn, cs);
-}
-
-/* A block traces 32 rays: warp 0 steps them, a ray a lane, and hands its segments through shared memory to warp 1,
- * which adds them to the rays' derivative lists meanwhile, four rays at a time with a lane per corner of the
+/* A block traces 32 rays: warps 0 and 1 step them, two lanes a ray, and hand the segments through shared memory to
+ * warp 2, which adds them to the rays' derivative lists meanwhile, four rays at a time with a lane per corner of the
  * coarse cell.  A round is kRound segments of every ray; the warps change buffers at its end.  With one lane doing
  * both, and sorting its list at the end, the lists took two thirds of the time (scattered searches, and an insertion
  * sort whose lanes wait for the longest): 8192 rays in 201x201x81 24.7 -> 9.7 ms. */
-constexpr int kRays = 32, kRound = 8, kRayBlock = 64;
+constexpr int kRays = 32, kRound = 8, kRayBlock = 96;
 constexpr int kMaxCoarse = 8192;   /* coarse coordinates of the three axes */
 constexpr int kSeen = 4096;   /* bits of a ray's filter of listed nodes */
 
@@ -223,7 +226,7 @@ __device__ __forceinline__ int coarse_cell(const float *g, int n, float v, unsig
     return 1;   /* not reached: the tracer ends a ray whose midpoint has no cell */
 }
 
-/* Warp 1: adds buffer `buf` to the lists.  A ray crosses several fine cells per coarse cell, and every segment in
+/* Warp 2: adds buffer `buf` to the lists.  A ray crosses several fine cells per coarse cell, and every segment in
  * one coarse cell adds to the same eight nodes: the lanes keep their sums.  On entering the next cell the
  * nodes that it shares with the last one come from the neighbour lanes; the others are new unless the filter
  * has seen them (4 % of the time by chance), when the list is searched. */
@@ -336,18 +339,30 @@ __device__ __forceinline__ float coarse_end(const float *g, int n)
     return m;
 }
 
-/* Warp 0: the rays, a ray a lane */
+__device__ __forceinline__ double other(double v) { return __shfl_xor_sync(0xffffffffu, v, 1); }
+__device__ __forceinline__ float other(float v) { return __shfl_xor_sync(0xffffffffu, v, 1); }
+__device__ __forceinline__ int other(int v) { return __shfl_xor_sync(0xffffffffu, v, 1); }
+
+/* Warps 0 and 1: the rays.  A segment is a chain of some 430 FP64 instructions, each of which takes its scheduler 64
+ * cycles for one lane as for 32, and of 1800 others for its two sincos and two atan2.  The two lanes of a ray hold the
+ * same state; where two of the chain's steps are the same operation on other operands (longitude and colatitude,
+ * the two sines of a gradient's denominators, the wall of constant colatitude and that of constant radius,
+ * whose equation has a = 1) each lane takes one, and they exchange the results: `second` is the lane's role.  Idle
+ * pairs step along on harmless values, without jumps, so that every exchange is one of whole warps.
+ * 8192 rays in 201x201x81: 9.5 -> 6.0 ms against a ray a lane. */
 __device__ __forceinline__ void trace_rays(const RayGridDev &g, const WallTrig &wt, const float *gx, const float *gy, const float *gz,
                                            RaySums &sh, const RayObsDev *obs, int nrays, int max_seg, fdgpu_ray_result &r)
 {
-    const int lane = threadIdx.x & 31;
-    const bool mine = lane < nrays;
-    const RayObsDev ob = obs[mine ? lane : 0];
+    const int ray = threadIdx.x >> 1;
+    const bool second = threadIdx.x & 1, mine = ray < nrays;
+    const RayObsDev ob = obs[mine ? ray : 0];
     const float xend = coarse_end(gx, g.nxc), yend = coarse_end(gy, g.nyc), zend = coarse_end(gz, g.nzc);
     const float *t = ob.t;
     const double x0 = g.x0, y0 = g.y0, z0 = g.z0, h = g.h, dq = g.dq, df = g.df;
     const int nx = g.nx, ny = g.ny, nz = g.nz;
-    const double tolmin = h * 1.E-6f, tolmax = h * 6.0f;
+    const float tolmin = __double2float_ru(h * 1.E-6f), tolmax = __double2float_ru(h * 6.0f);
+    const double hmil = h / 1000.f, df4 = 4 * df, dq4 = 4 * dq, h4 = 4 * h;
+    const float hmilf = __double2float_ru(hmil);
     const double xs = ob.xs, ys = ob.ys, zs = ob.zs;
     const int is = (int)round((xs - x0) / df), js = (int)round((ys - y0) / dq), ks = (int)round((zs - z0) / h);
     const int iscell = trunc_i((xs - x0) / df), jscell = trunc_i((ys - y0) / dq), kscell = trunc_i((zs - z0) / h);
@@ -357,21 +372,20 @@ __device__ __forceinline__ void trace_rays(const RayGridDev &g, const WallTrig &
 
     double xx = ex, yy = ey, zz = ez;
     int ie = ies, je = jes, ke = kes;
-    double xi = xis, yj = yjs, zk = zks;
-    long long ipt[8];
     int nseg = 0;
     bool live = false;
     float x2, y2, z2;   /* the station in the cartesian frame, for the last cells (src/sphrayderv.c:1812-1817) */
     do {
         if (!mine) break;
-        if (!corners(g, ie, je, ke, ipt)) { r.status = FDGPU_RAY_OUTSIDE; break; }
+        float tc8[8];
+        if (!corners(g, t, ie, je, ke, tc8)) { r.status = FDGPU_RAY_OUTSIDE; break; }
         bool notime = false;
-        for (int q = 0; q < 8; q++) notime = notime || t[ipt[q]] > 1.E9;
+        for (int q = 0; q < 8; q++) notime = notime || tc8[q] > 1.E9;
         if (notime) { r.status = FDGPU_RAY_NOTIME; break; }
 
         /* residual and hypocentre derivatives at the event (src/sphrayderv.c:1366-1441) */
         {
-            const double fx = (xx - xi) / df, fy = (yy - yj) / dq, fz = (zz - zk) / h;
+            const double fx = (xx - xis) / df, fy = (yy - yjs) / dq, fz = (zz - zks) / h;
             float ds[8];
             ds[0] = (1.f - fz) * (1.f - fy) * (1.f - fx);
             ds[1] = (1.f - fz) * (1.f - fy) * fx;
@@ -381,8 +395,6 @@ __device__ __forceinline__ void trace_rays(const RayGridDev &g, const WallTrig &
             ds[5] = fz * (1.f - fy) * fx;
             ds[6] = fz * fy * (1.f - fx);
             ds[7] = fz * fy * fx;
-            float tc8[8];
-            for (int q = 0; q < 8; q++) tc8[q] = t[ipt[q]];
             double dt = 0;
             for (int q = 0; q < 8; q++) dt += ds[q] * tc8[q];
             dt += 0.0f;
@@ -450,215 +462,218 @@ __device__ __forceinline__ void trace_rays(const RayGridDev &g, const WallTrig &
     for (int buf = 0;; buf ^= 1) {
         int count = 0;
         for (int step = 0; step < kRound && __any_sync(0xffffffffu, live); step++) {
-            /* no jump out of a segment's code: the lanes stay together */
-            bool go = live;
-            float dxs, dys, dzs;
-            double dlen, sinq, cosq;
-            float tv[8];
-            if (go) {
-                xi = df * ie + x0;
-                yj = dq * je + y0;
-                zk = h * ke + z0;
-                dxs = xx - xs, dys = yy - ys, dzs = zz - zs;
-                const float rs = kRearth - zz;
-                const float dqs = rs * dys;
-                sincos_rn(yy, &sinq, &cosq);
-                const float dfs = rs * sinq * dxs;
-                const float float_dlen = sqrtf(dfs * dfs + dqs * dqs + dzs * dzs);
-                dlen = float_dlen;
-                if ((ie == iscell && je == jscell && ke == kscell) || (dlen < (h / 1000.f))) {
-                    const float xm = xx - dxs * 0.5f, ym = yy - dys * 0.5f, zm = zz - dzs * 0.5f;
-                    go = false;
-                    if (xm < xend && ym < yend && zm < zend) {
-                        sh.seg[buf][count++][lane] = make_float4(xm, ym, zm, float_dlen);
-                        r.status = FDGPU_RAY_OK;
+            if (!live) {
+                xx = yy = 1.;
+                zz = 0.;
+                ie = je = ke = 0;
+            }
+            const double zk = h * ke + z0;
+            double sn, cs;
+            sincos_rn(second ? xx : yy, &sn, &cs);
+            const double sno = other(sn), cso = other(cs);
+            const double sinq = second ? sno : sn, cosq = second ? cso : cs;
+            const double sinf_ = second ? sn : sno, cosf_ = second ? cs : cso;
+
+            /* the distance to the station: the last segment in its cell or this near to it */
+            const float du = (second ? xx : yy) - (second ? xs : ys), dzs = zz - zs;
+            const float rs = kRearth - zz;
+            const float dfs1 = rs * sinq * du, dqs1 = rs * du;
+            const float part = second ? dfs1 : dqs1, parto = other(part);
+            const float dfs = second ? part : parto, dqs = second ? parto : part;
+            const float dlen = sqrtf(dfs * dfs + dqs * dqs + dzs * dzs);
+            const bool last = live && ((ie == iscell && je == jscell && ke == kscell) || dlen < hmilf);
+            if (last) {
+                const float mu = (second ? xx : yy) - du * 0.5f, zm = zz - dzs * 0.5f;
+                const unsigned pair = 3u << (threadIdx.x & 30);
+                const bool in = (second ? mu < xend : mu < yend) && zm < zend;
+                if (__all_sync(pair, in)) {
+                    float4 &m = sh.seg[buf][count][ray];
+                    if (second) {
+                        m.x = mu;
                     } else {
-                        r.status = FDGPU_RAY_COARSE;
+                        m.y = mu;
+                        m.z = zm;
+                        m.w = dlen;
                     }
-                } else if (nseg >= max_seg) {
-                    go = false;
-                    r.status = FDGPU_RAY_STEPS;
-                } else if (!corners(g, ie, je, ke, ipt)) {
-                    go = false;
-                    r.status = FDGPU_RAY_OUTSIDE;
+                    count++;
+                    r.status = FDGPU_RAY_OK;
                 } else {
-                    for (int q = 0; q < 8; q++) tv[q] = t[ipt[q]];
+                    r.status = FDGPU_RAY_COARSE;
                 }
-                live = go;
             }
             __syncwarp();
+            bool go = live && !last;
+            float tv[8] = {0.f, 1.f, 2.f, 4.f, 8.f, 16.f, 32.f, 64.f};
+            if (go && nseg >= max_seg) {
+                go = false;
+                r.status = FDGPU_RAY_STEPS;
+            }
+            if (go && !corners(g, t, ie, je, ke, tv)) {
+                go = false;
+                r.status = FDGPU_RAY_OUTSIDE;
+            }
+
+            /* the gradient */
+            const double r1 = kRearth - zk, r2 = r1 - h;
+            const double4 rw = walls(wt.row, g.ny, je, dq, y0), cw = walls(wt.col, g.nx, ie, df, x0);
+            const double sqm = second ? rw.z : rw.x;
+            const double lo = (second ? tv[3] - tv[2] : tv[1] - tv[0]) / (r1 * sqm);
+            const double hi = (second ? tv[7] - tv[6] : tv[5] - tv[4]) / (r2 * sqm);
+            const double fq = (second ? tv[6] + tv[7] - tv[4] - tv[5] : tv[2] + tv[3] - tv[0] - tv[1]) / (second ? r2 : r1);
+            const double loo = other(lo), hio = other(hi), fqo = other(fq);
+            const double sum0 = lo + loo + hi + hio, sum1 = fqo + fq;   /* the first lane's, the second's */
+            const double gd = -((second ? sum1 : sum0) / (second ? dq4 : df4)), gdo = other(gd);
+            double g0 = second ? gdo : gd, g1 = second ? gd : gdo;
+            double g2 = (tv[4] + tv[5] + tv[6] + tv[7] - tv[0] - tv[1] - tv[2] - tv[3]) / h4;
+
+            /* the direction */
+            const double ro = kRearth - zz;
+            const double xo = ro * sinq * cosf_, yo = ro * sinq * sinf_, zo = ro * cosq;
+            const double gm = sqrt(g0 * g0 + g1 * g1 + g2 * g2);
+            const double gu = (second ? g1 : g0) / gm, guo = other(gu);
+            const double sf = second ? guo : gu, sq = second ? gu : guo, sr = g2 / gm;
+            const double u1 = second ? cosf_ : -sinf_, u2 = second ? sinf_ : cosf_;
+            double su = u1 * sf + cosq * u2 * sq + sinq * u2 * sr, suo = other(su);
+            double sz = -sinq * sq + cosq * sr;
+            {
+                const double ax = second ? suo : su, ay = second ? su : suo;
+                const float smag = sqrtf((float)(ax * ax + ay * ay + sz * sz));
+                su /= smag;
+                sz /= smag;
+            }
+            suo = other(su);
+            double sx = second ? suo : su, sy = second ? su : suo;
+            if (ie >= (is - 2) && ie < (is + 2) && je >= (js - 2) && je < (js + 2) && ke >= (ks - 2) && ke < (ks + 2)) {
+                const double dx = x2 - xo, dy = y2 - yo, dz = z2 - zo;
+                const double dl = sqrt(dx * dx + dy * dy + dz * dz);
+                sx = dx / dl;
+                sy = dy / dl;
+                sz = dz / dl;
+            }
+            __syncwarp();
+
+            /* the walls: the first lane takes radius and longitude, the second colatitude */
+            const bool near0 = second ? below0(g1) : below0(g0);
+            const double sinw = second ? (near0 ? rw.x : rw.z) : (near0 ? cw.x : cw.z);
+            const double cosw = second ? (near0 ? rw.y : rw.w) : (near0 ? cw.y : cw.w);
+            const bool big = fabs(cosw) > fabs(sinw);
+            const double tn = (big ? sinw : cosw) / (big ? cosw : sinw), tn2 = tn * tn;
+            const double m1 = second && !big ? tn2 : 1., m2 = second ? (big ? tn2 : 1.) : -1.;
+            const double rwall = above0(g2) ? r1 : r2;
+            const double a = second ? (sx * sx + sy * sy) * m1 - sz * sz * m2 : 1.;
+            const double b = (xo * sx + yo * sy) * m1 - zo * sz * m2;
+            const double c = (xo * xo + yo * yo) * m1 - zo * zo * m2 - (second ? 0. : rwall * rwall);
+            const double quad = b * b - a * c, root = sqrt(quad);
+            const double n1 = -b + root, n2 = -b - root;
+            const double lin = big ? xo * tn - yo : yo * tn - xo, lden = big ? sy - sx * tn : sx - sy * tn;
+            const float v1 = (second ? n1 : lin) / (second ? a : lden);
+            const float v2 = n2 / a;
+            float du_ = kNone, dl_ = kNone;
+            if (not0(second ? g1 : g2) && quad >= 0) du_ = pmin(second ? v1 : (float)n1, v2);
+            if (not0(g0) && v1 > 0) dl_ = v1;   /* the first lane's */
+            const float duo = other(du_);
+            float dd[3] = {__shfl_sync(0xffffffffu, dl_, threadIdx.x & 30), second ? du_ : duo, second ? duo : du_};
+
+            const int back3 = iseg + isegm1 + isegm2;
+            if (below0(g0)) {
+                if (dd[0] < hmilf && (iseg == 1 || (back3 == 1 && nseg >= 3))) { g0 = 0.; dd[0] = kNone; }
+            } else if (above0(g0)) {
+                if (dd[0] < hmilf && (iseg == -1 || (back3 == -1 && nseg >= 3))) { g0 = 0; dd[0] = kNone; }
+            } else {
+                dd[0] = kNone;
+            }
+            if (below0(g1)) {
+                if (dd[1] < hmilf && (iseg == 20 || (back3 == 20 && nseg >= 3))) { g1 = 0.; dd[1] = kNone; }
+            } else if (above0(g1)) {
+                if (dd[1] < hmilf && (iseg == -20 || (back3 == -20 && nseg >= 3))) { g1 = 0; dd[1] = kNone; }
+            } else {
+                dd[1] = kNone;
+            }
+            if (above0(g2)) {
+                if (dd[2] < hmilf && (iseg == 300 || (back3 == 300 && nseg >= 3))) { g2 = 0.; dd[2] = kNone; }
+            } else if (below0(g2)) {
+                if (dd[2] < hmilf && (iseg == -300 || (back3 == -300 && nseg >= 3))) { g2 = 0; dd[2] = kNone; }
+            } else {
+                dd[2] = kNone;
+            }
+
+            float dist;
+            int md;
+            dfind(dd, &dist, &md, tolmin, tolmax);
+            const double d = dist == kNone ? -1e20 : (double)dist;
+
+            /* the next point */
+            const double pu = (second ? yo : xo) + d * (second ? sy : sx), puo = other(pu), zn = zo + d * sz;
+            const double xn = second ? puo : pu, yn = second ? pu : puo;
+            const double h2 = xn * xn + yn * yn;
+            const double rt = sqrt(second ? h2 : h2 + zn * zn);
+            const double ang = atan2_rn(second ? rt : yn, second ? zn : xn), ango = other(ang);
+            const double xnew = second ? ango : ang, ynew = second ? ang : ango;
+            const double znew = kRearth - __shfl_sync(0xffffffffu, rt, threadIdx.x & 30);
+            const float mu = ((second ? ynew : xnew) + (second ? yy : xx)) * 0.5, zm = (znew + zz) * 0.5;
+            /* its cell: the two coordinates that no wall gives */
+            const bool byq = second ? md == 2 : md == 0;
+            const double cu = byq ? ynew - y0 : second ? znew - z0 : xnew - x0;
+            const int cell = trunc_i(cu / (byq ? dq : second ? h : df)), cello = other(cell);
+            const int ca = second ? cello : cell, cb = second ? cell : cello;
+            const bool in = (second ? mu < yend : mu < xend) && zm < zend;
+            const bool inside = other((int)in) && in;
             if (go) {
-                const double r1 = kRearth - zk, r2 = r1 - h;
-                double sq1, cq1, sq2, cq2;
-                row_trig(g, wt, je, 0, &sq1, &cq1);   /* q1 = yj */
-                row_trig(g, wt, je, 1, &sq2, &cq2);   /* q2 = yj + dq */
-                double gradt[3];
-                gradt[0] = ((tv[1] - tv[0]) / (r1 * sq1) + (tv[3] - tv[2]) / (r1 * sq2) + (tv[5] - tv[4]) / (r2 * sq1)
-                            + (tv[7] - tv[6]) / (r2 * sq2)) / (4 * df);
-                gradt[1] = ((tv[2] + tv[3] - tv[0] - tv[1]) / r1 + (tv[6] + tv[7] - tv[4] - tv[5]) / r2) / (4 * dq);
-                gradt[2] = (tv[4] + tv[5] + tv[6] + tv[7] - tv[0] - tv[1] - tv[2] - tv[3]) / (4 * h);
-                gradt[0] = gradt[0] * -1;
-                gradt[1] = gradt[1] * -1;
-
-                double sinf_, cosf_;
-                sincos_rn(xx, &sinf_, &cosf_);
-                double ro = kRearth - zz;
-                const double xo = ro * sinq * cosf_, yo = ro * sinq * sinf_, zo = ro * cosq;
-                double sx, sy, sz;
-                if (ie >= (is - 2) && ie < (is + 2) && je >= (js - 2) && je < (js + 2) && ke >= (ks - 2)
-                    && ke < (ks + 2)) {
-                    const double dx = x2 - xo, dy = y2 - yo, dz = z2 - zo;
-                    const double dl = sqrt(dx * dx + dy * dy + dz * dz);
-                    sx = dx / dl;
-                    sy = dy / dl;
-                    sz = dz / dl;
-                } else {
-                    const double gradtm = sqrt(gradt[0] * gradt[0] + gradt[1] * gradt[1] + gradt[2] * gradt[2]);
-                    const double sf = gradt[0] / gradtm, sq = gradt[1] / gradtm, sr = gradt[2] / gradtm;
-                    sx = -sinf_ * sf + cosq * cosf_ * sq + sinq * cosf_ * sr;
-                    sy = cosf_ * sf + cosq * sinf_ * sq + sinq * sinf_ * sr;
-                    sz = -sinq * sq + cosq * sr;
-                    const float smag = sqrtf((float)(sx * sx + sy * sy + sz * sz));
-                    sx /= smag;
-                    sy /= smag;
-                    sz /= smag;
-                }
-
-                double dd[3];
-                double a, b, c, quad;
-                dd[2] = -1e20;
-                if (gradt[2] != 0) {
-                    ro = gradt[2] > 0 ? kRearth - zk : kRearth - zk - h;
-                    b = xo * sx + yo * sy + zo * sz;
-                    c = xo * xo + yo * yo + zo * zo - ro * ro;
-                    quad = b * b - c;
-                    if (quad >= 0) {
-                        const float d1 = -b + sqrt(quad);
-                        const float d2 = -b - sqrt(quad);
-                        dd[2] = pmin(d1, d2);
-                    }
-                }
-                dd[1] = -1e20;
-                if (gradt[1] != 0) {
-                    if (gradt[1] < 0) {
-                        sinq = sq1;
-                        cosq = cq1;
-                    } else {
-                        sinq = sq2;
-                        cosq = cq2;
-                    }
-                    if (fabs(cosq) > fabs(sinq)) {
-                        const double tanq = sinq / cosq, tansq = tanq * tanq;
-                        a = sx * sx + sy * sy - sz * sz * tansq;
-                        b = xo * sx + yo * sy - zo * sz * tansq;
-                        c = xo * xo + yo * yo - zo * zo * tansq;
-                    } else {
-                        const double ctanq = cosq / sinq, ctansq = ctanq * ctanq;
-                        a = (sx * sx + sy * sy) * ctansq - sz * sz;
-                        b = (xo * sx + yo * sy) * ctansq - zo * sz;
-                        c = (xo * xo + yo * yo) * ctansq - zo * zo;
-                    }
-                    quad = b * b - a * c;
-                    if (quad >= 0) {
-                        const float d1 = (-b + sqrt(quad)) / a;
-                        const float d2 = (-b - sqrt(quad)) / a;
-                        dd[1] = pmin(d1, d2);
-                    }
-                }
-                dd[0] = -1e20;
-                if (gradt[0] != 0) {
-                    col_trig(g, wt, ie, gradt[0] < 0 ? 0 : 1, &sinf_, &cosf_);
-                    float d1;
-                    if (fabs(cosf_) > fabs(sinf_)) {
-                        const double tanf_ = sinf_ / cosf_;
-                        d1 = (xo * tanf_ - yo) / (sy - sx * tanf_);
-                    } else {
-                        const double ctanf_ = cosf_ / sinf_;
-                        d1 = (yo * ctanf_ - xo) / (sx - sy * ctanf_);
-                    }
-                    if (d1 > 0) dd[0] = d1;
-                }
-
-                const int back3 = iseg + isegm1 + isegm2;
-                if (gradt[0] < 0) {
-                    if (dd[0] < h / 1000 && (iseg == 1 || (back3 == 1 && nseg >= 3))) { gradt[0] = 0.; dd[0] = -1e20; }
-                } else if (gradt[0] > 0) {
-                    if (dd[0] < h / 1000 && (iseg == -1 || (back3 == -1 && nseg >= 3))) { gradt[0] = 0; dd[0] = -1e20; }
-                } else {
-                    dd[0] = -1e20;
-                }
-                if (gradt[1] < 0) {
-                    if (dd[1] < h / 1000 && (iseg == 20 || (back3 == 20 && nseg >= 3))) { gradt[1] = 0.; dd[1] = -1e20; }
-                } else if (gradt[1] > 0) {
-                    if (dd[1] < h / 1000 && (iseg == -20 || (back3 == -20 && nseg >= 3))) { gradt[1] = 0; dd[1] = -1e20; }
-                } else {
-                    dd[1] = -1e20;
-                }
-                if (gradt[2] > 0) {
-                    if (dd[2] < h / 1000 && (iseg == 300 || (back3 == 300 && nseg >= 3))) { gradt[2] = 0.; dd[2] = -1e20; }
-                } else if (gradt[2] < 0) {
-                    if (dd[2] < h / 1000 && (iseg == -300 || (back3 == -300 && nseg >= 3))) { gradt[2] = 0; dd[2] = -1e20; }
-                } else {
-                    dd[2] = -1e20;
-                }
-
-                double d;
-                int md;
-                dfind(dd, &d, &md, tolmin, tolmax);
-                dlen = d;
-                const double xold = xx, yold = yy, zold = zz;
-                const double xn = xo + d * sx, yn = yo + d * sy, zn = zo + d * sz;
-                xx = atan2_rn(yn, xn);
-                yy = atan2_rn(sqrt(xn * xn + yn * yn), zn);
-                zz = kRearth - sqrt(xn * xn + yn * yn + zn * zn);
+                xx = xnew;
+                yy = ynew;
+                zz = znew;
                 nseg++;
                 isegm2 = isegm1;
                 isegm1 = iseg;
                 bool left = false;
                 if (md == 0) {
-                    je = trunc_i((yy - y0) / dq);
-                    ke = trunc_i((zz - z0) / h);
-                    if (gradt[0] < 0) {
+                    je = ca;
+                    ke = cb;
+                    if (below0(g0)) {
                         if (ie < 0) left = true; else { ie--; iseg = -1; }
                     } else {
                         if (ie >= nx - 1) left = true; else { ie++; iseg = 1; }
                     }
                 } else if (md == 1) {
-                    if (gradt[1] < 0) {
+                    if (below0(g1)) {
                         if (je < 0) left = true; else { je--; iseg = -20; }
                     } else {
                         if (je >= ny - 1) left = true; else { je++; iseg = 20; }
                     }
-                    if (!left) {
-                        ie = trunc_i((xx - x0) / df);
-                        ke = trunc_i((zz - z0) / h);
-                    }
+                    ie = ca;
+                    ke = cb;
                 } else {
-                    if (gradt[2] > 0) {
+                    if (above0(g2)) {
                         if (ke < 0) left = true; else { ke--; iseg = -300; }
                     } else {
                         if (ke >= nz - 1) left = true; else { ke++; iseg = 300; }
                     }
-                    if (!left) {
-                        ie = trunc_i((xx - x0) / df);
-                        je = trunc_i((yy - y0) / dq);
-                    }
+                    ie = ca;
+                    je = cb;
                 }
                 if (left || (xx < x0 || ie >= nx) || (yy < y0 || je >= ny) || (zz < z0 || ke >= nz)) {
                     r.status = FDGPU_RAY_LEFT;
-                    live = false;
-                }
-                const float xm = (xx + xold) * 0.5, ym = (yy + yold) * 0.5, zm = (zz + zold) * 0.5;
-                if (live && !(xm < xend && ym < yend && zm < zend)) {
+                    go = false;
+                } else if (!inside) {
                     r.status = FDGPU_RAY_COARSE;
-                    live = false;
+                    go = false;
+                } else {
+                    float4 &m = sh.seg[buf][count][ray];
+                    if (second) {
+                        m.y = mu;
+                    } else {
+                        m.x = mu;
+                        m.z = zm;
+                        m.w = (float)d;
+                    }
+                    count++;
                 }
-                if (live) sh.seg[buf][count++][lane] = make_float4(xm, ym, zm, (float)dlen);
             }
+            live = go;
             __syncwarp();
         }
-        sh.n[buf][lane] = count;
-        if (__syncthreads_and(!live)) break;   /* the buffer to the other warp */
+        if (!second) sh.n[buf][ray] = count;
+        if (__syncthreads_and(!live)) break;   /* the buffer to the last warp */
     }
     r.nseg = nseg;
 }
@@ -689,7 +704,7 @@ __global__ void __launch_bounds__(kRayBlock) ray_trace(RayGridDev g, WallTrig wt
     sorted = __syncthreads_and(sorted);
     fdgpu_ray_result r;
     memset(&r, 0, sizeof r);
-    if (threadIdx.x < 32) {
+    if (threadIdx.x < 2 * kRays) {
         trace_rays(g, wt, gx, gy, gz, sh, obs + first, nrays, max_seg, r);
     } else {
         for (int b = 0;; b ^= 1) {
@@ -702,15 +717,15 @@ __global__ void __launch_bounds__(kRayBlock) ray_trace(RayGridDev g, WallTrig wt
             if (sh.pos[e >> 3][e & 7] >= 0) lval[(size_t)out[e >> 3] * cap + sh.pos[e >> 3][e & 7]] = sh.sum[e >> 3][e & 7];
     }
     __syncthreads();
-    for (int q = threadIdx.x >> 5; q < nrays; q += 2) {
+    for (int q = threadIdx.x >> 5; q < nrays; q += kRayBlock / 32) {
         int nz = 0;
         for (int e = threadIdx.x & 31; e < sh.len[q]; e += 32) nz += lval[(size_t)out[q] * cap + e] != 0;
         nz = __reduce_add_sync(0xffffffffu, nz);
         if ((threadIdx.x & 31) == 0) sh.nnz[q] = nz;
     }
     __syncthreads();
-    if (threadIdx.x < nrays) {
-        const int q = threadIdx.x;
+    if (threadIdx.x < 2 * nrays && !(threadIdx.x & 1)) {
+        const int q = threadIdx.x >> 1;
         if (r.status == FDGPU_RAY_OK && sh.over[q]) r.status = FDGPU_RAY_STEPS;
         r.nnz = r.status == FDGPU_RAY_OK ? sh.nnz[q] : 0;
         nlist[out[q]] = sh.len[q];
