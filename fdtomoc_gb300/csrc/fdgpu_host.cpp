@@ -95,6 +95,7 @@ struct fdgpu_ctx {
      * record (fdgpu_station bytes): the launch-order table */
     std::map<std::string, long long> solve_ns;
     cudaStream_t stream = nullptr;
+    cudaMemPool_t pool = nullptr;   /* scratch of fdgpu_locate and fdgpu_raytrace (fdh_ctx_pool) */
     std::map<GeoKey, std::unique_ptr<Geo>> geos;
     BatchBufs batch;   /* the buffers of fdgpu_solve_device, kept for the next call */
     DevBuf model, fields;
@@ -194,8 +195,10 @@ extern "C" void fdgpu_destroy(fdgpu_ctx *ctx)
     FdDeviceScope dev_(ctx->device);
     cudaStreamSynchronize(ctx->stream);
     cudaStream_t s = ctx->stream;
+    cudaMemPool_t pool = ctx->pool;
     delete ctx;   /* frees every device buffer it holds */
     cudaStreamDestroy(s);
+    if (pool) cudaMemPoolDestroy(pool);   /* frees still in flight on a caller's stream finish first */
 }
 
 extern "C" const char *fdgpu_strerror(int s)
@@ -237,6 +240,29 @@ extern "C" int fdgpu_probe_fp64(fdgpu_ctx *ctx, double *gops)
 /* context access for the library's other translation units */
 extern "C" int fdh_ctx_device(const fdgpu_ctx *ctx) { return ctx->device; }
 extern "C" void *fdh_ctx_stream(const fdgpu_ctx *ctx) { return (void *)ctx->stream; }
+
+/* The context's memory pool.  The device's own pool gives freed memory back to the system at every
+ * synchronisation, so that each call mapped its scratch anew (the location of one event on 61x61x31
+ * takes 0.28 ms with this pool and one copy each way, 0.51 before; 8192 rays 7.2 ms, 8.0 before).  This one
+ * keeps up to 512 MB until the context is destroyed.  NULL if it cannot be made: the device's then serves. */
+extern "C" void *fdh_ctx_pool(fdgpu_ctx *ctx)
+{
+    if (!ctx->pool) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.handleTypes = cudaMemHandleTypeNone;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = ctx->device;
+        unsigned long long keep = 512ull << 20;
+        if (cudaMemPoolCreate(&ctx->pool, &props) != cudaSuccess) {
+            cudaGetLastError();
+            ctx->pool = nullptr;
+        } else if (cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+            cudaGetLastError();
+        }
+    }
+    return (void *)ctx->pool;
+}
 extern "C" int fdh_ctx_fail(fdgpu_ctx *ctx, int cuda_error, const char *what)
 {
     return cuda_fail(ctx, (cudaError_t)cuda_error, what);

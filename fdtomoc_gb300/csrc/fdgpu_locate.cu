@@ -747,30 +747,13 @@ __global__ void loc_states(const LocEvent *evs, int nev, int *state)
 
 extern "C" int fdh_ctx_device(const fdgpu_ctx *ctx);
 extern "C" void *fdh_ctx_stream(const fdgpu_ctx *ctx);
+extern "C" void *fdh_ctx_pool(fdgpu_ctx *ctx);
 extern "C" int fdh_ctx_fail(fdgpu_ctx *ctx, int cuda_error, const char *what);
 
 namespace {
 
 constexpr double kHpi = 1.570796f;          /* src/sphfdloc.c:74-75: float literals */
 constexpr double kDegrad = 0.017453292f;
-
-struct DevArena {
-    std::vector<void *> ptrs;
-    cudaStream_t s;
-    explicit DevArena(cudaStream_t st) : s(st) {}
-    ~DevArena()
-    {
-        for (void *p : ptrs) cudaFreeAsync(p, s);
-    }
-    template <class T> cudaError_t get(T **out, size_t n)
-    {
-        void *p = nullptr;
-        const cudaError_t e = cudaMallocAsync(&p, sizeof(T) * (n ? n : 1), s);
-        if (e == cudaSuccess) ptrs.push_back(p);
-        *out = static_cast<T *>(p);
-        return e;
-    }
-};
 
 }  // namespace
 
@@ -844,8 +827,16 @@ extern "C" int fdgpu_locate(fdgpu_ctx *ctx, const fdgpu_loc_grid *g, const float
     if (dev_.err) return FDGPU_ENODEV;
     cudaStream_t st = stream ? (cudaStream_t)stream : (cudaStream_t)fdh_ctx_stream(ctx);
 
-    std::vector<LocObsDev> hobs(nobs);
-    std::vector<unsigned char> hgood(nobs);
+    /* one block goes to the device, phases, active list and offsets, good flags, residuals, times and results, and
+     * its part from the flags on comes back: a copy each way */
+    auto up16 = [](size_t b) { return (b + 15) & ~(size_t)15; };
+    const size_t o_offs = up16(sizeof(LocObsDev) * nobs), o_act = o_offs + up16(sizeof(int) * (nev + 1));
+    const size_t o_good = o_act + up16(sizeof(int) * nev), o_res = o_good + up16(nobs);
+    const size_t o_tps = o_res + up16(sizeof(float) * nobs), o_out = o_tps + up16(sizeof(float) * nobs);
+    const size_t o_end = o_out + sizeof(fdgpu_loc_result) * nev;
+    std::vector<char> block(o_end, 0);
+    LocObsDev *hobs = reinterpret_cast<LocObsDev *>(block.data());
+    unsigned char *hgood = reinterpret_cast<unsigned char *>(block.data() + o_good);
     for (int k = 0; k < nobs; k++) {
         hobs[k].field = d_fields[obs[k].field];
         hobs[k].obstime = obs[k].obstime;
@@ -853,32 +844,27 @@ extern "C" int fdgpu_locate(fdgpu_ctx *ctx, const fdgpu_loc_grid *g, const float
         hobs[k].s_scaled = (g->ivs == 0 && obs[k].phase == 'S') ? 1 : 0;
         hgood[k] = obs[k].good ? 1 : 0;
     }
-    DevArena mem(st);
-    LocObsDev *dobs, *dlist;
+    std::memcpy(block.data() + o_offs, obs_offset, sizeof(int) * (nev + 1));
+    for (int e = 0; e < nev; e++) reinterpret_cast<int *>(block.data() + o_act)[e] = e;
+    FdArena mem(fdh_ctx_pool(ctx), st);
+    char *dblock;
+    LocObsDev *dlist;
     AxisPos *daxes = nullptr;
-    unsigned char *dgood;
     LocEvent *devs;
-    int *doffs, *dact, *dstate;
-    float *dres, *dtps;
-    fdgpu_loc_result *dout;
-    LOC_CU(mem.get(&dobs, nobs));
+    int *dstate;
+    LOC_CU(mem.get(&dblock, o_end));
+    LocObsDev *dobs = reinterpret_cast<LocObsDev *>(dblock);
+    int *doffs = reinterpret_cast<int *>(dblock + o_offs), *dact = reinterpret_cast<int *>(dblock + o_act);
+    unsigned char *dgood = reinterpret_cast<unsigned char *>(dblock + o_good);
+    float *dres = reinterpret_cast<float *>(dblock + o_res), *dtps = reinterpret_cast<float *>(dblock + o_tps);
+    fdgpu_loc_result *dout = reinterpret_cast<fdgpu_loc_result *>(dblock + o_out);
     LOC_CU(mem.get(&dlist, nobs));
     /* the windows' axis tables (see loc_refine) */
     const int ndmax = g->ndiv > g->ndiv2 ? g->ndiv : g->ndiv2, naxis = 2 * ndmax + 1;
     if (ndmax <= kDivMax) LOC_CU(mem.get(&daxes, (size_t)nev * 3 * naxis));
-    LOC_CU(mem.get(&dgood, nobs));
     LOC_CU(mem.get(&devs, nev));
-    LOC_CU(mem.get(&doffs, nev + 1));
-    LOC_CU(mem.get(&dact, nev));
     LOC_CU(mem.get(&dstate, nev));
-    LOC_CU(mem.get(&dres, nobs));
-    LOC_CU(mem.get(&dtps, nobs));
-    LOC_CU(mem.get(&dout, nev));
-    LOC_CU(cudaMemcpyAsync(dobs, hobs.data(), sizeof(LocObsDev) * nobs, cudaMemcpyHostToDevice, st));
-    LOC_CU(cudaMemcpyAsync(dgood, hgood.data(), nobs, cudaMemcpyHostToDevice, st));
-    LOC_CU(cudaMemcpyAsync(doffs, obs_offset, sizeof(int) * (nev + 1), cudaMemcpyHostToDevice, st));
-    LOC_CU(cudaMemsetAsync(dres, 0, sizeof(float) * nobs, st));
-    LOC_CU(cudaMemsetAsync(dtps, 0, sizeof(float) * nobs, st));
+    LOC_CU(cudaMemcpyAsync(dblock, block.data(), o_end, cudaMemcpyHostToDevice, st));
     loc_init<<<(nev + 127) / 128, 128, 0, st>>>(devs, doffs, nev);
     LOC_CU(cudaGetLastError());
 
@@ -896,7 +882,7 @@ extern "C" int fdgpu_locate(fdgpu_ctx *ctx, const fdgpu_loc_grid *g, const float
     for (int pass = 0; !act.empty(); pass++) {
         if (pass > 2 * kMaxObs + 4) return FDGPU_ESCHED;   /* each redo drops or recovers a phase */
         const int nact = (int)act.size();
-        LOC_CU(cudaMemcpyAsync(dact, act.data(), sizeof(int) * nact, cudaMemcpyHostToDevice, st));
+        if (pass > 0) LOC_CU(cudaMemcpyAsync(dact, act.data(), sizeof(int) * nact, cudaMemcpyHostToDevice, st));
         const int tw = (nact + 3) / 4;   /* a warp per event */
         loc_begin_pass<<<tw, 128, 0, st>>>(devs, dact, nact, dobs, dgood, dlist);
         if (ncoarse > 0) {
@@ -932,11 +918,11 @@ extern "C" int fdgpu_locate(fdgpu_ctx *ctx, const fdgpu_loc_grid *g, const float
     }
     loc_results<<<(nev + 127) / 128, 128, 0, st>>>(devs, nev, dout);
     LOC_CU(cudaGetLastError());
-    LOC_CU(cudaMemcpyAsync(results, dout, sizeof(fdgpu_loc_result) * nev, cudaMemcpyDeviceToHost, st));
-    LOC_CU(cudaMemcpyAsync(resmin, dres, sizeof(float) * nobs, cudaMemcpyDeviceToHost, st));
-    LOC_CU(cudaMemcpyAsync(tps, dtps, sizeof(float) * nobs, cudaMemcpyDeviceToHost, st));
-    LOC_CU(cudaMemcpyAsync(hgood.data(), dgood, nobs, cudaMemcpyDeviceToHost, st));
+    LOC_CU(cudaMemcpyAsync(hgood, dgood, o_end - o_good, cudaMemcpyDeviceToHost, st));
     LOC_CU(cudaStreamSynchronize(st));
+    std::memcpy(results, block.data() + o_out, sizeof(fdgpu_loc_result) * nev);
+    std::memcpy(resmin, block.data() + o_res, sizeof(float) * nobs);
+    std::memcpy(tps, block.data() + o_tps, sizeof(float) * nobs);
     for (int k = 0; k < nobs; k++) obs[k].good = hgood[k];
     return FDGPU_OK;
 }

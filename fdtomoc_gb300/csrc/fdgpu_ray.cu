@@ -27,6 +27,7 @@
 
 extern "C" int fdh_ctx_device(const fdgpu_ctx *ctx);
 extern "C" void *fdh_ctx_stream(const fdgpu_ctx *ctx);
+extern "C" void *fdh_ctx_pool(fdgpu_ctx *ctx);
 extern "C" int fdh_ctx_fail(fdgpu_ctx *ctx, int cuda_error, const char *what);
 
 namespace {
@@ -763,24 +764,6 @@ __global__ void ray_pack(const fdgpu_ray_result *__restrict__ res, const long lo
     }
 }
 
-struct Arena {
-    std::vector<void *> ptrs;
-    cudaStream_t s;
-    explicit Arena(cudaStream_t st) : s(st) {}
-    ~Arena()
-    {
-        for (void *p : ptrs) cudaFreeAsync(p, s);
-    }
-    template <class T> cudaError_t get(T **out, size_t n)
-    {
-        void *p = nullptr;
-        const cudaError_t e = cudaMallocAsync(&p, sizeof(T) * (n ? n : 1), s);
-        if (e == cudaSuccess) ptrs.push_back(p);
-        *out = static_cast<T *>(p);
-        return e;
-    }
-};
-
 }  // namespace
 
 #define RAY_CU(call)                                                        \
@@ -843,7 +826,7 @@ extern "C" int fdgpu_raytrace(fdgpu_ctx *ctx, const fdgpu_ray_grid *g, const flo
     std::memcpy(hc.data() + g->nxc, g->gy, sizeof(float) * g->nyc);
     std::memcpy(hc.data() + g->nxc + g->nyc, g->gz, sizeof(float) * g->nzc);
 
-    Arena mem(st);
+    FdArena mem(fdh_ctx_pool(ctx), st);
     RayObsDev *dobs;
     float *dcoarse, *lval, *ddu;
     int *lidx, *didx, *dn;
