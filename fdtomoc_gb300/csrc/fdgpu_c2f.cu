@@ -47,7 +47,7 @@ __global__ void c2f_slowness(const float *v, float *s, int n)
  * 401 x 401 x 161: 149 -> 61 us (3.4 TB/s) against a warp per row with every value's weights and slownesses
  * formed anew; 78 us with one node a thread in single registers, 76 with pairs and a division per value. */
 constexpr int kC2fBlock = 128;
-constexpr int kC2fZ = 24;   /* fine planes a thread walks; 16 take 3 % longer, 48 the same */
+constexpr int kC2fZ = 24;   /* fine planes a thread walks at most; 16 take 3 % longer, 48 the same */
 
 struct F2 {
     unsigned long long v;
@@ -75,12 +75,12 @@ __device__ __forceinline__ F2 add2(F2 a, F2 b)
 
 __global__ void __launch_bounds__(kC2fBlock) c2f_interp(const float *__restrict__ slow, const Axis *__restrict__ ax,
                                                         const Axis *__restrict__ ay, const Axis *__restrict__ az,
-                                                        int nx, int nxy, int nz, int nxc, int nxyc, int ncoarse,
+                                                        int nx, int nxy, int nz, int walk, int nxc, int nxyc, int ncoarse,
                                                         float *__restrict__ out, unsigned long long minus_zeros)
 {
     __shared__ float2 zg[kC2fZ], zf[kC2fZ];   /* weights of the planes below and above, for both halves */
     __shared__ int zcell[kC2fZ + 1];
-    const int k0 = blockIdx.y * kC2fZ, nk = min(kC2fZ, nz - k0);
+    const int k0 = blockIdx.y * walk, nk = min(walk, nz - k0);
     if (threadIdx.x < nk) {
         const Axis Z = az[k0 + threadIdx.x];
         zg[threadIdx.x] = make_float2(Z.omf, Z.omf);
@@ -231,6 +231,7 @@ struct fdgpu_c2f_plan {
     fdgpu_ctx *ctx = nullptr;
     int device = 0;
     int nx = 0, ny = 0, nz = 0, nxc = 0, nyc = 0, nzc = 0;
+    int sms = 1;
     char *mem = nullptr;   /* slowness (2 x coarse), axis tables */
     float *slow = nullptr;
     Axis *ax = nullptr, *ay = nullptr, *az = nullptr;
@@ -257,6 +258,7 @@ extern "C" int fdgpu_c2f_plan_create(fdgpu_ctx *ctx, const fdgpu_c2f_grid *g, fd
     p->device = dev;
     p->nx = nx; p->ny = ny; p->nz = nz;
     p->nxc = g->nxc; p->nyc = g->nyc; p->nzc = g->nzc;
+    if (cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || p->sms < 1) p->sms = 1;
     const size_t nc2 = 2 * (size_t)g->nxc * g->nyc * g->nzc;
     const size_t o_x = (sizeof(float) * nc2 + 255) & ~(size_t)255;
     const size_t o_y = o_x + ((sizeof(Axis) * nx + 255) & ~(size_t)255);
@@ -289,8 +291,13 @@ extern "C" int fdgpu_c2f_run(fdgpu_c2f_plan *p, const float *d_coarse, float *d_
     const int nc2 = 2 * p->nxc * p->nyc * p->nzc;
     c2f_slowness<<<(nc2 + 255) / 256 < 1024 ? (nc2 + 255) / 256 : 1024, 256, 0, st>>>(d_coarse, p->slow, nc2);
     const int nxy = p->nx * p->ny;
-    const dim3 grid((nxy + 2 * kC2fBlock - 1) / (2 * kC2fBlock), (p->nz + kC2fZ - 1) / kC2fZ);
-    c2f_interp<<<grid, kC2fBlock, 0, st>>>(p->slow, p->ax, p->ay, p->az, p->nx, nxy, p->nz, p->nxc, p->nxc * p->nyc,
+    const int across = (nxy + 2 * kC2fBlock - 1) / (2 * kC2fBlock);
+    /* a model too small for eight blocks an SM is split further along z, to one plane a thread: there the
+     * walk's latency is what takes the time (28 x 64 x 27: 16.6 us a call with 24 planes, 8.4 with one) */
+    int walk = kC2fZ;
+    while (walk > 1 && (long long)across * ((p->nz + walk - 1) / walk) < 8ll * p->sms) walk /= 2;
+    const dim3 grid(across, (p->nz + walk - 1) / walk);
+    c2f_interp<<<grid, kC2fBlock, 0, st>>>(p->slow, p->ax, p->ay, p->az, p->nx, nxy, p->nz, walk, p->nxc, p->nxc * p->nyc,
                                              p->nxc * p->nyc * p->nzc, d_fine, 0x8000000080000000ull);
     const cudaError_t e = cudaGetLastError();
     return e ? fdh_ctx_fail(p->ctx, (int)e, "c2f launch") : FDGPU_OK;
