@@ -39,14 +39,12 @@ namespace fdk {
 #define FB_EY 1.9073486328125e-06f        /* 2^-19 */
 #define FB_ET 9.094947017729282e-13f      /* 2^-40 */
 
-/* a positive normal double truncated to float on the integer pipe (NaN outside float's normal
- * range, which makes every later comparison fail) */
+/* a positive double truncated to float; NaN outside float's normal range, which makes every later
+ * comparison fail */
 __device__ __forceinline__ float d2f_trunc(double x)
 {
-    const long long b = __double_as_longlong(x);
-    const int e = (int)((b >> 52) & 0x7ff) - 1023 + 127;
-    if (b <= 0 || e < 1 || e > 254) return __int_as_float(0x7fc00000);
-    return __int_as_float((e << 23) | (int)((b >> 29) & 0x7fffff));
+    const float f = __double2float_rz(x);
+    return f >= 1.17549435e-38f && f < 3.40282347e38f ? f : __int_as_float(0x7fc00000);
 }
 
 /* truncated reciprocals of the two tabulated distances at (z,y) (see FD_N_INV32) */
@@ -108,12 +106,6 @@ __device__ __forceinline__ float lower_2d(const TrialDesc &d, const float *t18, 
     const float m = ((fabsf(b) + shi) * FB_EY + B * FB_EB) * i2a * 1.001f + FB_ET * T;
     if (__fadd_ru(t3, (-b - slo) * i2a + m) < fl) return fminf(__fadd_rd(t3, (slo - b) * i2a - m), 1.e10f);
     return __fadd_rd(t3, (-b - shi) * i2a - m);
-}
-
-/* trial value v (>= the returned bound lo) cannot lower a running minimum that is at most g */
-__device__ __forceinline__ bool bound_prunes(float lo, double g)
-{
-    return lo >= 0.f && !lt(1.e11, g) && !lt(f2d(lo), g);
 }
 
 }  // namespace fdk

@@ -35,49 +35,10 @@ namespace fdk {
 /* ---------------------------------------------------------------------------------------------- */
 /* exact helpers                                                                                   */
 
-/* The solver's code is several times the SM's instruction caches, so the helpers that are inlined in dozens of
- * places are kept as short as they can be: one test for the operands that need the general instruction. */
-
-/* float -> double on the integer pipe (normal numbers; zeros and anything else convert normally) */
-__device__ __forceinline__ double f2d(float f)
-{
-    const unsigned b = __float_as_uint(f);
-    if (((b >> 23) & 0xffu) - 1u >= 254u) return (double)f;
-    return __hiloint2double((int)(((b & 0x7fffffffu) >> 3) + 0x38000000u | (b & 0x80000000u)), (int)(b << 29));
-}
-
-/* Comparisons of finite doubles on the integer pipe (an FP64 compare occupies this GPU's FP64 unit
- * like any FP64 instruction, 64 cycles per warp).  Each gives exactly the double comparison's result,
- * signed zeros included, for the operands it states; none is used where an operand may be NaN. */
-
-/* a < b for finite a and b of any sign */
-__device__ __forceinline__ bool flt(double a, double b)
-{
-    const long long ia = __double_as_longlong(a), ib = __double_as_longlong(b);
-    if ((ia | ib) >= 0) return ia < ib;                       /* both non-negative */
-    if ((ia & ib) < 0) return ia > ib;                        /* both negative: the larger magnitude */
-    if (ia < 0) return (ia << 1) != 0 || (ib << 1) != 0;      /* a negative: below b unless both zero */
-    return false;                                             /* b negative, a not */
-}
-
-/* !(x >= 0.) for any x: negative and not -0, or NaN */
-__device__ __forceinline__ bool not_ge0(double x)
-{
-    const long long ix = __double_as_longlong(x);
-    return (ix < 0 && (ix << 1) != 0) || (ix & 0x7fffffffffffffffll) > 0x7ff0000000000000ll;
-}
-
-/* x * 2^k, exact: exponent arithmetic on the integer pipe when x and the result are normal;
- * zeros and subnormals take the floating-point multiply */
-template <int K>
-__device__ __forceinline__ double scale2k(double x)
-{
-    const int hi = __double2hiint(x), e = (hi >> 20) & 0x7ff;
-    constexpr int lo = K < 0 ? 1 - K : 1, n = 2046 - (K > 0 ? K : 0) - lo;
-    if ((unsigned)(e - lo) <= (unsigned)n) return __hiloint2double(hi + K * (1 << 20), __double2loint(x));
-    constexpr double p2 = K >= 0 ? (double)(1ll << (K >= 0 ? K : 0)) : 1.0 / (double)(1ll << (K < 0 ? -K : 0));
-    return x * p2;
-}
+/* Conversions, comparisons and products by powers of two are FP64 instructions, although each occupies the FP64 unit
+ * for 64 cycles: the solver waits for instructions to arrive from the caches in half of its cycles, so
+ * that sequences of four to twelve integer instructions in their place cost more (400 windows of 25 to 61: 186 ms
+ * with such sequences, 172 without; one of 27x20x21: 4.78 and 4.69). */
 
 /* RN(x / d) given inv = RN(1/d): q = RN(x*inv) then two exact-residual corrections.  Zero x keeps
  * its sign, as a true division would. */
@@ -136,27 +97,27 @@ __host__ __device__ constexpr int chain_class(fdn_chain c)
  * causality test against floor tmx; tie rule of fdsph3d (x1 preferred only if strictly smaller). */
 __device__ __forceinline__ double roots_3d(double b, double rad, double twoa, double i2a, double tmx)
 {
-    if (not_ge0(rad)) return 1.e11;
+    if (!(rad >= 0.)) return 1.e11;
     const double sq = __dsqrt_rn(rad);
     const double x1 = div_rn(-b + sq, twoa, i2a);
     const double x2 = div_rn(-b - sq, twoa, i2a);
-    const bool bad1 = flt(x1, tmx), bad2 = flt(x2, tmx);
+    const bool bad1 = x1 < tmx, bad2 = x2 < tmx;
     if (bad1) return bad2 ? 1.e11 : x2;
     if (bad2) return x1;
-    return flt(x1, x2) ? x1 : x2;
+    return x1 < x2 ? x1 : x2;
 }
 
 /* same, with the tie rule of fdsphne / fdsph2d (x2 preferred only if strictly smaller) */
 __device__ __forceinline__ double roots_2(double b, double rad, double twoa, double i2a, double tmx)
 {
-    if (not_ge0(rad)) return 1.e11;
+    if (!(rad >= 0.)) return 1.e11;
     const double sq = __dsqrt_rn(rad);
     const double x1 = div_rn(-b + sq, twoa, i2a);
     const double x2 = div_rn(-b - sq, twoa, i2a);
-    const bool bad1 = flt(x1, tmx), bad2 = flt(x2, tmx);
+    const bool bad1 = x1 < tmx, bad2 = x2 < tmx;
     if (bad1) return bad2 ? 1.e11 : x2;
     if (bad2) return x1;
-    return flt(x2, x1) ? x2 : x1;
+    return x2 < x1 ? x2 : x1;
 }
 
 }  // namespace fdk
