@@ -40,6 +40,9 @@ namespace fdk {
  * that sequences of four to twelve integer instructions in their place cost more (400 windows of 25 to 61: 186 ms
  * with such sequences, 172 without; one of 27x20x21: 4.78 and 4.69). */
 
+__device__ __forceinline__ double f2d(float f) { return (double)f; }
+__device__ __forceinline__ bool lt(double a, double b) { return a < b; }
+
 /* RN(x / d) given inv = RN(1/d): q = RN(x*inv) then two exact-residual corrections.  Zero x keeps
  * its sign, as a true division would. */
 __device__ __forceinline__ double div_rn(double x, double d, double inv)

@@ -489,13 +489,13 @@ __device__ __forceinline__ double shfl_d(double x, int src) { return __shfl_sync
 /* the accepted root of fdsphne / fdsph2d and of fdsph3d (tie rules of roots_2 and roots_3d) */
 __device__ __forceinline__ double pick_2(double x1, double x2, double tmx)
 {
-    const bool bad1 = x1 < tmx, bad2 = x2 < tmx;
-    return bad1 ? (bad2 ? 1.e11 : x2) : (bad2 ? x1 : (x2 < x1 ? x2 : x1));
+    const bool bad1 = lt(x1, tmx), bad2 = lt(x2, tmx);
+    return bad1 ? (bad2 ? 1.e11 : x2) : (bad2 ? x1 : (lt(x2, x1) ? x2 : x1));
 }
 __device__ __forceinline__ double pick_3(double x1, double x2, double tmx)
 {
-    const bool bad1 = x1 < tmx, bad2 = x2 < tmx;
-    return bad1 ? (bad2 ? 1.e11 : x2) : (bad2 ? x1 : (x1 < x2 ? x1 : x2));
+    const bool bad1 = lt(x1, tmx), bad2 = lt(x2, tmx);
+    return bad1 ? (bad2 ? 1.e11 : x2) : (bad2 ? x1 : (lt(x1, x2) ? x1 : x2));
 }
 
 /* Up to eight corner items (fdsph3d, as eval_3d), lanes 4g .. 4g+3 on item g.  Lane r holds terms r and
@@ -523,9 +523,9 @@ __device__ void eval_corners_quad(const fd_station_dev &sd, const TrialDesc *dsc
     for (int h = 0; h < 2; h++) {
         const int i = r + 4 * h;   /* term 7: the point itself, a slowness only */
         const int nb = i < 7 ? d.slot[i] : NB_POINT;
-        S[i] = (double)s18[nb];
+        S[i] = f2d(s18[nb]);
         if (i < 7) {
-            const double t = (double)t18[nb];
+            const double t = f2d(t18[nb]);
             if (h == 0) tr = t;
             tm = h == 0 ? t18[nb] : fmaxf(tm, t18[nb]);
             T[i] = t;
@@ -573,7 +573,7 @@ __device__ void eval_corners_quad(const fd_station_dev &sd, const TrialDesc *dsc
     const double sq = __dsqrt_rn(none ? 0.0 : rad);
     const double x = div_rn(-b + (r & 1 ? -sq : sq), 2. * a, i2a);
     const double x1 = shfl_d(x, lead), x2 = shfl_d(x, lead + 1);
-    if (r == 0 && g < n) ws.res[slot][K] = none ? 1.e11 : pick_3(x1, x2, (double)tm);
+    if (r == 0 && g < n) ws.res[slot][K] = none ? 1.e11 : pick_3(x1, x2, f2d(tm));
     __syncwarp();
 }
 
@@ -597,7 +597,7 @@ __device__ void eval_edges_quad(const fd_station_dev &sd, const TrialDesc *dsc, 
     apair_rt(sd.g, d.apair, z, y, a, i2a);
     const float fx = t18[d.slot[ne ? 4 : 1]], fy = t18[d.slot[2]], fz = t18[d.slot[ne ? 1 : 3]];
     float fl = fmaxf(fmaxf(fx, fy), fz);
-    const double tz = (double)fz, ta = (double)(r == 0 || r == 3 ? fx : fy);
+    const double tz = f2d(fz), ta = f2d(r == 0 || r == 3 ? fx : fy);
     const double df = ta - tz;
     const double q1 = div_rn(r & 1 ? ta : df, dd, iv);
     const double pq = q1 - shfl_d(q1, lane ^ 1);      /* p in lane 0, q in lane 2 */
@@ -606,7 +606,7 @@ __device__ void eval_edges_quad(const fd_station_dev &sd, const TrialDesc *dsc, 
     if (ne) {
         const float f0 = t18[d.slot[0]], f3 = t18[d.slot[3]];
         fl = fmaxf(fl, fmaxf(f0, f3));
-        d3 = (double)f0 - (double)f3;
+        d3 = f2d(f0) - f2d(f3);
         if (r == 0) dist_rt(sd.g, d.dcls[0], z + d.ddz[0], y + d.ddy[0], dd, iv);
     } else {
         fl = fmaxf(fl, fmaxf(ws.s0[slot], ws.s4[slot]));
@@ -616,7 +616,7 @@ __device__ void eval_edges_quad(const fd_station_dev &sd, const TrialDesc *dsc, 
     const double b = 2. * (shfl_d(q2, lead + 1) + shfl_d(q2, lead + 3));
     /* slownesses in the reference's order, one conversion a lane */
     const int so = ne ? (r == 3 ? NB_POINT : d.slot[r == 0 ? 1 : r == 1 ? 2 : 4]) : (r == 0 ? NB_POINT : d.slot[r]);
-    const double sl = (double)s18[so];
+    const double sl = f2d(s18[so]);
     const double sum = ((shfl_d(sl, lead) + shfl_d(sl, lead + 1)) + shfl_d(sl, lead + 2)) + shfl_d(sl, lead + 3);
     const double m = (r == 2 ? sum : v) * (r == 2 ? 0.25 * sum : v);
     const double c = ((shfl_d(m, lead + 1) + shfl_d(m, lead + 3)) + shfl_d(m, lead)) - shfl_d(m, lead + 2);
@@ -625,7 +625,7 @@ __device__ void eval_edges_quad(const fd_station_dev &sd, const TrialDesc *dsc, 
     const double sq = __dsqrt_rn(none ? 0.0 : rad);
     const double x = div_rn(-b + (r & 1 ? -sq : sq), 2. * a, i2a);
     const double x1 = shfl_d(x, lead), x2 = shfl_d(x, lead + 1);
-    if (r == 0 && g < n) ws.res[slot][K] = none ? 1.e11 : pick_2(x1, x2, (double)fl);
+    if (r == 0 && g < n) ws.res[slot][K] = none ? 1.e11 : pick_2(x1, x2, f2d(fl));
     __syncwarp();
 }
 
@@ -671,7 +671,7 @@ __device__ unsigned stale_pair(const fd_station_dev &sd, const TrialDesc *dsc, W
 {
     const float *t18 = ws.t[slot];
     const float dx = ws.s0[slot], dy = ws.s4[slot], dz = d2f_trunc(sd.g.h);   /* step lengths, put there with the context */
-    double g1 = (double)t18[NB_POINT];
+    double g1 = f2d(t18[NB_POINT]);
     float s0 = it0, s4 = it4;
     /* the last writer's slots are what remains of the writers before it */
     auto wrote = [&](unsigned writers) {
@@ -682,14 +682,14 @@ __device__ unsigned stale_pair(const fd_station_dev &sd, const TrialDesc *dsc, W
     auto lowest = [&](unsigned b) {
         for (; b; b &= b - 1) {
             const double v = ws.res[slot][__ffs(b) - 1];
-            if (v < g1) g1 = v;
+            if (lt(v, g1)) g1 = v;
         }
     };
     if (gm & 0xFu) {
         wrote(gm & 0xFu);
         lowest(gm & em & 0xFu);
     }
-    if ((gm & 0xF0u) && 1.0e9 < g1) {
+    if ((gm & 0xF0u) && lt(1.0e9, g1)) {
         wrote(gm & 0xF0u);
         lowest(gm & em & 0xF0u);
     }
@@ -1339,14 +1339,14 @@ __device__ bool commit_node(const fd_station_dev &sd, Shared &sh, const TrialDes
                             unsigned char *dag, unsigned &was, Counters cn)
 {
     const float *t18 = ws.t[slot], *s18 = ws.s[slot];
-    const double told = (double)t18[NB_POINT];
+    const double told = f2d(t18[NB_POINT]);
     const int z = ws.z[slot], y = ws.y[slot];
     double guess = told;
     const unsigned head = c_guards[F].head;
     int lastK = -1, writer = -1;   /* the last head trial that lowered the minimum; the last writer */
     double last_gb = 0.0, last_v = 0.0;
     auto take = [&](int K, double v) {
-        if (!(v < guess)) return false;
+        if (!lt(v, guess)) return false;
         if ((head >> K) & 1u) { lastK = K; last_gb = guess; last_v = v; }
         guess = v;
         return true;
@@ -1368,14 +1368,14 @@ __device__ bool commit_node(const fd_station_dev &sd, Shared &sh, const TrialDes
     };
     if (gm & 0xFu) writer = 31 - __clz((int)(gm & 0xFu));
     for (unsigned b = gm & em & 0xFu; b; b &= b - 1) take(__ffs(b) - 1, ws.res[slot][__ffs(b) - 1]);
-    if ((gm & 0xF0u) && 1.0e9 < guess)
+    if ((gm & 0xF0u) && lt(1.0e9, guess))
         for (unsigned b = gm & 0xF0u; b; b &= b - 1) contact(__ffs(b) - 1);
     bool win2d = false;
     for (unsigned b = gm & em & k2d; b; b &= b - 1) win2d |= take(__ffs(b) - 1, ws.res[slot][__ffs(b) - 1]);
-    if (((gm >> TK_NF) & 1u) && 1.0e9 < guess) contact(TK_NF);
+    if (((gm >> TK_NF) & 1u) && lt(1.0e9, guess)) contact(TK_NF);
     for (unsigned b = gm & em & (0x1Fu << TK_1D0); b; b &= b - 1) take(__ffs(b) - 1, ws.res[slot][__ffs(b) - 1]);
     if (permissive && win2d) return false;
-    if (guess < told && FD_OK(wh.p, (long long)sd.g.nx * sd.g.ny * sd.g.nz, 11)) {
+    if (lt(guess, told) && FD_OK(wh.p, (long long)sd.g.nx * sd.g.ny * sd.g.nz, 11)) {
         sd.T[wh.p] = __double2float_rn(guess);
         if (lastK >= 0) {
             /* only the last head trial that lowered the minimum sets the measure that is tested */

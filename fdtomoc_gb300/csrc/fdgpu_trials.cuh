@@ -192,7 +192,7 @@ __device__ __forceinline__ double factor_rt(const fd_geo_dev &g, int kind, int z
     case FK_DF: return g.df;
     case FK_R: return g.zrow[(long long)(FD_OK(z, g.nz, 4) ? z : 0) * FD_Z_N + FD_Z_R];
     case FK_S: return g.ysin[FD_OK(y, g.ny, 5) ? y : 0];
-    default: return (double)slow;
+    default: return f2d(slow);
     }
 }
 
@@ -211,11 +211,11 @@ __device__ __forceinline__ double eval_3d(const TrialDesc &d, const float *t18, 
     for (int i = 1; i < 7; i++) tmx = fmaxf(tmx, tf[i]);
     double t[7];
 #pragma unroll
-    for (int i = 0; i < 7; i++) t[i] = (double)tf[i];
-    double sum = (double)s18[d.slot[0]];
+    for (int i = 0; i < 7; i++) t[i] = f2d(tf[i]);
+    double sum = f2d(s18[d.slot[0]]);
 #pragma unroll
-    for (int i = 1; i < 7; i++) sum = sum + (double)s18[d.slot[i]];
-    sum = sum + (double)s18[NB_POINT];
+    for (int i = 1; i < 7; i++) sum = sum + f2d(s18[d.slot[i]]);
+    sum = sum + f2d(s18[NB_POINT]);
     const double slo = 0.125 * sum;
     const double sl16 = 2. * sum * slo;
     int zc = z + d.zmin, yc = y + d.ymin;
@@ -238,7 +238,7 @@ __device__ __forceinline__ double eval_3d(const TrialDesc &d, const float *t18, 
     }
     c = c - sl16;
     const double rad = b * b - 4. * a * c;
-    return roots_3d(b, rad, 2. * a, i2a, (double)tmx);
+    return roots_3d(b, rad, 2. * a, i2a, f2d(tmx));
 }
 
 /* fdsphne (src/sphfd.c:6016-6074) */
@@ -254,8 +254,8 @@ __device__ __forceinline__ double eval_ne(const TrialDesc &d, const float *t18, 
     for (int j = 0; j < 5; j++) dist_rt(g, d.dcls[j], z + d.ddz[j], y + d.ddy[j], dd[j], iv[j]);
     double a, i2a;
     apair_rt(g, d.apair, z, y, a, i2a);
-    const double t0 = (double)tf[0], t1 = (double)tf[1], t2 = (double)tf[2], t3 = (double)tf[3], t4 = (double)tf[4];
-    const double sum = (((double)s18[d.slot[1]] + (double)s18[d.slot[2]]) + (double)s18[d.slot[4]]) + (double)s18[NB_POINT];
+    const double t0 = f2d(tf[0]), t1 = f2d(tf[1]), t2 = f2d(tf[2]), t3 = f2d(tf[3]), t4 = f2d(tf[4]);
+    const double sum = ((f2d(s18[d.slot[1]]) + f2d(s18[d.slot[2]])) + f2d(s18[d.slot[4]])) + f2d(s18[NB_POINT]);
     const double slo = 0.25 * sum;
     /* d[] = d01 d12 d14 d25 d45 */
     const double dt1 = div_rn(t4 - t1, dd[2], iv[2]) - div_rn(t2, dd[3], iv[3]);
@@ -264,7 +264,7 @@ __device__ __forceinline__ double eval_ne(const TrialDesc &d, const float *t18, 
     const double b = 2. * (div_rn(dt1, dd[3], iv[3]) + div_rn(dt2, dd[4], iv[4]));
     const double c = ((dt1 * dt1 + dt2 * dt2) + dt3 * dt3) - sum * slo;
     const double rad = b * b - 4. * a * c;
-    return roots_2(b, rad, 2. * a, i2a, (double)tmx);
+    return roots_2(b, rad, 2. * a, i2a, f2d(tmx));
 }
 
 /* fdsph2d (src/sphfd.c:6077-6143) without its stale-slot test: returns both roots (x1 NaN when
@@ -278,8 +278,8 @@ __device__ __forceinline__ void eval_2d(const TrialDesc &d, const float *t18, co
     for (int j = 0; j < 4; j++) dist_rt(g, d.dcls[j], z + d.ddz[j], y + d.ddy[j], dd[j], iv[j]);
     double a, i2a;
     apair_rt(g, d.apair, z, y, a, i2a);
-    const double t1 = (double)tf1, t2 = (double)tf2, t3 = (double)tf3;
-    const double sum = (((double)s18[NB_POINT] + (double)s18[d.slot[1]]) + (double)s18[d.slot[2]]) + (double)s18[d.slot[3]];
+    const double t1 = f2d(tf1), t2 = f2d(tf2), t3 = f2d(tf3);
+    const double sum = ((f2d(s18[NB_POINT]) + f2d(s18[d.slot[1]])) + f2d(s18[d.slot[2]])) + f2d(s18[d.slot[3]]);
     const double slo = 0.25 * sum;
     /* d[] = d01 d02 d13 d23 */
     const double t1t3t2 = div_rn(t1 - t3, dd[2], iv[2]) - div_rn(t2, dd[1], iv[1]);
@@ -309,13 +309,13 @@ __device__ __forceinline__ double eval_nf(const TrialDesc &d, const float *t18, 
     double dd[3], iv[3];
 #pragma unroll
     for (int j = 0; j < 3; j++) dist_rt(g, d.dcls[j], z + d.ddz[j], y + d.ddy[j], dd[j], iv[j]);
-    const double slo = 0.5 * ((double)s18[NB_POINT] + (double)s18[d.slot[2]]);
-    const double t4t0 = div_rn((double)tf[4] - (double)tf[0], dd[0], iv[0]);
-    const double t1t3 = div_rn((double)tf[1] - (double)tf[3], dd[1], iv[1]);
+    const double slo = 0.5 * (f2d(s18[NB_POINT]) + f2d(s18[d.slot[2]]));
+    const double t4t0 = div_rn(f2d(tf[4]) - f2d(tf[0]), dd[0], iv[0]);
+    const double t1t3 = div_rn(f2d(tf[1]) - f2d(tf[3]), dd[1], iv[1]);
     double x = slo * slo - 0.25 * (t4t0 * t4t0 + t1t3 * t1t3);
     if (!(x >= 0.)) return 1.e11;
-    x = (double)tf[2] + dd[2] * __dsqrt_rn(x);
-    return x < (double)tchk ? 1.e11 : x;
+    x = f2d(tf[2]) + dd[2] * __dsqrt_rn(x);
+    return x < f2d(tchk) ? 1.e11 : x;
 }
 
 /* straight edge: t_nbr + 0.5*(s_point + s_nbr) times the step's factors (e.g. src/sphfd.c:1727-1755): along
@@ -324,7 +324,7 @@ __device__ __forceinline__ double eval_1d(const TrialDesc &d, const float *t18, 
                                           const fd_geo_dev &g, int z, int y)
 {
     const float ssum = s18[NB_POINT] + s18[d.slot[0]];
-    double x = 0.5 * (double)ssum;
+    double x = 0.5 * f2d(ssum);
     if (d.vn == 1) {
         x = x * g.h;
     } else {
@@ -333,7 +333,7 @@ __device__ __forceinline__ double eval_1d(const TrialDesc &d, const float *t18, 
         x = x * (d.vn == 2 ? g.dq : d.vk[1] == FK_S ? s : g.df);
         if (d.vn == 3) x = x * (d.vk[1] == FK_S ? g.df : s);
     }
-    return (double)t18[d.slot[0]] + x;
+    return f2d(t18[d.slot[0]]) + x;
 }
 
 /* head-wave denominator of a head trial: d01*s_point (2-D) or the 1-D chain ending in s_point */
@@ -343,7 +343,7 @@ __device__ __forceinline__ double head_den(const TrialDesc &d, const float *s18,
     if (d.kind == FDN_2D) {
         double d01, i01;
         dist_rt(g, d.dcls[0], z + d.ddz[0], y + d.ddy[0], d01, i01);
-        return d01 * (double)sp;
+        return d01 * f2d(sp);
     }
     double den = factor_rt(g, d.hk[0], z + d.hdz[0], y + d.hdy[0], sp);
     for (int j = 1; j < d.hn; j++) den = den * factor_rt(g, d.hk[j], z + d.hdz[j], y + d.hdy[j], sp);
