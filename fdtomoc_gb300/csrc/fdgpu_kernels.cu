@@ -132,7 +132,7 @@ struct WalkShared {
      * and wait pairs */
     int nq;
     int qhead[6], qtail[6], qcap[6], qbase[6];
-    int rqhead, rqtail, rqcap, idle, ndone, npark, nwait;
+    int rqhead, rqtail, rqcap, idle, ndone, npark, nwait, nphi;
     int status;
     int headw[8];
     unsigned long long exitkey;
@@ -1054,8 +1054,8 @@ __device__ __forceinline__ void graph_ready(const fd_station_dev &sd, Shared &sh
  * never becomes free again within a sweep, so the pairs of a point lie between its hash slot and the
  * first free one.  (A list of all the sweep's pairs, searched for every awaited point, cost up to half a
  * million cycles a wake-up on windows with thousands of waits.) */
-__device__ __forceinline__ unsigned wait_slot(int p) { return ((unsigned)p * 2654435761u) >> 16; }
-static_assert(FD_GWAIT_CAP == 1 << 16, "wait_slot");
+__device__ __forceinline__ unsigned wait_slot(int p) { return ((unsigned)p * 2654435761u) >> 15; }
+static_assert(FD_GWAIT_CAP == 1 << 17, "wait_slot");
 
 FD_COLD void wake_waiters(const fd_station_dev &sd, Shared &sh, int p)
 {
@@ -1624,10 +1624,150 @@ FD_COLD bool resume_waiter(const fd_station_dev &sd, Shared &sh, int w, float *s
     return false;
 }
 
+/* nodes of instances not complete that keys_above looks through; with more it waits for the event.  500 windows of 41
+ * to 301 a side: 6.42 s without the bound, 6.32 with it at 65536, 6.27 at 131072, 7.97 with no limit; 150 windows of
+ * 73 to 91: 319 to 335 ms without, 242 at 65536, 242 and 290 (two models) at 131072, 257 at 16384. */
+#ifndef FD_PHI_NODES
+#define FD_PHI_NODES 65536
+#endif
+
+/* every trial's value is at least the time of one of the node's six neighbours, as the trial reads it: the corner,
+ * new-edge and 2-D stencils and the new face reject a value below their times (of the 2-D slots, 1 to 3 are the
+ * trial's own), and a 1-D trial adds to one (slownesses are not negative, as the floors of the 1-D trials assume) */
+constexpr bool trials_above_a_neighbour()
+{
+    for (int f = 0; f < FDN_NFACE; f++)
+        for (int k = 0; k < FDN_NTRIAL; k++) {
+            const fdn_trial tr = fd_face_trials[f][k];
+            const int from = tr.kind == FDN_2D ? 1 : 0;
+            const int to = tr.kind == FDN_3D ? 7 : tr.kind == FDN_2D ? 4 : tr.kind == FDN_1D ? 1 : 5;
+            bool some = false;
+            for (int i = from; i < to; i++) {
+                const fdn_node n = tr.t[i];
+                some = some || n.du * n.du + n.dv * n.dv + n.w * n.w == 1;
+            }
+            if (!some) return false;
+        }
+    return true;
+}
+static_assert(trials_above_a_neighbour(), "keys_above");
+
+/* Whether every key of instance I that is not known yet is certainly above kw, so that the points before point w
+ * (key kw) are all known already; if not, w is registered on a node that stands against it, or on the event
+ * that all keys are known.  One warp.
+ *
+ * A missing key is the time of a node of an earlier instance that is not done.  Let S be all such nodes and phi
+ * the least time now at any of them or their six neighbours: no node of S ends below phi.  For take the first one,
+ * in the reference's order, that did: its old time is not below phi, and each trial's value is not below the time
+ * it reads at one of the six (trials_above_a_neighbour), which was done before (as read here), is of S and before it
+ * (not below phi, since it is the first), or is of an instance not before its own (not changed before it is
+ * evaluated).  The flags of an instance are all read before the times about its nodes, and instances go in
+ * order: a neighbour whose flag says done then has its final time.  A time that is no number or negative stands
+ * against everything.
+ *
+ * Why: without it such a point waits for the whole inner layer, and where border points inherit state (a fast layer
+ * at the grid's edge) the planes of a forward sweep run one after another, which made a few windows five times
+ * as long as the others.  Their batches and lists end with them: 150 windows of 73 to 91 319 -> 242 ms, 24 host
+ * stations of 49x45x33 96 -> 60, 48 served requests 91 -> 77; with all 26 neighbours instead of the six 251, 65 and 83. */
+FD_COLD bool keys_above(const fd_station_dev &sd, Shared &sh, WarpSmem &ws, int I, int w, float kw)
+{
+    const int lane = threadIdx.x & 31;
+    const GraphSmem gs = gsmem(sh);
+    unsigned *bits = reinterpret_cast<unsigned *>(&ws.res[0][0]);
+    constexpr int kBits = 8 * sizeof ws.res;   /* a flag per node of an instance; larger faces wait for the event */
+    if (vload(sd.scr.ginst[I].phi) > kw) return true;
+    bool event = vload(sh.w.nphi) >= FD_GPHI_CAP - FD_WARPS;   /* these waits leave the tables' room for the others */
+    for (int turn = 0; turn < 8 && !event; turn++) {   /* a turn more if the node found is done by now */
+        float phi = 1.e10f, worst = -2.f;   /* worst: the largest bound that is not above kw, at node zw */
+        int zw = -1, scanned = 0;
+        for (int J0 = 0; J0 < I && !event; J0 += 32) {
+            /* the instances that have nodes to come */
+            const int Jl = J0 + lane;
+            unsigned open = __ballot_sync(0xffffffffu, Jl < I && vload(gs.ndone[Jl < I ? Jl : 0]) < rect_n(gs.rect[Jl < I ? Jl : 0]));
+            for (; open; open &= open - 1) {
+                const GRect r = gs.rect[J0 + __ffs(open) - 1];
+                const int n = rect_n(r), nuf = r.nuf();
+                scanned += n;
+                if (n > kBits || scanned > FD_PHI_NODES) {
+                    event = true;
+                    break;
+                }
+                const fdn_frame fr = frame_of(r.face());
+                const int su = (int)t_stride(sd, fr.axis_u), sv = (int)t_stride(sd, fr.axis_v);
+                const int du = 32 % nuf, step = du * su + 32 / nuf * sv, wrap = sv - nuf * su;
+                const int base = inst_node(sd, r, 0);
+                unsigned any = 0;
+                int u = lane % nuf, q = base + u * su + lane / nuf * sv;
+                for (int j0 = 0; j0 < n; j0 += 128) {
+                    unsigned c[4];
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        c[k] = j0 + 32 * k + lane < n ? vload(sd.scr.gcnt[q]) : FD_DONEB;
+                        u += du;
+                        q += step;
+                        if (u >= nuf) {
+                            u -= nuf;
+                            q += wrap;
+                        }
+                    }
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        const unsigned m = __ballot_sync(0xffffffffu, !(c[k] & FD_DONEB));
+                        if (lane == 0 && j0 + 32 * k < n) bits[(j0 >> 5) + k] = m;
+                        any |= m;
+                    }
+                }
+                __syncwarp();
+                wfence(sh);
+                if (any) {
+                    for (int j0 = 0; j0 < n; j0 += 32) {
+                        if (!((bits[j0 >> 5] >> lane) & 1u)) continue;
+                        const int xyz = inst_xyz(r, j0 + lane);
+                        const int x = xyz & 1023, y = (xyz >> 10) & 1023, z = xyz >> 20;
+                        const int nx = sd.g.nx, nxy = nx * sd.g.ny, p = z * nxy + y * nx + x;
+                        const int o[7] = {0, x > 0 ? -1 : 0, x < nx - 1 ? 1 : 0, y > 0 ? -nx : 0, y < sd.g.ny - 1 ? nx : 0,
+                                          z > 0 ? -nxy : 0, z < sd.g.nz - 1 ? nxy : 0};
+                        float t[7];
+#pragma unroll
+                        for (int k = 0; k < 7; k++) t[k] = sd.T[p + o[k]];
+                        float lb = 1.e10f;
+#pragma unroll
+                        for (int k = 0; k < 7; k++) lb = t[k] >= 0.f ? fminf(lb, t[k]) : -1.f;
+                        phi = fminf(phi, lb);
+                        if (lb <= kw && lb > worst) {
+                            worst = lb;
+                            zw = p;
+                        }
+                    }
+                }
+                __syncwarp();
+            }
+        }
+        if (event) break;
+        for (int o = 16; o; o >>= 1) phi = fminf(phi, __shfl_xor_sync(0xffffffffu, phi, o));
+        if (phi > kw) {
+            if (lane == 0) atomicMax(reinterpret_cast<int *>(&sd.scr.ginst[I].phi), __float_as_int(phi));
+            return true;
+        }
+        const unsigned m = __reduce_max_sync(0xffffffffu, zw < 0 ? 0u : okey32(worst));
+        const int l = __ffs(__ballot_sync(0xffffffffu, zw >= 0 && okey32(worst) == m)) - 1;
+        if (l < 0) break;
+        zw = __shfl_sync(0xffffffffu, zw, l);
+        bool waits = false;
+        if (lane == 0) {
+            atomicAdd(&sh.w.nphi, 1);
+            waits = wait_point(sd, sh, w, zw);
+        }
+        if (__shfl_sync(0xffffffffu, waits, 0)) return false;
+    }
+    if (lane == 0) wait_event(sd, sh, w, I, 1);
+    return false;
+}
+
 /* Sweep graph: the same search for point w (packed coordinates), by the reference's order of face
  * instances and, within one, of keys.  Registers w on an instance event or a point when the
  * answer is not yet known.  One warp; true with the state and w's face when found. */
-FD_COLD bool resume_graph(const fd_station_dev &sd, Shared &sh, int w, float *st0, float *st4, int *face)
+FD_COLD bool resume_graph(const fd_station_dev &sd, Shared &sh, WarpSmem &ws, int w, float *st0, float *st4, int *face)
 {
     const int lane = threadIdx.x & 31;
     const GraphSmem gs = gsmem(sh);
@@ -1640,14 +1780,11 @@ FD_COLD bool resume_graph(const fd_station_dev &sd, Shared &sh, int w, float *st
     const int I = own_inst(ow);
     const GRect r = gs.rect[I];
     const int n = rect_n(r), nuf = r.nuf();
-    if (vload(gs.nkeyed[I]) < n) {   /* keys below w's not all known yet */
-        if (lane == 0) wait_event(sd, sh, w, I, 1);
-        return false;
-    }
     const fdn_frame fr = frame_of(r.face());
     const int su = (int)t_stride(sd, fr.axis_u), sv = (int)t_stride(sd, fr.axis_v);
     const int base = inst_node(sd, r, 0), in = fr.inner * (int)t_stride(sd, fr.axis_n);
     const int wu = coord(fr.axis_u, wx, wy, wz) - r.ulo, wv = coord(fr.axis_v, wx, wy, wz) - r.vlo;
+    if (vload(gs.nkeyed[I]) < n && !keys_above(sd, sh, ws, I, w, vload(sd.T[base + wu * su + wv * sv + in]))) return false;
     const unsigned long long kc = node_key(vload(sd.T[base + wu * su + wv * sv + in]), wv * nuf + wu);
     const int dv = 32 / nuf, du = 32 - dv * nuf;   /* 32 points on in fill order */
     for (int guard = 0; guard <= 2 * n + 2; guard++) {
@@ -1851,7 +1988,7 @@ __device__ void run_walk(const fd_station_dev &sd, Shared &sh, const CtaSmem &cs
             chunks++;
         } else {
             h = __shfl_sync(0xffffffffu, e, 0);
-            if (h < 0 || !(sh.graph ? resume_graph(sd, sh, h, &in0, &in4, &face) : resume_waiter(sd, sh, h, &in0, &in4))) continue;
+            if (h < 0 || !(sh.graph ? resume_graph(sd, sh, ws, h, &in0, &in4, &face) : resume_waiter(sd, sh, h, &in0, &in4))) continue;
         }
         warp_chunk(sd, sh, cs, ws, face, e, act == 2, in0, in4, dag, cn);
     }
@@ -1863,7 +2000,7 @@ __device__ void walk_reset(Shared &sh, int nq, int rqcap)
 {
     sh.w.nq = nq;
     for (int k = 0; k < 6; k++) { sh.w.qhead[k] = 0; sh.w.qtail[k] = 0; sh.w.qcap[k] = 0; sh.w.qbase[k] = 0; }
-    sh.w.rqhead = sh.w.rqtail = sh.w.idle = sh.w.ndone = sh.w.npark = 0;
+    sh.w.rqhead = sh.w.rqtail = sh.w.idle = sh.w.ndone = sh.w.npark = sh.w.nphi = 0;
     sh.w.rqcap = rqcap;
     sh.w.exitkey = 0ull;
 }
@@ -1993,6 +2130,7 @@ __device__ void graph_sweep(const fd_station_dev &sd, Shared &sh, CtaSmem &cs, W
                     if (sh.n > 0) {
                         if (ninst >= cap) { over = true; break; }
                         fd_ginst &gi = sd.scr.ginst[ninst];
+                        gi.phi = 0.f;
                         gi.ev[0] = gi.ev[1] = FD_EV_NONE; gi.exitkey = 0ull;
                         GRect &gr = gs.rect[ninst];
                         gr.fl = (short)(sh.layer << 3 | face);

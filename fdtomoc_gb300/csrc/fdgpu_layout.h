@@ -80,6 +80,8 @@ typedef struct {
     int ev[2];                     /* events "all keys final", "all points done": the first parked
                                       point waiting for it (gpark index), FD_EV_NONE, FD_EV_FIRED */
     unsigned long long exitkey;    /* largest key of a point that made a writer call (0: none) */
+    float phi;                     /* no key of the instance that is still missing lies below (keys_above) */
+    int pad;
 } fd_ginst;
 
 /* the largest sweep graph: grid extent, face instances (at most nx + ny + nz + 8); larger grids walk their
@@ -91,9 +93,10 @@ typedef struct {
 #define FD_EV_FIRED (-2)
 
 /* sizes of the small sweep-graph tables */
-#define FD_GWAIT_CAP 65536   /* (awaited point, waiting point) pairs, a hash table */
+#define FD_GPHI_CAP 65536    /* of the waits below, those for a bound on missing keys (keys_above) */
+#define FD_GWAIT_CAP 131072  /* (awaited point, waiting point) pairs, a hash table */
 #define FD_GPARK_CAP 65536   /* points parked on an instance event: (point, next in the event's list) */
-#define FD_GRQ_CAP 262144    /* resume queue */
+#define FD_GRQ_CAP 327680    /* resume queue */
 
 /* Face-walk scratch of one station, sized for its largest face m (34 bytes per point):
  * key 8m | rec 8m | pst 4m | queue 4m | rq 8m | dag 2m (+32). */

@@ -96,8 +96,7 @@ typedef struct {
                                  11 a second point waiting on one point, 12 a point found no
                                  earlier point to take its stencil state from, 14 a node that no
                                  face instance owns, 15 a wait table full, 17 a walk ran past its
-                                 bound, 18 a queue entry outside the walk's nodes, 100 + k a
-                                 cluster barrier k gave up (several CTAs per station only) */
+                                 bound, 18 a queue entry outside the walk's nodes */
     int32_t sm;               /* the SM whose CTA ran the solve */
     int32_t pad;
 } fdgpu_stats;
@@ -122,10 +121,9 @@ int fdgpu_station_from_par(int ac, char **av, fdgpu_station *st, char *velfile, 
 int fdgpu_solve_host(fdgpu_ctx *ctx, int n, const fdgpu_station *st, const float *velocity, int mnx, int mny,
                      int mnz, float *const *times, const float *const *init_times, fdgpu_stats *stats);
 
-/* CTAs (one per SM) that may cooperate on each station in later solves of this context, as one
- * thread-block cluster: 0 (the default) lets the library choose, 1, 2, 4 or 8 asks for that many.
- * The library currently caps it at 1 (multi-CTA solving is disabled in this build).  Results do not
- * depend on it.  No counterpart in the reference (one OpenMP thread per station). */
+/* CTAs (one per SM) that may cooperate on each station in later solves of this context: 0 (the default)
+ * lets the library choose, 1, 2, 4 or 8 asks for that many.  This build solves a station with one CTA
+ * whatever is asked for.  Results do not depend on it.  No counterpart in the reference (one OpenMP thread per station). */
 int fdgpu_set_cluster(fdgpu_ctx *ctx, int ctas_per_station);
 
 /* Bounds, in SM clock cycles, of the solver's waits in later solves of this context: a warp with
