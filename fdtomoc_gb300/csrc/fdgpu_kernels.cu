@@ -1427,6 +1427,22 @@ __device__ __forceinline__ Where locate(const fd_station_dev &sd, const Shared &
     return wh;
 }
 
+/* Queue a point whose 2-D trials (which) won without the state it inherits.  Its record, not read while it is pending,
+ * takes the lowest of their values: what that state must exceed to reject them all (exit_floor). */
+FD_COLD void defer(const fd_station_dev &sd, Shared &sh, const WarpSmem &ws, int slot, long long p, unsigned which, int e)
+{
+    if (sh.graph) {
+        double low = 1.e11;
+        for (; which; which &= which - 1) {
+            const double v = ws.res[slot][__ffs(which) - 1];
+            if (lt(v, low)) low = v;
+        }
+        sd.scr.grec[p].x = __double2float_ru(low);
+        wfence(sh);
+    }
+    enqueue_to(sh.graph ? sd.scr.grq : sd.scr.rq, sh.w.rqtail, sh.w.rqcap, sh, e);
+}
+
 /* a float from global to shared memory without a register (waited for with cp.async.wait_all): the
  * slownesses are first needed by the trials, after the guards that the times alone decide */
 __device__ __forceinline__ void copy_async4(float *dst, const float *src)
@@ -1435,9 +1451,11 @@ __device__ __forceinline__ void copy_async4(float *dst, const float *src)
 }
 
 /* Evaluate and commit one chunk of face F: lane l holds queue entry e (-1 for none).  A node given
- * with have_inherit uses (it0, it4) as the stencil state entering it.  All 32 lanes call. */
+ * with inherit kState uses (it0, it4) as the stencil state entering it; with kFloor it0 is a floor of that
+ * state's larger time, and the node commits if no 2-D trial wins above it.  All 32 lanes call. */
+enum { kNoState, kState, kFloor };
 __device__ void warp_chunk(const fd_station_dev &sd, Shared &sh, const CtaSmem &cs, WarpSmem &ws, int F, int e,
-                           bool have_inherit, float it0, float it4, unsigned char *dag, Counters cn)
+                           int inherit, float it0, float it4, unsigned char *dag, Counters cn)
 {
     const int lane = threadIdx.x & 31;
     const fdn_frame fr = frame_of(F);
@@ -1495,7 +1513,7 @@ __device__ void warp_chunk(const fd_station_dev &sd, Shared &sh, const CtaSmem &
         ws.s4[lane] = d2f_trunc(sd.g.zrow[(long long)(FD_OK(wh.z, sd.g.nz, 8) ? wh.z : 0) * FD_Z_N + FD_Z_RDQ]);
         if (em & 0xF0u) em = ne_prune(dsc, tr, em);
         /* a 2-D trial before any corner / new-edge call reads the state an earlier point left */
-        permissive = !have_inherit && (gm & 0xFu) == 0 && !((gm & 0xF0u) && t[NB_POINT] > 1.0e9f) && (gm & 0xFF00u);
+        permissive = inherit != kState && (gm & 0xFu) == 0 && !((gm & 0xF0u) && t[NB_POINT] > 1.0e9f) && (gm & 0xFF00u);
     }
     __syncwarp();
     const int n3 = push_items(ws.items, 0, em, 0xFu, lane);
@@ -1507,7 +1525,7 @@ __device__ void warp_chunk(const fd_station_dev &sd, Shared &sh, const CtaSmem &
     eval_items<0>(sd, dsc, ws, ws.items, n3, lane);
     eval_items<1>(sd, dsc, ws, ws.items + n3, n1 - n3, lane);
     __syncwarp();
-    const float lo = __int_as_float(0xff800000);   /* -inf: no stale floor */
+    const float lo = inherit == kFloor ? it0 : __int_as_float(0xff800000);   /* -inf: no stale floor */
     const float p0 = permissive ? lo : it0, p4 = permissive ? lo : it4;
     if (valid) em = stale_pair(sd, dsc, ws, lane, F, gm, em, p0, p4);
     __syncwarp();
@@ -1526,11 +1544,11 @@ __device__ void warp_chunk(const fd_station_dev &sd, Shared &sh, const CtaSmem &
     if (valid) {
         fin = commit_node(sd, sh, dsc, ws, lane, F, wh, gm, em, p0, p4, permissive, dag, was, cn);
         if (!fin) {
-            atomicAdd(reinterpret_cast<unsigned long long *>(&sh.w.deferred), 1ull);
+            if (inherit != kFloor) atomicAdd(reinterpret_cast<unsigned long long *>(&sh.w.deferred), 1ull);
             if (sh.nodefer)
                 atomicCAS(&sh.w.status, 0, 6);   /* excluded by the sweep's precondition */
             else
-                enqueue_to(sh.graph ? sd.scr.grq : sd.scr.rq, sh.w.rqtail, sh.w.rqcap, sh, e);
+                defer(sd, sh, ws, lane, wh.p, gm & em & k2d, e);
         }
     }
     if (sh.graph) graph_release(sd, sh, ws, F, fin, was, wh);
@@ -1668,106 +1686,160 @@ static_assert(trials_above_a_neighbour(), "keys_above");
  * Why: without it such a point waits for the whole inner layer, and where border points inherit state (a fast layer
  * at the grid's edge) the planes of a forward sweep run one after another, which made a few windows five times
  * as long as the others.  Their batches and lists end with them: 150 windows of 73 to 91 319 -> 242 ms, 24 host
- * stations of 49x45x33 96 -> 60, 48 served requests 91 -> 77; with all 26 neighbours instead of the six 251, 65 and 83. */
-FD_COLD bool keys_above(const fd_station_dev &sd, Shared &sh, WarpSmem &ws, int I, int w, float kw)
+ * stations of 49x45x33 96 -> 60, 48 served requests 91 -> 76; with all 26 neighbours instead of the six 251, 65 and 83. */
+struct OpenScan {
+    float phi;    /* the least time at the open nodes and their six neighbours (of instance wide: 26) */
+    int below;    /* the node with the largest such time that is not above thr, -1 if none is */
+    int of_wide;  /* a node of instance wide that is open, -1 if none is */
+};
+
+/* the open nodes of the instances before I; false if they are too many to look through */
+FD_COLD bool scan_open(const fd_station_dev &sd, Shared &sh, WarpSmem &ws, int I, int wide, float thr, OpenScan &out)
 {
     const int lane = threadIdx.x & 31;
     const GraphSmem gs = gsmem(sh);
     unsigned *bits = reinterpret_cast<unsigned *>(&ws.res[0][0]);
     constexpr int kBits = 8 * sizeof ws.res;   /* a flag per node of an instance; larger faces wait for the event */
-    if (vload(sd.scr.ginst[I].phi) > kw) return true;
-    bool event = vload(sh.w.nphi) >= FD_GPHI_CAP - FD_WARPS;   /* these waits leave the tables' room for the others */
-    for (int turn = 0; turn < 8 && !event; turn++) {   /* a turn more if the node found is done by now */
-        float phi = 1.e10f, worst = -2.f;   /* worst: the largest bound that is not above kw, at node zw */
-        int zw = -1, scanned = 0;
-        for (int J0 = 0; J0 < I && !event; J0 += 32) {
-            /* the instances that have nodes to come */
-            const int Jl = J0 + lane;
-            unsigned open = __ballot_sync(0xffffffffu, Jl < I && vload(gs.ndone[Jl < I ? Jl : 0]) < rect_n(gs.rect[Jl < I ? Jl : 0]));
-            for (; open; open &= open - 1) {
-                const GRect r = gs.rect[J0 + __ffs(open) - 1];
-                const int n = rect_n(r), nuf = r.nuf();
-                scanned += n;
-                if (n > kBits || scanned > FD_PHI_NODES) {
-                    event = true;
-                    break;
-                }
-                const fdn_frame fr = frame_of(r.face());
-                const int su = (int)t_stride(sd, fr.axis_u), sv = (int)t_stride(sd, fr.axis_v);
-                const int du = 32 % nuf, step = du * su + 32 / nuf * sv, wrap = sv - nuf * su;
-                const int base = inst_node(sd, r, 0);
-                unsigned any = 0;
-                int u = lane % nuf, q = base + u * su + lane / nuf * sv;
-                for (int j0 = 0; j0 < n; j0 += 128) {
-                    unsigned c[4];
+    if (vload(sh.w.nphi) >= FD_GPHI_CAP - FD_WARPS) return false;   /* these waits leave the tables' room for the others */
+    float phi = 1.e10f, worst = -2.f;
+    int zw = -1, zj = -1, scanned = 0;
+    for (int J0 = 0; J0 < I; J0 += 32) {
+        /* the instances that have nodes to come */
+        const int Jl = J0 + lane;
+        unsigned open = __ballot_sync(0xffffffffu, Jl < I && vload(gs.ndone[Jl < I ? Jl : 0]) < rect_n(gs.rect[Jl < I ? Jl : 0]));
+        for (; open; open &= open - 1) {
+            const int J = J0 + __ffs(open) - 1;
+            const GRect r = gs.rect[J];
+            const int n = rect_n(r), nuf = r.nuf();
+            scanned += n;
+            if (n > kBits || scanned > FD_PHI_NODES) return false;
+            const fdn_frame fr = frame_of(r.face());
+            const int su = (int)t_stride(sd, fr.axis_u), sv = (int)t_stride(sd, fr.axis_v);
+            const int du = 32 % nuf, step = du * su + 32 / nuf * sv, wrap = sv - nuf * su;
+            unsigned any = 0;
+            int u = lane % nuf, q = inst_node(sd, r, 0) + u * su + lane / nuf * sv;
+            for (int j0 = 0; j0 < n; j0 += 128) {
+                unsigned c[4];
 #pragma unroll
-                    for (int k = 0; k < 4; k++) {
-                        c[k] = j0 + 32 * k + lane < n ? vload(sd.scr.gcnt[q]) : FD_DONEB;
-                        u += du;
-                        q += step;
-                        if (u >= nuf) {
-                            u -= nuf;
-                            q += wrap;
-                        }
-                    }
-#pragma unroll
-                    for (int k = 0; k < 4; k++) {
-                        const unsigned m = __ballot_sync(0xffffffffu, !(c[k] & FD_DONEB));
-                        if (lane == 0 && j0 + 32 * k < n) bits[(j0 >> 5) + k] = m;
-                        any |= m;
+                for (int k = 0; k < 4; k++) {
+                    c[k] = j0 + 32 * k + lane < n ? vload(sd.scr.gcnt[q]) : FD_DONEB;
+                    u += du;
+                    q += step;
+                    if (u >= nuf) {
+                        u -= nuf;
+                        q += wrap;
                     }
                 }
-                __syncwarp();
-                wfence(sh);
-                if (any) {
-                    for (int j0 = 0; j0 < n; j0 += 32) {
-                        if (!((bits[j0 >> 5] >> lane) & 1u)) continue;
-                        const int xyz = inst_xyz(r, j0 + lane);
-                        const int x = xyz & 1023, y = (xyz >> 10) & 1023, z = xyz >> 20;
-                        const int nx = sd.g.nx, nxy = nx * sd.g.ny, p = z * nxy + y * nx + x;
-                        const int o[7] = {0, x > 0 ? -1 : 0, x < nx - 1 ? 1 : 0, y > 0 ? -nx : 0, y < sd.g.ny - 1 ? nx : 0,
-                                          z > 0 ? -nxy : 0, z < sd.g.nz - 1 ? nxy : 0};
-                        float t[7];
 #pragma unroll
-                        for (int k = 0; k < 7; k++) t[k] = sd.T[p + o[k]];
-                        float lb = 1.e10f;
-#pragma unroll
-                        for (int k = 0; k < 7; k++) lb = t[k] >= 0.f ? fminf(lb, t[k]) : -1.f;
-                        phi = fminf(phi, lb);
-                        if (lb <= kw && lb > worst) {
-                            worst = lb;
-                            zw = p;
-                        }
-                    }
+                for (int k = 0; k < 4; k++) {
+                    const unsigned m = __ballot_sync(0xffffffffu, !(c[k] & FD_DONEB));
+                    if (lane == 0 && j0 + 32 * k < n) bits[(j0 >> 5) + k] = m;
+                    any |= m;
                 }
-                __syncwarp();
             }
+            __syncwarp();
+            wfence(sh);
+            for (int j0 = 0; any && j0 < n; j0 += 32) {
+                if (!((bits[j0 >> 5] >> lane) & 1u)) continue;
+                const int xyz = inst_xyz(r, j0 + lane);
+                const int x = xyz & 1023, y = (xyz >> 10) & 1023, z = xyz >> 20;
+                const int nx = sd.g.nx, nxy = nx * sd.g.ny, p = z * nxy + y * nx + x;
+                const int xl = x > 0 ? -1 : 0, xh = x < nx - 1 ? 1 : 0, yl = y > 0 ? -nx : 0, yh = y < sd.g.ny - 1 ? nx : 0;
+                const int zl = z > 0 ? -nxy : 0, zh = z < sd.g.nz - 1 ? nxy : 0;
+                const int o[7] = {0, xl, xh, yl, yh, zl, zh};
+                float lb = 1.e10f;
+                float t[7];
+#pragma unroll
+                for (int k = 0; k < 7; k++) t[k] = sd.T[p + o[k]];
+#pragma unroll
+                for (int k = 0; k < 7; k++) lb = t[k] >= 0.f ? fminf(lb, t[k]) : -1.f;
+                if (J == wide) {
+                    for (int k = 0; k < 27; k++) {
+                        const float tk = sd.T[p + (k % 3 == 0 ? xl : k % 3 == 2 ? xh : 0) + (k / 3 % 3 == 0 ? yl : k / 3 % 3 == 2 ? yh : 0)
+                                              + (k / 9 == 0 ? zl : k / 9 == 2 ? zh : 0)];
+                        lb = tk >= 0.f ? fminf(lb, tk) : -1.f;
+                    }
+                    zj = p;
+                }
+                phi = fminf(phi, lb);
+                if (lb <= thr && lb > worst) {
+                    worst = lb;
+                    zw = p;
+                }
+            }
+            __syncwarp();
         }
-        if (event) break;
-        for (int o = 16; o; o >>= 1) phi = fminf(phi, __shfl_xor_sync(0xffffffffu, phi, o));
-        if (phi > kw) {
-            if (lane == 0) atomicMax(reinterpret_cast<int *>(&sd.scr.ginst[I].phi), __float_as_int(phi));
+    }
+    for (int o = 16; o; o >>= 1) phi = fminf(phi, __shfl_xor_sync(0xffffffffu, phi, o));
+    const unsigned m = __reduce_max_sync(0xffffffffu, zw < 0 ? 0u : okey32(worst));
+    const unsigned at = __ballot_sync(0xffffffffu, zw >= 0 && okey32(worst) == m);
+    out.phi = phi;
+    out.below = at ? __shfl_sync(0xffffffffu, zw, __ffs(at) - 1) : -1;
+    out.of_wide = (int)__reduce_max_sync(0xffffffffu, zj);
+    return true;
+}
+
+/* point w waits for open node p, found by scan_open; false if p is done already */
+__device__ bool wait_open(const fd_station_dev &sd, Shared &sh, int w, int p)
+{
+    bool waits = false;
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(&sh.w.nphi, 1);
+        waits = wait_point(sd, sh, w, p);
+    }
+    return __shfl_sync(0xffffffffu, waits, 0);
+}
+
+FD_COLD bool keys_above(const fd_station_dev &sd, Shared &sh, WarpSmem &ws, int I, int w, float kw)
+{
+    if (vload(sd.scr.ginst[I].phi) > kw) return true;
+    OpenScan o;
+    for (int turn = 0; turn < 8 && scan_open(sd, sh, ws, I, -1, kw, o); turn++) {   /* a turn more if the node is done by now */
+        if (o.phi > kw) {
+            if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<int *>(&sd.scr.ginst[I].phi), __float_as_int(o.phi));
             return true;
         }
-        const unsigned m = __reduce_max_sync(0xffffffffu, zw < 0 ? 0u : okey32(worst));
-        const int l = __ffs(__ballot_sync(0xffffffffu, zw >= 0 && okey32(worst) == m)) - 1;
-        if (l < 0) break;
-        zw = __shfl_sync(0xffffffffu, zw, l);
-        bool waits = false;
-        if (lane == 0) {
-            atomicAdd(&sh.w.nphi, 1);
-            waits = wait_point(sd, sh, w, zw);
-        }
-        if (__shfl_sync(0xffffffffu, waits, 0)) return false;
+        if (o.below >= 0 && wait_open(sd, sh, w, o.below)) return false;
     }
-    if (lane == 0) wait_event(sd, sh, w, I, 1);
+    if ((threadIdx.x & 31) == 0) wait_event(sd, sh, w, I, 1);
     return false;
+}
+
+/* Point w of instance I inherits the state of the last writer of instance J, which is not complete.  A floor of
+ * that state's larger time: the last writer is the last one that is done, whose record is there, or a node of J that
+ * is open now, and the times of the nodes about that one, when it is evaluated, are not below the least now at any open
+ * node before I, its six neighbours and, for J, its 26 (see keys_above).  A floor above the value that won
+ * without one (thr) is worth another look at the point: 1, with the floor.  Else it waits for an open node that stands
+ * against that (0), or is to wait for J (2).  Such points come first in their instance, where the state is that of
+ * the times J ends with, far above their own; waiting for J made the planes of the slowest windows run one after another:
+ * 400 windows of 25 to 61 166 and 143 ms (two models) -> 142 and 112, 48 served requests 76 and 50 -> 55 and 41. */
+FD_COLD int exit_floor(const fd_station_dev &sd, Shared &sh, WarpSmem &ws, int I, int J, int w, float thr, float *floor)
+{
+    const GRect rj = gsmem(sh).rect[J];
+    OpenScan o;
+    for (int turn = 0; turn < 8 && scan_open(sd, sh, ws, I, J, thr, o); turn++) {
+        wfence(sh);
+        /* after the flags: a point whose flag says done has put its key there */
+        const unsigned long long ek = vload(sd.scr.ginst[J].exitkey);
+        if (!ek || !FD_OK((long long)(ek & 0xffffffffu), rect_n(rj), 31)) return 2;
+        const int p = inst_node(sd, rj, (int)(ek & 0xffffffffu));
+        const float f = fminf(o.phi, fmaxf(vload(sd.scr.grec[p].x), vload(sd.scr.grec[p].y)));
+        if (f > thr) {
+            *floor = f;
+            return 1;
+        }
+        const int z = o.below >= 0 ? o.below : o.of_wide;
+        if (z < 0) return 2;
+        if (wait_open(sd, sh, w, z)) return 0;
+    }
+    return 2;
 }
 
 /* Sweep graph: the same search for point w (packed coordinates), by the reference's order of face
  * instances and, within one, of keys.  Registers w on an instance event or a point when the
  * answer is not yet known.  One warp; true with the state and w's face when found. */
-FD_COLD bool resume_graph(const fd_station_dev &sd, Shared &sh, WarpSmem &ws, int w, float *st0, float *st4, int *face)
+FD_COLD bool resume_graph(const fd_station_dev &sd, Shared &sh, WarpSmem &ws, int w, float *st0, float *st4, bool *floor_only,
+                          int *face)
 {
     const int lane = threadIdx.x & 31;
     const GraphSmem gs = gsmem(sh);
@@ -1816,7 +1888,8 @@ FD_COLD bool resume_graph(const fd_station_dev &sd, Shared &sh, WarpSmem &ws, in
         }
         done = warp_max_u64(done);
         pend = warp_max_u64(pend);
-        int verdict = 0;   /* 0 look again, 1 found, 2 waiting */
+        int verdict = 0;   /* 0 look again, 1 found, 2 waiting, 3 an earlier instance is not complete */
+        int before = -1;   /* that instance */
         float t0 = sh.carry_t0, t4 = sh.carry_t4;
         if (lane == 0) {
             if (pend > done) {
@@ -1836,7 +1909,7 @@ FD_COLD bool resume_graph(const fd_station_dev &sd, Shared &sh, WarpSmem &ws, in
                 verdict = 1;
                 for (int J = I - 1; J >= 0; J--) {
                     const GRect &rj = gs.rect[J];
-                    if (vload(gs.ndone[J]) < rect_n(rj)) { wait_event(sd, sh, w, J, 2); verdict = 2; break; }
+                    if (vload(gs.ndone[J]) < rect_n(rj)) { before = J; verdict = 3; break; }
                     wfence(sh);
                     const unsigned long long ek = vload(sd.scr.ginst[J].exitkey);
                     if (ek) {
@@ -1850,6 +1923,19 @@ FD_COLD bool resume_graph(const fd_station_dev &sd, Shared &sh, WarpSmem &ws, in
             }
         }
         verdict = __shfl_sync(0xffffffffu, verdict, 0);
+        if (verdict == 3) {
+            before = __shfl_sync(0xffffffffu, before, 0);
+            float f = 0.f;
+            const int can = exit_floor(sd, sh, ws, I, before, w, vload(sd.scr.grec[node_of(sd, w)].x), &f);
+            if (can == 1) {
+                *st0 = *st4 = f;
+                *floor_only = true;
+                *face = r.face();
+                return true;
+            }
+            if (can == 2 && lane == 0) wait_event(sd, sh, w, before, 2);
+            return false;
+        }
         if (verdict == 2) return false;
         if (verdict == 1) {
             *st0 = __shfl_sync(0xffffffffu, t0, 0);
@@ -1972,6 +2058,7 @@ __device__ void run_walk(const fd_station_dev &sd, Shared &sh, const CtaSmem &cs
         }
         int e = -1, face = sh.face;
         float in0 = 0.f, in4 = 0.f;
+        bool floor_only = false;
         if (lane < m) {
             e = read_entry((act == 1 ? queue : rq) + h, lane, sh);
             /* an entry outside the walk's nodes ends the walk with a status instead of an access */
@@ -1988,9 +2075,9 @@ __device__ void run_walk(const fd_station_dev &sd, Shared &sh, const CtaSmem &cs
             chunks++;
         } else {
             h = __shfl_sync(0xffffffffu, e, 0);
-            if (h < 0 || !(sh.graph ? resume_graph(sd, sh, ws, h, &in0, &in4, &face) : resume_waiter(sd, sh, h, &in0, &in4))) continue;
+            if (h < 0 || !(sh.graph ? resume_graph(sd, sh, ws, h, &in0, &in4, &floor_only, &face) : resume_waiter(sd, sh, h, &in0, &in4))) continue;
         }
-        warp_chunk(sd, sh, cs, ws, face, e, act == 2, in0, in4, dag, cn);
+        warp_chunk(sd, sh, cs, ws, face, e, act == 2 ? (floor_only ? kFloor : kState) : kNoState, in0, in4, dag, cn);
     }
     if (lane == 0 && chunks) atomicAdd(reinterpret_cast<unsigned long long *>(&sh.w.rounds), (unsigned long long)chunks);
 }
