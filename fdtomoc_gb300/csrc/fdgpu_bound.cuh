@@ -18,7 +18,7 @@
  *     largest reciprocal it is within 1408 2^-53 T^2 v^4 of the exact one; FB_E64 is 20 times that;
  *   - FB_EY covers the quotient (reciprocal, product and square root within 2^-21 each) and FB_ET T the
  *     FP64 path's own rounding of x.
- * Table doubles enter through truncation toward zero to FP32, on the integer pipe.  A NaN or an
+ * Table doubles enter through truncation toward zero to FP32.  A NaN or an
  * overflow anywhere makes the result NaN and the final comparison fail, so the caller evaluates the
  * trial in FP64.  (Error bounds carried along through every operation, the form this replaces, took 350
  * instructions a trial where this takes about 90.)

@@ -12,7 +12,6 @@
  *   - x / d for a geometric divisor d is RN(x/d) computed from the tabulated RN(1/d) with two
  *     fused-multiply-add corrections (Markstein's theorem; 5 FP64 ops instead of ~17 for a
  *     generic division on this part);
- *   - float->double conversions and power-of-two scalings are done on the integer pipe;
  *   - a stencil whose causality floor (the largest time it reads, which its accepted root can
  *     never be below) is already >= the running minimum is not evaluated: it cannot lower the
  *     minimum, and its only side effect, the stale (t0,t4) state, is still applied.

@@ -16,9 +16,9 @@
  * The one sequential coupling that is not a neighbour relation is the stale (t0,t4) pair of
  * fdsph2d (src/sphfd.c:6116-6121): a point whose first 2-D trial comes before any 3-D / new-edge
  * call of its own reads the pair left by the previous point in sort order.  Such a point is put
- * aside; when no other point is ready, the one with the smallest key has every smaller-key point
- * done, and its pair is the record of the largest-key earlier point that made a writer call (or
- * the face's entry pair).  This is rare (hundreds of points per million).
+ * aside if a 2-D value wins without that pair, and waits for the record of the largest-key earlier
+ * point that made a writer call (or the entry pair); bounds on the times still missing keep that wait
+ * short (keys_above, exit_floor).  This is rare on most grids (hundreds of points per million).
  *
  * Within a walk the warps of the CTA are independent workers that meet only at shared-memory
  * counters (see "warp workers" below); every wait among them is bounded and ends in an error
@@ -476,11 +476,11 @@ constexpr unsigned k1d = 0x1Fu << TK_1D0;
 /* ---- evaluation of the queued items ----
  *
  * An FP64 instruction occupies its sub-partition for 64 cycles whatever the number of active lanes, so a
- * stencil evaluated by one lane holds it for its whole serial length: 116 instructions for a corner, 70 for
+ * stencil evaluated by one lane holds it for its whole serial length: some 140 instructions for a corner, 85 for
  * a new-edge or a 2-D trial.  That is the right form for a warp full of items.  A chunk of a forward
  * sweep has one to five corners and rarely more than one of the others; there four lanes share an
  * item, each taking the products, divisions or sums that do not depend on one another, in the
- * reference's order within every sum: 49 and 38 instructions for up to eight items (two such passes for
+ * reference's order within every sum: some 60 and 45 instructions for up to eight items (two such passes for
  * nine to sixteen corners cost as much as one of the other form). */
 #define FD_QUAD 8
 
