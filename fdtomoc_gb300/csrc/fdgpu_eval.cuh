@@ -83,7 +83,7 @@ struct PointCtx {
 __device__ __forceinline__ const double *node_row(const fd_geo_dev &g, int z, int y)
 {
     if (!FD_OK(z, g.nz, 1) || !FD_OK(y, g.ny, 2)) { z = 0; y = 0; }
-    return g.node + ((long long)z * g.ny + y) * FD_N_N;
+    return g.node + (long long)(z * g.ny + y) * FD_N_N;   /* a face has at most 2^30 points */
 }
 
 /* canonical distance products of the new-edge / 2-D / new-face stencils */

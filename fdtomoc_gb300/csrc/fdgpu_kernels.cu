@@ -515,7 +515,7 @@ __device__ void eval_corners_quad(const fd_station_dev &sd, const TrialDesc *dsc
            *Q = &ws.res[lead + 3][TK_2D0];
     int zc = ws.z[slot] + d.zmin, yc = ws.y[slot] + d.ymin;
     if (!FD_OK(zc, sd.g.nz - 1, 6) || !FD_OK(yc, sd.g.ny - 1, 7)) { zc = 0; yc = 0; }
-    const double *C = sd.g.cell + ((long long)zc * (sd.g.ny - 1) + yc) * FD_C_N;
+    const double *C = sd.g.cell + (long long)(zc * (sd.g.ny - 1) + yc) * FD_C_N;
     const double a = C[d.a_idx], i2a = C[d.i2a_idx];
     float tm = 0.f;
     double tr = 0.0;
@@ -1093,7 +1093,7 @@ __device__ __forceinline__ unsigned graph_record(const fd_station_dev &sd, Share
 /* nodes of a chunk up to which a release gives each neighbour a lane (more: each node), in a sweep of
  * several faces and of one */
 #ifndef FD_FEW
-#define FD_FEW 12
+#define FD_FEW 16
 #endif
 #ifndef FD_FEW1
 #define FD_FEW1 6
@@ -1146,8 +1146,9 @@ __device__ __forceinline__ void release_one(const fd_station_dev &sd, Shared &sh
  *
  * Measured, commit and release of one chunk: 55 -> 28 thousand cycles at 3.8 nodes (27x20x21), 80 -> 50 at
  * 29 nodes (141x121x57), against a loop over the neighbours with a search of the six faces for each
- * owner and a key event inside it.  The two forms cost the same at about 12 nodes of a forward sweep (27
- * steps of the second form against 12 of the first) and at 6 of a one-face sweep (17 steps). */
+ * owner and a key event inside it.  The two forms cost the same at about 16 nodes of a forward sweep (27
+ * steps of the second form; 27x20x21 takes 2.5 % longer with the line at 8, 0.7 % at 12) and at 6 of a one-face
+ * sweep (17 steps; 4 and 10 measure the same). */
 __device__ void graph_release(const fd_station_dev &sd, Shared &sh, WarpSmem &ws, int F, bool fin, unsigned was,
                               const Where &wh)
 {
@@ -1479,9 +1480,10 @@ __device__ void warp_chunk(const fd_station_dev &sd, Shared &sh, const CtaSmem &
         ws.z[lane] = wh.z;
         ws.y[lane] = wh.y;
         float *tr = ws.t[lane], *sr = ws.s[lane];
-        const long long su = t_stride(sd, fr.axis_u), sv = t_stride(sd, fr.axis_v);
+        const int su = (int)t_stride(sd, fr.axis_u), sv = (int)t_stride(sd, fr.axis_v);
         const long long ssu = s_stride(sd, fr.axis_u), ssv = s_stride(sd, fr.axis_v);
-        const long long inner_t = fr.inner * t_stride(sd, fr.axis_n), inner_s = fr.inner * s_stride(sd, fr.axis_n);
+        const int inner_t = fr.inner * (int)t_stride(sd, fr.axis_n);   /* a plane has at most 2^30 nodes */
+        const long long inner_s = fr.inner * s_stride(sd, fr.axis_n);
         /* columns (bits 0-2) and rows (bits 3-5) of the block inside the grid */
         const unsigned inside = (wh.r.u > 0 ? 1u : 0u) | 2u | (wh.r.u < wh.r.nu - 1 ? 4u : 0u) | (wh.r.v > 0 ? 8u : 0u)
                                 | 16u | (wh.r.v < wh.r.nv - 1 ? 32u : 0u);
@@ -1492,7 +1494,7 @@ __device__ void warp_chunk(const fd_station_dev &sd, Shared &sh, const CtaSmem &
             const unsigned bits = 1u << (du + 1) | 8u << (dv + 1);
             t[nb] = 0.f;
             if ((inside & bits) == bits) {
-                const long long o = du * su + dv * sv + (w ? inner_t : 0ll);
+                const int o = du * su + dv * sv + (w ? inner_t : 0);
                 if (FD_OK(wh.p + o, (long long)sd.g.nx * sd.g.ny * sd.g.nz, 27)) {
                     t[nb] = pT[o];   /* the CTA's own stores keep its L1 current */
                     copy_async4(&sr[nb], pS + (du * ssu + dv * ssv + (w ? inner_s : 0ll)));

@@ -220,7 +220,7 @@ __device__ __forceinline__ double eval_3d(const TrialDesc &d, const float *t18, 
     const double sl16 = 2. * sum * slo;
     int zc = z + d.zmin, yc = y + d.ymin;
     if (!FD_OK(zc, g.nz - 1, 6) || !FD_OK(yc, g.ny - 1, 7)) { zc = 0; yc = 0; }
-    const double *C = g.cell + ((long long)zc * (g.ny - 1) + yc) * FD_C_N;
+    const double *C = g.cell + (long long)(zc * (g.ny - 1) + yc) * FD_C_N;
     const double a = C[d.a_idx], i2a = C[d.i2a_idx];
     double b = t[0] * C[d.prow[0]];
 #pragma unroll
