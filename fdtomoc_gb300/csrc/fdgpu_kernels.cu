@@ -1827,6 +1827,7 @@ FD_COLD int exit_floor(const fd_station_dev &sd, Shared &sh, WarpSmem &ws, int I
         const int p = inst_node(sd, rj, (int)(ek & 0xffffffffu));
         const float f = fminf(o.phi, fmaxf(vload(sd.scr.grec[p].x), vload(sd.scr.grec[p].y)));
         if (f > thr) {
+            if ((threadIdx.x & 31) == 0) atomicAdd(&sh.w.nphi, 1);   /* it may come back to the queue */
             *floor = f;
             return 1;
         }

@@ -93,7 +93,7 @@ typedef struct {
 #define FD_EV_FIRED (-2)
 
 /* sizes of the small sweep-graph tables */
-#define FD_GPHI_CAP 65536    /* of the waits below, those for a bound on missing keys (keys_above) */
+#define FD_GPHI_CAP 65536    /* of the waits and queue entries below, those that bounds cost (keys_above, exit_floor) */
 #define FD_GWAIT_CAP 131072  /* (awaited point, waiting point) pairs, a hash table */
 #define FD_GPARK_CAP 65536   /* points parked on an instance event: (point, next in the event's list) */
 #define FD_GRQ_CAP 327680    /* resume queue */
