@@ -75,12 +75,13 @@ __device__ __forceinline__ F2 add2(F2 a, F2 b)
 
 __global__ void __launch_bounds__(kC2fBlock) c2f_interp(const float *__restrict__ slow, const Axis *__restrict__ ax,
                                                         const Axis *__restrict__ ay, const Axis *__restrict__ az,
-                                                        int nx, int nxy, int nz, int walk, int nxc, int nxyc, int ncoarse,
+                                                        int nx, int nxy, int nz, int across, int walk, int nxc, int nxyc, int ncoarse,
                                                         float *__restrict__ out, unsigned long long minus_zeros)
 {
     __shared__ float2 zg[kC2fZ], zf[kC2fZ];   /* weights of the planes below and above, for both halves */
     __shared__ int zcell[kC2fZ + 1];
-    const int k0 = blockIdx.y * walk, nk = min(walk, nz - k0);
+    const int part = blockIdx.x / across, col = blockIdx.x - part * across;   /* a thin model has more parts than grid.y takes */
+    const int k0 = part * walk, nk = min(walk, nz - k0);
     if (threadIdx.x < nk) {
         const Axis Z = az[k0 + threadIdx.x];
         zg[threadIdx.x] = make_float2(Z.omf, Z.omf);
@@ -89,7 +90,7 @@ __global__ void __launch_bounds__(kC2fBlock) c2f_interp(const float *__restrict_
     }
     if (threadIdx.x == nk) zcell[nk] = -1;
     __syncthreads();
-    const int p = blockIdx.x * 2 * kC2fBlock + threadIdx.x;
+    const int p = col * 2 * kC2fBlock + threadIdx.x;
     if (p >= nxy) return;
     const bool two = p + kC2fBlock < nxy;
     const int p2 = two ? p + kC2fBlock : p;
@@ -296,8 +297,8 @@ extern "C" int fdgpu_c2f_run(fdgpu_c2f_plan *p, const float *d_coarse, float *d_
      * walk's latency is what takes the time (28 x 64 x 27: 16.6 us a call with 24 planes, 8.4 with one) */
     int walk = kC2fZ;
     while (walk > 1 && (long long)across * ((p->nz + walk - 1) / walk) < 8ll * p->sms) walk /= 2;
-    const dim3 grid(across, (p->nz + walk - 1) / walk);
-    c2f_interp<<<grid, kC2fBlock, 0, st>>>(p->slow, p->ax, p->ay, p->az, p->nx, nxy, p->nz, walk, p->nxc, p->nxc * p->nyc,
+    const int grid = across * ((p->nz + walk - 1) / walk);
+    c2f_interp<<<grid, kC2fBlock, 0, st>>>(p->slow, p->ax, p->ay, p->az, p->nx, nxy, p->nz, across, walk, p->nxc, p->nxc * p->nyc,
                                              p->nxc * p->nyc * p->nzc, d_fine, 0x8000000080000000ull);
     const cudaError_t e = cudaGetLastError();
     return e ? fdh_ctx_fail(p->ctx, (int)e, "c2f launch") : FDGPU_OK;

@@ -1,5 +1,6 @@
 """The c2f kernel's walk up z against the oracle, bit for bit: part and block remainders, cells of one plane and
-cells longer than a walked part, sizes that walk 1, 3, 6, 12 and 24 planes.  The slowness kernel's wide and plain forms against IEEE division: every
+cells longer than a walked part, sizes that walk 1, 3, 6, 12 and 24 planes, more parts than
+a grid has rows.  The slowness kernel's wide and plain forms against IEEE division: every
 alignment of its arrays, lengths about a vector and a block.  The reciprocal against the division, for all floats."""
 import ctypes as C
 import os
@@ -17,7 +18,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("nc,ig", [((2, 2, 2), (1, 1, 1)), ((3, 2, 25), (1, 1, 1)), ((2, 5, 2), (130, 1, 23)),
                                    ((9, 9, 3), (7, 3, 24)), ((4, 3, 4), (43, 1, 31)), ((6, 5, 9), (5, 9, 3)),
                                    ((41, 41, 4), (5, 5, 10)), ((41, 41, 7), (5, 5, 10)), ((41, 41, 13), (5, 5, 10)),
-                                   ((41, 41, 20), (5, 5, 10))])
+                                   ((41, 41, 20), (5, 5, 10)), ((2, 2, 2), (1, 1, 1_600_000))])
 def test_c2f_walk_equals_oracle(gpu_lib, nc, ig):
     rng = np.random.default_rng(5)
     nxc, nyc, nzc = nc
