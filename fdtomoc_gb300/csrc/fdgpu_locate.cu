@@ -21,7 +21,7 @@
  * 26 FP64 instructions a phase and trial, which held the FP64 units (2 lanes a clock on an SM) 86 % busy.
  * Here the residual along a row of trials is A - b f in pairs of floats (about 46 bits), A and b formed once per
  * row, cell and phase; its float is certain unless the value lies within the pairs' error of
- * a rounding boundary (res_pair), and only such residuals, about one in ten thousand, are formed in double.
+ * a rounding boundary (fd_pair.h), and only such residuals are formed in double.
  * The floats that enter the statistics are the reference's either way.
  *
  * Arithmetic: statistics in float, positions and trilinear weights in double, as the reference;
@@ -36,6 +36,7 @@
 #include <math.h>
 #include <stdint.h>
 
+#include "fd_pair.h"
 #include "fdgpu.h"
 #include "fdgpu_device.h"
 
@@ -327,79 +328,6 @@ __device__ __noinline__ float residual_exact(const LocObsDev &o, const float *t,
     return residual_d(o, cell_time(c, t), vpvs);
 }
 
-/* a pair of floats (h + l) */
-struct FF {
-    float h, l;
-};
-__device__ __forceinline__ FF ff_one_minus(FF f)
-{
-    const float h = 1.f - f.h;
-    return {h, ((1.f - h) - f.h) - f.l};
-}
-__device__ __forceinline__ FF ff_mul(FF a, FF b)
-{
-    const float p = a.h * b.h;
-    return {p, fmaf(a.h, b.h, -p) + fmaf(a.h, b.l, a.l * b.h)};
-}
-__device__ __forceinline__ FF ff_add(FF a, FF b)
-{
-    const float h = a.h + b.h, v = h - a.h;
-    return {h, ((a.h - (h - v)) + (b.h - v)) + (a.l + b.l)};
-}
-__device__ __forceinline__ FF ff_neg(FF a) { return {-a.h, -a.l}; }
-/* a - b, exact */
-__device__ __forceinline__ FF ff_diff(float a, float b) { return ff_add(FF{a, 0.f}, FF{-b, 0.f}); }
-__device__ __forceinline__ FF ff_scale(FF a, float s)
-{
-    const float p = a.h * s;
-    return {p, fmaf(a.l, s, fmaf(a.h, s, -p))};
-}
-
-/* A cell's residual along a row of trials: A - b f, from the times of the row's cell at t (x), t + nx (y), t + nxy
- * (z) and the row's weights.  Times enter as their differences from the corner's, t0: they are exact and of a
- * step's size, so the pairs' error is too.  It is within 100 u^2 D + 10 u^2 |obs - t0| (u = 2^-24, D the largest
- * difference: weights, products and sums, term by term), the reference's own within 2^-49 of the largest time:
- * m is above their sum. */
-__device__ __forceinline__ void row_coefficients(const LocObsDev &o, const float *t, int nx, int nxy, const FF w[4], float vpvs,
-                                                 float4 *ab, float *m)
-{
-    const float t0 = t[0];
-    float big = fabsf(t0), dmax = 0.f;
-    FF v[2] = {{0.f, 0.f}, {0.f, 0.f}};
-#pragma unroll
-    for (int k = 1; k < 8; k++) {
-        const float tk = t[(k & 1) + (k & 2 ? nx : 0) + (k & 4 ? nxy : 0)];
-        const FF d = ff_diff(tk, t0);
-        big = fmaxf(big, fabsf(tk));
-        dmax = fmaxf(dmax, fabsf(d.h));
-        v[k & 1] = ff_add(v[k & 1], ff_mul(w[k >> 1], d));
-    }
-    FF c = {t0, 0.f}, a = v[0], b = ff_add(v[1], ff_neg(v[0]));
-    float mag = 1.f;
-    if (o.s_scaled) {
-        c = ff_scale(c, vpvs);
-        a = ff_scale(a, vpvs);
-        b = ff_scale(b, vpvs);
-        mag = fmaxf(1.f, fabsf(vpvs));
-    }
-    c = ff_add(FF{o.obstime, 0.f}, ff_neg(c));
-    const FF A = ff_add(c, ff_neg(a));
-    *ab = make_float4(A.h, A.l, b.h, b.l);
-    *m = mag * (4.547473508864641e-13f * dmax + 3.552713678800501e-15f * big) + 5.684341886080802e-14f * fabsf(c.h);
-}
-
-/* The residual A - b f rounded to float, f = fh + fl: true and the reference's float if that is certain, that
- * is if A - b f - m and A - b f + m round to the same float; else the caller forms the residual in double. */
-__device__ __forceinline__ bool res_pair(const float4 &ab, float m, float fh, float fl, float *res)
-{
-    const float p = ab.z * fh, e = fmaf(ab.w, fh, fmaf(ab.z, fl, fmaf(ab.z, fh, -p)));
-    const float d = ab.x - p, v = d - ab.x;
-    const float low = ((ab.x - (d - v)) + (-p - v)) + (ab.y - e);
-    const float up = d + (low + m);
-    *res = up;
-    return up == d + (low - m);
-}
-
 /* (b), (c) refinements: trial c = (k * nsy + j) * nsx + i of the event's window (header comment).  A block's
  * consecutive trials lie on a few rows (j, k) and in at most three cells of each (segments); the phases go
  * through in tiles whose coefficients, a pair of floats for a and b and the margin m per segment, fit shared
@@ -411,9 +339,9 @@ constexpr int kDivMax = 64;   /* largest divisions of the axis tables; finer win
 __global__ void __launch_bounds__(kLocBlock) loc_refine(fdgpu_loc_grid g, const LocObsDev *list, LocEvent *evs,
                                                           const int *active, const AxisPos *axes, int naxis)
 {
-    __shared__ float4 cab[kCoef];
+    __shared__ fdp_row cab[kCoef];
     __shared__ float cm[kCoef];
-    __shared__ FF wrow[kLocBlock + 2][4];
+    __shared__ fdp_ff wrow[kLocBlock + 2][4];
     __shared__ int orow[kLocBlock + 2];
     const int e = active[blockIdx.y];
     LocEvent &ev = evs[e];
@@ -429,11 +357,7 @@ __global__ void __launch_bounds__(kLocBlock) loc_refine(fdgpu_loc_grid g, const 
     const int segs = nrows * ncx, tile = min(16, kCoef / segs);
     for (int r = threadIdx.x; r < nrows; r += kLocBlock) {
         const int row = row0 + r, k = row / nsy, j = row - k * nsy;
-        const FF fy = {ay[j].fh, ay[j].fl}, fz = {az[k].fh, az[k].fl}, gy = ff_one_minus(fy), gz = ff_one_minus(fz);
-        wrow[r][0] = ff_mul(gy, gz);
-        wrow[r][1] = ff_mul(fy, gz);
-        wrow[r][2] = ff_mul(gy, fz);
-        wrow[r][3] = ff_mul(fy, fz);
+        fdp_weights(fdp_pair(ay[j].fh, ay[j].fl), fdp_pair(az[k].fh, az[k].fl), wrow[r]);
         orow[r] = az[k].cell * nxy + ay[j].cell * nx;
     }
     float avres = 0.0f, rsq = 0.0f, fh = 0.f, fl = 0.f;
@@ -451,14 +375,14 @@ __global__ void __launch_bounds__(kLocBlock) loc_refine(fdgpu_loc_grid g, const 
         for (int x = threadIdx.x; x < nq * segs; x += kLocBlock) {
             const int q = x / segs, sg = x - q * segs, r = sg / ncx;
             const LocObsDev o = ob[q0 + q];
-            row_coefficients(o, o.field + orow[r] + cmin + (sg - r * ncx), nx, nxy, wrow[r], g.vpvs, &cab[x], &cm[x]);
+            fdp_coefficients(o.obstime, o.s_scaled, g.vpvs, o.field + orow[r] + cmin + (sg - r * ncx), nx, nxy, wrow[r], &cab[x], &cm[x]);
         }
         __syncthreads();
         if (c < ncand) {
             for (int q = 0; q < nq; q++) {
                 const LocObsDev &o = ob[q0 + q];
                 float res;
-                if (!res_pair(cab[q * segs + seg], cm[q * segs + seg], fh, fl, &res)) {
+                if (!fdp_residual(&cab[q * segs + seg], cm[q * segs + seg], fh, fl, &res)) {
                     const int k = row / nsy, j = row - k * nsy;
                     res = residual_exact(o, o.field + orow[row - row0] + ax[i].cell, nx, nxy, ax[i].f, ay[j].f, az[k].f, g.vpvs);
                 }
