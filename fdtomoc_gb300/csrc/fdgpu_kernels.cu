@@ -313,6 +313,12 @@ constexpr int kSmemBase = kCtaSmemBytes + FD_WARPS * (int)sizeof(WarpSmem);
 template <class T>
 __device__ __forceinline__ T vload(const T &x) { return *const_cast<const volatile T *>(&x); }
 
+/* A value that other warps may be changing, as one lane sees it: what a warp branches on before a collective.  (Each
+ * lane's own vload may give another value, and lanes that then go another way leave the collective's mask unmet.)
+ * All 32 lanes call. */
+template <class T>
+__device__ __forceinline__ T vload_warp(const T &x) { return __shfl_sync(0xffffffffu, vload(x), 0); }
+
 __device__ __forceinline__ void nb_off(int k, int &du, int &dv)
 {
     /* k = 0..7 over the 3x3 block without its centre, row by row */
@@ -1702,7 +1708,7 @@ FD_COLD bool scan_open(const fd_station_dev &sd, Shared &sh, WarpSmem &ws, int I
     const GraphSmem gs = gsmem(sh);
     unsigned *bits = reinterpret_cast<unsigned *>(&ws.res[0][0]);
     constexpr int kBits = 8 * sizeof ws.res;   /* a flag per node of an instance; larger faces wait for the event */
-    if (vload(sh.w.nphi) >= FD_GPHI_CAP - FD_WARPS) return false;   /* these waits leave the tables' room for the others */
+    if (vload_warp(sh.w.nphi) >= FD_GPHI_CAP - FD_WARPS) return false;   /* these waits leave the tables' room for the others */
     float phi = 1.e10f, worst = -2.f;
     int zw = -1, zj = -1, scanned = 0;
     for (int J0 = 0; J0 < I; J0 += 32) {
@@ -1794,7 +1800,7 @@ __device__ bool wait_open(const fd_station_dev &sd, Shared &sh, int w, int p)
 
 FD_COLD bool keys_above(const fd_station_dev &sd, Shared &sh, WarpSmem &ws, int I, int w, float kw)
 {
-    if (vload(sd.scr.ginst[I].phi) > kw) return true;
+    if (vload_warp(sd.scr.ginst[I].phi) > kw) return true;
     OpenScan o;
     for (int turn = 0; turn < 8 && scan_open(sd, sh, ws, I, -1, kw, o); turn++) {   /* a turn more if the node is done by now */
         if (o.phi > kw) {
@@ -1822,10 +1828,10 @@ FD_COLD int exit_floor(const fd_station_dev &sd, Shared &sh, WarpSmem &ws, int I
     for (int turn = 0; turn < 8 && scan_open(sd, sh, ws, I, J, thr, o); turn++) {
         wfence(sh);
         /* after the flags: a point whose flag says done has put its key there */
-        const unsigned long long ek = vload(sd.scr.ginst[J].exitkey);
+        const unsigned long long ek = vload_warp(sd.scr.ginst[J].exitkey);
         if (!ek || !FD_OK((long long)(ek & 0xffffffffu), rect_n(rj), 31)) return 2;
         const int p = inst_node(sd, rj, (int)(ek & 0xffffffffu));
-        const float f = fminf(o.phi, fmaxf(vload(sd.scr.grec[p].x), vload(sd.scr.grec[p].y)));
+        const float f = fminf(o.phi, fmaxf(vload_warp(sd.scr.grec[p].x), vload_warp(sd.scr.grec[p].y)));
         if (f > thr) {
             if ((threadIdx.x & 31) == 0) atomicAdd(&sh.w.nphi, 1);   /* it may come back to the queue */
             *floor = f;
@@ -1859,8 +1865,10 @@ FD_COLD bool resume_graph(const fd_station_dev &sd, Shared &sh, WarpSmem &ws, in
     const int su = (int)t_stride(sd, fr.axis_u), sv = (int)t_stride(sd, fr.axis_v);
     const int base = inst_node(sd, r, 0), in = fr.inner * (int)t_stride(sd, fr.axis_n);
     const int wu = coord(fr.axis_u, wx, wy, wz) - r.ulo, wv = coord(fr.axis_v, wx, wy, wz) - r.vlo;
-    if (vload(gs.nkeyed[I]) < n && !keys_above(sd, sh, ws, I, w, vload(sd.T[base + wu * su + wv * sv + in]))) return false;
-    const unsigned long long kc = node_key(vload(sd.T[base + wu * su + wv * sv + in]), wv * nuf + wu);
+    const float tw = vload_warp(sd.T[base + wu * su + wv * sv + in]);   /* final: w has been evaluated once */
+    if (vload_warp(gs.nkeyed[I]) < n && !keys_above(sd, sh, ws, I, w, tw)) return false;
+    wfence(sh);   /* the keys are read after the count, or the bound, that says they are there */
+    const unsigned long long kc = node_key(tw, wv * nuf + wu);
     const int dv = 32 / nuf, du = 32 - dv * nuf;   /* 32 points on in fill order */
     for (int guard = 0; guard <= 2 * n + 2; guard++) {
         /* among the instance's earlier points: the last writer that is done, and the last point that is
@@ -1929,7 +1937,7 @@ FD_COLD bool resume_graph(const fd_station_dev &sd, Shared &sh, WarpSmem &ws, in
         if (verdict == 3) {
             before = __shfl_sync(0xffffffffu, before, 0);
             float f = 0.f;
-            const int can = exit_floor(sd, sh, ws, I, before, w, vload(sd.scr.grec[node_of(sd, w)].x), &f);
+            const int can = exit_floor(sd, sh, ws, I, before, w, vload_warp(sd.scr.grec[node_of(sd, w)].x), &f);
             if (can == 1) {
                 *st0 = *st4 = f;
                 *floor_only = true;
