@@ -137,7 +137,8 @@ constexpr bool kinds_uniform()
 }
 
 /* the 1-D trials step along one axis from the point itself: the inner neighbour, then +u -u +v -v, with the
- * factors h (z), r dq (y), r df s or r s df (x) in this order */
+ * factors h (z), r dq (y), r df s or r s df (x) in this order; head_wave takes the length that a head trial's
+ * value is formed with for the one its head-wave measure is divided by */
 template <int F>
 constexpr bool steps_as_assumed()
 {
@@ -154,6 +155,11 @@ constexpr bool steps_as_assumed()
         if (axis == 0 && !((d.vk[1] == FK_DF && d.vk[2] == FK_S) || (d.vk[1] == FK_S && d.vk[2] == FK_DF))) return false;
         for (int j = 0; j < d.vn; j++)
             if (d.vdz[j] != 0 || d.vdy[j] != 0) return false;
+        /* a head trial's denominator: the step's factors, then the point's slowness */
+        if (!tr.head) continue;
+        if (d.hn != d.vn + 1 || d.hk[d.vn] != FK_SLOW) return false;
+        for (int j = 0; j < d.vn; j++)
+            if (d.hk[j] != d.vk[j] || d.hdz[j] != 0 || d.hdy[j] != 0) return false;
     }
     return true;
 }
