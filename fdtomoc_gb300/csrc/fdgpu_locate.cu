@@ -331,18 +331,32 @@ __device__ __noinline__ float residual_exact(const LocObsDev &o, const float *t,
 /* (b), (c) refinements: trial c = (k * nsy + j) * nsx + i of the event's window (header comment).  A block's
  * consecutive trials lie on a few rows (j, k) and in at most three cells of each (segments); the phases go
  * through in tiles whose coefficients, a pair of floats for a and b and the margin m per segment, fit shared
- * memory.  128 events x 32 phases, 41^3 trials: 14.7 -> 2.0 ms in the first refinement and
- * 0.6 in the second, against FP64. */
+ * memory.
+ *
+ * Residuals that are not certain.  Where the places in a cell are fractions of few bits (8 or 16 divisions) every tenth
+ * residual is a tie of two floats, and where times fit well the residuals are small and the margin a larger part of
+ * their last place.  Formed where they occur, one such residual costs its warp the 43 FP64 instructions of all 32
+ * lanes.  So a tile's uncertain residuals are listed, formed with full warps, and handed back before the sums.
+ * First and second refinement of 128 events x 32 phases, against FP64 throughout and against forming them where they
+ * occur: 41^3 trials 15.3 and 15.2 -> 2.03 and 0.58 -> 0.99 and 0.65 ms; 17^3 trials (8 divisions, scaled S) 1.20
+ * and 1.20 -> 1.41 and 0.24 -> 0.25 and 0.10. */
+constexpr int kTile = 12;     /* phases of a tile at most, their residuals in registers: with 16 four blocks no longer fit an SM */
 constexpr int kCoef = 1024;   /* coefficients of a tile: segments x phases */
+constexpr int kFix = 1024;    /* uncertain residuals formed together; with more a tile takes several rounds */
 constexpr int kDivMax = 64;   /* largest divisions of the axis tables; finer windows take loc_refine_fp64 */
+static_assert(kLocBlock <= 256 && kTile <= 256 && kTile <= kFix, "entries of the list: phase << 8 | thread");
 
-__global__ void __launch_bounds__(kLocBlock) loc_refine(fdgpu_loc_grid g, const LocObsDev *list, LocEvent *evs,
+__global__ void __launch_bounds__(kLocBlock, 4) loc_refine(fdgpu_loc_grid g, const LocObsDev *list, LocEvent *evs,
                                                           const int *active, const AxisPos *axes, int naxis)
 {
     __shared__ fdp_row cab[kCoef];
     __shared__ float cm[kCoef];
     __shared__ fdp_ff wrow[kLocBlock + 2][4];
     __shared__ int orow[kLocBlock + 2];
+    __shared__ float fixv[kFix];
+    __shared__ unsigned short fixq[kFix];
+    __shared__ int nfix;
+    constexpr unsigned kNone = 0xffffu;
     const int e = active[blockIdx.y];
     LocEvent &ev = evs[e];
     const int nsx = ev.nsx, nsy = ev.nsy, ncand = nsx * nsy * ev.nsz;
@@ -354,17 +368,16 @@ __global__ void __launch_bounds__(kLocBlock) loc_refine(fdgpu_loc_grid g, const 
     const int c = c0 + threadIdx.x, clast = min(c0 + kLocBlock, ncand) - 1;
     const int row0 = c0 / nsx, nrows = clast / nsx - row0 + 1;
     const int cmin = ax[0].cell, ncx = ax[nsx - 1].cell - cmin + 1;
-    const int segs = nrows * ncx, tile = min(16, kCoef / segs);
+    const int segs = nrows * ncx, tile = min(kTile, kCoef / segs);
     for (int r = threadIdx.x; r < nrows; r += kLocBlock) {
         const int row = row0 + r, k = row / nsy, j = row - k * nsy;
         fdp_weights(fdp_pair(ay[j].fh, ay[j].fl), fdp_pair(az[k].fh, az[k].fl), wrow[r]);
         orow[r] = az[k].cell * nxy + ay[j].cell * nx;
     }
     float avres = 0.0f, rsq = 0.0f, fh = 0.f, fl = 0.f;
-    int seg = 0, i = 0, row = 0;
+    int seg = 0;
     if (c < ncand) {
-        row = c / nsx;
-        i = c - row * nsx;
+        const int row = c / nsx, i = c - row * nsx;
         fh = ax[i].fh;
         fl = ax[i].fl;
         seg = (row - row0) * ncx + ax[i].cell - cmin;
@@ -378,17 +391,44 @@ __global__ void __launch_bounds__(kLocBlock) loc_refine(fdgpu_loc_grid g, const 
             fdp_coefficients(o.obstime, o.s_scaled, g.vpvs, o.field + orow[r] + cmin + (sg - r * ncx), nx, nxy, wrow[r], &cab[x], &cm[x]);
         }
         __syncthreads();
-        if (c < ncand) {
-            for (int q = 0; q < nq; q++) {
-                const LocObsDev &o = ob[q0 + q];
-                float res;
-                if (!fdp_residual(&cab[q * segs + seg], cm[q * segs + seg], fh, fl, &res)) {
-                    const int k = row / nsy, j = row - k * nsy;
-                    res = residual_exact(o, o.field + orow[row - row0] + ax[i].cell, nx, nxy, ax[i].f, ay[j].f, az[k].f, g.vpvs);
-                }
-                accumulate(res, o.pwt, avres, rsq);
+        float res[kTile];
+        unsigned open = 0;   /* phases whose residual is not certain */
+#pragma unroll
+        for (int q = 0; q < kTile; q++)
+            if (q < nq && !fdp_residual(&cab[q * segs + seg], cm[q * segs + seg], fh, fl, &res[q])) open |= 1u << q;
+        if (c >= ncand) open = 0;
+        while (__syncthreads_or(open != 0)) {
+            if (threadIdx.x == 0) nfix = 0;
+            __syncthreads();
+            int at = 0;
+            bool fits = false;
+            if (open) {
+                at = atomicAdd(&nfix, __popc(open));
+                fits = at + __popc(open) <= kFix;
+                int to = at;
+                for (unsigned b = open; b && to < kFix; b &= b - 1) fixq[to++] = (unsigned short)(fits ? (__ffs(b) - 1) << 8 | threadIdx.x : kNone);
+            }
+            __syncthreads();
+            const int n = min(nfix, kFix);
+            for (int x = threadIdx.x; x < n; x += kLocBlock) {
+                const unsigned it = fixq[x];
+                if (it == kNone) continue;
+                const LocObsDev &o = ob[q0 + (it >> 8)];
+                const int cc = c0 + (int)(it & 255u), row = cc / nsx, k = row / nsy;
+                const AxisPos &px = ax[cc - row * nsx];
+                fixv[x] = residual_exact(o, o.field + orow[row - row0] + px.cell, nx, nxy, px.f, ay[row - k * nsy].f, az[k].f, g.vpvs);
+            }
+            __syncthreads();
+            if (fits) {
+#pragma unroll
+                for (int q = 0; q < kTile; q++)
+                    if ((open >> q) & 1u) res[q] = fixv[at++];
+                open = 0;
             }
         }
+#pragma unroll
+        for (int q = 0; q < kTile; q++)
+            if (q < nq) accumulate(res[q], ob[q0 + q].pwt, avres, rsq);
     }
     unsigned long long key = ~0ull;
     if (c < ncand) key = trial_key(deviation(avres, rsq, ev.facs, ev.ngood), (unsigned)c);
