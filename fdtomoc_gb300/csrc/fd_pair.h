@@ -128,4 +128,23 @@ FDP_FN int fdp_residual(const fdp_row *ab, float m, float fh, float fl, float *r
     return up == d + (low - m);
 }
 
+/* obstime - t vpvs of a node's time, rounded to float: 1 and the reference's float if that is certain (the reference
+ * forms it in double and rounds once more).  With p + e the product and d + er the difference obstime - p, both exact as
+ * pairs, the value is d + (er - e), exactly; in float er - e and the margin's sums lose less than 4 u^2 (|obstime| + |p|).
+ * A tie of two floats is inside any margin, and with vpvs of few bits (7/4) every second time makes one.  But there er - e
+ * is a float, so that d + (er - e) is one rounding of the exact value; and the reference's double is exact as well while
+ * the operands lie within 2^4 and 2^24 of each other: all terms are multiples of 2^-48 |p| and of 2^-24 |obstime|. */
+FDP_FN int fdp_scaled_residual(float obstime, float t, float vpvs, float *res)
+{
+    const float p = t * vpvs, e = fmaf(t, vpvs, -p);
+    const float d = obstime - p, v = d - obstime, er = (obstime - (d - v)) + (-p - v);
+    const float low = er - e, size = fabsf(obstime) + fabsf(p), m = 1.4210854715202004e-14f * size;
+    const float up = d + (low + m);
+    *res = up;
+    if (up == d + (low - m)) return 1;
+    const float w = low - er;
+    *res = d + low;
+    return (er - (low - w)) + (-e - w) == 0.f && fabsf(obstime) <= 16.f * fabsf(p) && fabsf(p) <= 16777216.f * fabsf(obstime);
+}
+
 #endif

@@ -218,16 +218,11 @@ __device__ __noinline__ float residual_scaled(float obstime, float t, float vpvs
     return (float)((double)obstime - (double)t * (double)vpvs);
 }
 
-/* The same without FP64: the product and the difference are exact as pairs of floats, but for a last
- * rounding within 2^-46 of their size (the reference rounds once more to double: 2^-53); where that
- * could change the float, the reference's form decides. */
+/* the same in pairs of floats, which nearly always tell (fd_pair.h) */
 __device__ __forceinline__ float residual_scaled_pair(float obstime, float t, float vpvs)
 {
-    const float p = t * vpvs, e = fmaf(t, vpvs, -p);
-    const float d = obstime - p, v = d - obstime, er = (obstime - (d - v)) + (-p - v);
-    const float low = er - e, m = 1.4210854715202004e-14f * (fabsf(obstime) + fabsf(p));
-    const float up = d + (low + m), dn = d + (low - m);
-    return up == dn ? up : residual_scaled(obstime, t, vpvs);
+    float res;
+    return fdp_scaled_residual(obstime, t, vpvs, &res) ? res : residual_scaled(obstime, t, vpvs);
 }
 
 /* a phase as the coarse search reads it from shared memory, in one 16-byte load */

@@ -1,4 +1,4 @@
-"""The location's residuals in pairs of floats (fd_pair.h) against the reference's double form: the pair within its
+"""The location's residuals in pairs of floats (fd_pair.h), at nodes and between them, against the reference's double form: the pair within its
 margin of it, and every residual called certain the same float.  P phases and S phases scaled from a P field, near-zero
 residuals (where a float is least certain) among them, times up to 300 s that differ by 0.1 ms to 1 s within the
 cell, places on steps of the usual divisions, and places beyond the cell along z."""
@@ -58,6 +58,26 @@ void pair_check(uint64_t seed, long n, int scaled, double vpvs_, int ndiv, int b
         }
     }
 }
+/* out: [0] certain but another float, [1] certain */
+void node_check(uint64_t seed, long n, double vpvs_, int mode, long *out)
+{
+    const float vpvs = (float)vpvs_;
+    s = seed;
+    for (long i = 0; i < n; i++) {
+        float t = (float)(0.3 * pow(1000., uni())), obs, res;
+        if (mode == 0) obs = (float)((double)t * vpvs + 4. * (uni() - .5));          /* a pick's residual */
+        else if (mode == 1) obs = (float)((double)t * vpvs);                         /* none but a rounding */
+        else if (mode == 2) obs = (float)(t * pow(2., 60. * uni() - 30.) * (uni() < .5 ? -1. : 1.));   /* far apart */
+        else {   /* few bits: ties at every size */
+            t = (float)ldexp((double)(1 + (int)(uni() * 0xffffff)), (int)(uni() * 40.) - 20);
+            obs = (float)ldexp((double)(1 + (int)(uni() * 255.)), (int)(uni() * 60.) - 30);
+        }
+        if (fdp_scaled_residual(obs, t, vpvs, &res)) {
+            out[1]++;
+            out[0] += res != (float)((double)obs - (double)t * (double)vpvs);
+        }
+    }
+}
 """
 
 
@@ -80,3 +100,14 @@ def test_pair_residual_within_its_margin(lib, scaled, vpvs, ndiv, beyond):
     assert out[0] == 0, f"{out[0]} pairs outside their margin"
     assert out[1] == 0, f"{out[1]} certain residuals that are another float"
     assert out[2] > 100_000   # most are certain away from zero
+
+
+@pytest.mark.parametrize("vpvs", [1.75, 1.5, 2.0, 1.78, 1.0, -1.75, 1.7320508])
+def test_scaled_node_residual(lib, vpvs):
+    """Certain residuals are the reference's float; ties, of which a factor of few bits makes many, are certain too."""
+    for mode in range(4):
+        out = (C.c_long * 2)()
+        lib.node_check(C.c_uint64(88172645463325252 + mode), C.c_long(400_000), C.c_double(vpvs), mode, out)
+        assert out[0] == 0, f"{out[0]} certain residuals that are another float"
+        if mode < 2:
+            assert out[1] > 0.999 * 400_000, out[1]
