@@ -2762,16 +2762,22 @@ extern "C" cudaError_t fdk_selfcheck_read(unsigned long long *out)
 #endif
 
 /* slowness = 1/velocity, float division as the reference does it (src/sphfd.c:689-690).  Bound by HBM: 16-byte
- * loads, kV2sBatch of them in flight per thread, where both arrays allow it (`wide`); the rest element by element.
- * 401 x 401 x 161: 58.5 -> 34.3 us (6.0 TB/s) against a 4-byte load at a time. */
+ * loads, kV2sBatch of them in flight per thread, where both arrays allow it (`wide`); else 4-byte loads, as many in
+ * flight (the arrays may be one and the same, so that each load has to be written before the first store).
+ * 401 x 401 x 161: 58.5 -> 34.3 us (6.0 TB/s) against a 4-byte load at a time; off a 16-byte boundary 62.1 -> 45.7. */
 constexpr int kV2sBatch = 4, kV2sBlock = 256;
 
 __global__ void __launch_bounds__(kV2sBlock) fd_v2s(const float *v, float *s, long long n, int wide)
 {
     const long long first = (long long)blockIdx.x * kV2sBlock * kV2sBatch + threadIdx.x;
     if (!wide) {
+        float a[kV2sBatch];
+#pragma unroll
         for (int u = 0; u < kV2sBatch; u++)
-            if (first + u * kV2sBlock < n) s[first + u * kV2sBlock] = 1.0f / v[first + u * kV2sBlock];
+            if (first + u * kV2sBlock < n) a[u] = v[first + u * kV2sBlock];
+#pragma unroll
+        for (int u = 0; u < kV2sBatch; u++)
+            if (first + u * kV2sBlock < n) s[first + u * kV2sBlock] = 1.0f / a[u];
         return;
     }
     const long long n4 = n / 4;
