@@ -68,18 +68,6 @@ struct FaceT {
     __host__ __device__ static constexpr int off(int a, fdn_node n) { return a == AU ? n.du : a == AV ? n.dv : n.w * IN; }
 };
 
-/* What a face point needs from its surroundings: times and slownesses of the 3x3 block on the face
- * layer (w=0) and on the inner layer (w=1), and the indices that locate it. */
-struct PointCtx {
-    int u, v;                  /* face coordinates */
-    int z, y;                  /* grid z and y of the point */
-    int nu, nv;                /* grid extent along u and v */
-    int ulo, uhi, vlo, vhi;    /* current face rectangle */
-    long long pT;              /* index of the point in T */
-    float t[2][3][3];
-    float s[2][3][3];
-};
-
 __device__ __forceinline__ const double *node_row(const fd_geo_dev &g, int z, int y)
 {
     if (!FD_OK(z, g.nz, 1) || !FD_OK(y, g.ny, 2)) { z = 0; y = 0; }
@@ -92,8 +80,6 @@ __host__ __device__ constexpr int chain_class(fdn_chain c)
 {
     return c.n == 1 ? CH_H : c.n == 2 ? CH_RDQ : CH_RSDF;
 }
-
-#define FD_T(p, n) ((p).t[(n).w][(n).dv + 1][(n).du + 1])
 
 /* roots of a x^2 + b x + c = 0 (rad = b*b - 4ac already formed), with the reference's
  * causality test against floor tmx; tie rule of fdsph3d (x1 preferred only if strictly smaller). */

@@ -89,7 +89,6 @@ uint64_t bits(double x)
 
 struct fdgpu_ctx {
     int device = 0;
-    int cluster = 0;   /* CTAs per station: 0 automatic */
     long long wait_cycles = 0, walk_cycles = 0;   /* bounds of the solver's waits, 0: built-in */
     /* measured solve time (ns) of each station this context has solved, keyed by the station's
      * record (fdgpu_station bytes): the launch-order table */
@@ -282,8 +281,7 @@ extern "C" int fdgpu_set_cluster(fdgpu_ctx *ctx, int ctas_per_station)
 {
     if (!ctx || ctas_per_station < 0 || ctas_per_station > 8 || (ctas_per_station & (ctas_per_station - 1)))
         return FDGPU_EINVAL;
-    ctx->cluster = ctas_per_station;
-    return FDGPU_OK;
+    return FDGPU_OK;   /* a hint: one CTA solves a station */
 }
 
 /* the launch-order table on disk: "FDGPUORD", a record count, then per station its key length,

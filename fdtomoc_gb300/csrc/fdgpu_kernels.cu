@@ -148,8 +148,6 @@ struct Shared {
     float carry_t0, carry_t4;
     /* current face of a face walk */
     int face, layer, ulo, uhi, vlo, vhi, nuf, n, n_pad;
-    long long su, sv, sn, ssu, ssv, ssn;
-    int nu, nv;
     /* current sweep graph: on/off, face instances, points; per face, the 27-bit masks of the
      * neighbour offsets a node of that face reads, and of those in its inner plane */
     int graph, gok, ninst, single, nodefer;
@@ -158,8 +156,6 @@ struct Shared {
     unsigned ctxm[6], innm[6];
     unsigned rel[6][27];     /* see relation_word */
     int lstride, imax;       /* layout of the sweep-graph tables (see GraphSmem) */
-    unsigned long long red[FD_BLOCK / 32];
-    unsigned long long bcast;
     /* statistics */
     long long faces, node_updates;
     int sweeps;
@@ -198,40 +194,6 @@ __device__ __forceinline__ unsigned okey32(float f)
     unsigned b = __float_as_uint(f);
     if (b == 0x80000000u) b = 0u;
     return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
-}
-
-__device__ __forceinline__ unsigned long long block_min_u64(unsigned long long x, Shared &sh)
-{
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long y = __shfl_down_sync(0xffffffffu, x, o);
-        x = y < x ? y : x;
-    }
-    if ((threadIdx.x & 31) == 0) sh.red[threadIdx.x >> 5] = x;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned long long m = sh.red[0];
-        for (int w = 1; w < FD_BLOCK / 32; w++) m = sh.red[w] < m ? sh.red[w] : m;
-        sh.bcast = m;
-    }
-    __syncthreads();
-    return sh.bcast;
-}
-
-__device__ __forceinline__ unsigned long long block_max_u64(unsigned long long x, Shared &sh)
-{
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long y = __shfl_down_sync(0xffffffffu, x, o);
-        x = y > x ? y : x;
-    }
-    if ((threadIdx.x & 31) == 0) sh.red[threadIdx.x >> 5] = x;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned long long m = sh.red[0];
-        for (int w = 1; w < FD_BLOCK / 32; w++) m = sh.red[w] > m ? sh.red[w] : m;
-        sh.bcast = m;
-    }
-    __syncthreads();
-    return sh.bcast;
 }
 
 /* stencil evaluations by kind (3-D, new-edge, 2-D, new-face, 1-D): the warp's counts in its
@@ -1077,7 +1039,11 @@ FD_COLD void wake_waiters(const fd_station_dev &sd, Shared &sh, int p)
 
 /* node p (instance I, fill index i) is final: its record.  Returns its counter word as it was when it was
  * marked done: FD_WAITB if a point waits for it (the caller wakes those once it has used the time the
- * word takes to arrive). */
+ * word takes to arrive).
+ * The record and the exit key are both written before the done mark, but in no order between them: exit_floor, which reads
+ * the key and then the record, may see a key without its record.  It only does so of a point that was open when
+ * it read the flags, and then what it takes from the scan bounds that point's state, whatever the record holds (a NaN
+ * falls out in its minimum); whoever reads a record as such has seen its done mark first. */
 __device__ __forceinline__ unsigned graph_record(const fd_station_dev &sd, Shared &sh, long long p, int I, int i, bool writer,
                                                  float st0, float st4, float tin)
 {
@@ -1678,23 +1644,7 @@ constexpr bool trials_above_a_neighbour()
 }
 static_assert(trials_above_a_neighbour(), "keys_above");
 
-/* Whether every key of instance I that is not known yet is certainly above kw, so that the points before point w
- * (key kw) are all known already; if not, w is registered on a node that stands against it, or on the event
- * that all keys are known.  One warp.
- *
- * A missing key is the time of a node of an earlier instance that is not done.  Let S be all such nodes and phi
- * the least time now at any of them or their six neighbours: no node of S ends below phi.  For take the first one,
- * in the reference's order, that did: its old time is not below phi, and each trial's value is not below the time
- * it reads at one of the six (trials_above_a_neighbour), which was done before (as read here), is of S and before it
- * (not below phi, since it is the first), or is of an instance not before its own (not changed before it is
- * evaluated).  The flags of an instance are all read before the times about its nodes, and instances go in
- * order: a neighbour whose flag says done then has its final time.  A time that is no number or negative stands
- * against everything.
- *
- * Why: without it such a point waits for the whole inner layer, and where border points inherit state (a fast layer
- * at the grid's edge) the planes of a forward sweep run one after another, which made a few windows five times
- * as long as the others.  Their batches and lists end with them: 150 windows of 73 to 91 319 -> 242 ms, 24 host
- * stations of 49x45x33 96 -> 60, 48 served requests 91 -> 76; with all 26 neighbours instead of the six 251, 65 and 83. */
+/* what a look through the open nodes (not done) of earlier instances found: see keys_above and exit_floor */
 struct OpenScan {
     float phi;    /* the least time at the open nodes and their six neighbours (of instance wide: 26) */
     int below;    /* the node with the largest such time that is not above thr, -1 if none is */
@@ -1798,6 +1748,23 @@ __device__ bool wait_open(const fd_station_dev &sd, Shared &sh, int w, int p)
     return __shfl_sync(0xffffffffu, waits, 0);
 }
 
+/* Whether every key of instance I that is not known yet is certainly above kw, so that the points before point w
+ * (key kw) are all known already; if not, w is registered on a node that stands against it, or on the event
+ * that all keys are known.  One warp.
+ *
+ * A missing key is the time of a node of an earlier instance that is not done.  Let S be all such nodes and phi
+ * the least time now at any of them or their six neighbours: no node of S ends below phi.  For take the first one,
+ * in the reference's order, that did: its old time is not below phi, and each trial's value is not below the time
+ * it reads at one of the six (trials_above_a_neighbour), which was done before (as read here), is of S and before it
+ * (not below phi, since it is the first), or is of an instance not before its own (not changed before it is
+ * evaluated).  The flags of an instance are all read before the times about its nodes, and instances go in
+ * order: a neighbour whose flag says done then has its final time.  A time that is no number or negative stands
+ * against everything.
+ *
+ * Why: without it such a point waits for the whole inner layer, and where border points inherit state (a fast layer
+ * at the grid's edge) the planes of a forward sweep run one after another, which made a few windows five times
+ * as long as the others.  Their batches and lists end with them: 150 windows of 73 to 91 319 -> 242 ms, 24 host
+ * stations of 49x45x33 96 -> 60, 48 served requests 91 -> 76; with all 26 neighbours instead of the six 251, 65 and 83. */
 FD_COLD bool keys_above(const fd_station_dev &sd, Shared &sh, WarpSmem &ws, int I, int w, float kw)
 {
     if (vload_warp(sd.scr.ginst[I].phi) > kw) return true;
@@ -1827,7 +1794,7 @@ FD_COLD int exit_floor(const fd_station_dev &sd, Shared &sh, WarpSmem &ws, int I
     OpenScan o;
     for (int turn = 0; turn < 8 && scan_open(sd, sh, ws, I, J, thr, o); turn++) {
         wfence(sh);
-        /* after the flags: a point whose flag says done has put its key there */
+        /* after the flags: a point whose flag says done has put its key there (and its record: graph_record) */
         const unsigned long long ek = vload_warp(sd.scr.ginst[J].exitkey);
         if (!ek || !FD_OK((long long)(ek & 0xffffffffu), rect_n(rj), 31)) return 2;
         const int p = inst_node(sd, rj, (int)(ek & 0xffffffffu));
@@ -2166,10 +2133,8 @@ __device__ void face_walk(const fd_station_dev &sd, Shared &sh, CtaSmem &cs, War
 }
 
 /* face parameters of face `face` for the current walls (thread 0) */
-__device__ void setup_face(const fd_station_dev &sd, Shared &sh, int face)
+__device__ void setup_face(Shared &sh, int face)
 {
-    const int nx = sd.g.nx, ny = sd.g.ny, nz = sd.g.nz;
-    const long long nxy = (long long)nx * ny;
     /* walls: 0 z1, 1 z2, 2 x2, 3 x1, 4 y1, 5 y2 */
     const int x1 = sh.wall[3], x2 = sh.wall[2], y1 = sh.wall[4], y2 = sh.wall[5];
     const int z1 = sh.wall[0], z2 = sh.wall[1];
@@ -2177,19 +2142,10 @@ __device__ void setup_face(const fd_station_dev &sd, Shared &sh, int face)
     sh.layer = sh.wall[face];
     if (face < 2) {
         sh.ulo = x1 + 1; sh.uhi = x2 - 1; sh.vlo = y1 + 1; sh.vhi = y2 - 1;
-        sh.nu = nx; sh.nv = ny;
-        sh.su = 1; sh.sv = nx; sh.sn = nxy;
-        sh.ssu = 1; sh.ssv = sd.s_sy; sh.ssn = sd.s_sz;
     } else if (face < 4) {
         sh.ulo = y1 + 1; sh.uhi = y2 - 1; sh.vlo = z1 + 1; sh.vhi = z2 - 1;
-        sh.nu = ny; sh.nv = nz;
-        sh.su = nx; sh.sv = nxy; sh.sn = 1;
-        sh.ssu = sd.s_sy; sh.ssv = sd.s_sz; sh.ssn = 1;
     } else {
         sh.ulo = x1 + 1; sh.uhi = x2 - 1; sh.vlo = z1 + 1; sh.vhi = z2 - 1;
-        sh.nu = nx; sh.nv = nz;
-        sh.su = 1; sh.sv = nxy; sh.sn = nx;
-        sh.ssu = 1; sh.ssv = sd.s_sz; sh.ssn = sd.s_sy;
     }
     sh.nuf = sh.uhi - sh.ulo + 1;
     const int nvf = sh.vhi - sh.vlo + 1;
@@ -2224,7 +2180,7 @@ __device__ void graph_sweep(const fd_station_dev &sd, Shared &sh, CtaSmem &cs, W
             for (int face = 0; face < 6; face++) {
                 for (int ig = 1; ig <= sd.grow[face]; ig++) {
                     if (!sh.dflag[face]) continue;
-                    setup_face(sd, sh, face);
+                    setup_face(sh, face);
                     if (sh.n > 0) {
                         if (ninst >= cap) { over = true; break; }
                         fd_ginst &gi = sd.scr.ginst[ninst];
@@ -2487,7 +2443,7 @@ __device__ __forceinline__ void solve_station(const fd_station_dev &sd, int dag_
             for (int face = 0; face < 6; face++) {
                 for (int ig = 1; ig <= sd.grow[face]; ig++) {
                     if (!sh.dflag[face]) continue;
-                    if (tid == 0) setup_face(sd, sh, face);
+                    if (tid == 0) setup_face(sh, face);
                     __syncthreads();
                     if (sh.n > 0) face_walk(sd, sh, cs, ws, dag, cn);
                     __syncthreads();
