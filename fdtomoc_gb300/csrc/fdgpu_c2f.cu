@@ -38,7 +38,7 @@ __global__ void c2f_slowness(const float *v, float *s, int n)
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) s[i] = 1.f / v[i];
 }
 
-/* What bounds this is instruction issue (67 % of its slots, a third of them for pairs, which take two), then the
+/* What bounds this is instruction issue (71 % of its slots, a third of them for pairs, which take two), then the
  * HBM writes: eight products of weight and slowness, their sum and a reciprocal per value written.  A thread takes two (x, y) of the plane, kC2fBlock apart so that each store
  * of a warp is contiguous (the plane is, rows included), and walks up a part of z: the four weight products of
  * x and y are formed once, the coarse slownesses stay in registers until z enters the next coarse cell, where

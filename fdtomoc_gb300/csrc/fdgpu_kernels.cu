@@ -1129,10 +1129,12 @@ __device__ void graph_release(const fd_station_dev &sd, Shared &sh, WarpSmem &ws
     const unsigned mask = __ballot_sync(0xffffffffu, fin);
     const int m = __popc(mask);
     if (!m) return;
+    static_assert(26 * 32 * sizeof(int) <= sizeof ws.res, "a node takes its key once, after one of at most 26 x 32 releases");
     int *keyq = reinterpret_cast<int *>(&ws.res[0][0]);
     int *nkey = reinterpret_cast<int *>(&ws.cnt[5]);
     const int nx = sd.g.nx, ny = sd.g.ny;
     const bool few = m <= (sh.single ? FD_FEW1 : FD_FEW);
+    static_assert(FD_FEW <= 32 && FD_FEW1 <= 32 && 32 * sizeof(RelNode) <= sizeof ws.s0 + sizeof ws.s4 + sizeof ws.z + sizeof ws.y, "RelNode");
     RelNode *rn = reinterpret_cast<RelNode *>(ws.s0);   /* s0, s4, z, y: free after the commit */
     if (few && fin)
         rn[__popc(mask & ((1u << lane) - 1u))] = {pack_xyz(wh.x, wh.y, wh.z), (int)wh.p, wh.inst, lane};
@@ -1787,7 +1789,7 @@ FD_COLD bool keys_above(const fd_station_dev &sd, Shared &sh, WarpSmem &ws, int 
  * without one (thr) is worth another look at the point: 1, with the floor.  Else it waits for an open node that stands
  * against that (0), or is to wait for J (2).  Such points come first in their instance, where the state is that of
  * the times J ends with, far above their own; waiting for J made the planes of the slowest windows run one after another:
- * 400 windows of 25 to 61 166 and 143 ms (two models) -> 142 and 112, 48 served requests 76 and 50 -> 55 and 41. */
+ * 400 windows of 25 to 61 166 and 143 ms (two models) -> 141 and 119, 48 served requests 76 and 50 -> 60 and 38. */
 FD_COLD int exit_floor(const fd_station_dev &sd, Shared &sh, WarpSmem &ws, int I, int J, int w, float thr, float *floor)
 {
     const GRect rj = gsmem(sh).rect[J];
