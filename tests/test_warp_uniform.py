@@ -93,7 +93,7 @@ def violations(text):
     return wide, found
 
 
-def test_checker_sees_what_it_is_for():
+def test_finds_what_it_is_for():
     bad = "__device__ bool f(int a)\n{\n    if (vload(x) > a) return true;\n    return __any_sync(0xffffffffu, a);\n}\n"
     good = bad.replace("vload(x)", "vload_warp(x)")
     by_name = bad.replace("if (vload(x) > a)", "const int v = vload(x);\n    if (v > a)")
